@@ -213,6 +213,13 @@ int slm_integrate_fields_noalloc(const slm_params* p, const slm_launch* launch,
  * (NaN equals NaN), [1] the largest such bit pattern plus one (0: none). */
 int slm_selftest_div6(uint64_t* counts, void* stream);
 
+/* slm_selftest_unit -- no counterpart in the reference: checks on the device,
+ * over every finite float from 2^-60 up, that the square root the tracers' unit
+ * vectors use equals the IEEE root and that its reciprocal is near enough for
+ * both quotients to round as IEEE divisions.  counts: DEVICE [2] uint64:
+ * failures, and the largest failing bit pattern + 1 (0: none).  Asynchronous. */
+int slm_selftest_unit(uint64_t* counts, void* stream);
+
 /* slm_selftest_cvt_i8 -- no counterpart in the reference: checks on the
  * device, over all 2^32 float bit patterns, that the tracer's float -> char
  * conversion (one range test around the device's saturating conversion)

@@ -13,12 +13,15 @@
 // (a step is at most integrator_step_factor px, so a trajectory usually visits
 // a pixel several times in a row) and adds the merged count and length sum
 // with one 64-bit atomic each when it moves to another pixel.
-#include <cstring>
 #include "capi_util.cuh"
-#include "trace_common.cuh"
+#include "trace_fast.cuh"
 
 
 static_assert(sizeof(slm_tile) == 40, "slm_tile layout is part of the ABI");
+
+// Resident blocks of 256 threads per SM the field kernels are compiled for
+// (64 registers a thread; 48, five blocks, spill the RK4 step).
+constexpr int FIELD_BLOCKS = 4;
 
 namespace slm {
 
@@ -36,21 +39,28 @@ __device__ __forceinline__ void acc_flush(Acc& a, u64* __restrict__ slc, u64* __
     }
 }
 
-// writearray.cl:31-40: slt += (uint)(l+0.5), slc += 1
-__device__ __forceinline__ void acc_visit(Acc& a, uint32_t idx, float l, u64* __restrict__ slc,
+// *p += v if `on` (predicated: no branch around it)
+__device__ __forceinline__ void add_if(bool on, u64* p, u64 v) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q red.global.add.u64 [%1], %2;\n\t}"
+                 :
+                 : "r"((uint32_t)on), "l"(p), "l"(v));  // nothing here reads the sums
+}
+
+// writearray.cl:31-40: slt += (uint)(l+0.5), slc += 1, if `visits`
+__device__ __forceinline__ void acc_visit(Acc& a, uint32_t idx, float l, bool visits, u64* __restrict__ slc,
                                           u64* __restrict__ slt) {
-    const u64 v = __float2uint_rz(l + 0.5f);
-    // only the two atomics of a finished run branch; the bookkeeping is
-    // selects, so a warp whose lanes change pixel at different steps runs it
-    // once with every lane active
+    const uint32_t v = __float2uint_rz(l + 0.5f);
+    // selects and predicated atomics, no branch: some lane of a warp changes
+    // pixel in nearly every step
     const bool same = (idx == a.idx) && a.cnt;
-    if (!same && a.cnt) {
-        atomicAdd(slt + a.idx, a.sum);
-        atomicAdd(slc + a.idx, (u64)a.cnt);
+    const bool flush = visits && !same && a.cnt;
+    add_if(flush, slt + a.idx, a.sum);
+    add_if(flush, slc + a.idx, (u64)a.cnt);
+    if (visits) {
+        a.cnt = same ? a.cnt + 1u : 1u;
+        a.sum = (same ? a.sum : 0ull) + v;
+        a.idx = idx;
     }
-    a.cnt = same ? a.cnt + 1u : 1u;
-    a.sum = same ? a.sum + v : v;
-    a.idx = idx;
 }
 
 // State of one jittered field trajectory between steps.
@@ -58,31 +68,49 @@ struct FieldLane {
     Vec2 a;
     float l, dt;
     uint32_t n, rng;
-    uint32_t item, k;  // queue position and RK steps so far (kept only when recording)
+    uint32_t item, k;  // queue position and RK steps so far
     bool alive;
+    F2 t;              // 2^23 + pixel of a, and the byte offset of that
+    uint32_t off;      // pixel's vector in uv (kept for the fast step)
+};
+
+// A grid as a lane sees it: its geometry, the fast step's form of it, its
+// first pixel in the uv / mask arrays and the offset from a pixel's index
+// there to its accumulators.
+struct FieldGrid {
+    Geo g;
+    FastGeo f;
+    uint32_t base, acc_offset;
 };
 
 // Begin the trajectory of sub-pixel `sub` (= j*d + i) of the seed at `c`,
 // whose RNG stream is that of seed index `rng_idx`
-// (integratefields.cl:83-113; jittertrajectory.cl:56-62).  `mask` is the
-// grid's own; pixel indices are offset by `base` into slc/slt.
+// (integratefields.cl:83-113; jittertrajectory.cl:56-62).
+template <bool FAST>
 __device__ __forceinline__ void field_init(FieldLane& s, float2 c, uint32_t rng_idx, uint32_t sub,
                                            uint32_t item, const uint8_t* __restrict__ mask,
-                                           const slm_params& p, const Geo& g, uint32_t base,
-                                           Acc& acc, u64* __restrict__ slc, u64* __restrict__ slt) {
+                                           const slm_params& p, const FieldGrid& G, Acc& acc,
+                                           u64* __restrict__ slc, u64* __restrict__ slt) {
     const uint32_t d = p.subpixel_seed_point_density;
     const uint32_t j = sub / d, i = sub % d;
     s.a.x = c.x + ((float)i * p.subpixel_seed_step - p.subpixel_seed_halfspan);
     s.a.y = c.y + ((float)j * p.subpixel_seed_step - p.subpixel_seed_halfspan);
     s.rng = seed_rng(rng_idx);
+    // the fast draws form (state + 1) * A without wrapping the sum: the state
+    // whose successor wraps to 0 has the same successor as the modulus - 1
+    if (FAST && s.rng == 0xffffffffu) s.rng = LEHMER_M - 1u;
     s.l = 0.0f;
-    s.dt = g.dt_max;
+    s.dt = G.g.dt_max;
     s.n = 0;
     s.item = item;
     s.k = 0;
-    const uint32_t idx = pixel_of(s.a, p, g);
+    const uint32_t idx = G.base + pixel_of(s.a, p, G.g);
+    if (FAST) {
+        s.t = pixel_magic_clamped(s.a, p.pad_width_pp5, G.g.nxp, G.g.nyp);
+        s.off = 8u * idx;
+    }
     const bool masked = __ldg(mask + idx) != 0;
-    if (!masked) acc_visit(acc, base + idx, 0.0f, slc, slt);
+    acc_visit(acc, G.acc_offset + idx, 0.0f, !masked, slc, slt);
     s.alive = !masked && (0.0f < p.max_length) && (0u < p.max_n_steps);
 }
 
@@ -103,50 +131,74 @@ __device__ __forceinline__ void split_item(u64 item, uint32_t dd, uint32_t& pos,
 // `order` (optional) maps queue positions to seed indices, so trajectories can
 // be traced in any order; the RNG stream still follows the seed index, so no
 // trajectory changes.
+template <bool FAST>
 __device__ __forceinline__ void field_start(FieldLane& s, u64 item, uint32_t seed_begin,
                                             const float2* __restrict__ seeds,
                                             const uint32_t* __restrict__ order,
                                             const uint8_t* __restrict__ mask, const slm_params& p,
-                                            const Geo& g, Acc& acc, u64* __restrict__ slc,
+                                            const FieldGrid& G, Acc& acc, u64* __restrict__ slc,
                                             u64* __restrict__ slt) {
     const uint32_t d = p.subpixel_seed_point_density;
     uint32_t seed_off, sub;
     split_item(item, d * d, seed_off, sub);
     const uint32_t seed_idx = order ? __ldg(order + seed_begin + seed_off) : seed_begin + seed_off;
-    field_init(s, __ldg(seeds + seed_idx), seed_idx, sub, (uint32_t)item, mask, p, g, 0u, acc, slc, slt);
+    field_init<FAST>(s, __ldg(seeds + seed_idx), seed_idx, sub, (uint32_t)item, mask, p, G, acc, slc, slt);
 }
 
 // One pass of the while loop of jittered_trajectory with
 // runge_kutta_step_write_sl_data (rungekutta.cl:163-186).  The Euler branch
-// of that loop is unreachable (get_array_idx clamps into the grid).  P2:
-// trajectory_resolution and GRID_SCALE are powers of two (slm_pow2_steps).
-template <int ORDER, bool P2 = false>
+// of that loop is unreachable (get_array_idx clamps into the grid).  FAST:
+// the launch meets fast_params, and the grid fast_grid (GATED: or it has no
+// interior, so that every step is rk_step's).
+template <int ORDER, bool FAST, bool GATED>
 __device__ __forceinline__ void field_step(FieldLane& s, const uint8_t* __restrict__ mask,
                                            const float2* __restrict__ uv, const slm_params& p,
-                                           const Geo& g, uint32_t base, Acc& acc,
+                                           const FastConst& k, const FieldGrid& G, Acc& acc,
                                            u64* __restrict__ slc, u64* __restrict__ slt) {
-    const Step st = rk_step<ORDER, true, P2>(s.a, s.dt, s.rng, uv, p, g);
-    if (__ldg(mask + st.idx)) {
-        s.alive = false;
-        return;
+    float dl, dt;
+    uint32_t idx;
+    if (FAST) {
+        FastStep st;
+        const bool ok = step_fast<ORDER, true, GATED>(s.a, s.t, s.off, s.dt, G.g.cf, s.rng, uv, G.f, k, st);
+        float ex = st.d2.x - st.d1.x, ey = st.d2.y - st.d1.y;
+        dt = G.g.dt_max;
+        // rare: a guard failed, or the next dt is not DT_MAX by the cheap test
+        if (!ok || !(s.dt * s.dt * G.f.kerr >= __fmaf_rn(ey, ey, ex * ex))) {
+            if (!ok) {
+                st = step_exact<ORDER, true>(s.a, s.dt, s.rng, G.g.cf, uv, G.base, p, G.g.nxp, G.g.nyp);
+                ex = st.d2.x - st.d1.x;
+                ey = st.d2.y - st.d1.y;
+            }
+            dt = next_dt_fast(ex, ey, s.dt, G.g.dt_max, G.g.gs, G.f.gs_rcp, p.adjusted_max_error);
+        }
+        s.rng = st.rng;
+        s.off = st.off;
+        s.a = st.next;
+        s.t = st.t;
+        dl = quantised_length(__fmaf_rn(st.d2.y, st.d2.y, st.d2.x * st.d2.x));
+        idx = st.off >> 3;
+        s.alive = __ldg(mask + idx) == 0;
+    } else {
+        const Step st = rk_step<ORDER, true>(s.a, s.dt, s.rng, uv + G.base, p, G.g);
+        idx = G.base + st.idx;
+        const float err = vlen(div_gs(st.d2.x - st.d1.x, G.g), div_gs(st.d2.y - st.d1.y, G.g));
+        dl = vlen(st.d2.x, st.d2.y);
+        dt = next_dt(s.dt, err, p, G.g);
+        s.a = st.next;
+        s.alive = __ldg(mask + idx) == 0;
     }
-    const float err = vlen(div_gs<P2>(st.d2.x - st.d1.x, g), div_gs<P2>(st.d2.y - st.d1.y, g));
-    const float dl = vlen(st.d2.x, st.d2.y);
-    s.a = st.next;
-    if (dl < p.integration_halt_threshold) {
-        s.l = s.l + dl;
-        s.n += 1;
-        acc_visit(acc, base + st.idx, s.l, slc, slt);
-        s.alive = false;
-        return;
-    }
-    s.dt = next_dt(s.dt, err, p, g);
+    // a masked pixel ends the trajectory without a visit
     s.l = s.l + dl;
     s.n += 1;
-    acc_visit(acc, base + st.idx, s.l, slc, slt);
-    s.alive = (s.l < p.max_length) && (s.n < p.max_n_steps);
+    s.dt = dt;  // (a halted trajectory has no next step)
+    acc_visit(acc, G.acc_offset + idx, s.l, s.alive, slc, slt);
+    s.alive = s.alive && !(dl < p.integration_halt_threshold) && (s.l < p.max_length) && (s.n < p.max_n_steps);
 }
 
+// The grid of a launch's parameter block.
+__device__ __forceinline__ FieldGrid grid_of(const slm_params& p, const FastGeo& f) {
+    return FieldGrid{geo_of(p), f, 0u, 0u};
+}
 
 // per-trajectory RK step count, saturated to 16 bits, indexed by queue position
 template <bool RECORD>
@@ -166,85 +218,100 @@ __device__ __forceinline__ void warp_add_counters(u64 steps, u64 ntraj, u64* wor
     }
 }
 
-template <int ORDER, bool RECORD>
-__global__ void __launch_bounds__(256)
-k_fields_plain(const slm_params p, const float2* __restrict__ seeds, uint32_t seed_begin,
+// Steps of a lane's finished trajectories, gathered when the lane takes its
+// next one (a trajectory's own count is 32 bits wide, a launch's is not).
+struct LaneCount {
+    u64 steps, ntraj;
+};
+
+__device__ __forceinline__ void count_trajectory(LaneCount& c, FieldLane& s) {
+    c.steps += s.k;
+    s.k = 0;
+}
+
+template <int ORDER, bool RECORD, bool FAST>
+__global__ void __launch_bounds__(256, FIELD_BLOCKS)
+k_fields_plain(const __grid_constant__ slm_params p, const __grid_constant__ FastGeo f,
+               const __grid_constant__ FastConst k, const float2* __restrict__ seeds, uint32_t seed_begin,
                u64 n_items, const uint8_t* __restrict__ mask, const float2* __restrict__ uv,
                u64* __restrict__ slc, u64* __restrict__ slt, u64* __restrict__ work,
                const uint32_t* __restrict__ order, uint16_t* __restrict__ item_steps) {
     const u64 item = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    u64 steps = 0, ntraj = 0;
+    LaneCount c{0ull, 0ull};
     Acc acc{0u, 0u, 0ull};
-    const Geo g = geo_of(p);
+    const FieldGrid G = grid_of(p, f);
     if (item < n_items) {
         FieldLane s;
-        field_start(s, item, seed_begin, seeds, order, mask, p, g, acc, slc, slt);
-        ntraj = 1;
+        field_start<FAST>(s, item, seed_begin, seeds, order, mask, p, G, acc, slc, slt);
+        c.ntraj = 1;
         while (s.alive) {
-            field_step<ORDER>(s, mask, uv, p, g, 0u, acc, slc, slt);
-            steps++;
-            if (RECORD) s.k++;
+            field_step<ORDER, FAST, false>(s, mask, uv, p, k, G, acc, slc, slt);
+            s.k++;
         }
         record_end<RECORD>(s, item_steps);
+        count_trajectory(c, s);
         acc_flush(acc, slc, slt);
     }
-    warp_add_counters(steps, ntraj, work);
+    warp_add_counters(c.steps, c.ntraj, work);
+}
+
+// Queue positions for the warp's idle lanes (mask `idle`): the first one, or
+// none once the queue of n items is used up.
+__device__ __forceinline__ u64 take_items(u64* work, unsigned idle, unsigned lane, u64 n, bool& drained) {
+    const int leader = __ffs(idle) - 1;
+    const unsigned n_idle = __popc(idle);
+    u64 head = 0;
+    if ((int)lane == leader) head = atomicAdd(work, (u64)n_idle);
+    head = __shfl_sync(0xffffffffu, head, leader);
+    if (head + n_idle >= n) drained = true;
+    return head + __popc(idle & ((1u << lane) - 1u));
 }
 
 // Persistent form: the queue head work[0] must be 0 at launch.  Every loop
 // pass either hands queue items to idle lanes or advances every live
 // trajectory by one step, and each trajectory ends within max_n_steps steps,
 // so the loop ends; the exit test is warp-uniform.
-template <int ORDER, bool RECORD>
-__global__ void __launch_bounds__(256)
-k_fields_persistent(const slm_params p, const float2* __restrict__ seeds, uint32_t seed_begin,
+template <int ORDER, bool RECORD, bool FAST>
+__global__ void __launch_bounds__(256, FIELD_BLOCKS)
+k_fields_persistent(const __grid_constant__ slm_params p, const __grid_constant__ FastGeo f,
+                    const __grid_constant__ FastConst k, const float2* __restrict__ seeds, uint32_t seed_begin,
                     u64 n_items, const uint8_t* __restrict__ mask, const float2* __restrict__ uv,
                     u64* __restrict__ slc, u64* __restrict__ slt, u64* __restrict__ work,
                     const uint32_t* __restrict__ order, uint16_t* __restrict__ item_steps,
                     uint32_t refill_min) {
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
-    const Geo g = geo_of(p);
+    const FieldGrid G = grid_of(p, f);
     FieldLane s;
     s.alive = false;
+    s.k = 0;
     Acc acc{0u, 0u, 0ull};
-    u64 steps = 0, ntraj = 0;
+    LaneCount c{0ull, 0ull};
     bool drained = false;
     while (true) {
-        if (!drained) {
-            const unsigned idle = __ballot_sync(FULL, !s.alive);
-            if (idle && (idle == FULL || (uint32_t)__popc(idle) >= refill_min)) {
-                const int leader = __ffs(idle) - 1;
-                const unsigned n_idle = __popc(idle);
-                u64 base = 0;
-                if ((int)lane == leader) base = atomicAdd(work, (u64)n_idle);
-                base = __shfl_sync(FULL, base, leader);
-                if (base + n_idle >= n_items) drained = true;
-                if (!s.alive) {
-                    const u64 item = base + __popc(idle & ((1u << lane) - 1u));
-                    if (item < n_items) {
-                        field_start(s, item, seed_begin, seeds, order, mask, p, g, acc, slc, slt);
-                        ntraj++;
-                        if (!s.alive) record_end<RECORD>(s, item_steps);
-                    }
+        const unsigned idle = __ballot_sync(FULL, !s.alive);
+        if (!drained && (uint32_t)__popc(idle) >= refill_min) {
+            const u64 item = take_items(work, idle, lane, n_items, drained);
+            if (!s.alive) {
+                count_trajectory(c, s);
+                if (item < n_items) {
+                    field_start<FAST>(s, item, seed_begin, seeds, order, mask, p, G, acc, slc, slt);
+                    c.ntraj++;
+                    if (!s.alive) record_end<RECORD>(s, item_steps);
                 }
             }
-        }
-        if (!__any_sync(FULL, s.alive)) {
-            if (drained) break;
             continue;
         }
+        if (idle == FULL) break;
         if (s.alive) {
-            field_step<ORDER>(s, mask, uv, p, g, 0u, acc, slc, slt);
-            steps++;
-            if (RECORD) {
-                s.k++;
-                if (!s.alive) record_end<RECORD>(s, item_steps);
-            }
+            field_step<ORDER, FAST, false>(s, mask, uv, p, k, G, acc, slc, slt);
+            s.k++;
+            if (RECORD && !s.alive) record_end<RECORD>(s, item_steps);
         }
     }
+    count_trajectory(c, s);
     acc_flush(acc, slc, slt);
-    warp_add_counters(steps, ntraj, work);
+    warp_add_counters(c.steps, c.ntraj, work);
 }
 
 // ------------------------------------------------------------------ both directions
@@ -255,66 +322,60 @@ k_fields_persistent(const slm_params p, const float2* __restrict__ seeds, uint32
 // direction value of the step) and its accumulator offset (0, or up_stride
 // for the upstream slc/slt); every trajectory is the single-direction
 // kernels'.
-template <int ORDER, bool P2>
-__global__ void __launch_bounds__(256)
-k_fields_pair(const slm_params p, float cf_up, const float2* __restrict__ seeds, uint32_t seed_begin,
-              u64 n_items, const uint8_t* __restrict__ mask, const float2* __restrict__ uv,
+template <int ORDER, bool FAST>
+__global__ void __launch_bounds__(256, FIELD_BLOCKS)
+k_fields_pair(const __grid_constant__ slm_params p, const __grid_constant__ FastGeo f,
+              const __grid_constant__ FastConst k, float cf_up, const float2* __restrict__ seeds,
+              uint32_t seed_begin, u64 n_items, const uint8_t* __restrict__ mask, const float2* __restrict__ uv,
               u64* __restrict__ slc, u64* __restrict__ slt, uint32_t up_stride, u64* __restrict__ work,
               const uint32_t* __restrict__ order, const uint32_t* __restrict__ order_up,
               uint32_t refill_min) {
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const uint32_t dd = p.subpixel_seed_point_density * p.subpixel_seed_point_density;
-    const Geo g_down = geo_of(p);
-    Geo g_up = g_down;
-    g_up.cf = cf_up;
+    FieldGrid G = grid_of(p, f);
+    const float cf_down = G.g.cf;
     const u64 n_total = 2 * n_items;
     FieldLane s;
     s.alive = false;
-    bool up = false;
-    uint32_t base = 0;
+    s.k = 0;
     Acc acc{0u, 0u, 0ull};
-    u64 steps = 0, ntraj = 0, steps_up = 0;
+    LaneCount c{0ull, 0ull};
+    u64 steps_up = 0;
     bool drained = false;
     while (true) {
-        if (!drained) {
-            const unsigned idle = __ballot_sync(FULL, !s.alive);
-            if (idle && (idle == FULL || (uint32_t)__popc(idle) >= refill_min)) {
-                const int leader = __ffs(idle) - 1;
-                const unsigned n_idle = __popc(idle);
-                u64 head = 0;
-                if ((int)lane == leader) head = atomicAdd(work, (u64)n_idle);
-                head = __shfl_sync(FULL, head, leader);
-                if (head + n_idle >= n_total) drained = true;
-                if (!s.alive) {
-                    u64 item = head + __popc(idle & ((1u << lane) - 1u));
-                    if (item < n_total) {
-                        up = item >= n_items;
-                        if (up) item -= n_items;
-                        base = up ? up_stride : 0u;
-                        uint32_t pos, sub;
-                        split_item(item, dd, pos, sub);
-                        const uint32_t* o = up ? order_up : order;
-                        const uint32_t seed_idx = o ? __ldg(o + seed_begin + pos) : seed_begin + pos;
-                        field_init(s, __ldg(seeds + seed_idx), seed_idx, sub, (uint32_t)item, mask, p,
-                                   up ? g_up : g_down, base, acc, slc, slt);
-                        ntraj++;
-                    }
+        const unsigned idle = __ballot_sync(FULL, !s.alive);
+        if (!drained && (uint32_t)__popc(idle) >= refill_min) {
+            u64 item = take_items(work, idle, lane, n_total, drained);
+            if (!s.alive) {
+                if (G.acc_offset) steps_up += s.k;
+                count_trajectory(c, s);
+                if (item < n_total) {
+                    const bool up = item >= n_items;
+                    if (up) item -= n_items;
+                    G.acc_offset = up ? up_stride : 0u;
+                    G.g.cf = up ? cf_up : cf_down;
+                    uint32_t pos, sub;
+                    split_item(item, dd, pos, sub);
+                    const uint32_t* o = up ? order_up : order;
+                    const uint32_t seed_idx = o ? __ldg(o + seed_begin + pos) : seed_begin + pos;
+                    field_init<FAST>(s, __ldg(seeds + seed_idx), seed_idx, sub, (uint32_t)item, mask, p, G, acc, slc,
+                                     slt);
+                    c.ntraj++;
                 }
             }
-        }
-        if (!__any_sync(FULL, s.alive)) {
-            if (drained) break;
             continue;
         }
+        if (idle == FULL) break;
         if (s.alive) {
-            field_step<ORDER, P2>(s, mask, uv, p, up ? g_up : g_down, base, acc, slc, slt);
-            steps++;
-            steps_up += up;
+            field_step<ORDER, FAST, false>(s, mask, uv, p, k, G, acc, slc, slt);
+            s.k++;
         }
     }
+    if (G.acc_offset) steps_up += s.k;
+    count_trajectory(c, s);
     acc_flush(acc, slc, slt);
-    warp_add_counters(steps, ntraj, work);
+    warp_add_counters(c.steps, c.ntraj, work);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) steps_up += __shfl_xor_sync(FULL, steps_up, o);
     if (lane == 0) atomicAdd(work + 3, steps_up);
@@ -341,9 +402,9 @@ __device__ __forceinline__ uint32_t find_tile(const slm_tile* __restrict__ tiles
 // trajectory is computed exactly as a single-grid launch on its tile computes
 // it (RNG stream of the tile-local seed index).  work[3] receives 1 if a seed
 // falls outside its tile's range (an inconsistent table).
-template <int ORDER, bool RECORD>
-__global__ void __launch_bounds__(256, 5)
-k_fields_batched(const slm_params p, const slm_tile* __restrict__ tiles, uint32_t n_tiles,
+template <int ORDER, bool RECORD, bool FAST>
+__global__ void __launch_bounds__(256, FIELD_BLOCKS)
+k_fields_batched(const __grid_constant__ slm_params p, const __grid_constant__ FastConst k, const slm_tile* __restrict__ tiles, uint32_t n_tiles,
                  const float2* __restrict__ seeds, u64 n_items, const uint8_t* __restrict__ mask,
                  const float2* __restrict__ uv, u64* __restrict__ slc, u64* __restrict__ slt,
                  u64* __restrict__ work, const uint32_t* __restrict__ order,
@@ -353,63 +414,57 @@ k_fields_batched(const slm_params p, const slm_tile* __restrict__ tiles, uint32_
     const uint32_t dd = p.subpixel_seed_point_density * p.subpixel_seed_point_density;
     FieldLane s;
     s.alive = false;
-    Geo g = make_geo(2u, 2u, 0.0f, 0.0f, 1.0f);
-    uint32_t base = 0;
+    s.k = 0;
+    FieldGrid G{make_geo(2u, 2u, 0.0f, 0.0f, 1.0f), make_fast_geo(2u, 2u, 1.0f, 1.0f, 0.0f, 0u), 0u, 0u};
     Acc acc{0u, 0u, 0ull};
-    u64 steps = 0, ntraj = 0;
+    LaneCount c{0ull, 0ull};
     bool drained = false;
     while (true) {
-        if (!drained) {
-            const unsigned idle = __ballot_sync(FULL, !s.alive);
-            if (idle && (idle == FULL || (uint32_t)__popc(idle) >= refill_min)) {
-                const int leader = __ffs(idle) - 1;
-                const unsigned n_idle = __popc(idle);
-                u64 head = 0;
-                if ((int)lane == leader) head = atomicAdd(work, (u64)n_idle);
-                head = __shfl_sync(FULL, head, leader);
-                if (head + n_idle >= n_items) drained = true;
-                if (!s.alive) {
-                    const u64 item = head + __popc(idle & ((1u << lane) - 1u));
-                    if (item < n_items) {
-                        uint32_t pos, sub;
-                        split_item(item, dd, pos, sub);
-                        const uint32_t seed = order ? __ldg(order + pos) : pos;
-                        const uint32_t t = find_tile(tiles, n_tiles, seed);
-                        const slm_tile& T = tiles[t];
-                        const uint32_t local = seed - __ldg(&T.seed_begin);
-                        ntraj++;
-                        if (local < __ldg(&T.n_seeds)) {
-                            g = make_geo(__ldg(&T.nx_padded), __ldg(&T.ny_padded), __ldg(&T.combo_factor),
-                                         __ldg(&T.dt_max), __ldg(&T.grid_scale));
-                            base = (uint32_t)__ldg(&T.grid_offset);
-                            field_init(s, __ldg(seeds + seed), local, sub, (uint32_t)item, mask + base, p,
-                                       g, base, acc, slc, slt);
-                        } else {
-                            atomicOr(reinterpret_cast<unsigned long long*>(work + 3), 1ull);
-                            s.alive = false;
-                            s.item = (uint32_t)item;
-                            s.k = 0;
+        const unsigned idle = __ballot_sync(FULL, !s.alive);
+        if (!drained && (uint32_t)__popc(idle) >= refill_min) {
+            const u64 item = take_items(work, idle, lane, n_items, drained);
+            if (!s.alive) {
+                count_trajectory(c, s);
+                if (item < n_items) {
+                    uint32_t pos, sub;
+                    split_item(item, dd, pos, sub);
+                    const uint32_t seed = order ? __ldg(order + pos) : pos;
+                    const uint32_t t = find_tile(tiles, n_tiles, seed);
+                    const slm_tile& T = tiles[t];
+                    const uint32_t local = seed - __ldg(&T.seed_begin);
+                    c.ntraj++;
+                    if (local < __ldg(&T.n_seeds)) {
+                        G.g = make_geo(__ldg(&T.nx_padded), __ldg(&T.ny_padded), __ldg(&T.combo_factor),
+                                       __ldg(&T.dt_max), __ldg(&T.grid_scale));
+                        G.base = (uint32_t)__ldg(&T.grid_offset);
+                        if (FAST) {
+                            G.f = make_fast_geo(G.g.nxp, G.g.nyp, G.g.gs, G.g.dt_max, p.adjusted_max_error, G.base);
+                            // a tile the fast step cannot take has no interior pixel
+                            if (!fast_grid(G.g.nxp, G.g.nyp, G.base, G.g.cf, G.g.dt_max, p.trajectory_resolution))
+                                G.f.rx = -1.0f;
                         }
-                        if (!s.alive) record_end<RECORD>(s, item_steps);
+                        field_init<FAST>(s, __ldg(seeds + seed), local, sub, (uint32_t)item, mask, p, G, acc, slc, slt);
+                    } else {
+                        atomicOr(reinterpret_cast<unsigned long long*>(work + 3), 1ull);
+                        s.alive = false;
+                        s.item = (uint32_t)item;
+                        s.k = 0;
                     }
+                    if (!s.alive) record_end<RECORD>(s, item_steps);
                 }
             }
-        }
-        if (!__any_sync(FULL, s.alive)) {
-            if (drained) break;
             continue;
         }
+        if (idle == FULL) break;
         if (s.alive) {
-            field_step<ORDER>(s, mask + base, uv + base, p, g, base, acc, slc, slt);
-            steps++;
-            if (RECORD) {
-                s.k++;
-                if (!s.alive) record_end<RECORD>(s, item_steps);
-            }
+            field_step<ORDER, FAST, true>(s, mask, uv, p, k, G, acc, slc, slt);
+            s.k++;
+            if (RECORD && !s.alive) record_end<RECORD>(s, item_steps);
         }
     }
+    count_trajectory(c, s);
     acc_flush(acc, slc, slt);
-    warp_add_counters(steps, ntraj, work);
+    warp_add_counters(c.steps, c.ntraj, work);
 }
 
 // ------------------------------------------------------------------ trajectories
@@ -547,17 +602,25 @@ __global__ void k_fields_finish(const u64* __restrict__ acc, uint32_t nxy, uint3
 
 using namespace slm;
 
-// True when the step's two power-of-two shortcuts hold for the whole launch:
-// trajectory_resolution is a power of two (Quant) and GRID_SCALE is one whose
-// reciprocal is a normal float (pow2_reciprocal), the same tests the device
-// makes per step; the pair launch then runs the form without them.
-static bool pow2_steps(const slm_params& p) {
-    const uint32_t r = p.trajectory_resolution;
-    uint32_t b;
-    std::memcpy(&b, &p.grid_scale, sizeof b);
-    const uint32_t e = (b >> 23) & 0xffu;
-    const bool gs_pow2 = (b >> 31) == 0u && (b & 0x7fffffu) == 0u && e >= 1u && e <= 253u;
-    return r != 0u && (r & (r - 1u)) == 0u && gs_pow2;
+// The launch's steps can be evaluated by step_fast (else rk_step, the general form).
+static bool fast_steps(const slm_params& p) {
+    return fast_params(p) &&
+           fast_grid(p.nx_padded, p.ny_padded, 0u, p.combo_factor, p.dt_max, p.trajectory_resolution);
+}
+
+static FastGeo fast_geo_of(const slm_params& p) {
+    return make_fast_geo(p.nx_padded, p.ny_padded, p.grid_scale, p.dt_max, p.adjusted_max_error, 0u);
+}
+
+// Resident blocks per SM of a persistent launch: the caller's, else as many as fit.
+static int blocks_per_sm(const slm_launch& L, const void* kernel, int block, int* out) {
+    *out = L.blocks_per_sm;
+    if (*out <= 0) {
+        int occ = 0;
+        SLM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, block, 0));
+        *out = occ > 0 ? occ : 1;
+    }
+    return SLM_OK;
 }
 
 static int check_grid(const slm_params* p) {
@@ -578,26 +641,23 @@ static uint32_t refill_min(const slm_launch& L) {
     return L.chunk <= 1 ? 1u : (L.chunk >= 32 ? 32u : (uint32_t)L.chunk);
 }
 
-template <int ORDER, bool RECORD>
+template <int ORDER, bool RECORD, bool FAST>
 static int launch_fields(const slm_params* p, const slm_launch& L, int block, const float2* sp,
                          uint32_t begin, u64 n_items, const uint8_t* mask, const float2* u2, u64* slc,
                          u64* slt, u64* work, const uint32_t* order, uint16_t* rec, cudaStream_t s) {
     if (L.schedule == SLM_SCHED_PLAIN) {
         const u64 grid = (n_items + block - 1) / block;
         SLM_REQUIRE(grid < (1ull << 31), "too many trajectories for one launch");
-        k_fields_plain<ORDER, RECORD><<<(unsigned)grid, block, 0, s>>>(*p, sp, begin, n_items, mask, u2,
-                                                                      slc, slt, work, order, rec);
+        k_fields_plain<ORDER, RECORD, FAST><<<(unsigned)grid, block, 0, s>>>(*p, fast_geo_of(*p), make_fast_const(*p), sp, begin, n_items, mask, u2,
+                                                                            slc, slt, work, order, rec);
         SLM_LAUNCHED("k_fields_plain");
     } else if (L.schedule == SLM_SCHED_PERSISTENT) {
-        int per_sm = L.blocks_per_sm;
-        if (per_sm <= 0) {
-            int occ = 0;
-            SLM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fields_persistent<ORDER, RECORD>, block, 0));
-            per_sm = occ > 0 ? occ : 1;
-        }
+        int per_sm = 0;
+        const int rc = blocks_per_sm(L, (const void*)k_fields_persistent<ORDER, RECORD, FAST>, block, &per_sm);
+        if (rc) return rc;
         const unsigned grid = (unsigned)(num_sms() * per_sm);
-        k_fields_persistent<ORDER, RECORD><<<grid, block, 0, s>>>(*p, sp, begin, n_items, mask, u2, slc, slt,
-                                                                  work, order, rec, refill_min(L));
+        k_fields_persistent<ORDER, RECORD, FAST><<<grid, block, 0, s>>>(*p, fast_geo_of(*p), make_fast_const(*p), sp, begin, n_items, mask, u2, slc, slt,
+                                                                        work, order, rec, refill_min(L));
         SLM_LAUNCHED("k_fields_persistent");
     } else {
         set_error("unknown schedule %d", L.schedule);
@@ -606,23 +666,27 @@ static int launch_fields(const slm_params* p, const slm_launch& L, int block, co
     return SLM_OK;
 }
 
-template <int ORDER, bool RECORD>
+template <int ORDER, bool RECORD, bool FAST>
 static int launch_batched(const slm_params* p, const slm_launch& L, int block, const slm_tile* tiles,
                           uint32_t n_tiles, const float2* sp, u64 n_items, const uint8_t* mask,
                           const float2* u2, u64* slc, u64* slt, u64* work, const uint32_t* order,
                           uint16_t* rec, cudaStream_t s) {
-    int per_sm = L.blocks_per_sm;
-    if (per_sm <= 0) {
-        int occ = 0;
-        SLM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fields_batched<ORDER, RECORD>, block, 0));
-        per_sm = occ > 0 ? occ : 1;
-    }
+    int per_sm = 0;
+    const int rc = blocks_per_sm(L, (const void*)k_fields_batched<ORDER, RECORD, FAST>, block, &per_sm);
+    if (rc) return rc;
     const unsigned grid = (unsigned)(num_sms() * per_sm);
-    k_fields_batched<ORDER, RECORD><<<grid, block, 0, s>>>(*p, tiles, n_tiles, sp, n_items, mask, u2, slc, slt,
-                                                          work, order, rec, refill_min(L));
+    k_fields_batched<ORDER, RECORD, FAST><<<grid, block, 0, s>>>(*p, make_fast_const(*p), tiles, n_tiles, sp, n_items, mask, u2, slc, slt,
+                                                                work, order, rec, refill_min(L));
     SLM_LAUNCHED("k_fields_batched");
     return SLM_OK;
 }
+
+// f<ORDER, RECORD, FAST>(...) for run-time values of the three
+#define SLM_FIELDS_DISPATCH(f, rk4, record, fast, ...)                                             \
+    ((rk4) ? ((record) ? ((fast) ? f<4, true, true>(__VA_ARGS__) : f<4, true, false>(__VA_ARGS__))    \
+                       : ((fast) ? f<4, false, true>(__VA_ARGS__) : f<4, false, false>(__VA_ARGS__))) \
+           : ((record) ? ((fast) ? f<2, true, true>(__VA_ARGS__) : f<2, true, false>(__VA_ARGS__))    \
+                       : ((fast) ? f<2, false, true>(__VA_ARGS__) : f<2, false, false>(__VA_ARGS__))))
 
 extern "C" {
 
@@ -664,11 +728,8 @@ int slm_integrate_fields_scheduled(const slm_params* p, const slm_launch* launch
     const float2* sp = reinterpret_cast<const float2*>(seed_point);
     const float2* u2 = reinterpret_cast<const float2*>(uv);
     u64* w = (u64*)workspace;
-    if (L.integrator == SLM_RK4)
-        return item_steps ? launch_fields<4, true>(p, L, block, sp, begin, n_items, mask, u2, (u64*)slc, (u64*)slt, w, seed_order, item_steps, s)
-                          : launch_fields<4, false>(p, L, block, sp, begin, n_items, mask, u2, (u64*)slc, (u64*)slt, w, seed_order, nullptr, s);
-    return item_steps ? launch_fields<2, true>(p, L, block, sp, begin, n_items, mask, u2, (u64*)slc, (u64*)slt, w, seed_order, item_steps, s)
-                      : launch_fields<2, false>(p, L, block, sp, begin, n_items, mask, u2, (u64*)slc, (u64*)slt, w, seed_order, nullptr, s);
+    return SLM_FIELDS_DISPATCH(launch_fields, L.integrator == SLM_RK4, item_steps != nullptr, fast_steps(*p), p, L, block,
+                               sp, begin, n_items, mask, u2, (u64*)slc, (u64*)slt, w, seed_order, item_steps, s);
 }
 
 int slm_integrate_fields_pair(const slm_params* p_down, const slm_params* p_up, const slm_launch* launch,
@@ -709,31 +770,16 @@ int slm_integrate_fields_pair(const slm_params* p_down, const slm_params* p_up, 
     const u64 n_items = (u64)(p_down->n_seed_points - begin) * dd;
     const float2* sp = reinterpret_cast<const float2*>(seed_point);
     const float2* u2 = reinterpret_cast<const float2*>(uv);
-    const bool p2 = pow2_steps(*p_down);
-    int per_sm = L.blocks_per_sm;
-    if (per_sm <= 0) {
-        int occ = 0;
-        const void* fn = L.integrator == SLM_RK4 ? (p2 ? (const void*)k_fields_pair<4, true>
-                                                       : (const void*)k_fields_pair<4, false>)
-                                                 : (p2 ? (const void*)k_fields_pair<2, true>
-                                                       : (const void*)k_fields_pair<2, false>);
-        SLM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, block, 0));
-        per_sm = occ > 0 ? occ : 1;
-    }
+    const bool rk4 = L.integrator == SLM_RK4, fast = fast_steps(*p_down);
+    const auto kernel = rk4 ? (fast ? k_fields_pair<4, true> : k_fields_pair<4, false>)
+                            : (fast ? k_fields_pair<2, true> : k_fields_pair<2, false>);
+    int per_sm = 0;
+    rc = blocks_per_sm(L, (const void*)kernel, block, &per_sm);
+    if (rc) return rc;
     const unsigned grid = (unsigned)(num_sms() * per_sm);
     const uint32_t* o_up = seed_order_up ? seed_order_up : seed_order;
-#define SLM_PAIR_LAUNCH(ORD, P2)                                                                          \
-    k_fields_pair<ORD, P2><<<grid, block, 0, s>>>(*p_down, p_up->combo_factor, sp, begin, n_items, mask, u2, \
-                                                  (u64*)slc, (u64*)slt, (uint32_t)up_stride,              \
-                                                  (u64*)workspace, seed_order, o_up, refill_min(L))
-    if (L.integrator == SLM_RK4) {
-        if (p2) SLM_PAIR_LAUNCH(4, true);
-        else SLM_PAIR_LAUNCH(4, false);
-    } else {
-        if (p2) SLM_PAIR_LAUNCH(2, true);
-        else SLM_PAIR_LAUNCH(2, false);
-    }
-#undef SLM_PAIR_LAUNCH
+    kernel<<<grid, block, 0, s>>>(*p_down, fast_geo_of(*p_down), make_fast_const(*p_down), p_up->combo_factor, sp, begin, n_items, mask, u2, (u64*)slc, (u64*)slt,
+                                  (uint32_t)up_stride, (u64*)workspace, seed_order, o_up, refill_min(L));
     SLM_LAUNCHED("k_fields_pair");
     return SLM_OK;
 }
@@ -768,11 +814,8 @@ int slm_integrate_fields_batched(const slm_params* p, const slm_launch* launch, 
     const float2* sp = reinterpret_cast<const float2*>(seed_point);
     const float2* u2 = reinterpret_cast<const float2*>(uv);
     u64* w = (u64*)workspace;
-    if (L.integrator == SLM_RK4)
-        return item_steps ? launch_batched<4, true>(p, L, block, tiles, n_tiles, sp, n_items, mask, u2, (u64*)slc, (u64*)slt, w, seed_order, item_steps, s)
-                          : launch_batched<4, false>(p, L, block, tiles, n_tiles, sp, n_items, mask, u2, (u64*)slc, (u64*)slt, w, seed_order, nullptr, s);
-    return item_steps ? launch_batched<2, true>(p, L, block, tiles, n_tiles, sp, n_items, mask, u2, (u64*)slc, (u64*)slt, w, seed_order, item_steps, s)
-                      : launch_batched<2, false>(p, L, block, tiles, n_tiles, sp, n_items, mask, u2, (u64*)slc, (u64*)slt, w, seed_order, nullptr, s);
+    return SLM_FIELDS_DISPATCH(launch_batched, L.integrator == SLM_RK4, item_steps != nullptr, fast_params(*p), p, L, block,
+                               tiles, n_tiles, sp, n_items, mask, u2, (u64*)slc, (u64*)slt, w, seed_order, item_steps, s);
 }
 
 int slm_fields_finish(const uint64_t* acc, uint32_t nxy_padded, uint32_t density, double ds_scale_down,
@@ -914,6 +957,43 @@ __global__ void k_selftest_cvt_i8(u64* counts) {
         atomicAdd(counts, bad);
         atomicMax(counts + 1, last);
     }
+}
+
+// counts[0] += sums of squares s >= 2^-60 (and finite) for which the root or the
+// reciprocal of root_and_reciprocal could give a wrong quotient: the root is
+// not the IEEE square root, or with b = len 2^-k in [1, 2) and d = |y len - 1|
+//   d (b + 2^-23) >= 2^-23        (the residual correction could cross a midpoint)
+//   d > 2^-25 b (1 + 2^-18)       (the first quotient could be two ulps off)
+// counts[1] as for div6
+__global__ void k_selftest_unit(u64* counts) {
+    u64 bad = 0, last = 0;
+    const u64 lo = __float_as_uint(0x1p-100f), hi = 0x7f7fffffu;
+    for (u64 v = lo + (u64)blockIdx.x * blockDim.x + threadIdx.x; v <= hi; v += (u64)gridDim.x * blockDim.x) {
+        const float s = __uint_as_float((uint32_t)v);
+        float len, y;
+        root_and_reciprocal(s, len, y);
+        const double b = (double)__uint_as_float((__float_as_uint(len) & 0x7fffffu) | 0x3f800000u);
+        const double d = fabs((double)y * (double)len - 1.0);
+        const bool ok = len == __fsqrt_rn(s) && d * (b + 0x1p-23) < 0x1p-23 && d <= 0x1p-25 * b * (1.0 + 0x1p-18);
+        if (!ok) {
+            bad++;
+            last = v + 1;
+        }
+    }
+    if (bad) {
+        atomicAdd(counts, bad);
+        atomicMax(counts + 1, last);
+    }
+}
+
+extern "C" int slm_selftest_unit(uint64_t* counts, void* stream) {
+    clear_error();
+    SLM_REQUIRE(counts && aligned(counts, 8), "counts must be two 8-byte aligned device words");
+    cudaStream_t s = (cudaStream_t)stream;
+    SLM_CUDA(cudaMemsetAsync(counts, 0, 2 * sizeof(uint64_t), s));
+    k_selftest_unit<<<(unsigned)(num_sms() * 8), 256, 0, s>>>((u64*)counts);
+    SLM_LAUNCHED("k_selftest_unit");
+    return SLM_OK;
 }
 
 extern "C" int slm_selftest_div6(uint64_t* counts, void* stream) {

@@ -69,11 +69,8 @@ __device__ __forceinline__ Geo geo_of(const slm_params& p) {
 }
 
 // x / GRID_SCALE: a multiplication when GRID_SCALE is a power of two (both
-// are the correctly rounded value of the same quotient).  P2: the caller has
-// checked that it is (slm_pow2_steps), so the test is left out.
-template <bool P2 = false>
+// are the correctly rounded value of the same quotient).
 __device__ __forceinline__ float div_gs(float x, const Geo& g) {
-    if (P2) return x * g.gs_inv;
     return g.gs_inv != 0.0f ? x * g.gs_inv : __fdiv_rn(x, g.gs);
 }
 
@@ -116,21 +113,17 @@ __device__ __forceinline__ Vec2 sample_uv(Vec2 a, const float2* __restrict__ uv,
 
 // Quantisation scale.  When trajectory_resolution is a power of two (128 by
 // default) dividing by it is exactly a multiplication by its reciprocal.
-// P2: the caller has checked that it is, so the test is left out.
-template <bool P2 = false>
 struct Quant {
     float res, inv;
     bool pow2;
     __device__ __forceinline__ float operator()(float v) const {
         const float c = (float)cvt_i8(v * res);
-        if (P2) return c * inv;
         return pow2 ? c * inv : __fdiv_rn(c, res);
     }
 };
 
-template <bool P2 = false>
-__device__ __forceinline__ Quant<P2> make_quant(uint32_t r) {
-    Quant<P2> q;
+__device__ __forceinline__ Quant make_quant(uint32_t r) {
+    Quant q;
     q.res = (float)r;
     q.inv = __fdiv_rn(1.0f, (float)r);
     q.pow2 = r != 0u && (r & (r - 1u)) == 0u;
@@ -203,15 +196,14 @@ struct Step {
 };
 
 // RK2 (computestep.cl:42-57 / 86-106), or the RK4 extension (same
-// quantisation; d1 = approx(h k1) for the error estimate).  P2: the
-// trajectory resolution is a power of two (checked by the caller).
-template <int ORDER, bool JITTER, bool P2 = false>
+// quantisation; d1 = approx(h k1) for the error estimate).
+template <int ORDER, bool JITTER>
 __device__ __forceinline__ Step rk_step(Vec2 a, float dt, uint32_t& rng,
                                         const float2* __restrict__ uv, const slm_params& p,
                                         const Geo& g) {
     Step s;
     const float cf = g.cf;
-    const Quant<P2> quant = make_quant<P2>(p.trajectory_resolution);
+    const Quant quant = make_quant(p.trajectory_resolution);
     Vec2 k1 = sample_uv(a, uv, p, g);
     if (JITTER) k1 = jitter(k1, rng, p.jitter_magnitude);
     s.u1 = k1;

@@ -1,0 +1,409 @@
+// trace_fast.cuh -- the RK step of trace_common.cuh as straight-line code.
+//
+// The tracers are bound by instruction issue, not by memory: the plain form
+// of a jittered RK4 step (rk_step) is 815 thread instructions, most of them
+// the 17 IEEE divisions and 10 square roots, each with a range check, a branch
+// around its slow path and a convergence barrier, and the index clamps of the
+// four bilinear samples.  Here a step is evaluated without any of them and
+// with one test at its end: the step's values are those of rk_step bit for
+// bit when every guard below holds, and a lane for which one does not hold
+// (a sample next to the grid's edge, a NaN, an overflow, a component below
+// 2^-30, one generator state in 10^9) evaluates the step again with rk_step.
+//
+// What makes each shortcut exact:
+//
+//   unit vectors    u / |u| from one reciprocal square root estimate
+//                   (unit_fast): square root and quotients correctly rounded
+//                   by fused residuals (P. Markstein, "Computation of
+//                   elementary functions on the IBM RISC System/6000
+//                   processor", IBM J. Res. Dev. 34(1), 1990).  The root and
+//                   the reciprocal depend on the sum of squares alone, so
+//                   slm_selftest_unit checks every float of the guarded range.
+//   pixel index     trunc(v) for 0 <= v < 2^23 is v + 2^23 rounded towards
+//                   zero; the sum's low bits are the integer, so neither
+//                   conversion unit nor clamp is used (the clamps cannot bind
+//                   for samples within one pixel of an interior pixel).
+//   quantisation    trunc(|v| 2^k) the same way in one fused operation; the
+//                   host checks that a step is below 127 units.
+//   jitter draws    the generator's reduction without its last conditional
+//                   subtraction, which acts on 5 of 2^32 states (guarded).
+//   products by a power of two fused with the sum that follows (exact).
+//   adaptive dt     DT_MAX, without root and division, when a test with
+//                   margin shows the error small enough; else as next_dt.
+//
+// x and y of a step go through the packed two-float instructions of sm_100a
+// (each half rounded as the scalar instruction rounds it), which halve the
+// issue slots of the bilinear sums and the step's products.
+//
+// Measured (B200, both directions of 1024^2 incised relief, 2x2 seeds, RK4):
+// 815 -> 440 thread instructions per step; 4096^2 fan terrain, 1.64e10 RK4
+// steps: 505 -> 294 ms; 256^2 hills, RK2: 11.9 -> 6.8 ms.  What is left is
+// bound by the float units (80 % of the issue slots' worth of work: packed
+// operations take two cycles, the generator's wide products four), so
+// variants that trade slots for float work (wide products for the addresses
+// or the draws' reduction) measured 2 to 5 % slower, fewer or more resident
+// warps (24, 36, 38, 40 against 32 per SM) 0 to 4 % slower.
+#pragma once
+#include "trace_common.cuh"
+
+namespace slm {
+
+typedef u64 F2;  // two floats in a register pair: x low, y high
+
+__device__ __forceinline__ F2 pack2(float x, float y) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ F2 splat2(float v) { return pack2(v, v); }
+__device__ __forceinline__ void unpack2(F2 a, float& x, float& y) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 add2_rz(F2 a, F2 b) {
+    F2 r;
+    asm("add.rz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) {
+    F2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// three-operand minimum, NaN if any operand is
+__device__ __forceinline__ float min3_nan(float a, float b, float c) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+constexpr float FAST_MAGIC = 8388608.0f;           // 2^23
+constexpr uint32_t FAST_MAGIC_BITS = 0x4B000000u;  // its bit pattern
+constexpr float FAST_S_MIN = 0x1p-60f;             // least square of a component
+
+constexpr uint32_t LEHMER_M = 0xfffffffbu;
+
+// Square root of s and the reciprocal of that root, s >= 2^-60 and finite.
+// len is the IEEE square root and y the IEEE reciprocal of len, or off it
+// where that cannot change a quotient; slm_selftest_unit checks both over
+// the whole range.  The bias of 2^-44 (a 2^-21 part of an ulp) decides the
+// one tie the Newton step would round down, len = (2 - 2^-23) 2^k.
+__device__ __forceinline__ void root_and_reciprocal(float s, float& len, float& y) {
+    float y0;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(s));
+    // h = y0 / 2 by its exponent: the float units are the busier ones
+    const float g = __fmul_rn(s, y0), h = __uint_as_float(__float_as_uint(y0) - 0x800000u);
+    len = __fmaf_rn(__fmaf_rn(-g, g, s), h, g);
+    const float e = __fadd_rn(__fmaf_rn(-len, y0, 1.0f), 0x1p-44f);
+    y = __fmaf_rn(e, y0, y0);
+}
+
+// u / |u| as rk_step forms it: |u| = sqrt(x*x + y*y), both components divided
+// by it.  Exact, but for the sign of a zero component (which no later value
+// depends on), when s = x*x + y*y >= 2^-60 is finite and each component is
+// zero or at least 2^-103: the residuals are then exact.
+__device__ __forceinline__ F2 unit_fast(F2 u, float& xx, float& yy, float& s) {
+    unpack2(mul2(u, u), xx, yy);
+    s = __fadd_rn(xx, yy);
+    float len, r;
+    root_and_reciprocal(s, len, r);
+    const F2 r2 = splat2(r), q = mul2(u, r2);
+    return fma2(fma2(splat2(-len), q, u), r2, q);
+}
+
+// sqrt(x*x + y*y) of a quantised step (multiples of 2^-k, so the sum of
+// squares is 0 or above 2^-40; the added 2^-100 is absorbed unless it is 0,
+// where it keeps the estimate finite and the root 0)
+__device__ __forceinline__ float quantised_length(float s) {
+    float y0;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(__fadd_rn(s, 0x1p-100f)));
+    const float g = __fmul_rn(s, y0), h = __fmul_rn(0.5f, y0);
+    return __fmaf_rn(__fmaf_rn(-g, g, s), h, g);
+}
+
+// A grid as the fast step uses it.  Part of the launch's parameters in the
+// single-grid kernels, one per lane in the batched one.
+struct FastGeo {
+    uint32_t pitch;     // bytes of a grid row of vectors
+    uint32_t koff;      // byte offset of a pixel's vector: pitch * bits(2^23 + xi) + 8 * bits(2^23 + yi) + koff
+    uint32_t off_last;  // largest such offset whose four taps lie in the grid
+    float cx, cy;       // interior pixels: |xi - cx| <= rx, |yi - cy| <= ry, that is
+    float rx, ry;       //   2 <= xi <= nxp - 4 and 2 <= yi <= nyp - 4
+    float kerr;         // dt^2 kerr >= |d2 - d1|^2 implies a next dt of DT_MAX
+    float gs_rcp;       // IEEE reciprocal of GRID_SCALE
+};
+
+// base: the grid's first pixel in its arrays
+__host__ __device__ __forceinline__ FastGeo make_fast_geo(uint32_t nxp, uint32_t nyp, float gs, float dt_max,
+                                                          float adjusted_max_error, uint32_t base) {
+    FastGeo f;
+    f.pitch = 8u * nyp;
+    f.koff = 8u * base - (f.pitch + 8u) * FAST_MAGIC_BITS;
+    f.off_last = 8u * (base + nxp * nyp - nyp - 2u);
+    f.cx = 0.5f * (float)(nxp - 2u);
+    f.cy = 0.5f * (float)(nyp - 2u);
+    f.rx = 0.5f * ((float)nxp - 6.0f);
+    f.ry = 0.5f * ((float)nyp - 6.0f);
+    f.gs_rcp = 1.0f / gs;
+    const float k = adjusted_max_error * gs / dt_max;
+    f.kerr = (k > 0x1p-30f && k < 0x1p30f) ? k * k * (1.0f - 0x1p-16f) : -1.0f;  // -1: never by the test
+    return f;
+}
+
+// Constants of the fast step, formed on the host: the kernels' loops would
+// otherwise form them again in every step (they do not fit the registers).
+// As pairs, they are operands of the packed instructions.
+struct FastConst {
+    float2 pp5, pad, magic, one, half, two, mag, draw, draw0, div6_hi, div6_lo;
+    float res, inv, minus_magic_inv;
+};
+
+static inline FastConst make_fast_const(const slm_params& p) {
+    const auto both = [](float v) { return make_float2(v, v); };
+    FastConst k;
+    k.pp5 = both(p.pad_width_pp5);
+    k.pad = both((float)p.pad_width);
+    k.magic = both(FAST_MAGIC);
+    k.one = both(1.0f);
+    k.half = both(0.5f);
+    k.two = both(2.0f);
+    k.mag = both(p.jitter_magnitude);
+    k.draw = both(0x1p-32f);
+    k.draw0 = both(-0.5f);
+    k.div6_hi = both(0x1.555556p-3f);
+    k.div6_lo = both(-0x1.555556p-28f);
+    k.res = (float)p.trajectory_resolution;
+    k.inv = 1.0f / k.res;  // a power of two
+    k.minus_magic_inv = -FAST_MAGIC * k.inv;
+    return k;
+}
+
+__device__ __forceinline__ F2 as_f2(const float2& v) { return pack2(v.x, v.y); }
+
+// a + m where m is a product of its own rounding: the assembler joins a packed
+// product and the packed sum that follows into one fused operation whatever
+// its contraction flag says, so the sum is written as m * 1 + a with a 1 it
+// cannot see (exact, and one instruction as well).
+__device__ __forceinline__ F2 add2_product(F2 m, F2 a, const FastConst& k) { return fma2(m, as_f2(k.one), a); }
+
+// Whether a grid's steps can be evaluated by step_fast: quantised steps below
+// 127 units (so below a pixel, and no conversion wraps), coordinates that
+// 2^23 + i holds.  Grids below 8 pixels have no interior worth the test.
+__host__ __device__ __forceinline__ bool fast_grid(uint32_t nxp, uint32_t nyp, uint32_t base, float cf,
+                                                   float dt_max, uint32_t resolution) {
+    const float h = fabsf(cf) * dt_max;
+    return nxp >= 8u && nyp >= 8u && nxp <= (1u << 22) && nyp <= (1u << 22) &&
+           (u64)nxp * nyp + base <= (1ull << 29) &&  // 32-bit byte offsets
+           dt_max > 0.0f && h >= 0x1p-20f && h <= 0.99f && h * (float)resolution <= 126.0f && fabsf(cf) <= 0x1p30f;
+}
+
+// The conditions on the parameters all grids of a launch share: a resolution
+// that is a power of two, a jitter that keeps quotients normal, a dt rule
+// that never lengthens a step.
+__host__ __device__ __forceinline__ bool fast_params(const slm_params& p) {
+    const uint32_t r = p.trajectory_resolution;
+    const float m = fabsf(p.jitter_magnitude);
+    return r != 0u && (r & (r - 1u)) == 0u && r <= (1u << 20) && (m == 0.0f || (m >= 0x1p-40f && m <= 0x1p10f)) &&
+           p.adjusted_max_error >= 0.0f && p.pad_width < (1u << 20);
+}
+
+// 2^23 + clamped pixel index of a position, per axis (get_array_idx); the
+// clamp written so that NaN gives pixel 0, as axis_index
+__device__ __forceinline__ F2 pixel_magic_clamped(Vec2 a, float pp5, uint32_t nxp, uint32_t nyp) {
+    const float vx = fminf(fmaxf(a.x + pp5, 0.0f), (float)(nxp - 1u));
+    const float vy = fminf(fmaxf(a.y + pp5, 0.0f), (float)(nyp - 1u));
+    return pack2(__fadd_rz(vx, FAST_MAGIC), __fadd_rz(vy, FAST_MAGIC));
+}
+
+__device__ __forceinline__ uint32_t offset_from_magic(F2 t, const FastGeo& f) {
+    float tx, ty;
+    unpack2(t, tx, ty);
+    return f.pitch * __float_as_uint(tx) + (8u * __float_as_uint(ty) + f.koff);
+}
+
+// Bilinear flow at a, whose pixel is floor2 (at byte offset `off` of uv);
+// unnormalised.
+__device__ __forceinline__ F2 taps_fast(F2 a, F2 floor2, uint32_t off, const float2* __restrict__ uv,
+                                        const FastGeo& f, const FastConst& k) {
+    const F2 w = add2(sub2(a, floor2), as_f2(k.pad));
+    const F2 w1 = sub2(as_f2(k.one), w);
+    float wr, wu, wl, wd;
+    unpack2(w, wr, wu);
+    unpack2(w1, wl, wd);
+    const char* b = reinterpret_cast<const char*>(uv);
+    const F2* p = reinterpret_cast<const F2*>(b + off);
+    const F2* q = reinterpret_cast<const F2*>(b + (off + f.pitch));
+    const F2 q00 = __ldg(p), q01 = __ldg(p + 1), q10 = __ldg(q), q11 = __ldg(q + 1);
+    const F2 wl2 = splat2(wl), wr2 = splat2(wr);
+    const F2 lo = add2_product(mul2(q00, wl2), mul2(q10, wr2), k);
+    const F2 hi = add2_product(mul2(q01, wl2), mul2(q11, wr2), k);
+    return add2_product(mul2(lo, splat2(wd)), mul2(hi, splat2(wu)), k);
+}
+
+// one generator step: lehmer_next up to its conditional subtraction
+__device__ __forceinline__ uint32_t lehmer_fast(uint32_t s) {
+    const u64 p = (u64)s * 279470273u + 279470273u;
+    const uint32_t lo = (uint32_t)p, hi = (uint32_t)(p >> 32);
+    const uint32_t h5 = hi * 5u;
+    const uint32_t y = lo + h5;
+    return y < lo ? y + 5u : y;
+}
+
+// Guards gathered over one step: the least square of a sampled component or
+// sum of squares of a jittered vector (NaN if one is), the largest state.
+struct FastGuard {
+    float smallest;
+    uint32_t state;
+};
+
+// The unit flow vector at a stage's point, jittered.
+template <bool JITTER>
+__device__ __forceinline__ F2 stage_fast(F2 a, F2 floor2, uint32_t off, uint32_t& rng, FastGuard& gd, float& sj,
+                                         const float2* __restrict__ uv, const FastGeo& f, const FastConst& k) {
+    float xx, yy;
+    F2 u = unit_fast(taps_fast(a, floor2, off, uv, f, k), xx, yy, sj);
+    gd.smallest = min3_nan(gd.smallest, xx, yy);
+    if (JITTER) {
+        const uint32_t r0 = lehmer_fast(rng), r1 = lehmer_fast(r0);
+        rng = r1;
+        gd.state = max(gd.state, max(r0, r1));
+        // r * 2^-32 - 1/2 in one rounding (the product is exact)
+        const F2 r = fma2(pack2(__uint2float_rn(r0), __uint2float_rn(r1)), as_f2(k.draw), as_f2(k.draw0));
+        u = unit_fast(add2_product(mul2(r, as_f2(k.mag)), u, k), xx, yy, sj);
+    }
+    return u;
+}
+
+// the pixel of an intermediate point, without clamps
+__device__ __forceinline__ void locate_fast(F2 a, const FastGeo& f, const FastConst& k, F2& floor2, uint32_t& off) {
+    const F2 t = add2_rz(add2(a, as_f2(k.pp5)), as_f2(k.magic));
+    floor2 = sub2(t, as_f2(k.magic));
+    off = min(offset_from_magic(t, f), f.off_last);  // in the grid even when a guard will fail
+}
+
+// Quantisation to 1 / TRAJECTORY_RESOLUTION (a power of two), |v| res < 127
+__device__ __forceinline__ float quant_fast(float v, const FastConst& k) {
+    const float t = __fmaf_rz(fabsf(v), k.res, FAST_MAGIC);
+    return copysignf(__fmaf_rn(t, k.inv, k.minus_magic_inv), v);
+}
+
+struct FastStep {
+    Vec2 d1, d2, next, u1;
+    F2 t;          // 2^23 + pixel of next
+    uint32_t off;  // byte offset of that pixel's vector
+    uint32_t rng;
+};
+
+// rk_step for a lane whose guards failed
+template <int ORDER, bool JITTER>
+__device__ __noinline__ FastStep step_exact(Vec2 a, float dt, uint32_t rng, float cf, const float2* uv, uint32_t base,
+                                            const slm_params& p, uint32_t nxp, uint32_t nyp) {
+    const Geo g{nxp, nyp, cf, 0.0f, 0.0f, 0.0f};  // the step itself reads neither DT_MAX nor GRID_SCALE
+    const Step st = rk_step<ORDER, JITTER>(a, dt, rng, uv + base, p, g);
+    return FastStep{st.d1, st.d2, st.next, st.u1, pixel_magic_clamped(st.next, p.pad_width_pp5, nxp, nyp),
+                    8u * (base + st.idx), rng};
+}
+
+// One RK step from a0 (pixel t0 - 2^23, at byte offset off0 of the array uv)
+// with time step dt; true if every guard held and the values are rk_step's.
+// GATED: a lane outside the interior reads nothing (its grid may have none);
+// else it reads its clamped pixel's taps.
+template <int ORDER, bool JITTER, bool GATED>
+__device__ __forceinline__ bool step_fast(Vec2 a0, F2 t0, uint32_t off0, float dt, float cf, uint32_t rng,
+                                          const float2* __restrict__ uv, const FastGeo& f, const FastConst& k,
+                                          FastStep& o) {
+    const F2 a = pack2(a0.x, a0.y);
+    const F2 cf2 = splat2(cf), dt2 = splat2(dt);
+    F2 fl = sub2(t0, as_f2(k.magic));
+    float ix, iy;
+    unpack2(sub2(fl, pack2(f.cx, f.cy)), ix, iy);
+    const bool inside = fabsf(ix) <= f.rx && fabsf(iy) <= f.ry;
+    if (GATED && !inside) return false;
+    uint32_t off = min(off0, f.off_last);
+    FastGuard gd{FAST_S_MIN, 0u};
+    float s1, s2, s3, s4;  // sums of squares of the stages' last vectors
+    const F2 k1 = stage_fast<JITTER>(a, fl, off, rng, gd, s1, uv, f, k);
+    const F2 h1 = mul2(mul2(k1, cf2), dt2);
+    float hx, hy, sx, sy;
+    unpack2(h1, hx, hy);
+    o.d1.x = quant_fast(hx, k);
+    o.d1.y = quant_fast(hy, k);
+    if (ORDER == 2) {
+        const F2 d1 = pack2(o.d1.x, o.d1.y);
+        const F2 b = add2(a, d1);
+        locate_fast(b, f, k, fl, off);
+        const F2 k2 = stage_fast<JITTER>(b, fl, off, rng, gd, s2, uv, f, k);
+        gd.smallest = min3_nan(gd.smallest, s1, s2);
+        unpack2(mul2(as_f2(k.half), add2_product(mul2(mul2(k2, cf2), dt2), d1, k)), sx, sy);
+    } else {
+        const F2 b = fma2(as_f2(k.half), h1, a);
+        locate_fast(b, f, k, fl, off);
+        const F2 h2 = mul2(mul2(stage_fast<JITTER>(b, fl, off, rng, gd, s2, uv, f, k), cf2), dt2);
+        gd.smallest = min3_nan(gd.smallest, s1, s2);
+        const F2 c = fma2(as_f2(k.half), h2, a);
+        locate_fast(c, f, k, fl, off);
+        const F2 h3 = mul2(mul2(stage_fast<JITTER>(c, fl, off, rng, gd, s3, uv, f, k), cf2), dt2);
+        const F2 d = add2_product(h3, a, k);
+        locate_fast(d, f, k, fl, off);
+        const F2 h4 = mul2(mul2(stage_fast<JITTER>(d, fl, off, rng, gd, s4, uv, f, k), cf2), dt2);
+        gd.smallest = min3_nan(gd.smallest, s3, s4);
+        const F2 w = add2_product(h4, fma2(as_f2(k.two), h3, fma2(as_f2(k.two), h2, h1)), k);
+        // div6 without its range test: below 2^-120 both quantise to 0
+        unpack2(fma2(as_f2(k.div6_hi), w, mul2(as_f2(k.div6_lo), w)), sx, sy);
+    }
+    o.d2.x = quant_fast(sx, k);
+    o.d2.y = quant_fast(sy, k);
+    const F2 next = add2(a, pack2(o.d2.x, o.d2.y));
+    o.t = add2_rz(add2(next, as_f2(k.pp5)), as_f2(k.magic));
+    o.off = offset_from_magic(o.t, f);
+    o.rng = rng;
+    unpack2(next, o.next.x, o.next.y);
+    unpack2(k1, o.u1.x, o.u1.y);
+    bool ok = gd.smallest >= FAST_S_MIN && inside;
+    if (JITTER) ok = ok && gd.state < LEHMER_M;
+    else ok = ok && fabsf(sx) < 1.0f && fabsf(sy) < 1.0f;  // an infinite sum of squares gives NaN here
+    return ok;
+}
+
+// next_dt from the two quantised steps' difference (ex, ey), its two
+// quotients by GRID_SCALE, the root and the last quotient formed as in
+// unit_fast (gs_rcp: the IEEE reciprocal of GRID_SCALE; a quotient by it is
+// exact by the same theorem).  A time step or an error too small for exact
+// residuals takes the IEEE operations.
+__device__ __forceinline__ float next_dt_fast(float ex, float ey, float dt, float dt_max, float gs, float gs_rcp,
+                                              float adjusted_max_error) {
+    const float qx = __fmul_rn(ex, gs_rcp), qy = __fmul_rn(ey, gs_rcp);
+    const float x = __fmaf_rn(-__fmaf_rn(gs, qx, -ex), gs_rcp, qx);
+    const float y = __fmaf_rn(-__fmaf_rn(gs, qy, -ey), gs_rcp, qy);
+    const float s = __fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y));
+    const float n = __fmul_rn(adjusted_max_error, dt);
+    float cand;
+    if (s >= 0x1p-100f && n >= FAST_S_MIN) {
+        float err, r;
+        root_and_reciprocal(s, err, r);
+        const float q = __fmul_rn(n, r);
+        cand = __fmaf_rn(-__fmaf_rn(err, q, -n), r, q);
+    } else {
+        if (ex == 0.0f && ey == 0.0f) return dt_max;
+        const float err = vlen(__fdiv_rn(ex, gs), __fdiv_rn(ey, gs));
+        if (err == 0.0f) return dt_max;
+        cand = __fdiv_rn(n, err);
+    }
+    return fminf(dt_max, cand);
+}
+
+}  // namespace slm

@@ -232,3 +232,77 @@ def test_float_to_char_matches_x86_for_every_float():
     torch.cuda.synchronize()
     bad, last = (int(v) for v in counts.view(torch.int64).cpu().tolist())
     assert bad == 0, "{} inputs differ, e.g. bit pattern {:#010x}".format(bad, last - 1)
+
+
+def test_unit_vector_root_and_reciprocal_for_every_float():
+    """The fast step's square root equals the IEEE root and its reciprocal is
+    near enough for both quotients to round as IEEE divisions, over every
+    finite sum of squares from 2^-100 up."""
+    import ctypes
+
+    from slm_b200 import _lib
+    counts = torch.zeros(2, dtype=torch.uint64, device=DEV)
+    _lib.check(_lib.load().slm_selftest_unit(_lib.ptr(counts),
+                                             ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    bad, last = (int(v) for v in counts.view(torch.int64).cpu().tolist())
+    assert bad == 0, "{} inputs fail, e.g. bit pattern {:#010x}".format(bad, last - 1)
+
+
+def _patch(kind):
+    """Flow that the fast step's guards must hand to the general step."""
+    def apply(c):
+        uv = c.uv
+        if kind == "zero":
+            uv[9:14, 8:15] = 0.0
+        elif kind == "axis":
+            uv[6:20, 6:12] = (1.0, 0.0)
+            uv[20:30, 6:12] = (0.0, -1.0)
+        elif kind == "tiny":
+            uv[5:25, 5:25] *= np.float32(1e-33)
+        elif kind == "huge":
+            uv[5:25, 5:25] *= np.float32(3e19)
+        elif kind == "one small component":
+            uv[5:30, 5:30, 1] *= np.float32(1e-12)
+    return apply
+
+
+def _set(**kw):
+    def apply(c):
+        for k, v in kw.items():
+            setattr(c.info, k, v)
+    return apply
+
+
+# (case, change): the launches on either side of each rule that admits the
+# fast step (fast_params, fast_grid), and flows on either side of its guards
+STEP_EDGES = [
+    (dict(nx=33, ny=47, pad=0), None), (dict(nx=33, ny=47, pad=1, step=0.1), None), (dict(nx=33, ny=21, pad=7), None),
+    (dict(nx=3, ny=4, step=0.1), None), (dict(nx=4, ny=4, step=0.5), None), (dict(nx=5, ny=29, step=0.1), None),
+    (dict(nx=40, ny=40, step=0.98), None), (dict(nx=40, ny=40, step=0.999), None), (dict(nx=40, ny=40, step=1.5), None),
+    (dict(nx=40, ny=30), _set(trajectory_resolution=np.uint32(100))),
+    (dict(nx=40, ny=30, step=0.4), _set(trajectory_resolution=np.uint32(256))),
+    (dict(nx=40, ny=30), _set(trajectory_resolution=np.uint32(512))),
+    (dict(nx=40, ny=30, jitter=0.7), None), (dict(nx=40, ny=30, jitter=0.0), None),
+    (dict(nx=40, ny=30, jitter=1e-13), None), (dict(nx=40, ny=30, jitter=2000.0), None),
+    (dict(nx=40, ny=30), _set(adjusted_max_error=np.float32(0.0))),
+    (dict(nx=40, ny=30), _set(adjusted_max_error=np.float32(0.01))),
+    (dict(nx=36, ny=30), _patch("zero")), (dict(nx=36, ny=30, jitter=0.0), _patch("axis")),
+    (dict(nx=36, ny=30), _patch("tiny")), (dict(nx=36, ny=30), _patch("huge")),
+    (dict(nx=36, ny=30, jitter=0.0), _patch("one small component")),
+]
+
+
+@pytest.mark.parametrize("kw,change", STEP_EDGES)
+@pytest.mark.parametrize("integrator", [2, 4])
+def test_fields_at_the_edges_of_the_fast_step(kw, change, integrator):
+    c = Case(**{"seed": 11, "max_length": 60.0, **kw})
+    if change:
+        change(c)
+    for sign in (1.0, -1.0):
+        prm = c.params("INTEGRATE_FIELDS", sign)
+        oslc, oslt, osteps, ontraj = O.integrate_fields(prm, c.seeds, c.mask, c.uv, integrator=integrator,
+                                                        n_threads=4)
+        slc, slt, steps, ntraj = _gpu_fields(c, prm, "persistent", integrator)
+        assert np.array_equal(slc, oslc) and np.array_equal(slt, oslt)
+        assert (steps, ntraj) == (osteps, ontraj)
