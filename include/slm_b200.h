@@ -505,6 +505,19 @@ int slm_cnn_infer(const float* uv, uint32_t nx_padded, uint32_t ny_padded, uint3
                   const float* w1, const float* b1,
                   const float* w2, const float* b2, const float* w3, const float* b3,
                   float* out, void* stream);
+/* The same predictions for many seeds of one grid: formed once per pixel of
+ * the padded grid into workspace (device, 8-byte aligned,
+ * slm_cnn_infer_grid_workspace bytes; a seed's patch depends only on its
+ * pixel) and then picked for the seeds; seeds whose pixel is off the grid go
+ * through slm_cnn_infer's kernel.  Equal to slm_cnn_infer but for the order
+ * of the last layer's fp32 sums.  Cheaper from about one seed in eight
+ * pixels on. */
+size_t slm_cnn_infer_grid_workspace(uint32_t nx_padded, uint32_t ny_padded);
+int slm_cnn_infer_grid(const float* uv, uint32_t nx_padded, uint32_t ny_padded, uint32_t pad,
+                       const float* seed_point, const uint32_t* index, uint32_t n,
+                       const float* w1, const float* b1,
+                       const float* w2, const float* b2, const float* w3, const float* b3,
+                       float* out, void* workspace, size_t workspace_bytes, void* stream);
 /* order [n]: seed indices by column col of pred [n][stride], longest predicted
  * first, in n_bins equal bins over [lo, hi] (bins: n_bins uint32 scratch) */
 int slm_order_by_prediction(const float* pred, uint32_t stride, uint32_t col, uint32_t n,

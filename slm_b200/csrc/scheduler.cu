@@ -18,6 +18,7 @@
 // tcgen05 with bf16 operands and fp32 accumulators in tensor memory, split-K
 // for the weight gradients); inference is one fused kernel per warp of 16
 // seeds (mma.sync m16n8k16 bf16 -> fp32).
+#include <algorithm>
 #include <cuda_bf16.h>
 #include "capi_util.cuh"
 
@@ -142,6 +143,12 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// a seed whose pixel is not in the padded grid
+__device__ __forceinline__ bool off_grid(float2 sp, uint32_t nxp, uint32_t nyp, uint32_t pad) {
+    const int cx = (int)sp.x + (int)pad, cy = (int)sp.y + (int)pad;
+    return cx < 0 || cx >= (int)nxp || cy < 0 || cy >= (int)nyp;
+}
+
 // Shared-memory layout of the inference kernel (bf16 pairs as uint32):
 //   W1t [32 n][16 kpairs], W2t [64 n][64 kpairs], W3t [8 n][128 kpairs] (n-major,
 //   so a B fragment (k pair, n) is one 32-bit word); biases fp32; per warp an
@@ -161,7 +168,10 @@ k_cnn_infer(const float2* __restrict__ uv, uint32_t nxp, uint32_t nyp, uint32_t 
             const float2* __restrict__ seeds, const uint32_t* __restrict__ index, uint32_t n,
             const float* __restrict__ w1,
             const float* __restrict__ b1, const float* __restrict__ w2, const float* __restrict__ b2,
-            const float* __restrict__ w3, const float* __restrict__ b3, float* __restrict__ out) {
+            const float* __restrict__ w3, const float* __restrict__ b3, float* __restrict__ out,
+            const uint32_t* __restrict__ outside) {
+    // outside (NULL: every seed): only the seeds off the grid, if it counted any
+    if (outside && *outside == 0u) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     InferSmem& S = *reinterpret_cast<InferSmem*>(smem_raw);
     for (int i = threadIdx.x; i < 32 * 16; i += blockDim.x) {
@@ -185,6 +195,11 @@ k_cnn_infer(const float2* __restrict__ uv, uint32_t nxp, uint32_t nyp, uint32_t 
     const int gid = lane >> 2, tig = lane & 3;
     const uint32_t groups = (n + 15) / 16;
     for (uint32_t grp = blockIdx.x * INF_WARPS + warp; grp < groups; grp += gridDim.x * INF_WARPS) {
+        if (outside) {
+            const uint32_t s = grp * 16 + (lane & 15);
+            const float2 sp = seeds[index ? __ldg(index + min(s, n - 1)) : min(s, n - 1)];
+            if (!__any_sync(0xffffffffu, off_grid(sp, nxp, nyp, pad))) continue;
+        }
         // 16 seeds per warp pass; conv1 + conv2 in 4 quarters of 4 seeds
         for (int q = 0; q < 4; ++q) {
             for (int sl = 0; sl < 4; ++sl) {
@@ -274,17 +289,223 @@ k_cnn_infer(const float2* __restrict__ uv, uint32_t nxp, uint32_t nyp, uint32_t 
             const uint32_t s0 = grp * 16 + gid, s1 = s0 + 8;
             if (s0 < n) {
                 const size_t o = index ? __ldg(index + s0) : s0;
-                out[2 * o] = c3[0] + S.b3[0];
-                out[2 * o + 1] = c3[1] + S.b3[1];
+                if (!outside || off_grid(seeds[o], nxp, nyp, pad)) {
+                    out[2 * o] = c3[0] + S.b3[0];
+                    out[2 * o + 1] = c3[1] + S.b3[1];
+                }
             }
             if (s1 < n) {
                 const size_t o = index ? __ldg(index + s1) : s1;
-                out[2 * o] = c3[2] + S.b3[0];
-                out[2 * o + 1] = c3[3] + S.b3[1];
+                if (!outside || off_grid(seeds[o], nxp, nyp, pad)) {
+                    out[2 * o] = c3[2] + S.b3[0];
+                    out[2 * o + 1] = c3[3] + S.b3[1];
+                }
             }
         }
         __syncwarp();
     }
+}
+
+// ------------------------------------------------------------------ dense inference
+// Predictions for every pixel of a grid.  The patches of neighbouring seeds
+// overlap: conv1's output at a tile depends only on where the tile lies, and
+// conv2's on its position too, so over a grid each is formed once per pixel
+// position instead of 16 and 4 times per seed,
+//
+//   A1(Q) = bf16(relu(W1 uv[Q .. Q+3] + b1))         (pixels clamped to the grid)
+//   A2(Q) = bf16(relu(W2 A1(Q + 4(ei, ej)) + b2))
+//   out(P) = b3 + sum over u of W3_u A2(P - 8 + 8(ui, uj))
+//
+// 9.8 k products per pixel against 50 k per seed, and no patch gathers (2 KB
+// per seed).  The products, their order and the roundings are k_cnn_infer's up
+// to the dense layer, whose four positions are summed apart and then added.
+//
+// A block walks down a strip of GRID_OUT columns, GRID_ROWS rows at a time.
+// A1 and the dense layer's partial sums D stay in rings of rows in shared
+// memory, so nothing is formed twice along x and 64 / 56 times along y.
+// conv2 is 95 % of the work: a warp owns two 16-position tiles, so each weight
+// fragment read from shared memory serves two products; A2 never leaves the
+// registers (an accumulator's layout is the next product's operand layout).
+// Row strides of 20 and 68 words keep the fragment loads free of bank
+// conflicts.
+//
+// Measured (B200, 3.07 M seeds, one per pixel of 1500 x 2048, spatial order
+// included): 3.54 -> 0.375 ms; the grid kernel itself 0.27 ms (350 TFLOP/s of
+// mma.sync work, its fragment loads about as busy as the tensor pipe).
+constexpr int GRID_OUT = 56;              // output columns of a strip
+constexpr int GRID_Q = GRID_OUT + 8;      // A2 columns
+constexpr int GRID_A = 80;                // A1 columns: GRID_Q + 4, in tiles of 16
+constexpr int GRID_UV = GRID_A + 4;       // flow columns (GRID_A + 3 are read)
+constexpr int GRID_ROWS = 4;
+constexpr int GRID_THREADS = 256;
+
+struct GridSmem {
+    uint32_t uv[8][GRID_UV];              // rows of bf16 (u, v) pairs
+    uint32_t a1[8][GRID_A][16 + 4];
+    uint32_t w1[32][16 + 4], w2[64][64 + 4], w3[8][32 + 4];
+    float b1[32], b2[64];
+    float2 d[12][GRID_Q][4];              // [row][column][u]
+};
+
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const uint32_t* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+
+// flow rows k0 .. k0 + n - 1 (row k is pixel row x0 - 8 + k) into their slots
+__device__ __forceinline__ void grid_load_uv(GridSmem& S, const float2* __restrict__ uv, int nxp, int nyp, int x0,
+                                             int y0, int k0, int n) {
+    for (int i = threadIdx.x; i < n * GRID_UV; i += GRID_THREADS) {
+        const int k = k0 + i / GRID_UV, c = i % GRID_UV;
+        const int x = min(max(x0 - 8 + k, 0), nxp - 1), y = min(max(y0 - 8 + c, 0), nyp - 1);
+        const float2 v = __ldg(uv + (size_t)x * nyp + y);
+        S.uv[k & 7][c] = pack_bf16(v.x, v.y);
+    }
+}
+
+// A1 rows k0 .. k0 + GRID_ROWS - 1
+__device__ __forceinline__ void grid_conv1(GridSmem& S, int k0, int warp, int lane) {
+    const int gid = lane >> 2, tig = lane & 3;
+    for (int tile = warp; tile < GRID_ROWS * (GRID_A / 16); tile += GRID_THREADS / 32) {
+        const int k = k0 + tile / (GRID_A / 16), c0 = (tile % (GRID_A / 16)) * 16;
+        float c[4][4] = {};
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+            uint32_t a[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                a[r] = S.uv[(k + 2 * ks + (r >> 1)) & 7][c0 + gid + ((r & 1) ? 8 : 0) + tig];
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt)
+                mma_bf16(c[nt], a, S.w1[nt * 8 + gid][ks * 8 + tig], S.w1[nt * 8 + gid][ks * 8 + tig + 4]);
+        }
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+            const int o = nt * 8 + tig * 2;
+            S.a1[k & 7][c0 + gid][o / 2] = pack_bf16(fmaxf(c[nt][0] + S.b1[o], 0.0f), fmaxf(c[nt][1] + S.b1[o + 1], 0.0f));
+            S.a1[k & 7][c0 + gid + 8][o / 2] =
+                pack_bf16(fmaxf(c[nt][2] + S.b1[o], 0.0f), fmaxf(c[nt][3] + S.b1[o + 1], 0.0f));
+        }
+    }
+}
+
+// conv2 and the dense layer's products of rows k0 .. k0 + GRID_ROWS - 1: warp
+// w owns columns 32 (w & 1) .. + 31 of row k0 + w / 2
+__device__ __forceinline__ void grid_conv2(GridSmem& S, int k0, int warp, int lane) {
+    const int gid = lane >> 2, tig = lane & 3;
+    const int k = k0 + (warp >> 1), c0 = (warp & 1) * 32;
+    const int arow = (lane & 7) + ((lane >> 3) & 1) * 8, aword = (lane >> 4) * 4;
+    const int brow = (lane & 7) + (lane >> 4) * 8, bword = ((lane >> 3) & 1) * 4;
+    float c[2][8][4] = {};
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+        const int e = ks >> 1, slot = (k + 4 * (e >> 1)) & 7, at = c0 + 4 * (e & 1) + arow;
+        uint32_t a[2][4];
+        ldmatrix_x4(a[0], &S.a1[slot][at][(ks & 1) * 8 + aword]);
+        ldmatrix_x4(a[1], &S.a1[slot][at + 16][(ks & 1) * 8 + aword]);
+#pragma unroll
+        for (int np = 0; np < 4; ++np) {
+            uint32_t b[4];
+            ldmatrix_x4(b, &S.w2[np * 16 + brow][ks * 8 + bword]);
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                mma_bf16(c[t][2 * np], a[t], b[0], b[1]);
+                mma_bf16(c[t][2 * np + 1], a[t], b[2], b[3]);
+            }
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        float d[4] = {};
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+            uint32_t a[4];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float(&v)[4] = c[t][2 * ks + h];
+                const int o = (2 * ks + h) * 8 + tig * 2;
+                a[2 * h] = pack_bf16(fmaxf(v[0] + S.b2[o], 0.0f), fmaxf(v[1] + S.b2[o + 1], 0.0f));
+                a[2 * h + 1] = pack_bf16(fmaxf(v[2] + S.b2[o], 0.0f), fmaxf(v[3] + S.b2[o + 1], 0.0f));
+            }
+            mma_bf16(d, a, S.w3[gid][ks * 8 + tig], S.w3[gid][ks * 8 + tig + 4]);
+        }
+        // column 2u + o of the product is output o of position u
+        S.d[k % 12][c0 + 16 * t + gid][tig] = make_float2(d[0], d[1]);
+        S.d[k % 12][c0 + 16 * t + gid + 8][tig] = make_float2(d[2], d[3]);
+    }
+}
+
+// map [nxp][nyp] float2: the predictions of a seed at each pixel of the
+// padded grid.  Blocks: strips of GRID_OUT columns (x), row ranges (y) of
+// rows_per_block (a multiple of GRID_ROWS).
+__global__ void __launch_bounds__(GRID_THREADS, 2)
+k_cnn_grid(const float2* __restrict__ uv, int nxp, int nyp, int rows_per_block, const float* __restrict__ w1,
+           const float* __restrict__ b1, const float* __restrict__ w2, const float* __restrict__ b2,
+           const float* __restrict__ w3, const float* __restrict__ b3, float2* __restrict__ map) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    GridSmem& S = *reinterpret_cast<GridSmem*>(smem_raw);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int y0 = blockIdx.x * GRID_OUT, x0 = blockIdx.y * rows_per_block;
+    const int rows = min(rows_per_block, nxp - x0);
+    for (int i = threadIdx.x; i < 32 * 16; i += GRID_THREADS) {
+        const int n = i % 32, kp = i / 32;
+        S.w1[n][kp] = pack_bf16(w1[2 * kp * CNN_C1 + n], w1[(2 * kp + 1) * CNN_C1 + n]);
+    }
+    for (int i = threadIdx.x; i < 64 * 64; i += GRID_THREADS) {
+        const int n = i % 64, kp = i / 64;
+        S.w2[n][kp] = pack_bf16(w2[2 * kp * CNN_C2 + n], w2[(2 * kp + 1) * CNN_C2 + n]);
+    }
+    // dense weights as [2u + o][k pairs of position u]
+    for (int i = threadIdx.x; i < 8 * 32; i += GRID_THREADS) {
+        const int n = i / 32, kp = i % 32, h = 64 * (n >> 1) + 2 * kp;
+        S.w3[n][kp] = pack_bf16(w3[h * CNN_OUT + (n & 1)], w3[(h + 1) * CNN_OUT + (n & 1)]);
+    }
+    if (threadIdx.x < 32) S.b1[threadIdx.x] = b1[threadIdx.x];
+    if (threadIdx.x < 64) S.b2[threadIdx.x] = b2[threadIdx.x];
+    const float o0 = __ldg(b3), o1 = __ldg(b3 + 1);
+    grid_load_uv(S, uv, nxp, nyp, x0, y0, 0, 7);
+    __syncthreads();
+    grid_conv1(S, 0, warp, lane);
+    // rows k of A2 and D: pixel row x0 - 8 + k; outputs start at k = 8
+    for (int k0 = 0; k0 < rows + 8; k0 += GRID_ROWS) {
+        __syncthreads();  // the last pass's readers of the slots written next
+        grid_load_uv(S, uv, nxp, nyp, x0, y0, k0 + 7, 4);
+        __syncthreads();
+        grid_conv1(S, k0 + 4, warp, lane);
+        __syncthreads();
+        grid_conv2(S, k0, warp, lane);
+        __syncthreads();
+        if (k0 >= 8) {
+            for (int i = threadIdx.x; i < GRID_ROWS * GRID_OUT; i += GRID_THREADS) {
+                const int k = k0 + i / GRID_OUT, c = i % GRID_OUT;
+                const int x = x0 - 8 + k, y = y0 + c;
+                if (k - 8 >= rows || y >= nyp) continue;
+                const float2 d0 = S.d[(k - 8) % 12][c][0], d1 = S.d[(k - 8) % 12][c + 8][1];
+                const float2 d2 = S.d[k % 12][c][2], d3 = S.d[k % 12][c + 8][3];
+                map[(size_t)x * nyp + y] =
+                    make_float2((((d0.x + d1.x) + d2.x) + d3.x) + o0, (((d0.y + d1.y) + d2.y) + d3.y) + o1);
+            }
+        }
+    }
+}
+
+// out [n][2] from the map of predictions; *outside counts the seeds whose
+// pixel is not in the grid (k_cnn_infer takes those)
+__global__ void k_cnn_pick(const float2* __restrict__ map, uint32_t nxp, uint32_t nyp, uint32_t pad,
+                           const float2* __restrict__ seeds, const uint32_t* __restrict__ index, uint32_t n,
+                           float* __restrict__ out, uint32_t* __restrict__ outside) {
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= n) return;
+    const size_t i = index ? __ldg(index + j) : j;
+    const float2 sp = __ldg(seeds + i);
+    if (off_grid(sp, nxp, nyp, pad)) {
+        atomicAdd(outside, 1u);
+        return;
+    }
+    const float2 v = __ldg(map + (size_t)((int)sp.x + (int)pad) * nyp + ((int)sp.y + (int)pad));
+    out[2 * i] = v.x;
+    out[2 * i + 1] = v.y;
 }
 
 // ------------------------------------------------------------------ ordering
@@ -498,6 +719,23 @@ int slm_adam(float* w, float* wq, const float* g, float* m, float* v, uint64_t n
     return SLM_OK;
 }
 
+static int launch_infer(const float* uv, uint32_t nx_padded, uint32_t ny_padded, uint32_t pad,
+                        const float* seed_point, const uint32_t* index, uint32_t n, const float* w1, const float* b1,
+                        const float* w2, const float* b2, const float* w3, const float* b3, float* out,
+                        const uint32_t* outside, cudaStream_t s) {
+    const size_t smem = sizeof(InferSmem);
+    SLM_CUDA(cudaFuncSetAttribute(k_cnn_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const uint32_t groups = (n + 15) / 16;
+    unsigned grid = (groups + INF_WARPS - 1) / INF_WARPS;
+    const unsigned cap = (unsigned)num_sms() * 8u;
+    if (grid > cap) grid = cap;
+    k_cnn_infer<<<grid, INF_WARPS * 32, smem, s>>>(
+        reinterpret_cast<const float2*>(uv), nx_padded, ny_padded, pad,
+        reinterpret_cast<const float2*>(seed_point), index, n, w1, b1, w2, b2, w3, b3, out, outside);
+    SLM_LAUNCHED("k_cnn_infer");
+    return SLM_OK;
+}
+
 int slm_cnn_infer(const float* uv, uint32_t nx_padded, uint32_t ny_padded, uint32_t pad,
                   const float* seed_point, const uint32_t* index, uint32_t n, const float* w1,
                   const float* b1,
@@ -506,17 +744,53 @@ int slm_cnn_infer(const float* uv, uint32_t nx_padded, uint32_t ny_padded, uint3
     clear_error();
     if (n == 0) return SLM_OK;
     SLM_REQUIRE(uv && seed_point && w1 && b1 && w2 && b2 && w3 && b3 && out, "NULL buffer");
-    const size_t smem = sizeof(InferSmem);
-    SLM_CUDA(cudaFuncSetAttribute(k_cnn_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const uint32_t groups = (n + 15) / 16;
-    unsigned grid = (groups + INF_WARPS - 1) / INF_WARPS;
-    const unsigned cap = (unsigned)num_sms() * 8u;
-    if (grid > cap) grid = cap;
-    k_cnn_infer<<<grid, INF_WARPS * 32, smem, (cudaStream_t)stream>>>(
-        reinterpret_cast<const float2*>(uv), nx_padded, ny_padded, pad,
-        reinterpret_cast<const float2*>(seed_point), index, n, w1, b1, w2, b2, w3, b3, out);
-    SLM_LAUNCHED("k_cnn_infer");
-    return SLM_OK;
+    return launch_infer(uv, nx_padded, ny_padded, pad, seed_point, index, n, w1, b1, w2, b2, w3, b3, out, nullptr,
+                        (cudaStream_t)stream);
+}
+
+size_t slm_cnn_infer_grid_workspace(uint32_t nx_padded, uint32_t ny_padded) {
+    return (size_t)nx_padded * ny_padded * sizeof(float2) + 256;
+}
+
+int slm_cnn_infer_grid(const float* uv, uint32_t nx_padded, uint32_t ny_padded, uint32_t pad,
+                       const float* seed_point, const uint32_t* index, uint32_t n, const float* w1,
+                       const float* b1, const float* w2, const float* b2, const float* w3, const float* b3,
+                       float* out, void* workspace, size_t workspace_bytes, void* stream) {
+    clear_error();
+    if (n == 0) return SLM_OK;
+    SLM_REQUIRE(uv && seed_point && w1 && b1 && w2 && b2 && w3 && b3 && out && workspace, "NULL buffer");
+    SLM_REQUIRE(nx_padded > 0 && ny_padded > 0 && nx_padded < (1u << 24) && ny_padded < (1u << 24) &&
+                    (uint64_t)nx_padded * ny_padded < (1ull << 32),
+                "grid size");
+    const size_t need = slm_cnn_infer_grid_workspace(nx_padded, ny_padded);
+    SLM_REQUIRE(workspace_bytes >= need, "workspace holds %zu bytes, needs %zu", workspace_bytes, need);
+    SLM_REQUIRE(aligned(workspace, 8) && aligned(uv, 8) && aligned(seed_point, 8), "misaligned buffer");
+    cudaStream_t s = (cudaStream_t)stream;
+    float2* map = static_cast<float2*>(workspace);
+    uint32_t* outside = reinterpret_cast<uint32_t*>(map + (size_t)nx_padded * ny_padded);
+    SLM_CUDA(cudaMemsetAsync(outside, 0, sizeof(uint32_t), s));
+    // Row ranges: a block of `rows` rows forms rows + 8 of them (and stages the
+    // weights, about 8 rows' worth of time), and two blocks run on an SM at a
+    // time, so take the range count with the least waves x (rows + 16).
+    const uint32_t strips = (ny_padded + GRID_OUT - 1) / GRID_OUT, resident = 2u * (uint32_t)num_sms();
+    uint32_t rows = 0;
+    uint64_t best = ~0ull;
+    for (uint32_t r = 8; r <= 512; r += GRID_ROWS) {
+        const uint64_t blocks = (uint64_t)strips * ((nx_padded + r - 1) / r);
+        const uint64_t cost = (blocks + resident - 1) / resident * (r + 16);
+        if (cost < best) best = cost, rows = r;
+    }
+    const dim3 grid(strips, (nx_padded + rows - 1) / rows);
+    SLM_REQUIRE(grid.y < 65536, "nx_padded too large");
+    const size_t smem = sizeof(GridSmem);
+    SLM_CUDA(cudaFuncSetAttribute(k_cnn_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_cnn_grid<<<grid, GRID_THREADS, smem, s>>>(reinterpret_cast<const float2*>(uv), (int)nx_padded, (int)ny_padded,
+                                                (int)rows, w1, b1, w2, b2, w3, b3, map);
+    SLM_LAUNCHED("k_cnn_grid");
+    k_cnn_pick<<<(n + 255) / 256, 256, 0, s>>>(map, nx_padded, ny_padded, pad,
+                                               reinterpret_cast<const float2*>(seed_point), index, n, out, outside);
+    SLM_LAUNCHED("k_cnn_pick");
+    return launch_infer(uv, nx_padded, ny_padded, pad, seed_point, index, n, w1, b1, w2, b2, w3, b3, out, outside, s);
 }
 
 int slm_order_by_prediction(const float* pred, uint32_t stride, uint32_t col, uint32_t n, float lo,

@@ -338,3 +338,38 @@ def test_fields_spatial_order_identical():
         out.append((data.slc_array.copy(), data.slt_array.copy(), list(f.n_steps)))
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
     assert out[0][2] == out[1][2] and out[0][2][0] > 0
+
+
+@pytest.mark.parametrize("nxp,nyp,pad", [(1, 1, 0), (5, 3, 1), (20, 56, 2), (33, 57, 2), (31, 113, 0), (70, 64, 4),
+                                         (203, 55, 2)])
+def test_grid_predictions_equal_per_seed(nxp, nyp, pad, monkeypatch):
+    """Predictions formed once per pixel against the per-seed kernel: the same
+    products and activations, so they differ at most by the last layer's fp32
+    sums taken in another order -- 256 terms, one unit in the last place each
+    (2^-23) on either side.  Some seeds lie off the grid."""
+    import ctypes
+
+    from slm_b200 import _lib
+    rng = np.random.default_rng(nxp * 1000 + nyp)
+    uv = rng.standard_normal((nxp, nyp, 2)).astype(np.float32)
+    n = nxp * nyp + 37
+    seeds = np.stack([rng.integers(-pad, nxp - pad, n), rng.integers(-pad, nyp - pad, n)], 1).astype(np.float32)
+    seeds[::29] += np.float32(0.75)
+    seeds[5::31, 0] = -20.0 - pad
+    seeds[7::41, 1] = nyp + 3.0
+    w = _weights(4)
+    m = S.LengthModel(DEV, w)
+    uv_d, seeds_d = torch.from_numpy(uv).to(DEV), torch.from_numpy(seeds).to(DEV)
+    visit = torch.from_numpy(rng.permutation(n).astype(np.uint32)).to(DEV)
+    monkeypatch.setattr(S, "DENSE_SEEDS", 1)  # predict takes the grid form
+    got = m.predict(uv_d, nxp, nyp, pad, seeds_d, n, visit=visit)
+    ref = torch.full((n, 2), float("nan"), device=DEV)
+    P, W = _lib.ptr, m.W
+    _lib.check(m.L.slm_cnn_infer(P(uv_d), nxp, nyp, pad, P(seeds_d), None, n, P(W["w1"]), P(W["b1"]), P(W["w2"]),
+                                 P(W["b2"]), P(W["w3"]), P(W["b3"]), P(ref),
+                                 ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    c = LM.forward({k: v.cpu().numpy() for k, v in W.items()}, LM.gather(uv, pad, seeds))[1]
+    mag = np.abs(c["x3"]) @ np.abs(c["W"]["w3"]) + np.abs(c["W"]["b3"])
+    diff = (got.double() - ref.double()).abs().cpu().numpy()
+    assert np.all(diff <= 2 * 256 * 2.0 ** -23 * mag)
