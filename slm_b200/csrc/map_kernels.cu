@@ -43,7 +43,7 @@
 #include <type_traits>
 #include <vector>
 #include "capi_util.cuh"
-#include "trace_common.cuh"
+#include "trace_fast.cuh"
 
 #define MAP_ST_CAP 1u
 #define MAP_ST_OOB 2u
@@ -60,30 +60,37 @@ __device__ __forceinline__ Vec2 seed_vec(const float2* __restrict__ seeds, uint3
     return Vec2{s.x, s.y};
 }
 
-struct Move { float err, dl; bool stuck; };
+struct Move { float ex, ey, dl; bool stuck; };
 
 // the shared tail of every *_runge_kutta_step (rungekutta.cl:289-296 ...):
-// error, length, first-order fallback when stuck, move to the new point
-__device__ __forceinline__ Move rk_move(const Step& s, Vec2& vec, uint32_t& idx, const slm_params& p) {
+// the steps' difference, length, first-order fallback when stuck, move to the
+// new point
+__device__ __forceinline__ Move rk_move(const Step& s, Vec2& vec, uint32_t& idx, const slm_params& p,
+                                        const WalkGrid& wg) {
     Move m;
-    m.err = vlen(__fdiv_rn(s.d2.x - s.d1.x, p.grid_scale), __fdiv_rn(s.d2.y - s.d1.y, p.grid_scale));
-    Vec2 next = s.next;
-    m.dl = vlen(s.d2.x, s.d2.y);
+    m.ex = s.d2.x - s.d1.x;
+    m.ey = s.d2.y - s.d1.y;
+    m.dl = step_length(s.d2, wg);
     if (m.dl < p.integration_halt_threshold) {
-        next.x = vec.x + s.d1.x;
-        next.y = vec.y + s.d1.y;
-        m.dl = vlen(s.d1.x, s.d1.y);
+        vec.x = vec.x + s.d1.x;
+        vec.y = vec.y + s.d1.y;
+        m.dl = step_length(s.d1, wg);
+        idx = pixel_of(vec, p);
+    } else {
+        vec = s.next;
+        idx = s.idx;
     }
-    vec = next;
-    idx = pixel_of(next, p);
     m.stuck = m.dl < p.integration_halt_threshold;
     return m;
 }
 
+__device__ __forceinline__ float next_dt(float dt, const Move& m, const slm_params& p, const WalkGrid& wg) {
+    return walk_dt(m.ex, m.ey, dt, p, wg);
+}
+
 __device__ __forceinline__ Step rk_plain(Vec2 a, float dt, const float2* __restrict__ uv,
-                                         const slm_params& p) {
-    uint32_t rng = 0;
-    return rk_step<2, false>(a, dt, rng, uv, p);
+                                         const slm_params& p, const WalkGrid& wg) {
+    return plain_step<2>(a, dt, uv, p, wg);
 }
 
 // Brent's cycle detection on a walk's (vec, dt) state, which determines the
@@ -105,7 +112,8 @@ struct StateCycle {
 };
 
 // ------------------------------------------------------------------ connect
-__global__ void k_connect_channels(const slm_params p, uint32_t n, const float2* __restrict__ seeds,
+__global__ void k_connect_channels(const __grid_constant__ slm_params p, const __grid_constant__ WalkGrid wg,
+                                   uint32_t n, const float2* __restrict__ seeds,
                                    const uint8_t* __restrict__ mask, const float2* __restrict__ uv,
                                    uint32_t* mapping, uint32_t* status) {
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -117,19 +125,28 @@ __global__ void k_connect_channels(const slm_params p, uint32_t n, const float2*
     Vec2 vec = start, prev = start;
     float dt = p.dt_max;
     uint32_t idx = pixel_of(vec, p), prev_idx = idx, n_steps = 0, guard = 0;
+    // (vec, dt) determines the rest of the walk: once it repeats inside the
+    // start pixel (Brent) the walk circles there until n_steps reaches
+    // MAX_N_STEPS.  With that at or above INTERCHANNEL_MAX_N_STEPS nothing is
+    // flagged then, whatever is recorded until there, so it ends at once;
+    // walks stuck in pits and on flats are what the launch otherwise waits for.
+    const bool may_end = p.max_n_steps >= p.interchannel_max_n_steps;
+    StateCycle cyc;
+    cyc.init(vec, dt);
     while (prev_idx == idx && !mask[idx] && n_steps != p.max_n_steps) {
         if (++guard > MAP_LOOP_CAP) { atomicOr(status, MAP_ST_CAP); break; }
-        const Step s = rk_plain(vec, dt, uv, p);
+        const Step s = rk_plain(vec, dt, uv, p, wg);
         idx = s.idx;
         if (!mask[idx]) {
-            const Move m = rk_move(s, vec, idx, p);
-            if (!m.stuck) dt = next_dt(dt, m.err, p);
+            const Move m = rk_move(s, vec, idx, p, wg);
+            if (!m.stuck) dt = next_dt(dt, m, p, wg);
             if (n_steps < cap_rec) {
                 rec[2 * n_steps] = cvt_i8((vec.x - prev.x) * res);
                 rec[2 * n_steps + 1] = cvt_i8((vec.y - prev.y) * res);
             }
             n_steps++;
             if (!m.stuck) prev = vec;
+            if (may_end && prev_idx == idx && cyc.repeated(vec, dt)) return;
         }
     }
     // The second loop ends at n_steps == INTERCHANNEL_MAX_N_STEPS (every pass
@@ -142,11 +159,11 @@ __global__ void k_connect_channels(const slm_params p, uint32_t n, const float2*
     while (n_steps <= p.interchannel_max_n_steps && (mapping[idx] & p.is_channel) == 0 && !mask[idx]
            && n_steps != p.interchannel_max_n_steps) {
         if (++guard > MAP_LOOP_CAP) { atomicOr(status, MAP_ST_CAP); break; }
-        const Step s = rk_plain(vec, dt, uv, p);
+        const Step s = rk_plain(vec, dt, uv, p, wg);
         idx = s.idx;
         if (!mask[idx]) {
-            const Move m = rk_move(s, vec, idx, p);
-            if (!m.stuck) dt = next_dt(dt, m.err, p);
+            const Move m = rk_move(s, vec, idx, p, wg);
+            if (!m.stuck) dt = next_dt(dt, m, p, wg);
             if (n_steps < cap_rec) {
                 rec[2 * n_steps] = cvt_i8((vec.x - prev.x) * res);
                 rec[2 * n_steps + 1] = cvt_i8((vec.y - prev.y) * res);
@@ -170,7 +187,8 @@ __global__ void k_connect_channels(const slm_params p, uint32_t n, const float2*
 }
 
 // ------------------------------------------------------------------ channel heads
-__global__ void k_map_channel_heads(const slm_params p, uint32_t n, const float2* __restrict__ seeds,
+__global__ void k_map_channel_heads(const __grid_constant__ slm_params p, const __grid_constant__ WalkGrid wg,
+                                    uint32_t n, const float2* __restrict__ seeds,
                                     const uint8_t* __restrict__ mask, const float2* __restrict__ uv,
                                     uint32_t* mapping) {
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -186,11 +204,11 @@ __global__ void k_map_channel_heads(const slm_params p, uint32_t n, const float2
     StateCycle cyc;
     cyc.init(vec, dt);
     while (prev_idx == idx && !mask[idx] && n_steps < p.max_n_steps) {
-        const Step s = rk_plain(vec, dt, uv, p);
+        const Step s = rk_plain(vec, dt, uv, p, wg);
         idx = s.idx;
-        const Move m = rk_move(s, vec, idx, p);
+        const Move m = rk_move(s, vec, idx, p, wg);
         n_steps++;
-        dt = next_dt(dt, m.err, p);
+        dt = next_dt(dt, m, p, wg);
         if (prev_idx == idx && cyc.repeated(vec, dt)) return;
     }
     if (n_steps >= p.max_n_steps) return;
@@ -319,7 +337,8 @@ struct EventWriter {
     }
 };
 
-__global__ void k_count_paths(const slm_params p, uint32_t n, const float2* __restrict__ seeds,
+__global__ void k_count_paths(const __grid_constant__ slm_params p, const __grid_constant__ WalkGrid wg,
+                              uint32_t n, const float2* __restrict__ seeds,
                               const uint8_t* __restrict__ mask, const float2* __restrict__ uv,
                               u64* __restrict__ n_events, const u64* __restrict__ offsets,
                               uint32_t* __restrict__ events, uint32_t* __restrict__ tail_idx) {
@@ -345,11 +364,11 @@ __global__ void k_count_paths(const slm_params p, uint32_t n, const float2* __re
     float tdt = dt;
     uint32_t power = 1, lam = 0;
     while (!mask[idx] && n_steps < lim) {
-        const Step s = rk_plain(vec, dt, uv, p);
+        const Step s = rk_plain(vec, dt, uv, p, wg);
         idx = s.idx;
-        const Move m = rk_move(s, vec, idx, p);
+        const Move m = rk_move(s, vec, idx, p, wg);
         if (m.stuck) break;
-        dt = next_dt(dt, m.err, p);
+        dt = next_dt(dt, m, p, wg);
         n_steps++;
         if (prev_idx != idx) {
             w.event(idx);
@@ -372,10 +391,10 @@ __global__ void k_count_paths(const slm_params p, uint32_t n, const float2* __re
                     E = nfut;  // written after the pattern
                 }
                 for (uint32_t t = 1; t <= L; ++t) {
-                    const Step s2 = rk_plain(v2, d2, uv, p);
+                    const Step s2 = rk_plain(v2, d2, uv, p, wg);
                     i2 = s2.idx;
-                    const Move m2 = rk_move(s2, v2, i2, p);
-                    d2 = next_dt(d2, m2.err, p);
+                    const Move m2 = rk_move(s2, v2, i2, p, wg);
+                    d2 = next_dt(d2, m2, p, wg);
                     if (prev2 != i2) {
                         if (pass == 0) {
                             E++;
@@ -695,11 +714,11 @@ __global__ void k_segment_downchannels(const slm_params p, uint32_t n, const flo
 
 // segment_runge_kutta_step (rungekutta.cl:435-459): n_steps++ always, stuck ends
 __device__ __forceinline__ bool seg_move(const Step& s, Vec2& vec, uint32_t& idx, float& dt,
-                                         uint32_t& n_steps, const slm_params& p) {
-    const Move m = rk_move(s, vec, idx, p);
+                                         uint32_t& n_steps, const slm_params& p, const WalkGrid& wg) {
+    const Move m = rk_move(s, vec, idx, p, wg);
     n_steps++;
     if (m.stuck) return true;
-    dt = next_dt(dt, m.err, p);
+    dt = next_dt(dt, m, p, wg);
     return false;
 }
 
@@ -711,7 +730,8 @@ __device__ __forceinline__ bool seg_move(const Step& s, Vec2& vec, uint32_t& idx
 constexpr uint32_t WALK_PER_WARP = 256;
 
 template <class W>
-__global__ void __launch_bounds__(256) k_walks(W w, uint32_t n) {
+__global__ void __launch_bounds__(256)
+k_walks(const __grid_constant__ slm_params p, const __grid_constant__ WalkGrid wg, W w, uint32_t n) {
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -724,13 +744,13 @@ __global__ void __launch_bounds__(256) k_walks(W w, uint32_t n) {
         if (idle && next < hi) {
             const uint64_t mine = next + __popc(idle & ((1u << lane) - 1u));
             next += __popc(idle);
-            if (!alive && mine < hi) alive = w.start((uint32_t)mine);
+            if (!alive && mine < hi) alive = w.start((uint32_t)mine, p);
         }
         if (!__any_sync(FULL, alive)) {
             if (next >= hi) break;
             continue;
         }
-        if (alive) alive = w.step();
+        if (alive) alive = w.step(p, wg);
     }
 }
 
@@ -742,7 +762,6 @@ static unsigned walk_grid(uint32_t n) {
 // segment_hillslopes (segment.cl): from each hillslope pixel down to a thin
 // channel, whose label it takes
 struct SegHillWalk {
-    slm_params p;
     const float2* seeds;
     const uint8_t* mask;
     const float2* uv;
@@ -752,35 +771,35 @@ struct SegHillWalk {
     float dt;
     uint32_t idx, h, n_steps;
     StateCycle cyc;
-    __device__ bool start(uint32_t g) {
+    __device__ bool start(uint32_t g, const slm_params& p) {
         vec = seed_vec(seeds, g);
         idx = pixel_of(vec, p);
         h = idx;
         n_steps = 0;
         dt = p.dt_max;
         cyc.init(vec, dt);
-        return step_test();
+        return step_test(p);
     }
     // the loop test; false ends the walk (and writes its label)
-    __device__ bool step_test() {
+    __device__ bool step_test(const slm_params& p) {
         if (!mask[idx] && ((~mapping[idx]) & p.is_thinchannel) && n_steps < p.max_n_steps) return true;
-        finish();
+        finish(p);
         return false;
     }
-    __device__ void finish() {
+    __device__ void finish(const slm_params& p) {
         if (mapping[idx] & p.is_thinchannel) label[h] = label[idx];
     }
-    __device__ bool step() {
-        const Step s = rk_plain(vec, dt, uv, p);
+    __device__ bool step(const slm_params& p, const WalkGrid& wg) {
+        const Step s = rk_plain(vec, dt, uv, p, wg);
         idx = s.idx;
-        if (seg_move(s, vec, idx, dt, n_steps, p)) {
-            finish();
+        if (seg_move(s, vec, idx, dt, n_steps, p, wg)) {
+            finish(p);
             return false;
         }
         // a cycle of states that all continue the loop ends at the bound on a
         // pixel that is not a thin channel: no label
         if (cyc.repeated(vec, dt)) return false;
-        return step_test();
+        return step_test(p);
     }
 };
 
@@ -846,7 +865,6 @@ __global__ void k_subsegment_channel_edges(const slm_params p, uint32_t n,
 // subsegment_flanks (segment.cl:360-414): from each pixel down to a left
 // flank or thin channel; the left-flank bit when a left flank is reached
 struct SubsegFlankWalk {
-    slm_params p;
     const float2* seeds;
     const uint8_t* mask;
     const float2* uv;
@@ -856,36 +874,36 @@ struct SubsegFlankWalk {
     float dt;
     uint32_t idx, h, n_steps;
     StateCycle cyc;
-    __device__ bool start(uint32_t g) {
+    __device__ bool start(uint32_t g, const slm_params& p) {
         vec = seed_vec(seeds, g);
         idx = pixel_of(vec, p);
         h = idx;
         n_steps = 0;
         dt = p.dt_max;
         cyc.init(vec, dt);
-        return step_test();
+        return step_test(p);
     }
-    __device__ bool step_test() {
+    __device__ bool step_test(const slm_params& p) {
         if (!mask[idx] && ((~mapping[idx]) & p.is_leftflank) && ((~mapping[idx]) & p.is_thinchannel)
             && n_steps < p.max_n_steps)
             return true;
-        finish();
+        finish(p);
         return false;
     }
-    __device__ void finish() {
+    __device__ void finish(const slm_params& p) {
         if (mapping[idx] & p.is_leftflank) label[h] |= p.left_flank_addition;
     }
-    __device__ bool step() {
-        const Step s = rk_plain(vec, dt, uv, p);
+    __device__ bool step(const slm_params& p, const WalkGrid& wg) {
+        const Step s = rk_plain(vec, dt, uv, p, wg);
         idx = s.idx;
-        if (seg_move(s, vec, idx, dt, n_steps, p)) {
-            finish();
+        if (seg_move(s, vec, idx, dt, n_steps, p, wg)) {
+            finish(p);
             return false;
         }
         // a cycle of states that all continue the loop ends at the bound on a
         // pixel that is not left flank: no flank bit
         if (cyc.repeated(vec, dt)) return false;
-        return step_test();
+        return step_test(p);
     }
 };
 
@@ -962,7 +980,7 @@ struct LinkedSink {
 // of the item range at a time, so the stored paths fit the workspace).
 // The walk of item g into `sink`; returns its pair count.
 template <class Sink>
-__device__ u64 flank_walk(const slm_params& p, uint32_t g, const float2* __restrict__ seeds,
+__device__ u64 flank_walk(const slm_params& p, const WalkGrid& wg, uint32_t g, const float2* __restrict__ seeds,
                           const uint8_t* __restrict__ stop, const float2* __restrict__ uv, Sink& sink) {
     Vec2 vec = seed_vec(seeds, g);
     uint32_t idx = pixel_of(vec, p), n_steps = 0;
@@ -976,10 +994,10 @@ __device__ u64 flank_walk(const slm_params& p, uint32_t g, const float2* __restr
     float tdt = dt;
     uint32_t power = 1, lam = 0;
     while (!stop[idx] && n_steps < p.max_n_steps) {
-        const Step s = rk_plain(vec, dt, uv, p);
+        const Step s = rk_plain(vec, dt, uv, p, wg);
         const uint32_t q = s.idx;
         idx = q;
-        const bool stuck = seg_move(s, vec, idx, dt, n_steps, p);
+        const bool stuck = seg_move(s, vec, idx, dt, n_steps, p, wg);
         if (q != last.x || idx != last.y) {
             last = make_uint2(q, idx);
             sink.put(last);
@@ -1001,10 +1019,10 @@ __device__ u64 flank_walk(const slm_params& p, uint32_t g, const float2* __restr
                     sink.put(make_uint2(FLANK_PERIOD | E, nfut));
                 }
                 for (uint32_t t2 = 1; t2 <= L; ++t2) {
-                    const Step s2 = rk_plain(v2, d2, uv, p);
+                    const Step s2 = rk_plain(v2, d2, uv, p, wg);
                     const uint32_t q2 = s2.idx;
                     i2 = q2;
-                    seg_move(s2, v2, i2, d2, ns2, p);
+                    seg_move(s2, v2, i2, d2, ns2, p, wg);
                     if (q2 != l2.x || i2 != l2.y) {
                         l2 = make_uint2(q2, i2);
                         if (pass == 0) {
@@ -1030,7 +1048,7 @@ __device__ u64 flank_walk(const slm_params& p, uint32_t g, const float2* __restr
 
 // Items g0 .. g0+n-1: with pairs == NULL the pair counts into n_pairs[g],
 // else the pairs into pairs[offsets[g] - base ..].
-__global__ void k_flank_paths(const slm_params p, uint32_t g0, uint32_t n, const float2* __restrict__ seeds,
+__global__ void k_flank_paths(const __grid_constant__ slm_params p, const __grid_constant__ WalkGrid wg, uint32_t g0, uint32_t n, const float2* __restrict__ seeds,
                               const uint8_t* __restrict__ stop, const float2* __restrict__ uv,
                               u64* __restrict__ n_pairs, const u64* __restrict__ offsets, u64 base,
                               uint2* __restrict__ pairs) {
@@ -1038,7 +1056,7 @@ __global__ void k_flank_paths(const slm_params p, uint32_t g0, uint32_t n, const
     if (t >= n) return;
     const uint32_t g = g0 + t;
     ContigSink sink{pairs ? pairs + (offsets[g] - base) : nullptr, 0};
-    const u64 k = flank_walk(p, g, seeds, stop, uv, sink);
+    const u64 k = flank_walk(p, wg, g, seeds, stop, uv, sink);
     if (!pairs) n_pairs[g] = k;
 }
 
@@ -1046,7 +1064,7 @@ __global__ void k_flank_paths(const slm_params p, uint32_t g0, uint32_t n, const
 // (head block heads[g], NO_BLOCK for an empty path), its count into
 // n_pairs[g]; pool_ctr[0] counts the blocks taken, pool_ctr[1] is set when
 // the pool ran out (the counts are still exact).
-__global__ void k_flank_paths_linked(const slm_params p, uint32_t n, const float2* __restrict__ seeds,
+__global__ void k_flank_paths_linked(const __grid_constant__ slm_params p, const __grid_constant__ WalkGrid wg, uint32_t n, const float2* __restrict__ seeds,
                                      const uint8_t* __restrict__ stop, const float2* __restrict__ uv,
                                      u64* __restrict__ n_pairs, uint32_t* __restrict__ heads,
                                      uint2* __restrict__ pool, uint32_t cap_blocks, uint32_t* pool_ctr) {
@@ -1054,7 +1072,7 @@ __global__ void k_flank_paths_linked(const slm_params p, uint32_t n, const float
     if (g >= n) return;
     heads[g] = NO_BLOCK;
     LinkedSink sink{pool, pool_ctr, pool_ctr + 1, cap_blocks, NO_BLOCK, 0, heads + g, 0, true};
-    n_pairs[g] = flank_walk(p, g, seeds, stop, uv, sink);
+    n_pairs[g] = flank_walk(p, wg, g, seeds, stop, uv, sink);
 }
 
 // The label of pixel q as flank item g sees it: item g's own running value if
@@ -1459,7 +1477,8 @@ k_flank_settle(const slm_params p, uint32_t g0, uint32_t n, uint32_t side, const
 }
 
 // ------------------------------------------------------------------ hillslopes
-__global__ void k_hillslopes(const slm_params p, uint32_t n, const float2* __restrict__ seeds,
+__global__ void k_hillslopes(const __grid_constant__ slm_params p, const __grid_constant__ WalkGrid wg,
+                             uint32_t n, const float2* __restrict__ seeds,
                              const uint8_t* __restrict__ mask, const float2* __restrict__ uv,
                              uint32_t* link) {
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1474,11 +1493,11 @@ __global__ void k_hillslopes(const slm_params p, uint32_t n, const float2* __res
     uint32_t power = 1, lam = 0;
     while (prev_idx == idx && !mask[idx] && n_steps < 100u * p.max_n_steps) {
         prev_idx = idx;
-        const Step s = rk_plain(vec, dt, uv, p);
+        const Step s = rk_plain(vec, dt, uv, p, wg);
         idx = s.idx;
-        const Move m = rk_move(s, vec, idx, p);
+        const Move m = rk_move(s, vec, idx, p, wg);
         if (m.stuck) break;
-        dt = next_dt(dt, m.err, p);
+        dt = next_dt(dt, m, p, wg);
         n_steps++;
         if (idx == prev_idx && __float_as_uint(vec.x) == __float_as_uint(tv.x)
             && __float_as_uint(vec.y) == __float_as_uint(tv.y) && __float_as_uint(dt) == __float_as_uint(tdt))
@@ -1493,7 +1512,8 @@ __global__ void k_hillslopes(const slm_params p, uint32_t n, const float2* __res
     if (prev_idx != idx && !mask[idx]) link[prev_idx] = idx;
 }
 
-__global__ void k_hillslope_lengths(const slm_params p, uint32_t n, const float2* __restrict__ seeds,
+__global__ void k_hillslope_lengths(const __grid_constant__ slm_params p, const __grid_constant__ WalkGrid wg,
+                                    uint32_t n, const float2* __restrict__ seeds,
                                     const uint8_t* __restrict__ mask, const float2* __restrict__ uv,
                                     const uint32_t* __restrict__ mapping, float* traj_length) {
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1511,7 +1531,7 @@ __global__ void k_hillslope_lengths(const slm_params p, uint32_t n, const float2
     StateCycle cyc;
     cyc.init(vec, dt);
     while (((~mapping[idx]) & p.is_thinchannel) && n_steps < p.max_n_steps) {
-        const Step s = rk_plain(vec, dt, uv, p);
+        const Step s = rk_plain(vec, dt, uv, p, wg);
         idx = s.idx;
         if (mask[idx]) return;
         bool turned = false;
@@ -1521,11 +1541,11 @@ __global__ void k_hillslope_lengths(const slm_params p, uint32_t n, const float2
         } else if (moved_off && (mapping[idx] & from_flag)) {
             return;
         }
-        const Move m = rk_move(s, vec, idx, p);
+        const Move m = rk_move(s, vec, idx, p, wg);
         l = l + m.dl;
         n_steps++;
         if (m.stuck) return;
-        dt = next_dt(dt, m.err, p);
+        dt = next_dt(dt, m, p, wg);
         if (turned) cyc.init(vec, dt);
         else if (cyc.repeated(vec, dt)) return;
     }
@@ -1820,7 +1840,7 @@ int slm_connect_channels(const slm_params* p, uint32_t n, const float* seed_poin
     SLM_REQUIRE(status, "status word is NULL");
     SLM_CUDA(cudaMemsetAsync(status, 0, sizeof(uint32_t), SS));
     if (n == 0) return SLM_OK;
-    k_connect_channels<<<blocks_for(n, 128), 128, 0, SS>>>(*p, n, F2(seed_point), mask, F2(uv), mapping, status);
+    k_connect_channels<<<blocks_for(n, 128), 128, 0, SS>>>(*p, make_walk_grid(*p), n, F2(seed_point), mask, F2(uv), mapping, status);
     SLM_LAUNCHED("k_connect_channels");
     return SLM_OK;
 }
@@ -1831,7 +1851,7 @@ int slm_map_channel_heads(const slm_params* p, uint32_t n, const float* seed_poi
     int rc = map_checks(p, n, seed_point);
     if (rc) return rc;
     if (n == 0) return SLM_OK;
-    k_map_channel_heads<<<blocks_for(n, 128), 128, 0, SS>>>(*p, n, F2(seed_point), mask, F2(uv), mapping);
+    k_map_channel_heads<<<blocks_for(n, 128), 128, 0, SS>>>(*p, make_walk_grid(*p), n, F2(seed_point), mask, F2(uv), mapping);
     SLM_LAUNCHED("k_map_channel_heads");
     return SLM_OK;
 }
@@ -1867,7 +1887,7 @@ int slm_count_downchannels(const slm_params* p, uint32_t n, const float* seed_po
     u64* offsets = n_events + n;
     uint32_t* tails = reinterpret_cast<uint32_t*>(offsets + n + 1);
     uint32_t* events = tails + n;
-    k_count_paths<<<blocks_for(n, 128), 128, 0, SS>>>(*p, n, F2(seed_point), mask, F2(uv), n_events,
+    k_count_paths<<<blocks_for(n, 128), 128, 0, SS>>>(*p, make_walk_grid(*p), n, F2(seed_point), mask, F2(uv), n_events,
                                                      nullptr, nullptr, nullptr);
     SLM_LAUNCHED("k_count_paths");
     k_exclusive_scan<<<1, 1024, 0, SS>>>(n_events, n, offsets);
@@ -1882,7 +1902,7 @@ int slm_count_downchannels(const slm_params* p, uint32_t n, const float* seed_po
                   (unsigned long long)total);
         return SLM_ERR_CAPACITY;
     }
-    k_count_paths<<<blocks_for(n, 128), 128, 0, SS>>>(*p, n, F2(seed_point), mask, F2(uv), nullptr,
+    k_count_paths<<<blocks_for(n, 128), 128, 0, SS>>>(*p, make_walk_grid(*p), n, F2(seed_point), mask, F2(uv), nullptr,
                                                      offsets, events, tails);
     SLM_LAUNCHED("k_count_paths");
     SLM_REQUIRE(p->nxy_padded < 0xFFFFFFE0u, "grid too large for the count replay");
@@ -1972,8 +1992,8 @@ int slm_segment_hillslopes(const slm_params* p, uint32_t n, const float* seed_po
     int rc = map_checks(p, n, seed_point);
     if (rc) return rc;
     if (n == 0) return SLM_OK;
-    SegHillWalk w{*p, F2(seed_point), mask, F2(uv), mapping, label};
-    k_walks<SegHillWalk><<<walk_grid(n), 256, 0, SS>>>(w, n);
+    SegHillWalk w{F2(seed_point), mask, F2(uv), mapping, label};
+    k_walks<SegHillWalk><<<walk_grid(n), 256, 0, SS>>>(*p, make_walk_grid(*p), w, n);
     SLM_LAUNCHED("k_walks<SegHillWalk>");
     return SLM_OK;
 }
@@ -2003,8 +2023,8 @@ int slm_subsegment_flanks(const slm_params* p, uint32_t n, const float* seed_poi
     int rc = map_checks(p, n, seed_point);
     if (rc) return rc;
     if (n == 0) return SLM_OK;
-    SubsegFlankWalk w{*p, F2(seed_point), mask, F2(uv), mapping, label};
-    k_walks<SubsegFlankWalk><<<walk_grid(n), 256, 0, SS>>>(w, n);
+    SubsegFlankWalk w{F2(seed_point), mask, F2(uv), mapping, label};
+    k_walks<SubsegFlankWalk><<<walk_grid(n), 256, 0, SS>>>(*p, make_walk_grid(*p), w, n);
     SLM_LAUNCHED("k_walks<SubsegFlankWalk>");
     return SLM_OK;
 }
@@ -2093,7 +2113,7 @@ static int fix_flanks(const slm_params* p, uint32_t n, const float* seed_point, 
         settle_grid = (unsigned)(num_sms() * (occ > 0 ? occ : 1));
         const u64 cap_blocks = cap_pairs / FLANK_BLOCK;
         k_flank_paths_linked<<<blocks_for(n, 128), 128, 0, SS>>>(
-            *p, n, F2(seed_point), stop, F2(uv), n_pairs, heads, pairs,
+            *p, make_walk_grid(*p), n, F2(seed_point), stop, F2(uv), n_pairs, heads, pairs,
             (uint32_t)(cap_blocks < 0xfffffffeull ? cap_blocks : 0xfffffffeull), words + 3);
         SLM_LAUNCHED("k_flank_paths_linked");
         counted = true;
@@ -2120,7 +2140,7 @@ static int fix_flanks(const slm_params* p, uint32_t n, const float* seed_point, 
     //    item reads only initial labels and the final labels of lower-index
     //    owners, which earlier chunks have resolved.
     if (!counted) {
-        k_flank_paths<<<blocks_for(n, 128), 128, 0, SS>>>(*p, 0u, n, F2(seed_point), stop, F2(uv), n_pairs,
+        k_flank_paths<<<blocks_for(n, 128), 128, 0, SS>>>(*p, make_walk_grid(*p), 0u, n, F2(seed_point), stop, F2(uv), n_pairs,
                                                          nullptr, 0ull, nullptr);
         SLM_LAUNCHED("k_flank_paths");
     }
@@ -2162,7 +2182,7 @@ static int fix_flanks(const slm_params* p, uint32_t n, const float* seed_point, 
             u64 base = 0;
             SLM_CUDA(cudaMemcpyAsync(&base, offsets + a, sizeof(u64), cudaMemcpyDeviceToHost, SS));
             SLM_CUDA(cudaStreamSynchronize(SS));
-            k_flank_paths<<<blocks_for(m, 128), 128, 0, SS>>>(*p, a, m, F2(seed_point), stop, F2(uv), nullptr,
+            k_flank_paths<<<blocks_for(m, 128), 128, 0, SS>>>(*p, make_walk_grid(*p), a, m, F2(seed_point), stop, F2(uv), nullptr,
                                                              offsets, base, pairs);
             SLM_LAUNCHED("k_flank_paths");
             SLM_CUDA(cudaMemsetAsync(words + 1, 0, sizeof(uint32_t), SS));
@@ -2186,7 +2206,7 @@ static int fix_flanks(const slm_params* p, uint32_t n, const float* seed_point, 
         u64 base = 0;
         SLM_CUDA(cudaMemcpyAsync(&base, offsets + a, sizeof(u64), cudaMemcpyDeviceToHost, SS));
         SLM_CUDA(cudaStreamSynchronize(SS));
-        k_flank_paths<<<blocks_for(m, 128), 128, 0, SS>>>(*p, a, m, F2(seed_point), stop, F2(uv), nullptr,
+        k_flank_paths<<<blocks_for(m, 128), 128, 0, SS>>>(*p, make_walk_grid(*p), a, m, F2(seed_point), stop, F2(uv), nullptr,
                                                          offsets, base, pairs);
         SLM_LAUNCHED("k_flank_paths");
         uint32_t done = 0;
@@ -2239,7 +2259,7 @@ int slm_hillslopes(const slm_params* p, uint32_t n, const float* seed_point, con
     int rc = map_checks(p, n, seed_point);
     if (rc) return rc;
     if (n == 0) return SLM_OK;
-    k_hillslopes<<<blocks_for(n, 128), 128, 0, SS>>>(*p, n, F2(seed_point), mask, F2(uv), link);
+    k_hillslopes<<<blocks_for(n, 128), 128, 0, SS>>>(*p, make_walk_grid(*p), n, F2(seed_point), mask, F2(uv), link);
     SLM_LAUNCHED("k_hillslopes");
     return SLM_OK;
 }
@@ -2276,7 +2296,7 @@ int slm_hillslope_lengths(const slm_params* p, uint32_t n, const float* seed_poi
     int rc = map_checks(p, n, seed_point);
     if (rc) return rc;
     if (n == 0) return SLM_OK;
-    k_hillslope_lengths<<<blocks_for(n, 128), 128, 0, SS>>>(*p, n, F2(seed_point), mask, F2(uv), mapping,
+    k_hillslope_lengths<<<blocks_for(n, 128), 128, 0, SS>>>(*p, make_walk_grid(*p), n, F2(seed_point), mask, F2(uv), mapping,
                                                            traj_length);
     SLM_LAUNCHED("k_hillslope_lengths");
     return SLM_OK;

@@ -488,11 +488,15 @@ __device__ __forceinline__ void put_step(int8_t* rec, uint32_t n, float dx, floa
     reinterpret_cast<uint16_t*>(rec)[n] = (uint16_t)(lo | (hi << 8));
 }
 
+// One warp a block: a thousand trajectories are 32 warps, each as long as the
+// latency of its longest walk's steps, so they take an SM each.
+constexpr unsigned TRAJ_BLOCK = 32;
+
 // trajectory_record (trajectory.cl:41-80) with runge_kutta_step_record and
 // euler_step_record (rungekutta.cl:49-120)
 template <int ORDER>
-__global__ void __launch_bounds__(128)
-k_trajectory(const slm_params p, uint32_t n_chunk, const float2* __restrict__ seeds,
+__global__ void __launch_bounds__(TRAJ_BLOCK)
+k_trajectory(const __grid_constant__ slm_params p, const __grid_constant__ WalkGrid wg, uint32_t n_chunk, const float2* __restrict__ seeds,
              const uint8_t* __restrict__ mask, const float2* __restrict__ uv,
              int8_t* __restrict__ traj, uint16_t* __restrict__ nsteps_out,
              float* __restrict__ length_out) {
@@ -504,26 +508,24 @@ k_trajectory(const slm_params p, uint32_t n_chunk, const float2* __restrict__ se
     const float res = (float)p.trajectory_resolution;
     const float2 c = __ldg(seeds + seed_idx);
     Vec2 a{c.x, c.y}, prev = a;
-    uint32_t n = 0, rng = 0;
+    uint32_t n = 0;
     float l = 0.0f, dt = p.dt_max;
-    const Geo geo = geo_of(p);
-    uint32_t idx = pixel_of(a, p, geo);
+    uint32_t idx = pixel_of(a, p);
     while (!__ldg(mask + idx) && (l < p.max_length && n < p.max_n_steps)) {
-        const Step st = rk_step<ORDER, false>(a, dt, rng, uv, p, geo);
+        const Step st = plain_step<ORDER>(a, dt, uv, p, wg);
         idx = st.idx;
         if (!__ldg(mask + idx)) {
-            const float err = vlen(div_gs(st.d2.x - st.d1.x, geo), div_gs(st.d2.y - st.d1.y, geo));
-            Vec2 next = st.next;
-            float dl = vlen(st.d2.x, st.d2.y);
+            float dl = step_length(st.d2, wg);
             if (dl < p.integration_halt_threshold) {
-                next.x = a.x + st.d1.x;
-                next.y = a.y + st.d1.y;
-                dl = vlen(st.d1.x, st.d1.y);
+                a.x = a.x + st.d1.x;
+                a.y = a.y + st.d1.y;
+                dl = step_length(st.d1, wg);
+                idx = pixel_of(a, p);
+            } else {
+                a = st.next;
             }
-            a = next;
-            idx = pixel_of(next, p, geo);
             const bool stuck = dl < p.integration_halt_threshold;
-            if (!stuck) dt = next_dt(dt, err, p, geo);
+            if (!stuck) dt = walk_dt(st.d2.x - st.d1.x, st.d2.y - st.d1.y, dt, p, wg);
             l = l + dl;
             put_step(rec, n, a.x - prev.x, a.y - prev.y, res);
             n++;
@@ -849,13 +851,14 @@ int slm_integrate_trajectory(const slm_params* p, int32_t integrator, uint32_t n
     SLM_REQUIRE(aligned(trajectories, 2) && aligned(nsteps, 2) && aligned(length, 4),
                 "trajectory buffers misaligned");
     cudaStream_t s = (cudaStream_t)stream;
-    const unsigned block = 128, grid = (n_chunk + block - 1) / block;
+    const unsigned grid = (n_chunk + TRAJ_BLOCK - 1) / TRAJ_BLOCK;
+    const WalkGrid wg = make_walk_grid(*p);
     const float2* sp = reinterpret_cast<const float2*>(seed_point);
     const float2* u2 = reinterpret_cast<const float2*>(uv);
     if (integrator == SLM_RK4)
-        k_trajectory<4><<<grid, block, 0, s>>>(*p, n_chunk, sp, mask, u2, trajectories, nsteps, length);
+        k_trajectory<4><<<grid, TRAJ_BLOCK, 0, s>>>(*p, wg, n_chunk, sp, mask, u2, trajectories, nsteps, length);
     else
-        k_trajectory<2><<<grid, block, 0, s>>>(*p, n_chunk, sp, mask, u2, trajectories, nsteps, length);
+        k_trajectory<2><<<grid, TRAJ_BLOCK, 0, s>>>(*p, wg, n_chunk, sp, mask, u2, trajectories, nsteps, length);
     SLM_LAUNCHED("k_trajectory");
     return SLM_OK;
 }

@@ -406,4 +406,50 @@ __device__ __forceinline__ float next_dt_fast(float ex, float ey, float dt, floa
     return fminf(dt_max, cand);
 }
 
+// ------------------------------------------------------------------ plain walks
+// The un-jittered step of the trajectory recorder and the mapping walks,
+// which are bound by the latency of one step after another: by step_fast
+// where the launch admits it, else by rk_step.  Uniform in a launch.
+struct WalkGrid {
+    FastGeo f;
+    FastConst k;
+    uint32_t fast;
+};
+
+static inline WalkGrid make_walk_grid(const slm_params& p) {
+    WalkGrid w;
+    w.f = make_fast_geo(p.nx_padded, p.ny_padded, p.grid_scale, p.dt_max, p.adjusted_max_error, 0u);
+    w.k = make_fast_const(p);
+    w.fast = fast_params(p) &&
+             fast_grid(p.nx_padded, p.ny_padded, 0u, p.combo_factor, p.dt_max, p.trajectory_resolution);
+    return w;
+}
+
+template <int ORDER>
+__device__ __forceinline__ Step plain_step(Vec2 a, float dt, const float2* __restrict__ uv, const slm_params& p,
+                                           const WalkGrid& w) {
+    FastStep st;
+    bool ok = false;
+    if (w.fast) {
+        const F2 t = pixel_magic_clamped(a, p.pad_width_pp5, p.nx_padded, p.ny_padded);
+        ok = step_fast<ORDER, false, false>(a, t, offset_from_magic(t, w.f), dt, p.combo_factor, 0u, uv, w.f, w.k, st);
+    }
+    if (!ok) st = step_exact<ORDER, false>(a, dt, 0u, p.combo_factor, uv, 0u, p, p.nx_padded, p.ny_padded);
+    return Step{st.d1, st.d2, st.u1, st.next, st.off >> 3};
+}
+
+// |d| of a quantised step
+__device__ __forceinline__ float step_length(Vec2 d, const WalkGrid& w) {
+    return w.fast ? quantised_length(__fmaf_rn(d.y, d.y, d.x * d.x)) : vlen(d.x, d.y);
+}
+
+// the next time step after one of dt whose quantised steps differ by (ex, ey)
+__device__ __forceinline__ float walk_dt(float ex, float ey, float dt, const slm_params& p, const WalkGrid& w) {
+    if (w.fast) {
+        if (dt * dt * w.f.kerr >= __fmaf_rn(ey, ey, ex * ex)) return p.dt_max;
+        return next_dt_fast(ex, ey, dt, p.dt_max, p.grid_scale, w.f.gs_rcp, p.adjusted_max_error);
+    }
+    return next_dt(dt, vlen(__fdiv_rn(ex, p.grid_scale), __fdiv_rn(ey, p.grid_scale)), p);
+}
+
 }  // namespace slm
