@@ -25,14 +25,14 @@
 //   fix_right_flanks, fix_left_flanks  every work-item writes only its own
 //       pixel's label and reads labels along its RK path, so its result depends
 //       only on the final labels of lower-index items owning pixels on that
-//       path.  One persistent launch (k_flank_resolve) takes items in
-//       ascending order and walks each once, waiting for the final label of a
-//       lower-index owner it reads.  Fallback (a bounded wait ran out): paths
-//       are traced in parallel (k_flank_paths, compressed to the steps whose
-//       (compute pixel, moved-to pixel) pair changes), then items are
-//       resolved in rounds (k_flank_round): an item resolves once every
-//       lower-index owner it reads has resolved in an earlier round.  The
-//       lowest unresolved item always can, so both forms end.
+//       path.  Paths are traced in parallel (k_flank_paths_linked, compressed
+//       to the steps whose (compute pixel, moved-to pixel) pair changes), then
+//       one persistent launch (k_flank_settle) takes items in ascending order,
+//       each waiting for the final labels of the lower-index owners on its
+//       path.  Fallback (a bounded wait ran out): items are resolved in rounds
+//       (k_flank_round): an item resolves once every lower-index owner it
+//       reads has resolved in an earlier round.  The lowest unresolved item
+//       always can, so both forms end.
 //
 // Every loop is bounded; a cap that the reference would exceed (it would loop
 // on) or a neighbour index outside the grid sets a bit in the caller's status
@@ -918,9 +918,11 @@ __global__ void k_owner_map(const slm_params p, uint32_t n, const float2* __rest
 }
 
 // Stored flank paths: linked blocks of FLANK_BLOCK entries, FLANK_BLOCK - 1
-// pairs and the index of the next block.
+// pairs and the indices of the next and the previous block.  A path is named
+// by its last block, with FLANK_FORWARD set if it is settled from its start.
 constexpr uint32_t FLANK_BLOCK = 32;
 constexpr uint32_t NO_BLOCK = 0xffffffffu;
+constexpr uint32_t FLANK_FORWARD = 0x80000000u;
 
 // A block index for each calling lane of the warp (one atomic per call site
 // and warp); NO_BLOCK when the pool of cap blocks is used up.
@@ -940,6 +942,7 @@ __device__ __forceinline__ uint32_t take_block(uint32_t* taken, uint32_t cap) {
 struct ContigSink {
     uint2* out;
     u64 k;
+    __device__ void settle_forward() {}
     __device__ void put(uint2 e) {
         if (out) out[k] = e;
         ++k;
@@ -951,9 +954,10 @@ struct LinkedSink {
     uint32_t* taken;
     uint32_t* overflow;
     uint32_t cap, cur, f;
-    uint32_t* head;
     u64 k;
-    bool ok;
+    bool ok, forward;
+    __device__ void settle_forward() { forward = true; }
+    __device__ uint32_t name() const { return cur == NO_BLOCK ? NO_BLOCK : (forward ? cur | FLANK_FORWARD : cur); }
     __device__ void put(uint2 e) {
         ++k;
         if (!ok) return;
@@ -964,8 +968,8 @@ struct LinkedSink {
                 atomicOr(overflow, 1u);
                 return;
             }
-            if (cur == NO_BLOCK) *head = b;
-            else pool[(u64)cur * FLANK_BLOCK + (FLANK_BLOCK - 1)] = make_uint2(b, 0u);
+            if (cur != NO_BLOCK) pool[(u64)cur * FLANK_BLOCK + (FLANK_BLOCK - 1)].x = b;
+            pool[(u64)b * FLANK_BLOCK + (FLANK_BLOCK - 1)] = make_uint2(NO_BLOCK, cur);
             cur = b;
             f = 0;
         }
@@ -984,8 +988,13 @@ __device__ u64 flank_walk(const slm_params& p, const WalkGrid& wg, uint32_t g, c
                           const uint8_t* __restrict__ stop, const float2* __restrict__ uv, Sink& sink) {
     Vec2 vec = seed_vec(seeds, g);
     uint32_t idx = pixel_of(vec, p), n_steps = 0;
+    const uint32_t h = idx;
     float dt = p.dt_max;
     uint2 last = make_uint2(NO_OWNER, NO_OWNER);
+    // Whether the walk has computed off its own pixel: a pair that starts from
+    // that pixel afterwards reads the item's running label, so such a path is
+    // settled from its start, as are paths with a period record.
+    bool left_home = false;
     // As in count_downchannels: once (vec, dt) repeats bit for bit the
     // per-step pairs repeat with the period, so the rest of the walk is
     // stored as one period record {0x80000000|E, n} + the E pairs of a lap
@@ -999,6 +1008,8 @@ __device__ u64 flank_walk(const slm_params& p, const WalkGrid& wg, uint32_t g, c
         idx = q;
         const bool stuck = seg_move(s, vec, idx, dt, n_steps, p, wg);
         if (q != last.x || idx != last.y) {
+            if (left_home && last.y == h) sink.settle_forward();
+            left_home = left_home || q != h;
             last = make_uint2(q, idx);
             sink.put(last);
         }
@@ -1016,6 +1027,7 @@ __device__ u64 flank_walk(const slm_params& p, const WalkGrid& wg, uint32_t g, c
                 if (pass == 1) {
                     const uint32_t nfut = (R / L) * E + partial;
                     if (nfut == 0) break;
+                    sink.settle_forward();
                     sink.put(make_uint2(FLANK_PERIOD | E, nfut));
                 }
                 for (uint32_t t2 = 1; t2 <= L; ++t2) {
@@ -1061,18 +1073,18 @@ __global__ void k_flank_paths(const __grid_constant__ slm_params p, const __grid
 }
 
 // Items 0 .. n-1 in one pass: each path into linked blocks from the pool
-// (head block heads[g], NO_BLOCK for an empty path), its count into
+// (its name into names[g], NO_BLOCK for an empty path), its count into
 // n_pairs[g]; pool_ctr[0] counts the blocks taken, pool_ctr[1] is set when
 // the pool ran out (the counts are still exact).
 __global__ void k_flank_paths_linked(const __grid_constant__ slm_params p, const __grid_constant__ WalkGrid wg, uint32_t n, const float2* __restrict__ seeds,
                                      const uint8_t* __restrict__ stop, const float2* __restrict__ uv,
-                                     u64* __restrict__ n_pairs, uint32_t* __restrict__ heads,
+                                     u64* __restrict__ n_pairs, uint32_t* __restrict__ names,
                                      uint2* __restrict__ pool, uint32_t cap_blocks, uint32_t* pool_ctr) {
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n) return;
-    heads[g] = NO_BLOCK;
-    LinkedSink sink{pool, pool_ctr, pool_ctr + 1, cap_blocks, NO_BLOCK, 0, heads + g, 0, true};
+    LinkedSink sink{pool, pool_ctr, pool_ctr + 1, cap_blocks, NO_BLOCK, 0, 0, true, false};
     n_pairs[g] = flank_walk(p, wg, g, seeds, stop, uv, sink);
+    names[g] = sink.name();
 }
 
 // The label of pixel q as flank item g sees it: item g's own running value if
@@ -1178,44 +1190,64 @@ __global__ void k_flank_round(const slm_params p, uint32_t g0, uint32_t n, uint3
 // The stored paths of a chunk of flank items resolved in one persistent
 // launch instead of rounds.  Warps take items in ascending index from a
 // queue (warp-aggregated atomicAdd), so every item below one a lane holds
-// has been taken.  A lane scans its item's stored path as k_flank_round does;
-// at a read of a lower-index owner that has not resolved it stops, notes that
-// owner and its place in the path (the start of a period record when inside
-// one, with the running label there), and on later passes only polls the
-// owner's flag until it can go on.  The lowest unresolved item taken waits on
-// nothing unresolved, so some lane always advances.  A label is published
-// by a release store of its resolved flag, read with acquire.  The RK walks are traced in parallel
-// beforehand (k_flank_paths), so only the path scans lie on a chain of waits.
+// has been taken.  The RK walks are traced in parallel beforehand
+// (k_flank_paths), so only the path scans lie on a chain of waits.
+//
+// An item reads the labels of lower-index owners along its path, and those
+// wait for the owners further down in turn, so what bounds the launch is the
+// chain of waits.  A lane therefore scans its path from its END: the far
+// pixels are those whose owners are resolved first, and when the nearest
+// owner, the last of them, resolves, one pair is left to scan.  (From the
+// start, the scan of the whole path would begin only then: a chain of n
+// pixels costs n^2 / 2 pair scans.)  The pairs already scanned are held as
+// the function they apply to the item's label.  One scan step takes
+// lab -> v when v's segment (the bits but the flank bit) differs from lab's,
+// so a run of steps is one of
+//   identity;   lab -> v unless lab has v's segment;   lab -> v,
+// closed under putting one more step before it.  A pair at which the walk
+// stops (its label is on the other flank) drops everything after it.
+// Two kinds of path do not allow this and are scanned from their start, up to
+// a read of an unresolved owner at a time: those with a period record (walks
+// that circle until the step bound), and those that come back to the item's
+// own pixel, whose running label decides there.
+//
+// The lowest unresolved item taken waits on nothing unresolved, so some lane
+// always advances.  Each pixel has a 16-byte record, (owner, initial label)
+// and (final label, resolved): the second half is published by one 8-byte
+// store, so a reader needs no fence and one load.
 //
 // Every wait is bounded: a lane that polls FLANK_WAIT_LIMIT times in a row
 // sets bit 0 of *status, and every warp stops; the caller then resolves the
 // items in rounds (k_flank_round) from the initial labels.
 #define FLANK_WAIT_LIMIT (1u << 24)
 
-// the label of pixel q as item g reads it (flank_read's rules, with the
-// owner's flag, read with acquire, instead of its round); false and *wait_o
-// when the owner has not resolved.  Out of line, as flank_read.
-// a flag read that orders the loads after it (acquire), and the flag write
-// that publishes the stores before it (release), at GPU scope
-__device__ __forceinline__ uint32_t load_acquire(const uint32_t* a) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a) : "memory");
+struct __align__(16) FlankRec {
+    u64 init;   // owner | initial label << 32
+    u64 final;  // label | 1 << 32 once resolved, else 0
+};
+
+// both halves of a record in one load, each half read atomically, from L2
+__device__ __forceinline__ FlankRec load_rec(const FlankRec* r) {
+    FlankRec v;
+    asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.init), "=l"(v.final) : "l"(r) : "memory");
     return v;
 }
-__device__ __forceinline__ void store_release(uint32_t* a, uint32_t v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(a), "r"(v) : "memory");
+
+// (where several items have the same pixel, its owner's label is the one read)
+__device__ __forceinline__ void publish(FlankRec* rec, uint32_t* label, uint32_t g, uint32_t h, uint32_t lab) {
+    label[h] = lab;
+    if ((uint32_t)rec[h].init == g) *(volatile u64*)&rec[h].final = (u64)lab | (1ull << 32);
 }
 
-__device__ __noinline__ bool settle_read(uint32_t q, uint32_t g, uint32_t h, uint32_t lab_h,
-                                        const uint2* __restrict__ pix, const uint32_t* label,
-                                        const uint32_t* resolved, uint32_t& out, uint32_t& wait_o) {
-    if (q == h) { out = lab_h; return true; }
-    const uint2 oi = pix[q];  // (owner, initial label) in one load
-    const uint32_t o = oi.x;
-    if (o == NO_OWNER || o > g) { out = oi.y; return true; }
-    if (load_acquire(resolved + o) == 0u) { wait_o = o; return false; }
-    out = ((volatile const uint32_t*)label)[q];
-    return true;
+// the label of pixel q (not g's own) as item g reads it: the initial label if
+// q has no owner or a higher-index one, else the owner's final label; false
+// when that owner has not resolved
+__device__ __forceinline__ bool settle_read(uint32_t q, uint32_t g, const FlankRec* rec, uint32_t& out) {
+    const FlankRec r = load_rec(rec + q);
+    const uint32_t o = (uint32_t)r.init;
+    const bool first = o == NO_OWNER || o > g;
+    out = first ? (uint32_t)(r.init >> 32) : (uint32_t)r.final;
+    return first || (r.final >> 32) != 0ull;
 }
 
 // A stored path read pair by pair: a contiguous range (pairs[k], k <
@@ -1256,53 +1288,49 @@ struct LinkedPath {
 template <class P>
 struct SettleLane {
     P path;
-    uint32_t g, h, at, lab_h, wait_o, waited;
+    uint32_t g, h, at, lab_h, wait_q, waited;
     bool alive, waiting;
 };
 
-// Scan item state `w` on from its place in its path; 0: resolved (label
-// written), 2: blocked (w.path, w.at, w.lab_h at the place to resume,
-// w.wait_o set).
+// the item's label after its walk, which ended at pixel `at` reading v there
+// (lab itself at its own pixel): the segment's label, then the flank bit
+__device__ __forceinline__ uint32_t settle_end(uint32_t lab, uint32_t v, bool own, uint32_t at, uint32_t side,
+                                               const slm_params& p, const uint32_t* __restrict__ mapping) {
+    const uint32_t lfa = p.left_flank_addition;
+    if (own) v = lab;
+    else if ((lab & ~lfa) != (v & ~lfa)) lab = v;
+    if (side) {
+        if (((~v) & lfa) && !(mapping[at] & p.is_thinchannel)) lab &= ~lfa;
+    } else {
+        if (v & lfa) lab |= lfa;
+    }
+    return lab;
+}
+
+// Scan item state `w` on from its place in its path; true: resolved and
+// published, false: blocked (w.path, w.at, w.lab_h at the place to resume,
+// w.wait_q the pixel whose owner it waits for).
 template <class P>
-__device__ int settle_scan(SettleLane<P>& w, uint32_t side, const slm_params& p,
-                           const uint8_t* __restrict__ stop, const uint32_t* __restrict__ mapping,
-                           const uint2* __restrict__ pix, uint32_t* label, uint32_t* resolved) {
-    const uint32_t lfa = p.left_flank_addition, thin = p.is_thinchannel;
-    uint32_t v = 0;
+__device__ __noinline__ bool settle_scan(SettleLane<P>& w, uint32_t side, const slm_params& p,
+                            const uint32_t* __restrict__ mapping, FlankRec* rec, uint32_t* label) {
+    const uint32_t lfa = p.left_flank_addition;
     // one pair of the walk's label scan: 0 go on, 1 the walk stops, 2 wait
-    // (stop[q]: mask or thin channel at q; when the compute pixel is the
-    // current one its label is the one just read)
-    // The stop byte and both pixels' (owner, initial label) words are loaded
-    // together; each label is then settled as settle_read does.
+    // (a stored path's compute pixels are unmasked and off the thin channel)
     auto scan = [&](uint2 e) -> int {
         const uint32_t a = w.at, c = e.x;
-        const bool own_a = a == w.h, own_c = c == w.h, same = c == a;
-        const uint8_t st_a = stop[a];
-        const uint2 oa = own_a ? make_uint2(NO_OWNER, 0u) : pix[a];
-        const uint2 oc = (own_c || same) ? make_uint2(NO_OWNER, 0u) : pix[c];
-        if (st_a) return 1;
-        if (own_a) {
-            v = w.lab_h;
-        } else if (oa.x == NO_OWNER || oa.x > w.g) {
-            v = oa.y;
-        } else if (load_acquire(resolved + oa.x) == 0u) {
-            w.wait_o = oa.x;
+        uint32_t v = w.lab_h;
+        if (a != w.h && !settle_read(a, w.g, rec, v)) {
+            w.wait_q = a;
             return 2;
-        } else {
-            v = ((volatile const uint32_t*)label)[a];
         }
         const bool flank_ok = side ? (v & lfa) != 0u : ((~v) & lfa) != 0u;
         if (!flank_ok) return 1;
-        if (!same) {
-            if (own_c) {
+        if (c != a) {
+            if (c == w.h) {
                 v = w.lab_h;
-            } else if (oc.x == NO_OWNER || oc.x > w.g) {
-                v = oc.y;
-            } else if (load_acquire(resolved + oc.x) == 0u) {
-                w.wait_o = oc.x;
+            } else if (!settle_read(c, w.g, rec, v)) {
+                w.wait_q = c;
                 return 2;
-            } else {
-                v = ((volatile const uint32_t*)label)[c];
             }
         }
         if ((w.lab_h & ~lfa) != (v & ~lfa)) w.lab_h = v;
@@ -1313,7 +1341,7 @@ __device__ int settle_scan(SettleLane<P>& w, uint32_t side, const slm_params& p,
         const uint2 e = w.path.get();
         if ((e.x & FLANK_PERIOD) == 0u) {
             const int st = scan(e);
-            if (st == 2) return 2;
+            if (st == 2) return false;
             if (st == 1) { w.path.end(); break; }
             w.path.next();
             continue;
@@ -1354,31 +1382,110 @@ __device__ int settle_scan(SettleLane<P>& w, uint32_t side, const slm_params& p,
         if (st == 2) {
             w.at = at0;
             w.lab_h = lab0;
-            return 2;
+            return false;
         }
         if (st == 1) { w.path.end(); break; }
         w.path = pat;
         for (uint32_t i = 0; i < E; ++i) w.path.next();
     }
-    // after the walk: the label at the last pixel, then the flank bit
-    if (!settle_read(w.at, w.g, w.h, w.lab_h, pix, label, resolved, v, w.wait_o)) return 2;
-    if ((w.lab_h & ~lfa) != (v & ~lfa)) w.lab_h = v;
-    settle_read(w.at, w.g, w.h, w.lab_h, pix, label, resolved, v, w.wait_o);
-    if (side) {
-        if (((~v) & lfa) && !(mapping[w.at] & thin)) w.lab_h &= ~lfa;
-    } else {
-        if (v & lfa) w.lab_h |= lfa;
+    uint32_t v = 0;
+    const bool own = w.at == w.h;
+    if (!own && !settle_read(w.at, w.g, rec, v)) {
+        w.wait_q = w.at;
+        return false;
     }
-    label[w.h] = w.lab_h;
-    store_release(resolved + w.g, 1u);
+    publish(rec, label, w.g, w.h, settle_end(w.lab_h, v, own, w.at, side, p, mapping));
+    return true;
+}
+
+// A path scanned from its end: `left` pairs are unscanned, the last of them
+// (cur) at pool[blk][off]; the scanned ones apply `kind` / `val` to the label
+// and end the walk at pixel `at`, whose label is v_end (at == h: the item's).
+struct BackLane {
+    uint32_t blk, off;
+    u64 left;
+    uint2 cur;
+    uint32_t kind, val;  // 0 identity, 1 val unless of val's segment, 2 val
+    uint32_t at, v_end;
+    uint32_t seen_q, seen_v;  // the label read last
+    bool ended;               // v_end is known
+};
+
+// One step of such a scan: the label at the walk's end, then pair by pair.
+// 0: go on, 1: resolved and published, 2: blocked on pixel w.wait_q.
+template <class W>
+__device__ __forceinline__ int settle_back(W& w, BackLane& b, uint32_t side, const slm_params& p,
+                                           const uint32_t* __restrict__ mapping, const uint2* __restrict__ pool,
+                                           FlankRec* rec, uint32_t* label) {
+    const uint32_t lfa = p.left_flank_addition;
+    if (!b.ended) {
+        if (b.at != w.h && !settle_read(b.at, w.g, rec, b.v_end)) {
+            w.wait_q = b.at;
+            return 2;
+        }
+        b.seen_q = b.at;
+        b.seen_v = b.v_end;
+        b.ended = true;
+    }
+    if (b.left == 0) {
+        uint32_t lab = w.lab_h;
+        if (b.kind == 2u || (b.kind == 1u && ((lab ^ b.val) & ~lfa) != 0u)) lab = b.val;
+        publish(rec, label, w.g, w.h, settle_end(lab, b.v_end, b.at == w.h, b.at, side, p, mapping));
+        return 1;
+    }
+    // the pixel the pair starts from: where the pair before it moved to
+    uint2 before = make_uint2(0u, w.h);
+    uint32_t blk = b.blk, off = b.off;
+    if (b.left > 1) {
+        if (off == 0) {
+            blk = __ldg(&pool[(u64)blk * FLANK_BLOCK + (FLANK_BLOCK - 1)].y);
+            off = FLANK_BLOCK - 1;
+        }
+        --off;
+        before = __ldg(&pool[(u64)blk * FLANK_BLOCK + off]);
+    }
+    const uint32_t a = before.y, c = b.cur.x;
+    uint32_t va = w.lab_h, vc;  // (at its own pixel before it first leaves it: the initial label)
+    if (a != w.h && !settle_read(a, w.g, rec, va)) {
+        w.wait_q = a;
+        return 2;
+    }
+    const bool flank_ok = side ? (va & lfa) != 0u : ((~va) & lfa) != 0u;
+    if (!flank_ok) {
+        b.kind = 0u;
+        b.at = a;
+        b.v_end = va;
+    } else if (c != w.h) {
+        if (c == a) {
+            vc = va;
+        } else if (c == b.seen_q) {
+            vc = b.seen_v;
+        } else if (!settle_read(c, w.g, rec, vc)) {
+            w.wait_q = c;
+            return 2;
+        }
+        if (b.kind == 0u) {
+            b.kind = 1u;
+            b.val = vc;
+        } else if (b.kind == 1u) {
+            if (((b.val ^ vc) & ~lfa) == 0u) b.val = vc;
+            else b.kind = 2u;
+        }
+    }
+    b.seen_q = a;
+    b.seen_v = va;
+    b.cur = before;
+    b.blk = blk;
+    b.off = off;
+    --b.left;
     return 0;
 }
 
-// pix[q] = (owner[q], label_init[q]), read together by the settle scan
-__global__ void k_flank_pix(uint32_t nxy, const uint32_t* __restrict__ owner,
-                            const uint32_t* __restrict__ label_init, uint2* __restrict__ pix) {
+// the records before the settle
+__global__ void k_flank_rec(uint32_t nxy, const uint32_t* __restrict__ owner,
+                            const uint32_t* __restrict__ label_init, FlankRec* __restrict__ rec) {
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nxy; q += gridDim.x * blockDim.x)
-        pix[q] = make_uint2(owner[q], label_init[q]);
+        rec[q] = FlankRec{(u64)owner[q] | ((u64)label_init[q] << 32), 0ull};
 }
 
 // stop[q] = 1 where a flank walk's loop test ends regardless of labels
@@ -1388,25 +1495,27 @@ __global__ void k_flank_stop(uint32_t nxy, const uint8_t* __restrict__ mask, con
         stop[q] = (mask[q] || (mapping[q] & thin)) ? 1 : 0;
 }
 
-// Items g0 .. g0+n-1: with LinkedPath, item g's path starts at block
-// heads[g] and holds n_pairs[g] pairs in `store`; with ContigPath it is
-// store[offsets[g] - base .. offsets[g + 1] - base).
+// Items g0 .. g0+n-1: with LinkedPath, item g's path is names[g] with
+// n_pairs[g] pairs in `store`; with ContigPath it is
+// store[offsets[g] - base .. offsets[g + 1] - base), scanned from its start.
 template <class P>
 __global__ void __launch_bounds__(256)
-k_flank_settle(const slm_params p, uint32_t g0, uint32_t n, uint32_t side, const u64* __restrict__ offsets,
-               u64 base, const uint32_t* __restrict__ heads, const u64* __restrict__ n_pairs,
-               const uint2* __restrict__ store, const uint32_t* __restrict__ hpix,
-               const uint8_t* __restrict__ stop, const uint32_t* __restrict__ mapping,
-               const uint2* __restrict__ pix, uint32_t* label, uint32_t* resolved, uint32_t* queue_head,
+k_flank_settle(const __grid_constant__ slm_params p, uint32_t g0, uint32_t n, uint32_t side,
+               const u64* __restrict__ offsets, u64 base, const uint32_t* __restrict__ names,
+               const u64* __restrict__ n_pairs, const uint2* __restrict__ store, const uint32_t* __restrict__ hpix,
+               const uint32_t* __restrict__ mapping, FlankRec* rec, uint32_t* label, uint32_t* queue_head,
                uint32_t* status) {
+    constexpr bool LINKED = std::is_same<P, LinkedPath>::value;
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     SettleLane<P> w;
+    BackLane b;
+    bool back = false;
     w.alive = false;
     bool drained = false;
     for (uint32_t pass = 0;; ++pass) {
         // a lane that gave up stops every warp (the caller falls back)
-        if ((pass & 63u) == 0u) {
+        if ((pass & 255u) == 0u) {
             uint32_t stop_all = 0;
             if (lane == 0) stop_all = *(volatile const uint32_t*)status;
             if (__shfl_sync(FULL, stop_all, 0)) break;
@@ -1423,22 +1532,42 @@ k_flank_settle(const slm_params p, uint32_t g0, uint32_t n, uint32_t side, const
                     const uint32_t t = head + __popc(idle & ((1u << lane) - 1u));
                     if (t < n) {
                         w.g = g0 + t;
-                        if constexpr (std::is_same<P, LinkedPath>::value) {
-                            w.path.pool = store;
-                            w.path.blk = heads[w.g];
-                            w.path.off = 0;
-                            w.path.left = n_pairs[w.g];
+                        w.h = hpix[w.g];
+                        w.at = w.h;
+                        w.lab_h = (uint32_t)(rec[w.h].init >> 32);
+                        w.waited = 0;
+                        w.waiting = false;
+                        w.alive = true;
+                        if constexpr (LINKED) {
+                            const uint32_t name = names[w.g];
+                            const u64 k = n_pairs[w.g];
+                            back = name == NO_BLOCK || (name & FLANK_FORWARD) == 0u;
+                            if (back) {
+                                b.left = k;
+                                b.kind = 0u;
+                                b.at = w.h;
+                                b.v_end = w.lab_h;
+                                b.ended = false;
+                                if (k) {
+                                    b.blk = name;
+                                    b.off = (uint32_t)((k - 1) % (FLANK_BLOCK - 1));
+                                    b.cur = __ldg(&store[(u64)b.blk * FLANK_BLOCK + b.off]);
+                                    b.at = b.cur.y;
+                                }
+                            } else {
+                                uint32_t blk = name & ~FLANK_FORWARD;
+                                for (u64 j = (k - 1) / (FLANK_BLOCK - 1); j > 0; --j)
+                                    blk = __ldg(&store[(u64)blk * FLANK_BLOCK + (FLANK_BLOCK - 1)].y);
+                                w.path.pool = store;
+                                w.path.blk = blk;
+                                w.path.off = 0;
+                                w.path.left = k;
+                            }
                         } else {
                             w.path.pairs = store;
                             w.path.k = offsets[w.g] - base;
                             w.path.k_end = offsets[w.g + 1] - base;
                         }
-                        w.h = hpix[w.g];
-                        w.at = w.h;
-                        w.lab_h = pix[w.h].y;
-                        w.waited = 0;
-                        w.waiting = false;
-                        w.alive = true;
                     }
                 }
             }
@@ -1449,30 +1578,35 @@ k_flank_settle(const slm_params p, uint32_t g0, uint32_t n, uint32_t side, const
         }
         bool idle_pass = true;  // this lane did nothing but wait this pass
         if (w.alive) {
+            int st;
             bool go = true;
-            if (w.waiting) {
-                if (load_acquire(resolved + w.wait_o) == 0u) {
-                    go = false;
-                    if (++w.waited >= FLANK_WAIT_LIMIT) {
-                        atomicOr(status, 1u);
-                        w.alive = false;
-                    }
-                } else {
-                    w.waiting = false;
-                    w.waited = 0;
+            if (LINKED && back) {
+                st = settle_back(w, b, side, p, mapping, store, rec, label);
+            } else {
+                // a forward scan is resumed once the owner it waits for is resolved
+                if (w.waiting) go = (load_rec(rec + w.wait_q).final >> 32) != 0ull;
+                st = 2;
+                if (go) {
+                    SettleLane<P> t = w;  // (its address is taken; w stays in registers)
+                    st = settle_scan(t, side, p, mapping, rec, label) ? 1 : 2;
+                    w = t;
                 }
+                w.waiting = st == 2;
             }
-            if (go) {
-                idle_pass = false;
-                if (settle_scan(w, side, p, stop, mapping, pix, label, resolved) == 2)
-                    w.waiting = true;
-                else
+            if (st == 2) {
+                if (++w.waited >= FLANK_WAIT_LIMIT) {
+                    atomicOr(status, 1u);
                     w.alive = false;
+                }
+            } else {
+                w.waited = 0;
+                idle_pass = false;
+                if (st == 1) w.alive = false;
             }
         }
         // a warp whose every lane only waited backs off, leaving the issue
         // slots to warps that scan
-        if (__all_sync(FULL, idle_pass)) __nanosleep(256);
+        if (__all_sync(FULL, idle_pass)) __nanosleep(64);
     }
 }
 
@@ -2046,7 +2180,7 @@ size_t slm_fix_flanks_workspace(uint32_t n_seeds, uint32_t nxy_padded, uint64_t 
     return (size_t)(2 * (size_t)n_seeds + 1) * sizeof(u64) + (size_t)n_seeds * 3 * sizeof(uint32_t)
          + (size_t)nxy_padded * 2 * sizeof(uint32_t) + 8 * sizeof(uint32_t) + 256
          + scan_scratch_words(n_seeds) * sizeof(u64) + ((size_t)nxy_padded + 16)
-         + ((size_t)nxy_padded * sizeof(uint2) + 16) + (size_t)n_pairs * sizeof(uint2);
+         + ((size_t)nxy_padded * sizeof(FlankRec) + 16) + (size_t)n_pairs * sizeof(uint2);
 }
 
 // restore the labels and flags before the rounds start over
@@ -2071,8 +2205,8 @@ static int fix_flanks(const slm_params* p, uint32_t n, const float* seed_point, 
     u64* offsets = n_pairs + n;
     uint32_t* hpix = reinterpret_cast<uint32_t*>(offsets + n + 1);
     uint32_t* resolved = hpix + n;
-    uint32_t* heads = resolved + n;
-    uint32_t* owner = heads + n;
+    uint32_t* names = resolved + n;
+    uint32_t* owner = names + n;
     uint32_t* label_init = owner + nxy;
     // [0] rounds: resolved count; [1] queue head; [2] status; [3] pool blocks
     // taken; [4] pool ran out
@@ -2083,8 +2217,8 @@ static int fix_flanks(const slm_params* p, uint32_t n, const float* seed_point, 
     uint8_t* stop = reinterpret_cast<uint8_t*>(scan_scratch + scan_scratch_words(n));
     pa = reinterpret_cast<uintptr_t>(stop + nxy);
     pa = (pa + 15) & ~(uintptr_t)15;
-    uint2* pix = reinterpret_cast<uint2*>(pa);
-    uint2* pairs = pix + nxy;  // the path store
+    FlankRec* rec = reinterpret_cast<FlankRec*>(pa);
+    uint2* pairs = reinterpret_cast<uint2*>(rec + nxy);  // the path store
     const u64 cap_pairs = (workspace_bytes - fixed) / sizeof(uint2);
     SLM_CUDA(cudaMemsetAsync(owner, 0xff, (size_t)nxy * sizeof(uint32_t), SS));
     SLM_CUDA(cudaMemsetAsync(resolved, 0, (size_t)n * sizeof(uint32_t), SS));
@@ -2094,8 +2228,8 @@ static int fix_flanks(const slm_params* p, uint32_t n, const float* seed_point, 
     SLM_LAUNCHED("k_owner_map");
     k_flank_stop<<<(unsigned)(num_sms() * 8), 256, 0, SS>>>(nxy, mask, mapping, p->is_thinchannel, stop);
     SLM_LAUNCHED("k_flank_stop");
-    k_flank_pix<<<(unsigned)(num_sms() * 8), 256, 0, SS>>>(nxy, owner, label_init, pix);
-    SLM_LAUNCHED("k_flank_pix");
+    k_flank_rec<<<(unsigned)(num_sms() * 8), 256, 0, SS>>>(nxy, owner, label_init, rec);
+    SLM_LAUNCHED("k_flank_rec");
     if (required_bytes) *required_bytes = fixed;
 
     // 1. Every walk traced once into linked blocks, then settled in one
@@ -2113,8 +2247,8 @@ static int fix_flanks(const slm_params* p, uint32_t n, const float* seed_point, 
         settle_grid = (unsigned)(num_sms() * (occ > 0 ? occ : 1));
         const u64 cap_blocks = cap_pairs / FLANK_BLOCK;
         k_flank_paths_linked<<<blocks_for(n, 128), 128, 0, SS>>>(
-            *p, make_walk_grid(*p), n, F2(seed_point), stop, F2(uv), n_pairs, heads, pairs,
-            (uint32_t)(cap_blocks < 0xfffffffeull ? cap_blocks : 0xfffffffeull), words + 3);
+            *p, make_walk_grid(*p), n, F2(seed_point), stop, F2(uv), n_pairs, names, pairs,
+            (uint32_t)(cap_blocks < FLANK_FORWARD - 1u ? cap_blocks : FLANK_FORWARD - 1u), words + 3);
         SLM_LAUNCHED("k_flank_paths_linked");
         counted = true;
         uint32_t ran_out = 0;
@@ -2122,8 +2256,8 @@ static int fix_flanks(const slm_params* p, uint32_t n, const float* seed_point, 
         SLM_CUDA(cudaStreamSynchronize(SS));
         if (!ran_out) {
             k_flank_settle<LinkedPath><<<settle_grid, 256, 0, SS>>>(
-                *p, 0u, n, side, nullptr, 0ull, heads, n_pairs, pairs, hpix, stop, mapping, pix, label, resolved,
-                words + 1, words + 2);
+                *p, 0u, n, side, nullptr, 0ull, names, n_pairs, pairs, hpix, mapping, rec, label, words + 1,
+                words + 2);
             SLM_LAUNCHED("k_flank_settle");
             uint32_t st = 0;
             SLM_CUDA(cudaMemcpyAsync(&st, words + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost, SS));
@@ -2187,8 +2321,8 @@ static int fix_flanks(const slm_params* p, uint32_t n, const float* seed_point, 
             SLM_LAUNCHED("k_flank_paths");
             SLM_CUDA(cudaMemsetAsync(words + 1, 0, sizeof(uint32_t), SS));
             k_flank_settle<ContigPath><<<grid, 256, 0, SS>>>(*p, a, m, side, offsets, base, nullptr, nullptr,
-                                                             pairs, hpix, stop, mapping, pix, label, resolved,
-                                                             words + 1, words + 2);
+                                                             pairs, hpix, mapping, rec, label, words + 1,
+                                                             words + 2);
             SLM_LAUNCHED("k_flank_settle");
         }
         uint32_t st = 0;
