@@ -993,12 +993,16 @@ __device__ u64 flank_walk(const slm_params& p, const WalkGrid& wg, uint32_t g, c
     uint2 last = make_uint2(NO_OWNER, NO_OWNER);
     // Whether the walk has computed off its own pixel: a pair that starts from
     // that pixel afterwards reads the item's running label, so such a path is
-    // settled from its start, as are paths with a period record.
+    // settled from its start.
     bool left_home = false;
     // As in count_downchannels: once (vec, dt) repeats bit for bit the
-    // per-step pairs repeat with the period, so the rest of the walk is
-    // stored as one period record {0x80000000|E, n} + the E pairs of a lap
-    // (after every step `last` is that step's pair, so each lap merges alike).
+    // per-step pairs repeat with the period (after every step `last` is that
+    // step's pair, so each lap merges alike).  Unless a lap passes through the
+    // item's own pixel, every lap reads the same labels: it stops the scan where
+    // the first lap does, and two laps in a row leave the label one lap leaves.
+    // So one lap and the last, partial one are stored in place of all of them.
+    // With the own pixel in it the lap is stored as a period record
+    // {0x80000000|E, n} + the E pairs of a lap.
     Vec2 tv = vec;
     float tdt = dt;
     uint32_t power = 1, lam = 0;
@@ -1019,22 +1023,35 @@ __device__ u64 flank_walk(const slm_params& p, const WalkGrid& wg, uint32_t g, c
             && __float_as_uint(dt) == __float_as_uint(tdt) && n_steps < p.max_n_steps) {
             const uint32_t L = lam, R = p.max_n_steps - n_steps, Rm = R % L;
             uint32_t E = 0, partial = 0;
-            for (int pass = 0; pass < 2; ++pass) {
+            bool own = last.y == h, record = false;
+            // pass 0 counts a lap's pairs, pass 1 stores them, pass 2 the
+            // partial lap's
+            for (int pass = 0; pass < 3; ++pass) {
                 Vec2 v2 = vec;
                 float d2 = dt;
-                uint32_t i2 = idx, ns2 = 0;
+                uint32_t i2 = idx, ns2 = 0, steps = L;
                 uint2 l2 = last;
                 if (pass == 1) {
                     const uint32_t nfut = (R / L) * E + partial;
                     if (nfut == 0) break;
-                    sink.settle_forward();
-                    sink.put(make_uint2(FLANK_PERIOD | E, nfut));
+                    record = own;
+                    if (record) {
+                        sink.settle_forward();
+                        sink.put(make_uint2(FLANK_PERIOD | E, nfut));
+                    } else if (R < L) {
+                        continue;
+                    }
                 }
-                for (uint32_t t2 = 1; t2 <= L; ++t2) {
+                if (pass == 2) {
+                    if (record) break;
+                    steps = Rm;
+                }
+                for (uint32_t t2 = 1; t2 <= steps; ++t2) {
                     const Step s2 = rk_plain(v2, d2, uv, p, wg);
                     const uint32_t q2 = s2.idx;
                     i2 = q2;
                     seg_move(s2, v2, i2, d2, ns2, p, wg);
+                    own = own || i2 == h;
                     if (q2 != l2.x || i2 != l2.y) {
                         l2 = make_uint2(q2, i2);
                         if (pass == 0) {
@@ -1206,10 +1223,9 @@ __global__ void k_flank_round(const slm_params p, uint32_t g0, uint32_t n, uint3
 //   identity;   lab -> v unless lab has v's segment;   lab -> v,
 // closed under putting one more step before it.  A pair at which the walk
 // stops (its label is on the other flank) drops everything after it.
-// Two kinds of path do not allow this and are scanned from their start, up to
-// a read of an unresolved owner at a time: those with a period record (walks
-// that circle until the step bound), and those that come back to the item's
-// own pixel, whose running label decides there.
+// Paths that come back to the item's own pixel, whose running label decides
+// there, do not allow this and are scanned from their start, up to a read of
+// an unresolved owner at a time.
 //
 // The lowest unresolved item taken waits on nothing unresolved, so some lane
 // always advances.  Each pixel has a 16-byte record, (owner, initial label)
