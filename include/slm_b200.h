@@ -553,10 +553,9 @@ int slm_create_seeds(const uint8_t* mask, uint32_t nx_padded, uint32_t ny_padded
  * rows in the same order, and the same generator state), built in DEVICE
  * memory: argwhere by the order-preserving compaction of slm_pick_seeds; the
  * swap partners drawn on the host with the same generator, by a thread of
- * its own; the Fisher-Yates swaps applied on the device in reservation
- * rounds (a swap runs once it is the earliest pending swap on both of its
- * rows), chunk by chunk (4 M swaps, in sequential order) as their partners
- * are drawn, which replaces the host's random-access pass over the rows.  Replaces create_seeds
+ * its own; the permutation the Fisher-Yates swaps compose to formed on the
+ * device, row by row, from the partners as they are drawn, which replaces the
+ * host's random-access pass over the rows.  Replaces create_seeds
  * (python/streamlines/useful.py:470-517) for callers that trace on the GPU.
  *   mask        DEVICE [nx_padded][ny_padded] uint8 (nonzero = masked)
  *   seed_point  DEVICE [capacity][2] float32, 8-byte aligned
@@ -564,8 +563,8 @@ int slm_create_seeds(const uint8_t* mask, uint32_t nx_padded, uint32_t ny_padded
  *   generator_state  host [625] or NULL, as slm_create_seeds
  *   workspace   DEVICE, 256-byte aligned, slm_create_seeds_device_workspace
  *               (nx_padded * ny_padded) bytes
- * Synchronises the stream (it reads back the row count and, per round, the
- * number of swaps still pending). */
+ * Synchronises the stream (it reads back the row count, and the partners'
+ * copies must have left host memory). */
 size_t slm_create_seeds_device_workspace(uint64_t n_pixels);
 int slm_create_seeds_device(const uint8_t* mask, uint32_t nx_padded, uint32_t ny_padded, uint32_t pad,
                             int do_shuffle, uint32_t rng_seed, float* seed_point, uint64_t capacity,
