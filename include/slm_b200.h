@@ -214,10 +214,11 @@ int slm_integrate_fields_noalloc(const slm_params* p, const slm_launch* launch,
 int slm_selftest_div6(uint64_t* counts, void* stream);
 
 /* slm_selftest_unit -- no counterpart in the reference: checks on the device,
- * over every finite float from 2^-60 up, that the square root the tracers' unit
- * vectors use equals the IEEE root and that its reciprocal is near enough for
- * both quotients to round as IEEE divisions.  counts: DEVICE [2] uint64:
- * failures, and the largest failing bit pattern + 1 (0: none).  Asynchronous. */
+ * over every finite float from 2^-100 up, that the square root behind the
+ * unit vectors equals the IEEE root and that the reciprocals of it and of the
+ * floats next to it are near enough for quotients by them to round as IEEE
+ * divisions.  counts: DEVICE [2] uint64: failures, and the largest failing
+ * bit pattern + 1 (0: none).  Asynchronous. */
 int slm_selftest_unit(uint64_t* counts, void* stream);
 
 /* slm_selftest_cvt_i8 -- no counterpart in the reference: checks on the

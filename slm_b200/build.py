@@ -20,7 +20,7 @@ OBJ = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libslm_b200.so")
 SOURCES = ["capi.cu", "trace.cu", "kde.cu", "map_kernels.cu", "scheduler.cu", "map_device.cu", "preprocess.cu",
            "seeds.cpp", "seeds_device.cu", "gemm_tc.cu", "fmm.cu"]
-HEADERS = ["trace_common.cuh", "trace_fast.cuh", "capi_util.cuh", "mt19937.hpp"]
+HEADERS = ["trace_common.cuh", "trace_fast.cuh", "unit_math.cuh", "capi_util.cuh", "mt19937.hpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC = os.environ.get("NVCC", "nvcc")
 

@@ -962,22 +962,24 @@ __global__ void k_selftest_cvt_i8(u64* counts) {
     }
 }
 
-// counts[0] += sums of squares s >= 2^-60 (and finite) for which the root or the
-// reciprocal of root_and_reciprocal could give a wrong quotient: the root is
-// not the IEEE square root, or with b = len 2^-k in [1, 2) and d = |y len - 1|
-//   d (b + 2^-23) >= 2^-23        (the residual correction could cross a midpoint)
-//   d > 2^-25 b (1 + 2^-18)       (the first quotient could be two ulps off)
-// counts[1] as for div6
+// counts[0] += floats s from 2^-100 up for which unit_math.cuh could give a wrong
+// root or quotient: the root is not the IEEE square root, or the reciprocal
+// of the root or of a float next to it (a length whose square is s but for its
+// low bits) breaks one of the two bounds there.  counts[1] as for div6
 __global__ void k_selftest_unit(u64* counts) {
     u64 bad = 0, last = 0;
-    const u64 lo = __float_as_uint(0x1p-100f), hi = 0x7f7fffffu;
-    for (u64 v = lo + (u64)blockIdx.x * blockDim.x + threadIdx.x; v <= hi; v += (u64)gridDim.x * blockDim.x) {
+    for (u64 v = (u64)ROOT_MIN_BITS + (u64)blockIdx.x * blockDim.x + threadIdx.x; v <= ROOT_MAX_BITS;
+         v += (u64)gridDim.x * blockDim.x) {
         const float s = __uint_as_float((uint32_t)v);
-        float len, y;
-        root_and_reciprocal(s, len, y);
-        const double b = (double)__uint_as_float((__float_as_uint(len) & 0x7fffffu) | 0x3f800000u);
-        const double d = fabs((double)y * (double)len - 1.0);
-        const bool ok = len == __fsqrt_rn(s) && d * (b + 0x1p-23) < 0x1p-23 && d <= 0x1p-25 * b * (1.0 + 0x1p-18);
+        const float y0 = rsqrt_estimate(s), root = root_from(s, y0);
+        bool ok = root == __fsqrt_rn(s);
+        for (int k = -1; k <= 1; ++k) {
+            const float len = __uint_as_float(__float_as_uint(root) + (uint32_t)k);
+            const float y = reciprocal_from(len, y0);
+            const double b = (double)__uint_as_float((__float_as_uint(len) & 0x7fffffu) | 0x3f800000u);
+            const double d = fabs((double)y * (double)len - 1.0);
+            ok = ok && d * (b + 0x1p-23) < 0x1p-23 && d <= 0x1p-25 * b * (1.0 + 0x1p-18);
+        }
         if (!ok) {
             bad++;
             last = v + 1;

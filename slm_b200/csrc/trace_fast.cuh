@@ -12,13 +12,8 @@
 //
 // What makes each shortcut exact:
 //
-//   unit vectors    u / |u| from one reciprocal square root estimate
-//                   (unit_fast): square root and quotients correctly rounded
-//                   by fused residuals (P. Markstein, "Computation of
-//                   elementary functions on the IBM RISC System/6000
-//                   processor", IBM J. Res. Dev. 34(1), 1990).  The root and
-//                   the reciprocal depend on the sum of squares alone, so
-//                   slm_selftest_unit checks every float of the guarded range.
+//   unit vectors    u / |u| from one reciprocal square root estimate, square
+//                   root and quotients correctly rounded (unit_math.cuh).
 //   pixel index     trunc(v) for 0 <= v < 2^23 is v + 2^23 rounded towards
 //                   zero; the sum's low bits are the integer, so neither
 //                   conversion unit nor clamp is used (the clamps cannot bind
@@ -45,6 +40,7 @@
 // warps (24, 36, 38, 40 against 32 per SM) 0 to 4 % slower.
 #pragma once
 #include "trace_common.cuh"
+#include "unit_math.cuh"
 
 namespace slm {
 
@@ -97,21 +93,6 @@ constexpr float FAST_S_MIN = 0x1p-60f;             // least square of a componen
 
 constexpr uint32_t LEHMER_M = 0xfffffffbu;
 
-// Square root of s and the reciprocal of that root, s >= 2^-60 and finite.
-// len is the IEEE square root and y the IEEE reciprocal of len, or off it
-// where that cannot change a quotient; slm_selftest_unit checks both over
-// the whole range.  The bias of 2^-44 (a 2^-21 part of an ulp) decides the
-// one tie the Newton step would round down, len = (2 - 2^-23) 2^k.
-__device__ __forceinline__ void root_and_reciprocal(float s, float& len, float& y) {
-    float y0;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(s));
-    // h = y0 / 2 by its exponent: the float units are the busier ones
-    const float g = __fmul_rn(s, y0), h = __uint_as_float(__float_as_uint(y0) - 0x800000u);
-    len = __fmaf_rn(__fmaf_rn(-g, g, s), h, g);
-    const float e = __fadd_rn(__fmaf_rn(-len, y0, 1.0f), 0x1p-44f);
-    y = __fmaf_rn(e, y0, y0);
-}
-
 // u / |u| as rk_step forms it: |u| = sqrt(x*x + y*y), both components divided
 // by it.  Exact, but for the sign of a zero component (which no later value
 // depends on), when s = x*x + y*y >= 2^-60 is finite and each component is
@@ -119,8 +100,8 @@ __device__ __forceinline__ void root_and_reciprocal(float s, float& len, float& 
 __device__ __forceinline__ F2 unit_fast(F2 u, float& xx, float& yy, float& s) {
     unpack2(mul2(u, u), xx, yy);
     s = __fadd_rn(xx, yy);
-    float len, r;
-    root_and_reciprocal(s, len, r);
+    const float y0 = rsqrt_estimate(s);
+    const float len = root_from(s, y0), r = reciprocal_from(len, y0);
     const F2 r2 = splat2(r), q = mul2(u, r2);
     return fma2(fma2(splat2(-len), q, u), r2, q);
 }
@@ -129,10 +110,7 @@ __device__ __forceinline__ F2 unit_fast(F2 u, float& xx, float& yy, float& s) {
 // squares is 0 or above 2^-40; the added 2^-100 is absorbed unless it is 0,
 // where it keeps the estimate finite and the root 0)
 __device__ __forceinline__ float quantised_length(float s) {
-    float y0;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(__fadd_rn(s, 0x1p-100f)));
-    const float g = __fmul_rn(s, y0), h = __fmul_rn(0.5f, y0);
-    return __fmaf_rn(__fmaf_rn(-g, g, s), h, g);
+    return root_from(s, rsqrt_estimate(__fadd_rn(s, 0x1p-100f)));
 }
 
 // A grid as the fast step uses it.  Part of the launch's parameters in the
@@ -386,17 +364,14 @@ __device__ __forceinline__ bool step_fast(Vec2 a0, F2 t0, uint32_t off0, float d
 // residuals takes the IEEE operations.
 __device__ __forceinline__ float next_dt_fast(float ex, float ey, float dt, float dt_max, float gs, float gs_rcp,
                                               float adjusted_max_error) {
-    const float qx = __fmul_rn(ex, gs_rcp), qy = __fmul_rn(ey, gs_rcp);
-    const float x = __fmaf_rn(-__fmaf_rn(gs, qx, -ex), gs_rcp, qx);
-    const float y = __fmaf_rn(-__fmaf_rn(gs, qy, -ey), gs_rcp, qy);
+    const float x = quotient_from(ex, gs, gs_rcp), y = quotient_from(ey, gs, gs_rcp);
     const float s = __fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y));
     const float n = __fmul_rn(adjusted_max_error, dt);
     float cand;
     if (s >= 0x1p-100f && n >= FAST_S_MIN) {
-        float err, r;
-        root_and_reciprocal(s, err, r);
-        const float q = __fmul_rn(n, r);
-        cand = __fmaf_rn(-__fmaf_rn(err, q, -n), r, q);
+        const float y0 = rsqrt_estimate(s);
+        const float err = root_from(s, y0);
+        cand = quotient_from(n, err, reciprocal_from(err, y0));
     } else {
         if (ex == 0.0f && ey == 0.0f) return dt_max;
         const float err = vlen(__fdiv_rn(ex, gs), __fdiv_rn(ey, gs));

@@ -152,3 +152,56 @@ def test_preprocess_full_size_properties():
     full = r1.uv_array[1000 + 2 + 2:1000 + 62 + 2, 2:-2].cpu().numpy()
     part = o["uv_array"][2 + 2:62 + 2, 2:-2]
     assert _same(full, part)
+
+
+# relief on either side of the float32 path's guards, strip and row-range
+# edges, thresholds that float32 does not hold
+EDGES = [
+    (dict(nx=28, ny=28, seed=21), dict()), (dict(nx=3, ny=29, seed=22), dict(pixel_size=3.0)),
+    (dict(nx=131, ny=57, seed=23), dict(scale=1e-25)), (dict(nx=40, ny=113, seed=24), dict(scale=1e20, pixel_size=1e-12)),
+    (dict(nx=61, ny=56, seed=25), dict(scale=1e-42)), (dict(nx=50, ny=60, seed=26), dict(pixel_size=1e12)),
+    (dict(nx=50, ny=60, seed=27, plateaus=True), dict(plane=True)), (dict(nx=66, ny=84, seed=28), dict(infs=True)),
+    (dict(nx=70, ny=70, seed=29, noise=0.6), dict(vecsum_threshold=1e-30)),
+    (dict(nx=70, ny=70, seed=30, noise=0.6), dict(vecsum_threshold=1e30, divergence_threshold=-0.1,
+                                                   curl_threshold=0.1)),
+    (dict(nx=300, ny=280, seed=31, noise=0.6, dtype=np.float64), dict(vecsum_threshold=0.5)),
+]
+
+
+@pytest.mark.parametrize("relief,how", EDGES)
+@pytest.mark.parametrize("normalize", [True, False])
+@pytest.mark.filterwarnings("ignore")
+def test_preprocess_at_the_edges_of_the_float_path(relief, how, normalize):
+    how = dict(how)
+    roi = _roi(**relief)
+    roi = (roi * roi.dtype.type(how.pop("scale", 1.0))).astype(roi.dtype)
+    if how.pop("plane", False):
+        roi[:, 20:40] = np.arange(roi.shape[0], dtype=roi.dtype)[:, None]  # one gradient component is 0
+        roi[10:30, 45:] = 7.0                                              # flat
+    if how.pop("infs", False):
+        roi[::17, ::13] = np.inf
+        roi[5::29, 3::11] = -np.inf
+    pixel_size = how.pop("pixel_size", 1.0)
+    o = D.conditioned_uv(roi, pixel_size, 2, do_normalize_speed=normalize, **how)
+    r = _gpu(roi, pixel_size, 2, normalize, **how)
+    for k in EXACT:
+        assert _same(getattr(r, k), o[k]), k
+    assert r.n_loops == o["n_loops"]
+
+
+def test_preprocess_without_the_optional_outputs():
+    import ctypes
+
+    import torch
+
+    from slm_b200 import _lib
+    from slm_b200._lib import SlmPreprocessParams
+    roi = torch.from_numpy(_roi(90, 75, 33)).cuda()
+    full = _gpu(roi, 1.0, 2, download=False)
+    uv = torch.zeros_like(full.uv_array)
+    prm = SlmPreprocessParams(1.0, 0.95, -0.5, 0.0, 2, 1)
+    _lib.check(_lib.load().slm_preprocess(_lib.ptr(roi), 0, 90, 75, ctypes.byref(prm), _lib.ptr(uv), None, None, None,
+                                          None, None, None, None, None, None,
+                                          ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    assert torch.equal(uv, full.uv_array)
