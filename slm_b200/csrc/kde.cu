@@ -14,6 +14,7 @@
 // partial pdf float [n_hist_bins^2], pdf float [n_pdf_points] or
 // [n_pdf_points^2].  The rows and cols passes take the kernel weights they
 // reuse from a per-block shared-memory table.
+#include <algorithm>
 #include <cmath>
 #include "capi_util.cuh"
 
@@ -32,17 +33,39 @@ __device__ __forceinline__ double k_sample(uint32_t kind, double x, double w) {
     }
 }
 
+constexpr uint32_t HIST_BLOCK = 512;
+
 // float -> uint as C's truncation through a 64-bit integer
 __device__ __forceinline__ uint32_t f2u(float v) { return (uint32_t)__float2ll_rz(v); }
 
-__global__ void k_histogram_univariate(const slm_params p, const float* __restrict__ data,
-                                       uint32_t n, uint32_t* __restrict__ hist) {
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= n) return;
-    const float bin_x = __fdiv_rn(data[g] - p.logx_min, p.logx_range);
-    uint32_t idx = f2u(bin_x * (float)p.n_hist_bins);
-    idx = idx < p.n_hist_bins - 1u ? idx : p.n_hist_bins - 1u;
-    atomicAdd(hist + idx, 1u);
+__device__ __forceinline__ uint32_t bin_univariate(float v, const slm_params& p) {
+    const float bin_x = __fdiv_rn(v - p.logx_min, p.logx_range);
+    const uint32_t idx = f2u(bin_x * (float)p.n_hist_bins);
+    return idx < p.n_hist_bins - 1u ? idx : p.n_hist_bins - 1u;
+}
+
+// A univariate histogram has few bins for its data (2048 for a grid's pixels),
+// so counting in memory is a queue of atomics at each popular bin.  With
+// LOCAL a block counts in shared memory and adds its bins at the end: 2 M
+// values in 2048 bins take 232 us without, 11 us with (B200).
+template <bool LOCAL>
+__global__ void __launch_bounds__(HIST_BLOCK)
+k_histogram_univariate(const slm_params p, const float* __restrict__ data, uint32_t n,
+                       uint32_t* __restrict__ hist) {
+    extern __shared__ uint32_t bins[];
+    if (LOCAL) {
+        for (uint32_t b = threadIdx.x; b < p.n_hist_bins; b += HIST_BLOCK) bins[b] = 0u;
+        __syncthreads();
+    }
+    uint32_t* count = LOCAL ? bins : hist;
+    const uint32_t stride = gridDim.x * HIST_BLOCK;
+    for (uint64_t g = (uint64_t)blockIdx.x * HIST_BLOCK + threadIdx.x; g < n; g += stride)
+        atomicAdd(count + bin_univariate(__ldg(data + g), p), 1u);
+    if (LOCAL) {
+        __syncthreads();
+        for (uint32_t b = threadIdx.x; b < p.n_hist_bins; b += HIST_BLOCK)
+            if (bins[b]) atomicAdd(hist + b, bins[b]);
+    }
 }
 
 __global__ void k_histogram_bivariate(const slm_params p, const float2* __restrict__ data,
@@ -60,32 +83,47 @@ __global__ void k_histogram_bivariate(const slm_params p, const float2* __restri
     atomicAdd(hist + (iy + nb * ix), 1u);
 }
 
-// one thread per pdf point (kde.cl:426-526)
-__global__ void k_pdf_univariate(const slm_params p, const uint32_t* __restrict__ hist,
-                                 float* __restrict__ pdf) {
-    const uint32_t pdf_idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pdf_idx >= p.n_pdf_points) return;
+// one thread per pdf point (kde.cl:426-526).  The weight of (k, h) is every
+// point's: the block forms PDF_TABLE of them at a time in shared memory (an
+// exponential and divisions each), in the order the points use them.
+constexpr uint32_t PDF_BLOCK = 32, PDF_TABLE = 1024;
+
+__global__ void __launch_bounds__(PDF_BLOCK)
+k_pdf_univariate(const slm_params p, const uint32_t* __restrict__ hist, float* __restrict__ pdf) {
+    __shared__ double table[PDF_TABLE];
+    const uint32_t pdf_idx = blockIdx.x * PDF_BLOCK + threadIdx.x;
     const uint32_t nbpp = p.n_hist_bins / p.n_pdf_points;
     const double half_dx = (double)__fdiv_rn(p.pdf_dx, 2.0f);
+    const uint64_t total = ((uint64_t)p.n_kdf_part_points_x + 1u) * nbpp;
     double acc = 0.0, kw = 0.0;
-    for (uint32_t k = 0; k <= p.n_kdf_part_points_x; ++k) {
-        const double edge = (double)k * (double)p.pdf_dx - half_dx;
-        const int32_t col_r = (int32_t)(pdf_idx + k);
-        const int32_t col_l = (int32_t)(pdf_idx - k + 1u);
-        const bool ok_r = col_r < (int32_t)p.n_pdf_points;
-        const bool ok_l = (k != 0u) && (col_l > 0);
-        for (uint32_t h = 0; h < nbpp; ++h) {
-            const double x = edge + (double)p.bin_dx * ((double)h + 0.5);
-            const double kv = k_sample(p.kdf_kind, x, (double)p.kdf_width_x);
-            const uint32_t hr = (uint32_t)col_r * nbpp + h;
-            const uint32_t hl = (uint32_t)col_l * nbpp - h - 1u;
-            if (ok_r) acc += (double)hist[hr] * kv;
-            if (ok_l) acc += (double)hist[hl] * kv;
-            if (ok_r) kw += kv;
-            if (ok_l) kw += kv;
+    uint32_t k = 0, h = 0;  // of the weight at hand
+    for (uint64_t t0 = 0; t0 < total; t0 += PDF_TABLE) {
+        const uint32_t m = (uint32_t)(total - t0 < PDF_TABLE ? total - t0 : PDF_TABLE);
+        __syncthreads();
+        for (uint32_t t = threadIdx.x; t < m; t += PDF_BLOCK) {
+            const uint32_t tk = (uint32_t)((t0 + t) / nbpp), th = (uint32_t)((t0 + t) % nbpp);
+            const double edge = (double)tk * (double)p.pdf_dx - half_dx;
+            table[t] = k_sample(p.kdf_kind, edge + (double)p.bin_dx * ((double)th + 0.5), (double)p.kdf_width_x);
+        }
+        __syncthreads();
+        if (pdf_idx >= p.n_pdf_points) continue;
+        for (uint32_t t = 0; t < m; ++t) {
+            const double kv = table[t];
+            const int32_t col_r = (int32_t)(pdf_idx + k);
+            const int32_t col_l = (int32_t)(pdf_idx - k + 1u);
+            if (col_r < (int32_t)p.n_pdf_points) {
+                acc += (double)__ldg(hist + ((uint32_t)col_r * nbpp + h)) * kv;
+            }
+            if (k != 0u && col_l > 0) acc += (double)__ldg(hist + ((uint32_t)col_l * nbpp - h - 1u)) * kv;
+            if (col_r < (int32_t)p.n_pdf_points) kw += kv;
+            if (k != 0u && col_l > 0) kw += kv;
+            if (++h == nbpp) {
+                h = 0;
+                ++k;
+            }
         }
     }
-    pdf[pdf_idx] = (float)((double)(float)acc / kw);
+    if (pdf_idx < p.n_pdf_points) pdf[pdf_idx] = (float)((double)(float)acc / kw);
 }
 
 // one thread per histogram bin; weights k_sample(k, n_y + 0.5), k = 0..n_y,
@@ -188,8 +226,19 @@ int slm_histogram_univariate(const slm_params* p, const float* sl, uint32_t n_da
     if (rc) return rc;
     if (n_data == 0) return SLM_OK;
     SLM_REQUIRE(sl && hist, "NULL buffer");
-    const unsigned block = 256, grid = (n_data + block - 1) / block;
-    k_histogram_univariate<<<grid, block, 0, (cudaStream_t)stream>>>(*p, sl, n_data, hist);
+    // Counted in shared memory where the bins fit and a block's values are at
+    // least four a bin (below that, adding the bins up costs more than the
+    // atomics it saves); as many blocks as that leaves, two an SM at most.
+    const uint32_t by_values = n_data / std::max(4u * p->n_hist_bins, 4096u);
+    const uint32_t wide = (uint32_t)num_sms() * 2u;
+    if (by_values >= 1 && p->n_hist_bins <= 12288u) {
+        const unsigned grid = std::min(by_values, wide);
+        k_histogram_univariate<true><<<grid, HIST_BLOCK, p->n_hist_bins * sizeof(uint32_t), (cudaStream_t)stream>>>(
+            *p, sl, n_data, hist);
+    } else {
+        const unsigned grid = std::min((n_data + HIST_BLOCK - 1) / HIST_BLOCK, wide * 8u);
+        k_histogram_univariate<false><<<grid, HIST_BLOCK, 0, (cudaStream_t)stream>>>(*p, sl, n_data, hist);
+    }
     SLM_LAUNCHED("k_histogram_univariate");
     return SLM_OK;
 }
@@ -213,8 +262,8 @@ int slm_pdf_univariate(const slm_params* p, const uint32_t* hist, float* pdf, vo
     int rc = check_kde(p, false);
     if (rc) return rc;
     SLM_REQUIRE(hist && pdf, "NULL buffer");
-    const unsigned block = 128, grid = (p->n_pdf_points + block - 1) / block;
-    k_pdf_univariate<<<grid, block, 0, (cudaStream_t)stream>>>(*p, hist, pdf);
+    const unsigned grid = (p->n_pdf_points + PDF_BLOCK - 1) / PDF_BLOCK;
+    k_pdf_univariate<<<grid, PDF_BLOCK, 0, (cudaStream_t)stream>>>(*p, hist, pdf);
     SLM_LAUNCHED("k_pdf_univariate");
     return SLM_OK;
 }

@@ -122,3 +122,24 @@ def test_channel_threshold_from_device_pdf():
     o.locate_threshold()
     assert o.mode_i == d.mode_i
     assert o.channel_threshold_i == d.channel_threshold_i
+
+
+@pytest.mark.parametrize("nb,npp,n", [(256, 128, 4095), (256, 128, 4096), (2048, 256, 8191), (2048, 256, 8193),
+                                      (12288, 128, 60001), (12289 + 127, 128, 60001), (64, 64, 1000003),
+                                      (4096, 33, 1)])
+def test_univariate_histogram_in_shared_memory_and_not(nb, npp, n):
+    """Sizes on either side of the rule for counting in shared memory; the pdf
+    with more, fewer and as many weights as its table holds."""
+    nb -= nb % npp
+    rng = np.random.default_rng(nb + n)
+    d, _ = univariate("gaussian", n_hist_bins=nb, n_pdf_points=npp, n=20000, bandwidth=6.0)
+    prm = kde.kde_params(d, "pdf_univariate")
+    data = rng.choice(np.ascontiguousarray(d.logx_data.reshape(-1), dtype=np.float32), n)
+    hist_d = torch.full((nb,), 3, dtype=torch.int32, device="cuda").view(torch.uint32)  # added to, not cleared
+    kernels.histogram_univariate(prm, torch.from_numpy(data).cuda(), hist_d)
+    pdf_d = torch.zeros(npp, dtype=torch.float32, device="cuda")
+    hist_o = O.histogram_univariate(prm, data)
+    kernels.pdf_univariate(prm, torch.from_numpy(hist_o).cuda(), pdf_d)
+    torch.cuda.synchronize()
+    assert np.array_equal(hist_d.cpu().numpy(), hist_o + 3)
+    _close(pdf_d.cpu().numpy(), O.pdf_univariate(prm, hist_o))
