@@ -287,6 +287,18 @@ int slm_pdf_bivariate_rows(const slm_params* p, const uint32_t* hist, float* par
 /* pdf_bivariate_cols (opencl/kde.cl:249-361): partial -> pdf [n_pdf_points^2] float */
 int slm_pdf_bivariate_cols(const slm_params* p, const float* partial, float* pdf, void* stream);
 
+/* slm_column_moments -- no counterpart in the reference (NumPy's std of the
+ * data, kde.py:71-82, 151-158): per column c of data [n_rows][cols] (cols 1 or
+ * 2), out[2c] = the sum of d and out[2c+1] = the sum of d^2, d = value - the
+ * column's first value, in double; the column's variance is
+ * (out[2c+1] - out[2c]^2 / n_rows) / n_rows.  The sums' order is fixed.
+ * workspace: slm_column_moments_workspace(cols) bytes, 8-byte aligned. */
+size_t slm_column_moments_workspace(uint32_t cols);
+int slm_column_moments(const float* data, uint64_t n_rows, uint32_t cols, double* out, void* workspace,
+                       size_t workspace_bytes, void* stream);
+/* slm_scale_counts: out[i] = (double)hist[i] / scale (kde.py:113-114) */
+int slm_scale_counts(const uint32_t* hist, uint64_t n, double scale, double* out, void* stream);
+
 /* ---- channel / segment / hillslope mapping ----
  * One entry point per reference mapping kernel, same buffers in the same
  * order after (params, n_seeds, seed_point).  Results equal the reference's

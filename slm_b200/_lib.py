@@ -73,6 +73,9 @@ SIGNATURES = {
     "slm_histogram_bivariate": (ctypes.c_int, [_P, _P, _U, _P, _P]),
     "slm_pdf_univariate": (ctypes.c_int, [_P, _P, _P, _P]),
     "slm_pdf_bivariate_rows": (ctypes.c_int, [_P, _P, _P, _P]),
+    "slm_column_moments_workspace": (ctypes.c_size_t, [_U]),
+    "slm_column_moments": (ctypes.c_int, [_P, ctypes.c_uint64, _U, _P, _P, ctypes.c_size_t, _P]),
+    "slm_scale_counts": (ctypes.c_int, [_P, ctypes.c_uint64, ctypes.c_double, _P, _P]),
     "slm_pdf_bivariate_cols": (ctypes.c_int, [_P, _P, _P, _P]),
     "slm_connect_channels": (ctypes.c_int, [_P, _U, _P, _P, _P, _P, _P, _P]),
     "slm_map_channel_heads": (ctypes.c_int, [_P, _U, _P, _P, _P, _P, _P]),

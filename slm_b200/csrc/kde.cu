@@ -200,6 +200,63 @@ __global__ void k_pdf_bivariate_cols(const slm_params p, const float* __restrict
     pdf[pdf_idx] = (float)(acc / kw);
 }
 
+// ------------------------------------------------------------------ spread of the data
+// Sums of d and d^2, d = value - the column's first value, per column of rows
+// of COLS floats, in double.  Each block sums a fixed range of rows, and one
+// block then adds the blocks' sums in order, so the result does not depend on
+// the order blocks run in.
+constexpr uint32_t MOMENT_BLOCK = 256;
+
+template <int COLS>
+__device__ __forceinline__ void block_sum(double (&v)[2 * COLS], double* out) {
+    __shared__ double part[MOMENT_BLOCK / 32][2 * COLS];
+#pragma unroll
+    for (int c = 0; c < 2 * COLS; ++c)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_xor_sync(0xffffffffu, v[c], o);
+    if ((threadIdx.x & 31u) == 0)
+        for (int c = 0; c < 2 * COLS; ++c) part[threadIdx.x >> 5][c] = v[c];
+    __syncthreads();
+    if (threadIdx.x < 2 * COLS) {
+        double s = 0.0;
+        for (uint32_t w = 0; w < MOMENT_BLOCK / 32; ++w) s += part[w][threadIdx.x];
+        out[threadIdx.x] = s;
+    }
+}
+
+template <int COLS>
+__global__ void __launch_bounds__(MOMENT_BLOCK)
+k_moments(const float* __restrict__ data, uint64_t n, uint64_t rows_per_block, double* __restrict__ partial) {
+    const uint64_t lo = (uint64_t)blockIdx.x * rows_per_block;
+    const uint64_t hi = lo + rows_per_block < n ? lo + rows_per_block : n;
+    double v[2 * COLS] = {}, first[COLS];
+    for (int c = 0; c < COLS; ++c) first[c] = (double)__ldg(data + c);
+    for (uint64_t i = lo + threadIdx.x; i < hi; i += MOMENT_BLOCK)
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) {
+            const double d = (double)__ldg(data + COLS * i + c) - first[c];
+            v[2 * c] += d;
+            v[2 * c + 1] += d * d;
+        }
+    block_sum<COLS>(v, partial + (uint64_t)blockIdx.x * 2 * COLS);
+}
+
+template <int COLS>
+__global__ void __launch_bounds__(MOMENT_BLOCK)
+k_moments_sum(const double* __restrict__ partial, uint32_t blocks, double* __restrict__ out) {
+    double v[2 * COLS] = {};
+    for (uint32_t b = threadIdx.x; b < blocks; b += MOMENT_BLOCK)
+#pragma unroll
+        for (int c = 0; c < 2 * COLS; ++c) v[c] += partial[(uint64_t)b * 2 * COLS + c];
+    block_sum<COLS>(v, out);
+}
+
+// out[i] = hist[i] / scale
+__global__ void k_scale_counts(const uint32_t* __restrict__ hist, uint64_t n, double scale, double* __restrict__ out) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = __ddiv_rn((double)hist[i], scale);
+}
+
 }  // namespace slm
 
 using namespace slm;
@@ -298,6 +355,44 @@ int slm_pdf_bivariate_cols(const slm_params* p, const float* partial, float* pdf
     const unsigned block = 128, grid = (unsigned)((n + block - 1) / block);
     k_pdf_bivariate_cols<<<grid, block, smem, (cudaStream_t)stream>>>(*p, partial, pdf);
     SLM_LAUNCHED("k_pdf_bivariate_cols");
+    return SLM_OK;
+}
+
+// the block count is fixed, so the sums' order is
+static constexpr uint32_t MOMENT_BLOCKS = 512;
+
+size_t slm_column_moments_workspace(uint32_t cols) { return (size_t)MOMENT_BLOCKS * 2 * cols * sizeof(double); }
+
+int slm_column_moments(const float* data, uint64_t n_rows, uint32_t cols, double* out, void* workspace,
+                       size_t workspace_bytes, void* stream) {
+    clear_error();
+    SLM_REQUIRE(data && out && workspace && n_rows > 0, "NULL buffer or no rows");
+    SLM_REQUIRE(cols == 1 || cols == 2, "cols must be 1 or 2");
+    SLM_REQUIRE(workspace_bytes >= slm_column_moments_workspace(cols), "workspace holds %zu bytes, needs %zu",
+                workspace_bytes, slm_column_moments_workspace(cols));
+    SLM_REQUIRE(aligned(out, 8) && aligned(workspace, 8) && aligned(data, 4), "misaligned buffer");
+    cudaStream_t s = (cudaStream_t)stream;
+    double* partial = static_cast<double*>(workspace);
+    const uint64_t rows = (n_rows + MOMENT_BLOCKS - 1) / MOMENT_BLOCKS;
+    const uint32_t blocks = (uint32_t)((n_rows + rows - 1) / rows);
+    if (cols == 1) {
+        k_moments<1><<<blocks, MOMENT_BLOCK, 0, s>>>(data, n_rows, rows, partial);
+        k_moments_sum<1><<<1, MOMENT_BLOCK, 0, s>>>(partial, blocks, out);
+    } else {
+        k_moments<2><<<blocks, MOMENT_BLOCK, 0, s>>>(data, n_rows, rows, partial);
+        k_moments_sum<2><<<1, MOMENT_BLOCK, 0, s>>>(partial, blocks, out);
+    }
+    SLM_LAUNCHED("k_moments");
+    return SLM_OK;
+}
+
+int slm_scale_counts(const uint32_t* hist, uint64_t n, double scale, double* out, void* stream) {
+    clear_error();
+    if (n == 0) return SLM_OK;
+    SLM_REQUIRE(hist && out && aligned(out, 8), "NULL or misaligned buffer");
+    SLM_REQUIRE(n < (1ull << 39), "too many counts");
+    k_scale_counts<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(hist, n, scale, out);
+    SLM_LAUNCHED("k_scale_counts");
     return SLM_OK;
 }
 

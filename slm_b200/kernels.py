@@ -154,3 +154,29 @@ def pdf_bivariate_cols(params, partial, pdf, stream=None):
     _need(partial, torch.float32, nb * nb, "partial pdf")
     _need(pdf, torch.float32, np_ * np_, "pdf")
     check(_lib.load().slm_pdf_bivariate_cols(sref(params), ptr(partial), ptr(pdf), _stream(stream)))
+
+
+def column_std(data, stream=None):
+    """The standard deviation of each column of a float32 tensor [n] or
+    [n][2], formed in double and rounded to float32 (NumPy scalars; waits for
+    the result)."""
+    import math
+
+    import numpy as np
+    lib = _lib.load()
+    _need(data, torch.float32, None, "data")
+    n, cols = int(data.shape[0]), int(data.shape[1]) if data.dim() == 2 else 1
+    ws = torch.empty(int(lib.slm_column_moments_workspace(cols)), dtype=torch.uint8, device=data.device)
+    out = torch.empty(2 * cols, dtype=torch.float64, device=data.device)
+    check(lib.slm_column_moments(ptr(data), n, cols, ptr(out), ptr(ws), ws.numel(), _stream(stream)))
+    m = out.tolist()
+    var = [(m[2 * c + 1] - m[2 * c] * m[2 * c] / n) / n for c in range(cols)]
+    return [np.float32(math.sqrt(v)) if v > 0.0 else np.float32(0.0 if v <= 0.0 else v) for v in var]
+
+
+def scale_counts(hist, scale, stream=None):
+    """``hist / scale`` (uint32 counts, a double) as a float64 tensor."""
+    _need(hist, torch.uint32, None, "histogram")
+    out = torch.empty(hist.shape, dtype=torch.float64, device=hist.device)
+    check(_lib.load().slm_scale_counts(ptr(hist), int(hist.numel()), float(scale), ptr(out), _stream(stream)))
+    return out

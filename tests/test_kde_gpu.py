@@ -143,3 +143,17 @@ def test_univariate_histogram_in_shared_memory_and_not(nb, npp, n):
     torch.cuda.synchronize()
     assert np.array_equal(hist_d.cpu().numpy(), hist_o + 3)
     _close(pdf_d.cpu().numpy(), O.pdf_univariate(prm, hist_o))
+
+
+@pytest.mark.parametrize("n", [1, 255, 512, 513, 131073, 1000003])
+@pytest.mark.parametrize("cols", [1, 2])
+def test_column_std_against_64_bits(n, cols):
+    """Formed in double from n values of |x| < 30 with spread >= 0.5 and rounded
+    once to float32: within 2^-24 of the 64-bit value, but for the double sums'
+    own error (n 2^-53 of them, below 2^-30)."""
+    rng = np.random.default_rng(n * 3 + cols)
+    x = (3.0 + rng.standard_normal((n, cols)) * np.array([0.8, 0.5])[:cols]).astype(np.float32)
+    got = kernels.column_std(torch.from_numpy(x if cols == 2 else x[:, 0].copy()).cuda())
+    want = x.astype(np.float64).std(axis=0)
+    for g, w in zip(got, want):
+        assert g.dtype == np.float32 and abs(float(g) - w) <= w * (2.0 ** -24 + 2.0 ** -30)
