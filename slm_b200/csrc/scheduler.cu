@@ -19,6 +19,7 @@
 // for the weight gradients); inference is one fused kernel per warp of 16
 // seeds (mma.sync m16n8k16 bf16 -> fp32).
 #include <algorithm>
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include "capi_util.cuh"
 
@@ -80,22 +81,48 @@ __global__ void k_relu_backward(const float* __restrict__ da, const float* __res
     if (i < n) dz[i] = z[i] > 0.0f ? da[i] : 0.0f;
 }
 
-// column sums of dZ [rows][cols] added into db[cols]
-__global__ void k_bias_grad(const float* __restrict__ dz, size_t rows, int cols, float* __restrict__ db) {
-    const int c = blockIdx.x;
+// Column sums of dZ [rows][cols] added into db[cols].  A cluster of BIAS_CTAS
+// blocks takes 32 columns (one a lane, so rows are read whole; with fewer
+// columns a warp reads 32 / width rows at once), each warp every
+// (BIAS_CTAS * 32)th of the rows; the warps' sums are added in order by the
+// first block, which reads the others' shared memory, so the result does not
+// depend on the order they run in.  65536 x 32: 57 us with a block a column,
+// 22 us now (B200), what the eight SMs read from L2.
+constexpr uint32_t BIAS_CTAS = 8, BIAS_THREADS = 1024;
+
+__global__ void __cluster_dims__(BIAS_CTAS, 1, 1) __launch_bounds__(BIAS_THREADS)
+k_bias_grad(const float* __restrict__ dz, size_t rows, int cols, uint32_t width, float* __restrict__ db) {
+    __shared__ float part[BIAS_THREADS / 32][32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t rank = blockIdx.x % BIAS_CTAS;
+    const int c = (int)((blockIdx.x / BIAS_CTAS) * 32u + lane % width);
+    const uint32_t per_warp = 32u / width;  // rows a warp reads at once
+    const size_t step = (size_t)BIAS_CTAS * (BIAS_THREADS / 32) * per_warp;
     float s = 0.0f;
-    for (size_t r = threadIdx.x; r < rows; r += blockDim.x) s += dz[r * cols + c];
+    if (c < cols) {
+        size_t r = ((size_t)rank * (BIAS_THREADS / 32) + warp) * per_warp + lane / width;
+        for (; r + 15 * step < rows; r += 16 * step) {  // sixteen loads in flight
+            float v[16];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    __shared__ float part[32];
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        float t = threadIdx.x < (blockDim.x >> 5) ? part[threadIdx.x] : 0.0f;
+            for (int j = 0; j < 16; ++j) v[j] = __ldg(dz + (r + j * step) * cols + c);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        if (threadIdx.x == 0) atomicAdd(db + c, t);
+            for (int j = 0; j < 16; ++j) s += v[j];
+        }
+        for (; r < rows; r += step) s += __ldg(dz + r * cols + c);
     }
+    for (uint32_t o = width; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    part[warp][lane] = s;
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    cluster.sync();
+    if (rank == 0 && warp == 0 && lane < width && c < cols) {
+        float t = 0.0f;
+        for (uint32_t b = 0; b < BIAS_CTAS; ++b) {
+            const float* p = cluster.map_shared_rank(&part[0][0], b);
+            for (uint32_t w = 0; w < BIAS_THREADS / 32; ++w) t += p[w * 32 + lane];
+        }
+        db[c] += t;
+    }
+    cluster.sync();  // the other blocks' shared memory stays until it is read
 }
 
 // dY = 2 W (Y - T) inv_n, loss += sum W (Y - T)^2 inv_n (W = 1 without weights)
@@ -694,7 +721,10 @@ int slm_relu_backward(const float* da, const float* z, uint64_t n, float* dz, vo
 int slm_bias_grad(const float* dz, uint64_t rows, int cols, float* db, void* stream) {
     clear_error();
     SLM_REQUIRE(cols > 0, "cols must be > 0");
-    k_bias_grad<<<cols, 256, 0, (cudaStream_t)stream>>>(dz, rows, cols, db);
+    uint32_t width = 1;  // lanes side by side on a row
+    while (width < 32u && width < (uint32_t)cols) width <<= 1;
+    const unsigned groups = (unsigned)((cols + 31) / 32);
+    k_bias_grad<<<groups * BIAS_CTAS, BIAS_THREADS, 0, (cudaStream_t)stream>>>(dz, rows, cols, width, db);
     SLM_LAUNCHED("k_bias_grad");
     return SLM_OK;
 }

@@ -373,3 +373,23 @@ def test_grid_predictions_equal_per_seed(nxp, nyp, pad, monkeypatch):
     mag = np.abs(c["x3"]) @ np.abs(c["W"]["w3"]) + np.abs(c["W"]["b3"])
     diff = (got.double() - ref.double()).abs().cpu().numpy()
     assert np.all(diff <= 2 * 256 * 2.0 ** -23 * mag)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 1), (7, 2), (255, 3), (256, 33), (4096, 2), (65536, 32), (65537, 31),
+                                       (130001, 64), (300, 200)])
+def test_bias_grad_column_sums(rows, cols):
+    """Column sums in fp32 of values in [-1, 1]: rows terms summed in at most
+    rows / 256 + 300 additions one after another (a warp's rows, then the
+    warps), each within 2^-24 of a partial sum of at most rows."""
+    import ctypes
+
+    from slm_b200 import _lib
+    g = torch.Generator().manual_seed(rows * 7 + cols)
+    dz = (torch.rand((rows, cols), generator=g) * 2 - 1).to(DEV)
+    db = torch.full((cols,), 0.5, device=DEV)
+    _lib.check(_lib.load().slm_bias_grad(_lib.ptr(dz), rows, cols, _lib.ptr(db),
+                                         ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    want = dz.double().sum(0) + 0.5
+    bound = (rows / 256 + 301) * 2.0 ** -24 * (dz.double().abs().sum(0) + 0.5)
+    assert torch.all((db.double() - want).abs() <= bound)
