@@ -46,14 +46,17 @@ __device__ __forceinline__ void add_if(bool on, u64* p, u64 v) {
                  : "r"((uint32_t)on), "l"(p), "l"(v));  // nothing here reads the sums
 }
 
-// writearray.cl:31-40: slt += (uint)(l+0.5), slc += 1, if `visits`
+// writearray.cl:31-40: slt += (uint)(l+0.5), slc += 1, if `visits`.  A lane on
+// a trajectory has a run open (its start opened or continued one), so the
+// visits of its steps need not ask.
+template <bool OPEN>
 __device__ __forceinline__ void acc_visit(Acc& a, uint32_t idx, float l, bool visits, u64* __restrict__ slc,
                                           u64* __restrict__ slt) {
     const uint32_t v = __float2uint_rz(l + 0.5f);
     // selects and predicated atomics, no branch: some lane of a warp changes
     // pixel in nearly every step
-    const bool same = (idx == a.idx) && a.cnt;
-    const bool flush = visits && !same && a.cnt;
+    const bool same = idx == a.idx && (OPEN || a.cnt);
+    const bool flush = visits && !same && (OPEN || a.cnt);
     add_if(flush, slt + a.idx, a.sum);
     add_if(flush, slc + a.idx, (u64)a.cnt);
     if (visits) {
@@ -67,8 +70,8 @@ __device__ __forceinline__ void acc_visit(Acc& a, uint32_t idx, float l, bool vi
 struct FieldLane {
     Vec2 a;
     float l, dt;
-    uint32_t n, rng;
-    uint32_t item, k;  // queue position and RK steps so far
+    uint32_t n, rng;   // RK steps so far (the one that ends on a masked pixel included)
+    uint32_t item;     // queue position
     bool alive;
     F2 t;              // 2^23 + pixel of a, and the byte offset of that
     uint32_t off;      // pixel's vector in uv (kept for the fast step)
@@ -103,14 +106,13 @@ __device__ __forceinline__ void field_init(FieldLane& s, float2 c, uint32_t rng_
     s.dt = G.g.dt_max;
     s.n = 0;
     s.item = item;
-    s.k = 0;
     const uint32_t idx = G.base + pixel_of(s.a, p, G.g);
     if (FAST) {
         s.t = pixel_magic_clamped(s.a, p.pad_width_pp5, G.g.nxp, G.g.nyp);
         s.off = 8u * idx;
     }
     const bool masked = __ldg(mask + idx) != 0;
-    acc_visit(acc, G.acc_offset + idx, 0.0f, !masked, slc, slt);
+    acc_visit<false>(acc, G.acc_offset + idx, 0.0f, !masked, slc, slt);
     s.alive = !masked && (0.0f < p.max_length) && (0u < p.max_n_steps);
 }
 
@@ -191,7 +193,7 @@ __device__ __forceinline__ void field_step(FieldLane& s, const uint8_t* __restri
     s.l = s.l + dl;
     s.n += 1;
     s.dt = dt;  // (a halted trajectory has no next step)
-    acc_visit(acc, G.acc_offset + idx, s.l, s.alive, slc, slt);
+    acc_visit<true>(acc, G.acc_offset + idx, s.l, s.alive, slc, slt);
     s.alive = s.alive && !(dl < p.integration_halt_threshold) && (s.l < p.max_length) && (s.n < p.max_n_steps);
 }
 
@@ -203,7 +205,7 @@ __device__ __forceinline__ FieldGrid grid_of(const slm_params& p, const FastGeo&
 // per-trajectory RK step count, saturated to 16 bits, indexed by queue position
 template <bool RECORD>
 __device__ __forceinline__ void record_end(const FieldLane& s, uint16_t* __restrict__ item_steps) {
-    if (RECORD) item_steps[s.item] = (uint16_t)(s.k < 65535u ? s.k : 65535u);
+    if (RECORD) item_steps[s.item] = (uint16_t)(s.n < 65535u ? s.n : 65535u);
 }
 
 __device__ __forceinline__ void warp_add_counters(u64 steps, u64 ntraj, u64* work) {
@@ -225,8 +227,8 @@ struct LaneCount {
 };
 
 __device__ __forceinline__ void count_trajectory(LaneCount& c, FieldLane& s) {
-    c.steps += s.k;
-    s.k = 0;
+    c.steps += s.n;
+    s.n = 0;
 }
 
 template <int ORDER, bool RECORD, bool FAST>
@@ -246,7 +248,6 @@ k_fields_plain(const __grid_constant__ slm_params p, const __grid_constant__ Fas
         c.ntraj = 1;
         while (s.alive) {
             field_step<ORDER, FAST, false>(s, mask, uv, p, k, G, acc, slc, slt);
-            s.k++;
         }
         record_end<RECORD>(s, item_steps);
         count_trajectory(c, s);
@@ -267,10 +268,14 @@ __device__ __forceinline__ u64 take_items(u64* work, unsigned idle, unsigned lan
     return head + __popc(idle & ((1u << lane) - 1u));
 }
 
-// Persistent form: the queue head work[0] must be 0 at launch.  Every loop
-// pass either hands queue items to idle lanes or advances every live
-// trajectory by one step, and each trajectory ends within max_n_steps steps,
-// so the loop ends; the exit test is warp-uniform.
+// Persistent form: the queue head work[0] must be 0 at launch.  A warp hands
+// queue items to its idle lanes, then advances every live trajectory step by
+// step until refill_min lanes (all, once the queue is used up) are idle; each
+// trajectory ends within max_n_steps steps, so the loops end; their tests are
+// warp-uniform.  The stepping is a loop of its own, closed by one vote, and not
+// a branch of a loop that asks for idle lanes, the queue's end and live lanes in
+// turn: 263 -> 251 thread instructions per RK2 step, 295 -> 289 ms for 4096^2
+// fan terrain, RK4, 6.80 -> 6.51 ms for 256^2 hills, RK2.
 template <int ORDER, bool RECORD, bool FAST>
 __global__ void __launch_bounds__(256, FIELD_BLOCKS)
 k_fields_persistent(const __grid_constant__ slm_params p, const __grid_constant__ FastGeo f,
@@ -284,13 +289,15 @@ k_fields_persistent(const __grid_constant__ slm_params p, const __grid_constant_
     const FieldGrid G = grid_of(p, f);
     FieldLane s;
     s.alive = false;
-    s.k = 0;
+    s.n = 0;
     Acc acc{0u, 0u, 0ull};
     LaneCount c{0ull, 0ull};
     bool drained = false;
+    unsigned live = 0;
     while (true) {
-        const unsigned idle = __ballot_sync(FULL, !s.alive);
-        if (!drained && (uint32_t)__popc(idle) >= refill_min) {
+        // here at least refill_min lanes are idle
+        if (!drained) {
+            const unsigned idle = ~live;
             const u64 item = take_items(work, idle, lane, n_items, drained);
             if (!s.alive) {
                 count_trajectory(c, s);
@@ -300,14 +307,18 @@ k_fields_persistent(const __grid_constant__ slm_params p, const __grid_constant_
                     if (!s.alive) record_end<RECORD>(s, item_steps);
                 }
             }
-            continue;
+            live = __ballot_sync(FULL, s.alive);
+            if (!drained && (uint32_t)__popc(~live) >= refill_min) continue;
         }
-        if (idle == FULL) break;
-        if (s.alive) {
-            field_step<ORDER, FAST, false>(s, mask, uv, p, k, G, acc, slc, slt);
-            s.k++;
-            if (RECORD && !s.alive) record_end<RECORD>(s, item_steps);
-        }
+        if (live == 0u) break;
+        const int keep = drained ? 0 : 32 - (int)refill_min;
+        do {
+            if (s.alive) {
+                field_step<ORDER, FAST, false>(s, mask, uv, p, k, G, acc, slc, slt);
+                if (RECORD && !s.alive) record_end<RECORD>(s, item_steps);
+            }
+            live = __ballot_sync(FULL, s.alive);
+        } while (__popc(live) > keep);
     }
     count_trajectory(c, s);
     acc_flush(acc, slc, slt);
@@ -338,17 +349,19 @@ k_fields_pair(const __grid_constant__ slm_params p, const __grid_constant__ Fast
     const u64 n_total = 2 * n_items;
     FieldLane s;
     s.alive = false;
-    s.k = 0;
+    s.n = 0;
     Acc acc{0u, 0u, 0ull};
     LaneCount c{0ull, 0ull};
     u64 steps_up = 0;
     bool drained = false;
+    unsigned live = 0;
     while (true) {
-        const unsigned idle = __ballot_sync(FULL, !s.alive);
-        if (!drained && (uint32_t)__popc(idle) >= refill_min) {
+        // here at least refill_min lanes are idle
+        if (!drained) {
+            const unsigned idle = ~live;
             u64 item = take_items(work, idle, lane, n_total, drained);
             if (!s.alive) {
-                if (G.acc_offset) steps_up += s.k;
+                if (G.acc_offset) steps_up += s.n;
                 count_trajectory(c, s);
                 if (item < n_total) {
                     const bool up = item >= n_items;
@@ -364,15 +377,19 @@ k_fields_pair(const __grid_constant__ slm_params p, const __grid_constant__ Fast
                     c.ntraj++;
                 }
             }
-            continue;
+            live = __ballot_sync(FULL, s.alive);
+            if (!drained && (uint32_t)__popc(~live) >= refill_min) continue;
         }
-        if (idle == FULL) break;
-        if (s.alive) {
-            field_step<ORDER, FAST, false>(s, mask, uv, p, k, G, acc, slc, slt);
-            s.k++;
-        }
+        if (live == 0u) break;
+        const int keep = drained ? 0 : 32 - (int)refill_min;
+        do {
+            if (s.alive) {
+                field_step<ORDER, FAST, false>(s, mask, uv, p, k, G, acc, slc, slt);
+            }
+            live = __ballot_sync(FULL, s.alive);
+        } while (__popc(live) > keep);
     }
-    if (G.acc_offset) steps_up += s.k;
+    if (G.acc_offset) steps_up += s.n;
     count_trajectory(c, s);
     acc_flush(acc, slc, slt);
     warp_add_counters(c.steps, c.ntraj, work);
@@ -414,14 +431,16 @@ k_fields_batched(const __grid_constant__ slm_params p, const __grid_constant__ F
     const uint32_t dd = p.subpixel_seed_point_density * p.subpixel_seed_point_density;
     FieldLane s;
     s.alive = false;
-    s.k = 0;
+    s.n = 0;
     FieldGrid G{make_geo(2u, 2u, 0.0f, 0.0f, 1.0f), make_fast_geo(2u, 2u, 1.0f, 1.0f, 0.0f, 0u), 0u, 0u};
     Acc acc{0u, 0u, 0ull};
     LaneCount c{0ull, 0ull};
     bool drained = false;
+    unsigned live = 0;
     while (true) {
-        const unsigned idle = __ballot_sync(FULL, !s.alive);
-        if (!drained && (uint32_t)__popc(idle) >= refill_min) {
+        // here at least refill_min lanes are idle
+        if (!drained) {
+            const unsigned idle = ~live;
             const u64 item = take_items(work, idle, lane, n_items, drained);
             if (!s.alive) {
                 count_trajectory(c, s);
@@ -448,19 +467,22 @@ k_fields_batched(const __grid_constant__ slm_params p, const __grid_constant__ F
                         atomicOr(reinterpret_cast<unsigned long long*>(work + 3), 1ull);
                         s.alive = false;
                         s.item = (uint32_t)item;
-                        s.k = 0;
                     }
                     if (!s.alive) record_end<RECORD>(s, item_steps);
                 }
             }
-            continue;
+            live = __ballot_sync(FULL, s.alive);
+            if (!drained && (uint32_t)__popc(~live) >= refill_min) continue;
         }
-        if (idle == FULL) break;
-        if (s.alive) {
-            field_step<ORDER, FAST, true>(s, mask, uv, p, k, G, acc, slc, slt);
-            s.k++;
-            if (RECORD && !s.alive) record_end<RECORD>(s, item_steps);
-        }
+        if (live == 0u) break;
+        const int keep = drained ? 0 : 32 - (int)refill_min;
+        do {
+            if (s.alive) {
+                field_step<ORDER, FAST, true>(s, mask, uv, p, k, G, acc, slc, slt);
+                if (RECORD && !s.alive) record_end<RECORD>(s, item_steps);
+            }
+            live = __ballot_sync(FULL, s.alive);
+        } while (__popc(live) > keep);
     }
     count_trajectory(c, s);
     acc_flush(acc, slc, slt);
@@ -636,8 +658,10 @@ static int check_grid(const slm_params* p) {
 }
 
 // slm_launch.chunk: a warp takes queue items once at least this many of its
-// lanes are idle (or all are); 0 selects 4, which measured best on the 2048^2
-// and 8192^2 RK4 workloads (fewer refill passes run by one or two lanes).
+// lanes are idle (or all are); 0 selects 4: a pass over one or two idle lanes
+// costs the warp as much as one over many.  Measured with 1, 2, 3, 4, 6, 8: 405,
+// 323, 296, 289, 292, 300 ms for 4096^2 fan terrain, RK4; 6.75, 6.53, 6.56,
+// 6.51, 6.60, 6.68 ms for 256^2 hills, RK2.
 static uint32_t refill_min(const slm_launch& L) {
     if (L.chunk == 0) return 4u;
     return L.chunk <= 1 ? 1u : (L.chunk >= 32 ? 32u : (uint32_t)L.chunk);

@@ -31,8 +31,8 @@
 // issue slots of the bilinear sums and the step's products.
 //
 // Measured (B200, both directions of 1024^2 incised relief, 2x2 seeds, RK4):
-// 815 -> 440 thread instructions per step; 4096^2 fan terrain, 1.64e10 RK4
-// steps: 505 -> 294 ms; 256^2 hills, RK2: 11.9 -> 6.8 ms.  What is left is
+// 815 -> 428 thread instructions per step; 4096^2 fan terrain, 1.64e10 RK4
+// steps: 505 -> 289 ms; 256^2 hills, RK2: 11.9 -> 6.5 ms.  What is left is
 // bound by the float units (80 % of the issue slots' worth of work: packed
 // operations take two cycles, the generator's wide products four), so
 // variants that trade slots for float work (wide products for the addresses
