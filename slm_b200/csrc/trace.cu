@@ -46,6 +46,15 @@ __device__ __forceinline__ void add_if(bool on, u64* p, u64 v) {
                  : "r"((uint32_t)on), "l"(p), "l"(v));  // nothing here reads the sums
 }
 
+// *p if `on`, else 1 (predicated: no branch around it)
+__device__ __forceinline__ uint32_t load_if(bool on, const uint8_t* p) {
+    uint32_t v;
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %1, 0;\n\tmov.u32 %0, 1;\n\t@q ld.global.nc.u8 %0, [%2];\n\t}"
+        : "=r"(v)
+        : "r"((uint32_t)on), "l"(p));
+    return v;
+}
+
 // writearray.cl:31-40: slt += (uint)(l+0.5), slc += 1, if `visits`.  A lane on
 // a trajectory has a run open (its start opened or continued one), so the
 // visits of its steps need not ask.
@@ -55,15 +64,16 @@ __device__ __forceinline__ void acc_visit(Acc& a, uint32_t idx, float l, bool vi
     const uint32_t v = __float2uint_rz(l + 0.5f);
     // selects and predicated atomics, no branch: some lane of a warp changes
     // pixel in nearly every step
-    const bool same = idx == a.idx && (OPEN || a.cnt);
-    const bool flush = visits && !same && (OPEN || a.cnt);
+    const bool open = OPEN || a.cnt != 0u;
+    const bool same = (idx == a.idx) & open;
+    const bool flush = visits & !same & open;
     add_if(flush, slt + a.idx, a.sum);
     add_if(flush, slc + a.idx, (u64)a.cnt);
-    if (visits) {
-        a.cnt = same ? a.cnt + 1u : 1u;
-        a.sum = (same ? a.sum : 0ull) + v;
-        a.idx = idx;
-    }
+    const uint32_t cnt = (same ? a.cnt : 0u) + 1u;
+    const u64 sum = (same ? a.sum : 0ull) + v;
+    a.cnt = visits ? cnt : a.cnt;
+    a.sum = visits ? sum : a.sum;
+    a.idx = visits ? idx : a.idx;
 }
 
 // State of one jittered field trajectory between steps.
@@ -86,34 +96,51 @@ struct FieldGrid {
     uint32_t base, acc_offset;
 };
 
-// Begin the trajectory of sub-pixel `sub` (= j*d + i) of the seed at `c`,
-// whose RNG stream is that of seed index `rng_idx`
-// (integratefields.cl:83-113; jittertrajectory.cl:56-62).
+// A trajectory ready to start: its first point, generator state and pixel (in
+// the uv / mask arrays), its queue position, and what its kernel adds.
+struct FieldStart {
+    Vec2 a;
+    uint32_t rng, idx, item, tag;
+};
+
+// The start of sub-pixel `sub` (= j*d + i) of the seed at `c`, whose RNG
+// stream is that of seed index `rng_idx` (integratefields.cl:83-113;
+// jittertrajectory.cl:56-62), on the grid of geometry g and first pixel
+// `base`; false if it lies on a masked pixel (a trajectory without visits or
+// steps).
 template <bool FAST>
-__device__ __forceinline__ void field_init(FieldLane& s, float2 c, uint32_t rng_idx, uint32_t sub,
-                                           uint32_t item, const uint8_t* __restrict__ mask,
-                                           const slm_params& p, const FieldGrid& G, Acc& acc,
-                                           u64* __restrict__ slc, u64* __restrict__ slt) {
+__device__ __forceinline__ bool start_at(FieldStart& st, float2 c, uint32_t rng_idx, uint32_t sub,
+                                         const uint8_t* __restrict__ mask, const slm_params& p, const Geo& g,
+                                         uint32_t base) {
     const uint32_t d = p.subpixel_seed_point_density;
     const uint32_t j = sub / d, i = sub % d;
-    s.a.x = c.x + ((float)i * p.subpixel_seed_step - p.subpixel_seed_halfspan);
-    s.a.y = c.y + ((float)j * p.subpixel_seed_step - p.subpixel_seed_halfspan);
-    s.rng = seed_rng(rng_idx);
+    st.a.x = c.x + ((float)i * p.subpixel_seed_step - p.subpixel_seed_halfspan);
+    st.a.y = c.y + ((float)j * p.subpixel_seed_step - p.subpixel_seed_halfspan);
+    st.rng = seed_rng(rng_idx);
     // the fast draws form (state + 1) * A without wrapping the sum: the state
     // whose successor wraps to 0 has the same successor as the modulus - 1
-    if (FAST && s.rng == 0xffffffffu) s.rng = LEHMER_M - 1u;
+    if (FAST && st.rng == 0xffffffffu) st.rng = LEHMER_M - 1u;
+    st.idx = base + pixel_of(st.a, p, g);
+    return __ldg(mask + st.idx) == 0;
+}
+
+// Put the lane on the trajectory `st` of the grid G: its first visit.
+template <bool FAST>
+__device__ __forceinline__ void field_begin(FieldLane& s, const FieldStart& st, const slm_params& p,
+                                            const FieldGrid& G, Acc& acc, u64* __restrict__ slc,
+                                            u64* __restrict__ slt) {
+    s.a = st.a;
+    s.rng = st.rng;
     s.l = 0.0f;
     s.dt = G.g.dt_max;
     s.n = 0;
-    s.item = item;
-    const uint32_t idx = G.base + pixel_of(s.a, p, G.g);
+    s.item = st.item;
     if (FAST) {
         s.t = pixel_magic_clamped(s.a, p.pad_width_pp5, G.g.nxp, G.g.nyp);
-        s.off = 8u * idx;
+        s.off = 8u * st.idx;
     }
-    const bool masked = __ldg(mask + idx) != 0;
-    acc_visit<false>(acc, G.acc_offset + idx, 0.0f, !masked, slc, slt);
-    s.alive = !masked && (0.0f < p.max_length) && (0u < p.max_n_steps);
+    acc_visit<false>(acc, G.acc_offset + st.idx, 0.0f, true, slc, slt);
+    s.alive = (0.0f < p.max_length) && (0u < p.max_n_steps);
 }
 
 // queue item -> (queue position, sub-pixel index)
@@ -128,23 +155,22 @@ __device__ __forceinline__ void split_item(u64 item, uint32_t dd, uint32_t& pos,
     }
 }
 
-// Start trajectory `item` = (seed - seed_begin) * d*d + j*d + i of one grid.
+// The start of trajectory `item` = (seed - seed_begin) * d*d + j*d + i of one
+// grid.
 //
 // `order` (optional) maps queue positions to seed indices, so trajectories can
 // be traced in any order; the RNG stream still follows the seed index, so no
 // trajectory changes.
 template <bool FAST>
-__device__ __forceinline__ void field_start(FieldLane& s, u64 item, uint32_t seed_begin,
-                                            const float2* __restrict__ seeds,
-                                            const uint32_t* __restrict__ order,
-                                            const uint8_t* __restrict__ mask, const slm_params& p,
-                                            const FieldGrid& G, Acc& acc, u64* __restrict__ slc,
-                                            u64* __restrict__ slt) {
+__device__ __forceinline__ bool start_of(FieldStart& st, u64 item, uint32_t seed_begin,
+                                         const float2* __restrict__ seeds, const uint32_t* __restrict__ order,
+                                         const uint8_t* __restrict__ mask, const slm_params& p, const Geo& g) {
     const uint32_t d = p.subpixel_seed_point_density;
-    uint32_t seed_off, sub;
-    split_item(item, d * d, seed_off, sub);
-    const uint32_t seed_idx = order ? __ldg(order + seed_begin + seed_off) : seed_begin + seed_off;
-    field_init<FAST>(s, __ldg(seeds + seed_idx), seed_idx, sub, (uint32_t)item, mask, p, G, acc, slc, slt);
+    uint32_t pos, sub;
+    split_item(item, d * d, pos, sub);
+    const uint32_t seed_idx = order ? __ldg(order + seed_begin + pos) : seed_begin + pos;
+    st.item = (uint32_t)item;
+    return start_at<FAST>(st, __ldg(seeds + seed_idx), seed_idx, sub, mask, p, g, 0u);
 }
 
 // One pass of the while loop of jittered_trajectory with
@@ -152,26 +178,34 @@ __device__ __forceinline__ void field_start(FieldLane& s, u64 item, uint32_t see
 // of that loop is unreachable (get_array_idx clamps into the grid).  FAST:
 // the launch meets fast_params, and the grid fast_grid (GATED: or it has no
 // interior, so that every step is rk_step's).
-template <int ORDER, bool FAST, bool GATED>
+//
+// All lanes of a warp run it together (WARP): those without a live trajectory
+// compute along on whatever point they have, reading within the grid, and
+// leave no visit and no count.
+template <int ORDER, bool FAST, bool GATED, bool WARP>
 __device__ __forceinline__ void field_step(FieldLane& s, const uint8_t* __restrict__ mask,
                                            const float2* __restrict__ uv, const slm_params& p,
                                            const FastConst& k, const FieldGrid& G, Acc& acc,
                                            u64* __restrict__ slc, u64* __restrict__ slt) {
     float dl, dt;
     uint32_t idx;
+    const bool on = !WARP || s.alive;
     if (FAST) {
         FastStep st;
         const bool ok = step_fast<ORDER, true, GATED>(s.a, s.t, s.off, s.dt, G.g.cf, s.rng, uv, G.f, k, st);
         float ex = st.d2.x - st.d1.x, ey = st.d2.y - st.d1.y;
         dt = G.g.dt_max;
         // rare: a guard failed, or the next dt is not DT_MAX by the cheap test
-        if (!ok || !(s.dt * s.dt * G.f.kerr >= __fmaf_rn(ey, ey, ex * ex))) {
-            if (!ok) {
-                st = step_exact<ORDER, true>(s.a, s.dt, s.rng, G.g.cf, uv, G.base, p, G.g.nxp, G.g.nyp);
-                ex = st.d2.x - st.d1.x;
-                ey = st.d2.y - st.d1.y;
+        const bool rare = on & !(ok & (s.dt * s.dt * G.f.kerr >= __fmaf_rn(ey, ey, ex * ex)));
+        if (WARP ? __any_sync(0xffffffffu, rare) : rare) {
+            if (rare) {
+                if (!ok) {
+                    st = step_exact<ORDER, true>(s.a, s.dt, s.rng, G.g.cf, uv, G.base, p, G.g.nxp, G.g.nyp);
+                    ex = st.d2.x - st.d1.x;
+                    ey = st.d2.y - st.d1.y;
+                }
+                dt = next_dt_fast(ex, ey, s.dt, G.g.dt_max, G.g.gs, G.f.gs_rcp, p.adjusted_max_error);
             }
-            dt = next_dt_fast(ex, ey, s.dt, G.g.dt_max, G.g.gs, G.f.gs_rcp, p.adjusted_max_error);
         }
         s.rng = st.rng;
         s.off = st.off;
@@ -179,7 +213,7 @@ __device__ __forceinline__ void field_step(FieldLane& s, const uint8_t* __restri
         s.t = st.t;
         dl = quantised_length(__fmaf_rn(st.d2.y, st.d2.y, st.d2.x * st.d2.x));
         idx = st.off >> 3;
-        s.alive = __ldg(mask + idx) == 0;
+        s.alive = load_if(on, mask + idx) == 0u;
     } else {
         const Step st = rk_step<ORDER, true>(s.a, s.dt, s.rng, uv + G.base, p, G.g);
         idx = G.base + st.idx;
@@ -191,10 +225,10 @@ __device__ __forceinline__ void field_step(FieldLane& s, const uint8_t* __restri
     }
     // a masked pixel ends the trajectory without a visit
     s.l = s.l + dl;
-    s.n += 1;
+    s.n += (uint32_t)on;
     s.dt = dt;  // (a halted trajectory has no next step)
     acc_visit<true>(acc, G.acc_offset + idx, s.l, s.alive, slc, slt);
-    s.alive = s.alive && !(dl < p.integration_halt_threshold) && (s.l < p.max_length) && (s.n < p.max_n_steps);
+    s.alive = s.alive & !(dl < p.integration_halt_threshold) & (s.l < p.max_length) & (s.n < p.max_n_steps);
 }
 
 // The grid of a launch's parameter block.
@@ -244,10 +278,15 @@ k_fields_plain(const __grid_constant__ slm_params p, const __grid_constant__ Fas
     const FieldGrid G = grid_of(p, f);
     if (item < n_items) {
         FieldLane s;
-        field_start<FAST>(s, item, seed_begin, seeds, order, mask, p, G, acc, slc, slt);
+        FieldStart st;
+        s.alive = false;
+        s.n = 0;
+        s.item = (uint32_t)item;
+        if (start_of<FAST>(st, item, seed_begin, seeds, order, mask, p, G.g))
+            field_begin<FAST>(s, st, p, G, acc, slc, slt);
         c.ntraj = 1;
         while (s.alive) {
-            field_step<ORDER, FAST, false>(s, mask, uv, p, k, G, acc, slc, slt);
+            field_step<ORDER, FAST, false, false>(s, mask, uv, p, k, G, acc, slc, slt);
         }
         record_end<RECORD>(s, item_steps);
         count_trajectory(c, s);
@@ -256,26 +295,102 @@ k_fields_plain(const __grid_constant__ slm_params p, const __grid_constant__ Fas
     warp_add_counters(c.steps, c.ntraj, work);
 }
 
-// Queue positions for the warp's idle lanes (mask `idle`): the first one, or
-// none once the queue of n items is used up.
-__device__ __forceinline__ u64 take_items(u64* work, unsigned idle, unsigned lane, u64 n, bool& drained) {
-    const int leader = __ffs(idle) - 1;
-    const unsigned n_idle = __popc(idle);
-    u64 head = 0;
-    if ((int)lane == leader) head = atomicAdd(work, (u64)n_idle);
-    head = __shfl_sync(0xffffffffu, head, leader);
-    if (head + n_idle >= n) drained = true;
-    return head + __popc(idle & ((1u << lane) - 1u));
+// The loop of a persistent warp: take trajectories from the queue (its head,
+// work[0], must be 0 at launch), start them on idle lanes, advance every live
+// one step by step until refill_min lanes (all, once nothing is left to start)
+// are idle.  Each trajectory ends within max_n_steps steps, so the loops end;
+// their tests are warp-uniform.
+//   prepare(item, st)  form the start of queue item `item`, false if it has none
+//   place(st)          make the lane's grid that of st
+//
+// Starts are formed 32 at a time, by all lanes, into a stash in shared memory
+// that idle lanes draw on: a start costs half a step's instructions and four
+// dependent loads, and formed by the two to four idle lanes it cost the warp as
+// much as by 32 (2.8 steps' time, every 15 steps, where a trajectory is 122
+// steps long).  Near the end of the queue (four trajectories a lane left, more
+// than all the stashes hold) a warp takes only as many as it has idle lanes, so
+// that none waits in one warp's stash while another's lanes idle: with one or
+// two a lane 256^2 hills take 6.8 ms, not 6.2.
+//
+// The stepping is a loop of its own, closed by one vote, and its lanes step
+// together (field_step), so that it has no branch that could diverge but for
+// the rare one.  Measured, with the stash 2 lanes idle at a refill, without 4:
+// 4096^2 fan terrain, RK4 (122 steps a trajectory): 289 -> 278 ms; odd incised
+// relief, RK4 (92): 43.7 -> 42.4 ms; 256^2 hills, RK2 (880): 6.5 -> 6.5 ms; 24
+// tiles, RK2 (740): 104 -> 102 ms.
+template <int ORDER, bool RECORD, bool FAST, bool GATED, class Prepare, class Place>
+__device__ __forceinline__ void field_loop(FieldLane& s, LaneCount& c, Acc& acc, FieldGrid& G, u64 n_items,
+                                           uint32_t refill_min, const slm_params& p, const FastConst& k,
+                                           const uint8_t* __restrict__ mask, const float2* __restrict__ uv,
+                                           u64* __restrict__ slc, u64* __restrict__ slt, u64* __restrict__ work,
+                                           uint16_t* __restrict__ item_steps, Prepare prepare, Place place) {
+    __shared__ FieldStart stashes[256 / 32][32];
+    const unsigned FULL = 0xffffffffu;
+    const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    FieldStart* stash = stashes[threadIdx.x >> 5];
+    const u64 plenty = 4ull * gridDim.x * blockDim.x;
+    unsigned live = 0, held = 0;  // lanes on a trajectory; starts in the stash
+    bool drained = false, bulk = n_items > plenty;
+    while (true) {
+        // here at least refill_min lanes are idle
+        if (held != 0u || !drained) {
+            const unsigned idle = ~live;
+            if (held == 0u) {
+                const unsigned want = bulk ? 32u : (unsigned)__popc(idle);
+                u64 head = 0;
+                if (lane == 0u) head = atomicAdd(work, (u64)want);
+                head = __shfl_sync(FULL, head, 0);
+                drained = head + want >= n_items;
+                bulk = head + want + plenty < n_items;
+                const u64 item = head + lane;
+                FieldStart st;
+                bool ok = false;
+                if (lane < want && item < n_items) {
+                    c.ntraj++;
+                    ok = prepare(item, st);
+                    if (RECORD && !ok) item_steps[item] = 0;
+                }
+                const unsigned ready = __ballot_sync(FULL, ok);
+                if (ok) stash[__popc(ready & below)] = st;
+                held = __popc(ready);
+                __syncwarp();
+            }
+            const unsigned rank = __popc(idle & below);
+            if (!s.alive && rank < held) {
+                const FieldStart st = stash[held - 1u - rank];
+                place(st);
+                count_trajectory(c, s);
+                field_begin<FAST>(s, st, p, G, acc, slc, slt);
+                if (RECORD && !s.alive) record_end<RECORD>(s, item_steps);
+            }
+            __syncwarp();  // the stash is read before it is written again
+            held -= min(held, (unsigned)__popc(idle));
+            live = __ballot_sync(FULL, s.alive);
+            if ((held != 0u || !drained) && (uint32_t)__popc(~live) >= refill_min) continue;
+        }
+        if (live == 0u) break;
+        const int keep = held == 0u && drained ? 0 : 32 - (int)refill_min;
+        do {
+            if (FAST) {
+                const bool on = s.alive;
+                field_step<ORDER, FAST, GATED, true>(s, mask, uv, p, k, G, acc, slc, slt);
+                if (RECORD && on && !s.alive) record_end<RECORD>(s, item_steps);
+            } else if (s.alive) {
+                field_step<ORDER, FAST, GATED, false>(s, mask, uv, p, k, G, acc, slc, slt);
+                if (RECORD && !s.alive) record_end<RECORD>(s, item_steps);
+            }
+            live = __ballot_sync(FULL, s.alive);
+        } while (__popc(live) > keep);
+    }
 }
 
-// Persistent form: the queue head work[0] must be 0 at launch.  A warp hands
-// queue items to its idle lanes, then advances every live trajectory step by
-// step until refill_min lanes (all, once the queue is used up) are idle; each
-// trajectory ends within max_n_steps steps, so the loops end; their tests are
-// warp-uniform.  The stepping is a loop of its own, closed by one vote, and not
-// a branch of a loop that asks for idle lanes, the queue's end and live lanes in
-// turn: 263 -> 251 thread instructions per RK2 step, 295 -> 289 ms for 4096^2
-// fan terrain, RK4, 6.80 -> 6.51 ms for 256^2 hills, RK2.
+// After the loop: the lanes' last runs and counts.
+__device__ __forceinline__ void field_end(FieldLane& s, LaneCount& c, Acc& acc, u64* slc, u64* slt, u64* work) {
+    count_trajectory(c, s);
+    acc_flush(acc, slc, slt);
+    warp_add_counters(c.steps, c.ntraj, work);
+}
+
 template <int ORDER, bool RECORD, bool FAST>
 __global__ void __launch_bounds__(256, FIELD_BLOCKS)
 k_fields_persistent(const __grid_constant__ slm_params p, const __grid_constant__ FastGeo f,
@@ -284,45 +399,15 @@ k_fields_persistent(const __grid_constant__ slm_params p, const __grid_constant_
                     u64* __restrict__ slc, u64* __restrict__ slt, u64* __restrict__ work,
                     const uint32_t* __restrict__ order, uint16_t* __restrict__ item_steps,
                     uint32_t refill_min) {
-    const unsigned FULL = 0xffffffffu;
-    const unsigned lane = threadIdx.x & 31u;
-    const FieldGrid G = grid_of(p, f);
-    FieldLane s;
-    s.alive = false;
-    s.n = 0;
+    FieldGrid G = grid_of(p, f);
+    FieldLane s{};
     Acc acc{0u, 0u, 0ull};
     LaneCount c{0ull, 0ull};
-    bool drained = false;
-    unsigned live = 0;
-    while (true) {
-        // here at least refill_min lanes are idle
-        if (!drained) {
-            const unsigned idle = ~live;
-            const u64 item = take_items(work, idle, lane, n_items, drained);
-            if (!s.alive) {
-                count_trajectory(c, s);
-                if (item < n_items) {
-                    field_start<FAST>(s, item, seed_begin, seeds, order, mask, p, G, acc, slc, slt);
-                    c.ntraj++;
-                    if (!s.alive) record_end<RECORD>(s, item_steps);
-                }
-            }
-            live = __ballot_sync(FULL, s.alive);
-            if (!drained && (uint32_t)__popc(~live) >= refill_min) continue;
-        }
-        if (live == 0u) break;
-        const int keep = drained ? 0 : 32 - (int)refill_min;
-        do {
-            if (s.alive) {
-                field_step<ORDER, FAST, false>(s, mask, uv, p, k, G, acc, slc, slt);
-                if (RECORD && !s.alive) record_end<RECORD>(s, item_steps);
-            }
-            live = __ballot_sync(FULL, s.alive);
-        } while (__popc(live) > keep);
-    }
-    count_trajectory(c, s);
-    acc_flush(acc, slc, slt);
-    warp_add_counters(c.steps, c.ntraj, work);
+    field_loop<ORDER, RECORD, FAST, false>(
+        s, c, acc, G, n_items, refill_min, p, k, mask, uv, slc, slt, work, item_steps,
+        [&](u64 item, FieldStart& st) { return start_of<FAST>(st, item, seed_begin, seeds, order, mask, p, G.g); },
+        [](const FieldStart&) {});
+    field_end(s, c, acc, slc, slt, work);
 }
 
 // ------------------------------------------------------------------ both directions
@@ -341,61 +426,30 @@ k_fields_pair(const __grid_constant__ slm_params p, const __grid_constant__ Fast
               u64* __restrict__ slc, u64* __restrict__ slt, uint32_t up_stride, u64* __restrict__ work,
               const uint32_t* __restrict__ order, const uint32_t* __restrict__ order_up,
               uint32_t refill_min) {
-    const unsigned FULL = 0xffffffffu;
-    const unsigned lane = threadIdx.x & 31u;
-    const uint32_t dd = p.subpixel_seed_point_density * p.subpixel_seed_point_density;
     FieldGrid G = grid_of(p, f);
     const float cf_down = G.g.cf;
-    const u64 n_total = 2 * n_items;
-    FieldLane s;
-    s.alive = false;
-    s.n = 0;
+    FieldLane s{};
     Acc acc{0u, 0u, 0ull};
     LaneCount c{0ull, 0ull};
     u64 steps_up = 0;
-    bool drained = false;
-    unsigned live = 0;
-    while (true) {
-        // here at least refill_min lanes are idle
-        if (!drained) {
-            const unsigned idle = ~live;
-            u64 item = take_items(work, idle, lane, n_total, drained);
-            if (!s.alive) {
-                if (G.acc_offset) steps_up += s.n;
-                count_trajectory(c, s);
-                if (item < n_total) {
-                    const bool up = item >= n_items;
-                    if (up) item -= n_items;
-                    G.acc_offset = up ? up_stride : 0u;
-                    G.g.cf = up ? cf_up : cf_down;
-                    uint32_t pos, sub;
-                    split_item(item, dd, pos, sub);
-                    const uint32_t* o = up ? order_up : order;
-                    const uint32_t seed_idx = o ? __ldg(o + seed_begin + pos) : seed_begin + pos;
-                    field_init<FAST>(s, __ldg(seeds + seed_idx), seed_idx, sub, (uint32_t)item, mask, p, G, acc, slc,
-                                     slt);
-                    c.ntraj++;
-                }
-            }
-            live = __ballot_sync(FULL, s.alive);
-            if (!drained && (uint32_t)__popc(~live) >= refill_min) continue;
-        }
-        if (live == 0u) break;
-        const int keep = drained ? 0 : 32 - (int)refill_min;
-        do {
-            if (s.alive) {
-                field_step<ORDER, FAST, false>(s, mask, uv, p, k, G, acc, slc, slt);
-            }
-            live = __ballot_sync(FULL, s.alive);
-        } while (__popc(live) > keep);
-    }
+    field_loop<ORDER, false, FAST, false>(
+        s, c, acc, G, 2 * n_items, refill_min, p, k, mask, uv, slc, slt, work, nullptr,
+        [&](u64 item, FieldStart& st) {
+            const bool up = item >= n_items;
+            st.tag = up;
+            return start_of<FAST>(st, up ? item - n_items : item, seed_begin, seeds, up ? order_up : order, mask, p,
+                                  G.g);
+        },
+        [&](const FieldStart& st) {
+            if (G.acc_offset) steps_up += s.n;
+            G.acc_offset = st.tag ? up_stride : 0u;
+            G.g.cf = st.tag ? cf_up : cf_down;
+        });
     if (G.acc_offset) steps_up += s.n;
-    count_trajectory(c, s);
-    acc_flush(acc, slc, slt);
-    warp_add_counters(c.steps, c.ntraj, work);
+    field_end(s, c, acc, slc, slt, work);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) steps_up += __shfl_xor_sync(FULL, steps_up, o);
-    if (lane == 0) atomicAdd(work + 3, steps_up);
+    for (int o = 16; o > 0; o >>= 1) steps_up += __shfl_xor_sync(0xffffffffu, steps_up, o);
+    if ((threadIdx.x & 31u) == 0u) atomicAdd(work + 3, steps_up);
 }
 
 // ------------------------------------------------------------------ batched tiles
@@ -426,67 +480,44 @@ k_fields_batched(const __grid_constant__ slm_params p, const __grid_constant__ F
                  const float2* __restrict__ uv, u64* __restrict__ slc, u64* __restrict__ slt,
                  u64* __restrict__ work, const uint32_t* __restrict__ order,
                  uint16_t* __restrict__ item_steps, uint32_t refill_min) {
-    const unsigned FULL = 0xffffffffu;
-    const unsigned lane = threadIdx.x & 31u;
     const uint32_t dd = p.subpixel_seed_point_density * p.subpixel_seed_point_density;
-    FieldLane s;
-    s.alive = false;
-    s.n = 0;
+    FieldLane s{};
     FieldGrid G{make_geo(2u, 2u, 0.0f, 0.0f, 1.0f), make_fast_geo(2u, 2u, 1.0f, 1.0f, 0.0f, 0u), 0u, 0u};
     Acc acc{0u, 0u, 0ull};
     LaneCount c{0ull, 0ull};
-    bool drained = false;
-    unsigned live = 0;
-    while (true) {
-        // here at least refill_min lanes are idle
-        if (!drained) {
-            const unsigned idle = ~live;
-            const u64 item = take_items(work, idle, lane, n_items, drained);
-            if (!s.alive) {
-                count_trajectory(c, s);
-                if (item < n_items) {
-                    uint32_t pos, sub;
-                    split_item(item, dd, pos, sub);
-                    const uint32_t seed = order ? __ldg(order + pos) : pos;
-                    const uint32_t t = find_tile(tiles, n_tiles, seed);
-                    const slm_tile& T = tiles[t];
-                    const uint32_t local = seed - __ldg(&T.seed_begin);
-                    c.ntraj++;
-                    if (local < __ldg(&T.n_seeds)) {
-                        G.g = make_geo(__ldg(&T.nx_padded), __ldg(&T.ny_padded), __ldg(&T.combo_factor),
-                                       __ldg(&T.dt_max), __ldg(&T.grid_scale));
-                        G.base = (uint32_t)__ldg(&T.grid_offset);
-                        if (FAST) {
-                            G.f = make_fast_geo(G.g.nxp, G.g.nyp, G.g.gs, G.g.dt_max, p.adjusted_max_error, G.base);
-                            // a tile the fast step cannot take has no interior pixel
-                            if (!fast_grid(G.g.nxp, G.g.nyp, G.base, G.g.cf, G.g.dt_max, p.trajectory_resolution))
-                                G.f.rx = -1.0f;
-                        }
-                        field_init<FAST>(s, __ldg(seeds + seed), local, sub, (uint32_t)item, mask, p, G, acc, slc, slt);
-                    } else {
-                        atomicOr(reinterpret_cast<unsigned long long*>(work + 3), 1ull);
-                        s.alive = false;
-                        s.item = (uint32_t)item;
-                    }
-                    if (!s.alive) record_end<RECORD>(s, item_steps);
-                }
+    const auto tile_geo = [&](const slm_tile& T) {
+        return make_geo(__ldg(&T.nx_padded), __ldg(&T.ny_padded), __ldg(&T.combo_factor), __ldg(&T.dt_max),
+                        __ldg(&T.grid_scale));
+    };
+    field_loop<ORDER, RECORD, FAST, true>(
+        s, c, acc, G, n_items, refill_min, p, k, mask, uv, slc, slt, work, item_steps,
+        [&](u64 item, FieldStart& st) {
+            uint32_t pos, sub;
+            split_item(item, dd, pos, sub);
+            const uint32_t seed = order ? __ldg(order + pos) : pos;
+            st.item = (uint32_t)item;
+            st.tag = find_tile(tiles, n_tiles, seed);
+            const slm_tile& T = tiles[st.tag];
+            const uint32_t local = seed - __ldg(&T.seed_begin);
+            if (local >= __ldg(&T.n_seeds)) {
+                atomicOr(reinterpret_cast<unsigned long long*>(work + 3), 1ull);
+                return false;
             }
-            live = __ballot_sync(FULL, s.alive);
-            if (!drained && (uint32_t)__popc(~live) >= refill_min) continue;
-        }
-        if (live == 0u) break;
-        const int keep = drained ? 0 : 32 - (int)refill_min;
-        do {
-            if (s.alive) {
-                field_step<ORDER, FAST, true>(s, mask, uv, p, k, G, acc, slc, slt);
-                if (RECORD && !s.alive) record_end<RECORD>(s, item_steps);
+            return start_at<FAST>(st, __ldg(seeds + seed), local, sub, mask, p, tile_geo(T),
+                                  (uint32_t)__ldg(&T.grid_offset));
+        },
+        [&](const FieldStart& st) {
+            const slm_tile& T = tiles[st.tag];
+            G.g = tile_geo(T);
+            G.base = (uint32_t)__ldg(&T.grid_offset);
+            if (FAST) {
+                G.f = make_fast_geo(G.g.nxp, G.g.nyp, G.g.gs, G.g.dt_max, p.adjusted_max_error, G.base);
+                // a tile the fast step cannot take has no interior pixel
+                if (!fast_grid(G.g.nxp, G.g.nyp, G.base, G.g.cf, G.g.dt_max, p.trajectory_resolution))
+                    G.f.rx = -1.0f;
             }
-            live = __ballot_sync(FULL, s.alive);
-        } while (__popc(live) > keep);
-    }
-    count_trajectory(c, s);
-    acc_flush(acc, slc, slt);
-    warp_add_counters(c.steps, c.ntraj, work);
+        });
+    field_end(s, c, acc, slc, slt, work);
 }
 
 // ------------------------------------------------------------------ trajectories
@@ -657,13 +688,12 @@ static int check_grid(const slm_params* p) {
     return SLM_OK;
 }
 
-// slm_launch.chunk: a warp takes queue items once at least this many of its
-// lanes are idle (or all are); 0 selects 4: a pass over one or two idle lanes
-// costs the warp as much as one over many.  Measured with 1, 2, 3, 4, 6, 8: 405,
-// 323, 296, 289, 292, 300 ms for 4096^2 fan terrain, RK4; 6.75, 6.53, 6.56,
-// 6.51, 6.60, 6.68 ms for 256^2 hills, RK2.
+// slm_launch.chunk: a warp starts trajectories once at least this many of its
+// lanes are idle (or all are); 0 selects 2.  Measured with 1, 2, 3, 4: 274.9,
+// 273.5, 276.2, 278 ms for 4096^2 fan terrain, RK4, where a trajectory ends every
+// fourth step of a warp; within 1 % of one another where they are longer.
 static uint32_t refill_min(const slm_launch& L) {
-    if (L.chunk == 0) return 4u;
+    if (L.chunk == 0) return 2u;
     return L.chunk <= 1 ? 1u : (L.chunk >= 32 ? 32u : (uint32_t)L.chunk);
 }
 

@@ -32,7 +32,7 @@
 //
 // Measured (B200, both directions of 1024^2 incised relief, 2x2 seeds, RK4):
 // 815 -> 428 thread instructions per step; 4096^2 fan terrain, 1.64e10 RK4
-// steps: 505 -> 289 ms; 256^2 hills, RK2: 11.9 -> 6.5 ms.  What is left is
+// steps: 505 -> 278 ms; 256^2 hills, RK2: 11.9 -> 6.5 ms.  What is left is
 // bound by the float units (80 % of the issue slots' worth of work: packed
 // operations take two cycles, the generator's wide products four), so
 // variants that trade slots for float work (wide products for the addresses
@@ -298,8 +298,8 @@ __device__ __noinline__ FastStep step_exact(Vec2 a, float dt, uint32_t rng, floa
 
 // One RK step from a0 (pixel t0 - 2^23, at byte offset off0 of the array uv)
 // with time step dt; true if every guard held and the values are rk_step's.
-// GATED: a lane outside the interior reads nothing (its grid may have none);
-// else it reads its clamped pixel's taps.
+// GATED: a lane outside the interior reads nothing (its grid may have none) and
+// stays where it is; else it reads its clamped pixel's taps.
 template <int ORDER, bool JITTER, bool GATED>
 __device__ __forceinline__ bool step_fast(Vec2 a0, F2 t0, uint32_t off0, float dt, float cf, uint32_t rng,
                                           const float2* __restrict__ uv, const FastGeo& f, const FastConst& k,
@@ -309,8 +309,15 @@ __device__ __forceinline__ bool step_fast(Vec2 a0, F2 t0, uint32_t off0, float d
     F2 fl = sub2(t0, as_f2(k.magic));
     float ix, iy;
     unpack2(sub2(fl, pack2(f.cx, f.cy)), ix, iy);
-    const bool inside = fabsf(ix) <= f.rx && fabsf(iy) <= f.ry;
-    if (GATED && !inside) return false;
+    const bool inside = (fabsf(ix) <= f.rx) & (fabsf(iy) <= f.ry);
+    if (GATED && !inside) {
+        o.d1 = o.d2 = o.u1 = Vec2{0.0f, 0.0f};
+        o.next = a0;
+        o.t = t0;
+        o.off = off0;
+        o.rng = rng;
+        return false;
+    }
     uint32_t off = min(off0, f.off_last);
     FastGuard gd{FAST_S_MIN, 0u};
     float s1, s2, s3, s4;  // sums of squares of the stages' last vectors
@@ -351,9 +358,9 @@ __device__ __forceinline__ bool step_fast(Vec2 a0, F2 t0, uint32_t off0, float d
     o.rng = rng;
     unpack2(next, o.next.x, o.next.y);
     unpack2(k1, o.u1.x, o.u1.y);
-    bool ok = gd.smallest >= FAST_S_MIN && inside;
-    if (JITTER) ok = ok && gd.state < LEHMER_M;
-    else ok = ok && fabsf(sx) < 1.0f && fabsf(sy) < 1.0f;  // an infinite sum of squares gives NaN here
+    bool ok = (gd.smallest >= FAST_S_MIN) & inside;
+    if (JITTER) ok = ok & (gd.state < LEHMER_M);
+    else ok = ok & (fabsf(sx) < 1.0f) & (fabsf(sy) < 1.0f);  // an infinite sum of squares gives NaN here
     return ok;
 }
 

@@ -306,3 +306,29 @@ def test_fields_at_the_edges_of_the_fast_step(kw, change, integrator):
         slc, slt, steps, ntraj = _gpu_fields(c, prm, "persistent", integrator)
         assert np.array_equal(slc, oslc) and np.array_equal(slt, oslt)
         assert (steps, ntraj) == (osteps, ontraj)
+
+
+@pytest.mark.parametrize("chunk", [1, 2, 7, 32])
+@pytest.mark.parametrize("block,size,max_length", [(32, (120, 110), 30.0), (64, (61, 79), 30.0), (32, (9, 8), 30.0),
+                                                   (32, (120, 110), 0.0)])
+def test_fields_refill_takes_every_trajectory_once(block, size, max_length, chunk):
+    """The persistent warps' stash of ready trajectories (32 at a time while
+    many are left, as many as there are idle lanes near the queue's end) gives
+    the sums, counts and step records of one thread per trajectory, starts on
+    masked pixels included."""
+    c = Case(nx=size[0], ny=size[1], density=2, step=0.5, max_length=max_length, seed=17)
+    c.mask[np.random.default_rng(3).random(c.mask.shape) < 0.1] = True
+    seeds, mask, uv = _dev(c)
+    prm = c.params("INTEGRATE_FIELDS", 1.0)
+    order = torch.from_numpy(np.random.default_rng(4).permutation(int(prm.n_seed_points)).astype(np.int32))
+    got = []
+    for schedule in ("plain", "persistent"):
+        slc = torch.zeros(prm.nxy_padded, dtype=torch.uint64, device=DEV)
+        slt, work = torch.zeros_like(slc), kernels.workspace(DEV)
+        steps = torch.full((4 * int(prm.n_seed_points),), 9, dtype=torch.int16, device=DEV).view(torch.uint16)
+        kernels.integrate_fields(prm, seeds, mask, uv, slc, slt, work, schedule=schedule, block_threads=block,
+                                 blocks_per_sm=1, chunk=chunk, order=order.to(DEV).view(torch.uint32), item_steps=steps)
+        torch.cuda.synchronize()
+        got.append([t.cpu().numpy() for t in (slc, slt, steps, work[1:3])])
+    for plain, persistent in zip(*got):
+        assert np.array_equal(plain, persistent)
