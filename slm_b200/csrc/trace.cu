@@ -315,9 +315,9 @@ k_fields_plain(const __grid_constant__ slm_params p, const __grid_constant__ Fas
 // The stepping is a loop of its own, closed by one vote, and its lanes step
 // together (field_step), so that it has no branch that could diverge but for
 // the rare one.  Measured, with the stash 2 lanes idle at a refill, without 4:
-// 4096^2 fan terrain, RK4 (122 steps a trajectory): 289 -> 278 ms; odd incised
-// relief, RK4 (92): 43.7 -> 42.4 ms; 256^2 hills, RK2 (880): 6.5 -> 6.5 ms; 24
-// tiles, RK2 (740): 104 -> 102 ms.
+// 4096^2 fan terrain, RK4 (122 steps a trajectory): 289 -> 274 ms; odd incised
+// relief, RK4 (92): 43.7 -> 41.3 ms; 256^2 hills, RK2 (880): 6.5 -> 6.2 ms; 24
+// tiles, RK2 (740): 104 -> 94.5 ms (make_fast_geo's wider interior included).
 template <int ORDER, bool RECORD, bool FAST, bool GATED, class Prepare, class Place>
 __device__ __forceinline__ void field_loop(FieldLane& s, LaneCount& c, Acc& acc, FieldGrid& G, u64 n_items,
                                            uint32_t refill_min, const slm_params& p, const FastConst& k,

@@ -32,7 +32,7 @@
 //
 // Measured (B200, both directions of 1024^2 incised relief, 2x2 seeds, RK4):
 // 815 -> 428 thread instructions per step; 4096^2 fan terrain, 1.64e10 RK4
-// steps: 505 -> 278 ms; 256^2 hills, RK2: 11.9 -> 6.5 ms.  What is left is
+// steps: 505 -> 274 ms; 256^2 hills, RK2: 11.9 -> 6.2 ms.  What is left is
 // bound by the float units (80 % of the issue slots' worth of work: packed
 // operations take two cycles, the generator's wide products four), so
 // variants that trade slots for float work (wide products for the addresses
@@ -120,7 +120,7 @@ struct FastGeo {
     uint32_t koff;      // byte offset of a pixel's vector: pitch * bits(2^23 + xi) + 8 * bits(2^23 + yi) + koff
     uint32_t off_last;  // largest such offset whose four taps lie in the grid
     float cx, cy;       // interior pixels: |xi - cx| <= rx, |yi - cy| <= ry, that is
-    float rx, ry;       //   2 <= xi <= nxp - 4 and 2 <= yi <= nyp - 4
+    float rx, ry;       //   1 <= xi <= nxp - 3 and 1 <= yi <= nyp - 3 (one less on long axes)
     float kerr;         // dt^2 kerr >= |d2 - d1|^2 implies a next dt of DT_MAX
     float gs_rcp;       // IEEE reciprocal of GRID_SCALE
 };
@@ -134,8 +134,14 @@ __host__ __device__ __forceinline__ FastGeo make_fast_geo(uint32_t nxp, uint32_t
     f.off_last = 8u * (base + nxp * nyp - nyp - 2u);
     f.cx = 0.5f * (float)(nxp - 2u);
     f.cy = 0.5f * (float)(nyp - 2u);
-    f.rx = 0.5f * ((float)nxp - 6.0f);
-    f.ry = 0.5f * ((float)nyp - 6.0f);
+    // A step's samples lie at most 0.99 pixels from its start (fast_grid) and
+    // the coordinates' rounding stays below the other 0.01 up to 2^16: no clamp
+    // can bind for a start one pixel (at its upper side two) inside the grid.
+    // With the usual padding of 2 that is every pixel of the region; with one
+    // pixel less, as beyond 2^16, its last row and column are not, and 3 % of
+    // a warp's steps on 256^2 meet one (24 tiles, RK2: 102 ms, now 95).
+    f.rx = 0.5f * ((float)nxp - (nxp <= 65536u ? 4.0f : 6.0f));
+    f.ry = 0.5f * ((float)nyp - (nyp <= 65536u ? 4.0f : 6.0f));
     f.gs_rcp = 1.0f / gs;
     const float k = adjusted_max_error * gs / dt_max;
     f.kerr = (k > 0x1p-30f && k < 0x1p30f) ? k * k * (1.0f - 0x1p-16f) : -1.0f;  // -1: never by the test

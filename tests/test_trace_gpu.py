@@ -278,6 +278,8 @@ def _set(**kw):
 # fast step (fast_params, fast_grid), and flows on either side of its guards
 STEP_EDGES = [
     (dict(nx=33, ny=47, pad=0), None), (dict(nx=33, ny=47, pad=1, step=0.1), None), (dict(nx=33, ny=21, pad=7), None),
+    (dict(nx=65533, ny=4, step=0.9, max_length=3.0, density=1), None),
+    (dict(nx=4, ny=65531, step=0.9, max_length=3.0, density=1), None),
     (dict(nx=3, ny=4, step=0.1), None), (dict(nx=4, ny=4, step=0.5), None), (dict(nx=5, ny=29, step=0.1), None),
     (dict(nx=40, ny=40, step=0.98), None), (dict(nx=40, ny=40, step=0.999), None), (dict(nx=40, ny=40, step=1.5), None),
     (dict(nx=40, ny=30), _set(trajectory_resolution=np.uint32(100))),
