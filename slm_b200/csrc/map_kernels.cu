@@ -25,7 +25,7 @@
 //   fix_right_flanks, fix_left_flanks  every work-item writes only its own
 //       pixel's label and reads labels along its RK path, so its result depends
 //       only on the final labels of lower-index items owning pixels on that
-//       path.  Paths are traced in parallel (k_flank_paths_linked, compressed
+//       path.  Paths are traced in parallel (FlankWalk, compressed
 //       to the steps whose (compute pixel, moved-to pixel) pair changes), then
 //       one persistent launch (k_flank_settle) takes items in ascending order,
 //       each waiting for the final labels of the lower-index owners on its
@@ -723,21 +723,20 @@ __device__ __forceinline__ bool seg_move(const Step& s, Vec2& vec, uint32_t& idx
 }
 
 // Per-pixel walks with warp-local refill: warp w owns items
-// [w * WALK_PER_WARP, (w + 1) * WALK_PER_WARP); a lane whose walk ends takes
-// the warp's next item at once (a ballot, no global counter), so a warp's
-// lanes stay busy however uneven their walks are.  Each item's walk is the
-// one-thread-per-item walk, so results are unchanged.
-constexpr uint32_t WALK_PER_WARP = 256;
-
+// [w * per_warp, (w + 1) * per_warp); a lane whose walk ends takes the warp's
+// next item at once (a ballot, no global counter), so a warp's lanes stay busy
+// however uneven their walks are (waiting for 3, 6 or 10 idle lanes measured 1
+// to 7 % slower, runs of 32 items dealt to the warps in turn the same).  Each
+// item's walk is the one-thread-per-item walk, so results are unchanged.
 template <class W>
 __global__ void __launch_bounds__(256)
-k_walks(const __grid_constant__ slm_params p, const __grid_constant__ WalkGrid wg, W w, uint32_t n) {
+k_walks(const __grid_constant__ slm_params p, const __grid_constant__ WalkGrid wg, W w, uint32_t n,
+        uint32_t per_warp) {
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t lo = warp * WALK_PER_WARP;
-    const uint64_t hi = lo + WALK_PER_WARP < n ? lo + WALK_PER_WARP : n;
-    uint64_t next = lo;
+    const uint64_t hi = min((warp + 1) * per_warp, (uint64_t)n);
+    uint64_t next = warp * per_warp;
     bool alive = false;
     while (true) {
         const unsigned idle = __ballot_sync(FULL, !alive);
@@ -745,18 +744,24 @@ k_walks(const __grid_constant__ slm_params p, const __grid_constant__ WalkGrid w
             const uint64_t mine = next + __popc(idle & ((1u << lane) - 1u));
             next += __popc(idle);
             if (!alive && mine < hi) alive = w.start((uint32_t)mine, p);
-        }
-        if (!__any_sync(FULL, alive)) {
-            if (next >= hi) break;
-            continue;
+        } else if (idle == FULL) {
+            break;
         }
         if (alive) alive = w.step(p, wg);
     }
 }
 
-static unsigned walk_grid(uint32_t n) {
-    const uint64_t warps = ((uint64_t)n + WALK_PER_WARP - 1) / WALK_PER_WARP;
-    return (unsigned)((warps + 7) / 8);  // 8 warps per block of 256
+// Items of a warp: an even share of the warps that the SMs hold (28 each), up
+// to 256: few walks are spread a few to a warp, whose steps take turns with its
+// lanes' different branches, and many refill their lanes.  Blocks of 64 threads,
+// so that one wave of them fills the SMs (with 256 a quarter of the flank walks'
+// blocks waited for a second: 4.08, now 2.65 ms for 1024^2 incised relief).
+template <class W>
+static void launch_walks(const slm_params& p, const W& w, uint32_t n, cudaStream_t s) {
+    const uint32_t wanted = (uint32_t)num_sms() * 28u;
+    const uint32_t per_warp = std::min(256u, (n + wanted - 1) / wanted);
+    const uint32_t warps = (n + per_warp - 1) / per_warp;
+    k_walks<W><<<(warps + 1) / 2, 64, 0, s>>>(p, make_walk_grid(p), w, n, per_warp);
 }
 
 // segment_hillslopes (segment.cl): from each hillslope pixel down to a thin
@@ -936,173 +941,202 @@ __device__ __forceinline__ uint32_t take_block(uint32_t* taken, uint32_t cap) {
     return b < cap ? b : NO_BLOCK;
 }
 
-// Where a flank walk's pairs go: counted only (out == NULL), a contiguous
-// range, or linked blocks taken from a pool as needed (counting goes on
-// after the pool runs out; *overflow is then set).
+// Where the flank walks' pairs go: only counted into n_pairs, in contiguous
+// ranges pairs[offsets[g] - base ..] of a chunk of the items, or in linked blocks
+// taken from a pool as needed (each path's name into names[g], NO_BLOCK for an
+// empty path; counter[0] counts the blocks taken, counter[1] is set when the
+// pool ran out: the counts are still exact).
+struct FlankOut {
+    u64* n_pairs;
+    const u64* offsets;
+    u64 base;
+    uint32_t* names;
+    uint2* pairs;
+    uint32_t* counter;
+    uint32_t cap_blocks;
+};
+
 struct ContigSink {
-    uint2* out;
+    uint2* to;
     u64 k;
+    __device__ void open(const FlankOut& o, uint32_t g, bool) {
+        to = o.pairs ? o.pairs + (o.offsets[g] - o.base) : nullptr;
+        k = 0;
+    }
+    __device__ void close(const FlankOut& o, uint32_t g) {
+        if (!o.pairs) o.n_pairs[g] = k;
+    }
     __device__ void settle_forward() {}
-    __device__ void put(uint2 e) {
-        if (out) out[k] = e;
+    __device__ void put(const FlankOut&, uint2 e) {
+        if (to) to[k] = e;
         ++k;
     }
 };
 
 struct LinkedSink {
-    uint2* pool;
-    uint32_t* taken;
-    uint32_t* overflow;
-    uint32_t cap, cur, f;
+    uint32_t cur, f;   // the block, its entries used; none and full without a block
     u64 k;
-    bool ok, forward;
-    __device__ void settle_forward() { forward = true; }
-    __device__ uint32_t name() const { return cur == NO_BLOCK ? NO_BLOCK : (forward ? cur | FLANK_FORWARD : cur); }
-    __device__ void put(uint2 e) {
-        ++k;
-        if (!ok) return;
-        if (cur == NO_BLOCK || f == FLANK_BLOCK - 1) {
-            const uint32_t b = take_block(taken, cap);
-            if (b == NO_BLOCK) {
-                ok = false;
-                atomicOr(overflow, 1u);
-                return;
-            }
-            if (cur != NO_BLOCK) pool[(u64)cur * FLANK_BLOCK + (FLANK_BLOCK - 1)].x = b;
-            pool[(u64)b * FLANK_BLOCK + (FLANK_BLOCK - 1)] = make_uint2(NO_BLOCK, cur);
-            cur = b;
-            f = 0;
+    uint32_t forward;  // FLANK_FORWARD or 0
+    // a path that `goes` has a pair: its first block is taken with those of the
+    // walks that start with it
+    __device__ void open(const FlankOut& o, uint32_t, bool goes) {
+        cur = NO_BLOCK;
+        f = FLANK_BLOCK;
+        k = 0;
+        forward = 0u;
+        if (goes) next(o);
+    }
+    __device__ void close(const FlankOut& o, uint32_t g) {
+        o.n_pairs[g] = k;
+        o.names[g] = cur == NO_BLOCK ? NO_BLOCK : cur | forward;
+    }
+    __device__ void settle_forward() { forward = FLANK_FORWARD; }
+    __device__ void next(const FlankOut& o) {
+        const uint32_t b = take_block(o.counter, o.cap_blocks);
+        if (b == NO_BLOCK) {
+            f = FLANK_BLOCK;
+            atomicOr(o.counter + 1, 1u);
+            return;
         }
-        pool[(u64)cur * FLANK_BLOCK + f++] = e;
+        if (cur != NO_BLOCK) o.pairs[(u64)cur * FLANK_BLOCK + (FLANK_BLOCK - 1)].x = b;
+        o.pairs[(u64)b * FLANK_BLOCK + (FLANK_BLOCK - 1)] = make_uint2(NO_BLOCK, cur);
+        cur = b;
+        f = 0;
+    }
+    __device__ void put(const FlankOut& o, uint2 e) {
+        ++k;
+        if (f == FLANK_BLOCK - 1) next(o);
+        if (f < FLANK_BLOCK - 1) o.pairs[(u64)cur * FLANK_BLOCK + f++] = e;
     }
 };
 
-// Steps of a flank walk up to its label-independent end (mask, thin channel,
-// step cap, stuck), as (compute pixel, moved-to pixel) pairs; consecutive
-// equal pairs are stored once.  With pairs == nullptr only counts.
-// Items g0 .. g0+n-1; paths are stored at pairs[offsets[g] - base] (a chunk
-// of the item range at a time, so the stored paths fit the workspace).
-// The walk of item g into `sink`; returns its pair count.
+// Steps of a flank item's walk up to its label-independent end (mask, thin
+// channel, step cap, stuck), as (compute pixel, moved-to pixel) pairs;
+// consecutive equal pairs are stored once.
+//
+// As in count_downchannels: once (vec, dt) repeats bit for bit the per-step
+// pairs repeat with the period (after every step `last` is that step's pair, so
+// each lap merges alike).  Unless a lap passes through the item's own pixel,
+// every lap reads the same labels: it stops the scan where the first lap does,
+// and two laps in a row leave the label one lap leaves.  So one lap and the
+// last, partial one are stored in place of all of them.  With the own pixel in
+// it the lap is stored as a period record {0x80000000|E, n} + the E pairs of a
+// lap.  The laps are walked again from the repeated state: COUNT forms a lap's
+// E and the partial one's pairs, LAP stores the one, PART the other.  A walk is
+// at any time one RK step from its next state, in whichever of these it is, so
+// that the lanes of a warp step together (k_walks).  Measured for the right flanks
+// of 1024^2 incised relief (1.05e6 walks of 200 steps): a thread per item, 11
+// lanes live a step, 3.58 ms; now 22 lanes, 2.65 ms, bound by issue (159 warp
+// instructions a step, 123 of them the walk's own) and its last long walks.
 template <class Sink>
-__device__ u64 flank_walk(const slm_params& p, const WalkGrid& wg, uint32_t g, const float2* __restrict__ seeds,
-                          const uint8_t* __restrict__ stop, const float2* __restrict__ uv, Sink& sink) {
-    Vec2 vec = seed_vec(seeds, g);
-    uint32_t idx = pixel_of(vec, p), n_steps = 0;
-    const uint32_t h = idx;
-    float dt = p.dt_max;
-    uint2 last = make_uint2(NO_OWNER, NO_OWNER);
-    // Whether the walk has computed off its own pixel: a pair that starts from
-    // that pixel afterwards reads the item's running label, so such a path is
-    // settled from its start.
-    bool left_home = false;
-    // As in count_downchannels: once (vec, dt) repeats bit for bit the
-    // per-step pairs repeat with the period (after every step `last` is that
-    // step's pair, so each lap merges alike).  Unless a lap passes through the
-    // item's own pixel, every lap reads the same labels: it stops the scan where
-    // the first lap does, and two laps in a row leave the label one lap leaves.
-    // So one lap and the last, partial one are stored in place of all of them.
-    // With the own pixel in it the lap is stored as a period record
-    // {0x80000000|E, n} + the E pairs of a lap.
-    Vec2 tv = vec;
-    float tdt = dt;
-    uint32_t power = 1, lam = 0;
-    while (!stop[idx] && n_steps < p.max_n_steps) {
+struct FlankWalk {
+    enum : uint32_t { WALK, COUNT, LAP, PART };
+    const float2* seeds;
+    const uint8_t* stop;
+    const float2* uv;
+    FlankOut out;
+    uint32_t g0;  // the first item
+    Sink sink;
+    Vec2 vec, tv;
+    float dt, tdt;
+    uint32_t g, h, idx, n_steps, phase;
+    // t steps since the checkpoint (tv, tdt), of `steps` until the next one
+    uint32_t t, steps;
+    uint2 last, lap_last;
+    uint32_t lap, R, E, partial;
+    // left_home: the walk has computed off its own pixel: a pair that starts
+    // from that pixel afterwards reads the item's running label, so such a path
+    // is settled from its start.  own: a lap passes through that pixel.
+    uint32_t left_home, own;
+
+    __device__ bool start(uint32_t item, const slm_params& p) {
+        g = g0 + item;
+        vec = seed_vec(seeds, g);
+        idx = pixel_of(vec, p);
+        h = idx;
+        n_steps = 0;
+        dt = p.dt_max;
+        last = make_uint2(NO_OWNER, NO_OWNER);
+        left_home = own = 0u;
+        tv = vec;
+        tdt = dt;
+        t = 0;
+        steps = 1;
+        phase = WALK;
+        const bool goes = !stop[idx] && n_steps < p.max_n_steps;
+        sink.open(out, g, goes);
+        if (!goes) sink.close(out, g);
+        return goes;
+    }
+    __device__ bool finish() {
+        sink.close(out, g);
+        return false;
+    }
+    // from the repeated state (tv, tdt) through n steps once more
+    __device__ bool again(uint32_t ph, uint32_t n) {
+        if (n == 0u) return finish();
+        phase = ph;
+        vec = tv;
+        dt = tdt;
+        last = lap_last;
+        t = 0;
+        steps = n;
+        return true;
+    }
+    __device__ bool step(const slm_params& p, const WalkGrid& wg) {
         const Step s = rk_plain(vec, dt, uv, p, wg);
         const uint32_t q = s.idx;
         idx = q;
         const bool stuck = seg_move(s, vec, idx, dt, n_steps, p, wg);
-        if (q != last.x || idx != last.y) {
-            if (left_home && last.y == h) sink.settle_forward();
-            left_home = left_home || q != h;
-            last = make_uint2(q, idx);
-            sink.put(last);
+        const bool moved = (q != last.x) | (idx != last.y), walk = phase == WALK, count = phase == COUNT;
+        if (walk & moved) {
+            if (left_home & (uint32_t)(last.y == h)) sink.settle_forward();
+            left_home |= (uint32_t)(q != h);
         }
-        if (stuck) break;
-        lam++;
-        if (__float_as_uint(vec.x) == __float_as_uint(tv.x) && __float_as_uint(vec.y) == __float_as_uint(tv.y)
-            && __float_as_uint(dt) == __float_as_uint(tdt) && n_steps < p.max_n_steps) {
-            const uint32_t L = lam, R = p.max_n_steps - n_steps, Rm = R % L;
-            uint32_t E = 0, partial = 0;
-            bool own = last.y == h, record = false;
-            // pass 0 counts a lap's pairs, pass 1 stores them, pass 2 the
-            // partial lap's
-            for (int pass = 0; pass < 3; ++pass) {
-                Vec2 v2 = vec;
-                float d2 = dt;
-                uint32_t i2 = idx, ns2 = 0, steps = L;
-                uint2 l2 = last;
-                if (pass == 1) {
-                    const uint32_t nfut = (R / L) * E + partial;
-                    if (nfut == 0) break;
-                    record = own;
-                    if (record) {
-                        sink.settle_forward();
-                        sink.put(make_uint2(FLANK_PERIOD | E, nfut));
-                    } else if (R < L) {
-                        continue;
-                    }
-                }
-                if (pass == 2) {
-                    if (record) break;
-                    steps = Rm;
-                }
-                for (uint32_t t2 = 1; t2 <= steps; ++t2) {
-                    const Step s2 = rk_plain(v2, d2, uv, p, wg);
-                    const uint32_t q2 = s2.idx;
-                    i2 = q2;
-                    seg_move(s2, v2, i2, d2, ns2, p, wg);
-                    own = own || i2 == h;
-                    if (q2 != l2.x || i2 != l2.y) {
-                        l2 = make_uint2(q2, i2);
-                        if (pass == 0) {
-                            E++;
-                            if (t2 <= Rm) partial++;
-                        } else {
-                            sink.put(l2);
-                        }
-                    }
-                }
+        if (moved) last = make_uint2(q, idx);
+        if (moved & !count) sink.put(out, last);
+        ++t;
+        if (walk) {
+            if (stuck) return finish();
+            const bool more = n_steps < p.max_n_steps;
+            if (more & (__float_as_uint(vec.x) == __float_as_uint(tv.x)) &
+                (__float_as_uint(vec.y) == __float_as_uint(tv.y)) & (__float_as_uint(dt) == __float_as_uint(tdt))) {
+                lap = t;
+                R = p.max_n_steps - n_steps;
+                E = partial = 0;
+                own = idx == h;
+                lap_last = last;
+                return again(COUNT, lap);
             }
-            break;
+            if (t == steps) {
+                tv = vec;
+                tdt = dt;
+                steps <<= 1;
+                t = 0;
+            }
+            return !stop[idx] & more ? true : finish();
         }
-        if (lam == power) {
-            tv = vec;
-            tdt = dt;
-            power <<= 1;
-            lam = 0;
+        own |= (uint32_t)(idx == h) & (uint32_t)count;
+        if (count & moved) {
+            E++;
+            if (t <= R % lap) partial++;
         }
+        if (t < steps) return true;
+        if (count) {
+            const uint32_t nfut = (R / lap) * E + partial;
+            if (nfut == 0u) return finish();
+            if (own) {
+                sink.settle_forward();
+                sink.put(out, make_uint2(FLANK_PERIOD | E, nfut));
+            } else if (R < lap) {
+                return again(PART, R % lap);
+            }
+            return again(LAP, lap);
+        }
+        if (phase == LAP && !own) return again(PART, R % lap);
+        return finish();
     }
-    return sink.k;
-}
-
-// Items g0 .. g0+n-1: with pairs == NULL the pair counts into n_pairs[g],
-// else the pairs into pairs[offsets[g] - base ..].
-__global__ void k_flank_paths(const __grid_constant__ slm_params p, const __grid_constant__ WalkGrid wg, uint32_t g0, uint32_t n, const float2* __restrict__ seeds,
-                              const uint8_t* __restrict__ stop, const float2* __restrict__ uv,
-                              u64* __restrict__ n_pairs, const u64* __restrict__ offsets, u64 base,
-                              uint2* __restrict__ pairs) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    const uint32_t g = g0 + t;
-    ContigSink sink{pairs ? pairs + (offsets[g] - base) : nullptr, 0};
-    const u64 k = flank_walk(p, wg, g, seeds, stop, uv, sink);
-    if (!pairs) n_pairs[g] = k;
-}
-
-// Items 0 .. n-1 in one pass: each path into linked blocks from the pool
-// (its name into names[g], NO_BLOCK for an empty path), its count into
-// n_pairs[g]; pool_ctr[0] counts the blocks taken, pool_ctr[1] is set when
-// the pool ran out (the counts are still exact).
-__global__ void k_flank_paths_linked(const __grid_constant__ slm_params p, const __grid_constant__ WalkGrid wg, uint32_t n, const float2* __restrict__ seeds,
-                                     const uint8_t* __restrict__ stop, const float2* __restrict__ uv,
-                                     u64* __restrict__ n_pairs, uint32_t* __restrict__ names,
-                                     uint2* __restrict__ pool, uint32_t cap_blocks, uint32_t* pool_ctr) {
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= n) return;
-    LinkedSink sink{pool, pool_ctr, pool_ctr + 1, cap_blocks, NO_BLOCK, 0, 0, true, false};
-    n_pairs[g] = flank_walk(p, wg, g, seeds, stop, uv, sink);
-    names[g] = sink.name();
-}
+};
 
 // The label of pixel q as flank item g sees it: item g's own running value if
 // q is g's pixel; the initial label if q has no owner or a higher-index owner;
@@ -1208,7 +1242,7 @@ __global__ void k_flank_round(const slm_params p, uint32_t g0, uint32_t n, uint3
 // launch instead of rounds.  Warps take items in ascending index from a
 // queue (warp-aggregated atomicAdd), so every item below one a lane holds
 // has been taken.  The RK walks are traced in parallel beforehand
-// (k_flank_paths), so only the path scans lie on a chain of waits.
+// (FlankWalk), so only the path scans lie on a chain of waits.
 //
 // An item reads the labels of lower-index owners along its path, and those
 // wait for the owners further down in turn, so what bounds the launch is the
@@ -2143,7 +2177,7 @@ int slm_segment_hillslopes(const slm_params* p, uint32_t n, const float* seed_po
     if (rc) return rc;
     if (n == 0) return SLM_OK;
     SegHillWalk w{F2(seed_point), mask, F2(uv), mapping, label};
-    k_walks<SegHillWalk><<<walk_grid(n), 256, 0, SS>>>(*p, make_walk_grid(*p), w, n);
+    launch_walks(*p, w, n, SS);
     SLM_LAUNCHED("k_walks<SegHillWalk>");
     return SLM_OK;
 }
@@ -2174,7 +2208,7 @@ int slm_subsegment_flanks(const slm_params* p, uint32_t n, const float* seed_poi
     if (rc) return rc;
     if (n == 0) return SLM_OK;
     SubsegFlankWalk w{F2(seed_point), mask, F2(uv), mapping, label};
-    k_walks<SubsegFlankWalk><<<walk_grid(n), 256, 0, SS>>>(*p, make_walk_grid(*p), w, n);
+    launch_walks(*p, w, n, SS);
     SLM_LAUNCHED("k_walks<SubsegFlankWalk>");
     return SLM_OK;
 }
@@ -2204,6 +2238,17 @@ static int flank_restart(uint32_t* label, const uint32_t* label_init, uint32_t* 
                          uint32_t nxy, cudaStream_t s) {
     SLM_CUDA(cudaMemcpyAsync(label, label_init, (size_t)nxy * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
     SLM_CUDA(cudaMemsetAsync(resolved, 0, (size_t)n * sizeof(uint32_t), s));
+    return SLM_OK;
+}
+
+// the paths of items a .. a+m-1, contiguous from pairs[0]
+static int launch_flank_chunk(const slm_params& p, uint32_t a, uint32_t m, const float2* seeds, const uint8_t* stop,
+                              const float2* uv, const u64* offsets, u64 base, uint2* pairs, cudaStream_t s) {
+    FlankWalk<ContigSink> w{seeds, stop, uv};
+    w.out = FlankOut{nullptr, offsets, base, nullptr, pairs};
+    w.g0 = a;
+    launch_walks(p, w, m, s);
+    SLM_LAUNCHED("k_walks<FlankWalk<ContigSink>>");
     return SLM_OK;
 }
 
@@ -2262,10 +2307,11 @@ static int fix_flanks(const slm_params* p, uint32_t n, const float* seed_point, 
         SLM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_flank_settle<LinkedPath>, 256, 0));
         settle_grid = (unsigned)(num_sms() * (occ > 0 ? occ : 1));
         const u64 cap_blocks = cap_pairs / FLANK_BLOCK;
-        k_flank_paths_linked<<<blocks_for(n, 128), 128, 0, SS>>>(
-            *p, make_walk_grid(*p), n, F2(seed_point), stop, F2(uv), n_pairs, names, pairs,
-            (uint32_t)(cap_blocks < FLANK_FORWARD - 1u ? cap_blocks : FLANK_FORWARD - 1u), words + 3);
-        SLM_LAUNCHED("k_flank_paths_linked");
+        FlankWalk<LinkedSink> w{F2(seed_point), stop, F2(uv)};
+        w.out = FlankOut{n_pairs, nullptr, 0ull, names, pairs, words + 3,
+                         (uint32_t)(cap_blocks < FLANK_FORWARD - 1u ? cap_blocks : FLANK_FORWARD - 1u)};
+        launch_walks(*p, w, n, SS);
+        SLM_LAUNCHED("k_walks<FlankWalk<LinkedSink>>");
         counted = true;
         uint32_t ran_out = 0;
         SLM_CUDA(cudaMemcpyAsync(&ran_out, words + 4, sizeof(uint32_t), cudaMemcpyDeviceToHost, SS));
@@ -2290,9 +2336,10 @@ static int fix_flanks(const slm_params* p, uint32_t n, const float* seed_point, 
     //    item reads only initial labels and the final labels of lower-index
     //    owners, which earlier chunks have resolved.
     if (!counted) {
-        k_flank_paths<<<blocks_for(n, 128), 128, 0, SS>>>(*p, make_walk_grid(*p), 0u, n, F2(seed_point), stop, F2(uv), n_pairs,
-                                                         nullptr, 0ull, nullptr);
-        SLM_LAUNCHED("k_flank_paths");
+        FlankWalk<ContigSink> w{F2(seed_point), stop, F2(uv)};
+        w.out = FlankOut{n_pairs};
+        launch_walks(*p, w, n, SS);
+        SLM_LAUNCHED("k_walks<FlankWalk<ContigSink>>");
     }
     rc = exclusive_scan(n_pairs, n, offsets, scan_scratch, SS);
     if (rc) return rc;
@@ -2332,9 +2379,8 @@ static int fix_flanks(const slm_params* p, uint32_t n, const float* seed_point, 
             u64 base = 0;
             SLM_CUDA(cudaMemcpyAsync(&base, offsets + a, sizeof(u64), cudaMemcpyDeviceToHost, SS));
             SLM_CUDA(cudaStreamSynchronize(SS));
-            k_flank_paths<<<blocks_for(m, 128), 128, 0, SS>>>(*p, make_walk_grid(*p), a, m, F2(seed_point), stop, F2(uv), nullptr,
-                                                             offsets, base, pairs);
-            SLM_LAUNCHED("k_flank_paths");
+            rc = launch_flank_chunk(*p, a, m, F2(seed_point), stop, F2(uv), offsets, base, pairs, SS);
+            if (rc) return rc;
             SLM_CUDA(cudaMemsetAsync(words + 1, 0, sizeof(uint32_t), SS));
             k_flank_settle<ContigPath><<<grid, 256, 0, SS>>>(*p, a, m, side, offsets, base, nullptr, nullptr,
                                                              pairs, hpix, mapping, rec, label, words + 1,
@@ -2356,9 +2402,8 @@ static int fix_flanks(const slm_params* p, uint32_t n, const float* seed_point, 
         u64 base = 0;
         SLM_CUDA(cudaMemcpyAsync(&base, offsets + a, sizeof(u64), cudaMemcpyDeviceToHost, SS));
         SLM_CUDA(cudaStreamSynchronize(SS));
-        k_flank_paths<<<blocks_for(m, 128), 128, 0, SS>>>(*p, make_walk_grid(*p), a, m, F2(seed_point), stop, F2(uv), nullptr,
-                                                         offsets, base, pairs);
-        SLM_LAUNCHED("k_flank_paths");
+        rc = launch_flank_chunk(*p, a, m, F2(seed_point), stop, F2(uv), offsets, base, pairs, SS);
+        if (rc) return rc;
         uint32_t done = 0;
         for (uint32_t r0 = round; done < m; ++round) {
             if (round - r0 > m + 1) {

@@ -389,3 +389,13 @@ def test_exclusive_scan_u64(n):
                                         ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
     want = np.concatenate([[0], np.cumsum(x, dtype=np.uint64)])
     assert np.array_equal(out.cpu().numpy().view(np.uint64), want)
+
+
+@pytest.mark.parametrize("kw", [dict(nx=23, ny=31, seed=13), dict(nx=420, ny=380, seed=10, channel_pct=93.0)])
+def test_mapping_walks_one_to_a_warp_and_refilled(kw):
+    """The per-pixel walks with a share of one item a warp (712 pixels) and of
+    more than a warp's lanes (159 600 pixels), flank paths included."""
+    c, info, data = pipeline_case(**kw)
+    run = DeviceVsOracle()
+    assert M.map_channels_segments(None, info, data, runner=run)
+    assert run.mismatches == [], run.mismatches
