@@ -17,8 +17,8 @@
 //   count_downchannels  the RK walk from each head is independent of the
 //       shared state except for where it stops, so every head's sequence of
 //       newly entered pixels is traced in parallel (k_count_paths), then one
-//       thread replays the integer updates (count, link, flags) head by head
-//       with the reference's early stop (k_count_replay);
+//       warp replays the integer updates (count, link, flags) head by head
+//       with the reference's early stop (k_count_replay_warp);
 //   flag_downchannels, segment_downchannels, prune_channel_heads  link walks
 //       and neighbour checks with no RK arithmetic, replayed in seed order by
 //       one thread;
@@ -49,7 +49,6 @@
 #define MAP_ST_OOB 2u
 #define MAP_LOOP_CAP (1u << 26)
 #define CONNECT_REC_MAX 256
-#define CNT_PREFETCH 16u
 #define NO_OWNER 0xffffffffu
 #define FLANK_PERIOD 0x80000000u
 
@@ -265,6 +264,12 @@ __global__ void __launch_bounds__(1024) k_prune_channel_heads(const slm_params p
     }
 }
 
+// n items spread over the warps that the SMs hold of the walk kernels (28 each)
+static uint32_t walk_share(uint32_t n) {
+    const uint32_t warps = (uint32_t)num_sms() * 28u;
+    return n / warps + (n % warps ? 1u : 0u);
+}
+
 // ------------------------------------------------------------------ count / flag
 // Phase A of count_downchannels: the pixels each head's walk enters, in order,
 // up to the walk's state-independent end; with events == nullptr only counts.
@@ -283,6 +288,7 @@ constexpr uint32_t CNT_KIND = 0xC0000000u;
 
 struct EventWriter {
     uint32_t* out;  // null: count words only
+    u64 cap;        // words `out` holds (the count goes on beyond them)
     u64 k;          // words written
     uint32_t ring[2 * CNT_PMAX];
     uint32_t nlit;  // literals in the ring (capped at 2*CNT_PMAX)
@@ -290,7 +296,7 @@ struct EventWriter {
     uint32_t pat[CNT_PMAX];
     uint32_t reps;  // events matched by the open repeat record
     __device__ void put(uint32_t w) {
-        if (out) out[k] = w;
+        if (out && k < cap) out[k] = w;
         k++;
     }
     __device__ void close_repeat() {
@@ -337,19 +343,29 @@ struct EventWriter {
     }
 };
 
+// Into events[g * slot ..] if slot is nonzero (a path that is longer is only
+// counted, and *too_long set), else into events[offsets[g] ..].  A head's walk is
+// a thread; per_warp of them to a warp (walk_share): the launch takes as long as its
+// longest walk, and a warp's steps take turns with its lanes' branches.  640
+// heads of 1024^2 incised relief, 32 to a warp and walked three times: 3 x 457
+// us; now once, one to a warp: 271 us.
 __global__ void k_count_paths(const __grid_constant__ slm_params p, const __grid_constant__ WalkGrid wg,
-                              uint32_t n, const float2* __restrict__ seeds,
+                              uint32_t n, uint32_t per_warp, const float2* __restrict__ seeds,
                               const uint8_t* __restrict__ mask, const float2* __restrict__ uv,
-                              u64* __restrict__ n_events, const u64* __restrict__ offsets,
-                              uint32_t* __restrict__ events, uint32_t* __restrict__ tail_idx) {
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= n) return;
+                              u64* __restrict__ n_events, const u64* __restrict__ offsets, uint32_t slot,
+                              uint32_t* __restrict__ events, uint32_t* __restrict__ tail_idx,
+                              uint32_t* too_long) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t item = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per_warp + lane;
+    if (lane >= per_warp || item >= n) return;
+    const uint32_t g = (uint32_t)item;
     Vec2 vec = seed_vec(seeds, g);
     float dt = p.dt_max;
     uint32_t idx = pixel_of(vec, p), prev_idx = idx, n_steps = 0;
     const uint32_t lim = 1000u * p.max_n_steps;
     EventWriter w;
-    w.out = events ? events + offsets[g] : nullptr;
+    w.out = events ? events + (slot ? (u64)g * slot : offsets[g]) : nullptr;
+    w.cap = slot ? (u64)slot : ~0ull;
     w.k = 0;
     w.nlit = 0;
     w.P = 0;
@@ -419,8 +435,11 @@ __global__ void k_count_paths(const __grid_constant__ slm_params p, const __grid
         }
     }
     w.close_repeat();
-    if (events) tail_idx[g] = idx;
-    else n_events[g] = w.k;
+    tail_idx[g] = idx;
+    if (slot) {
+        n_events[g] = w.k;
+        if (w.k > slot) atomicOr(too_long, 1u);
+    }
 }
 
 // The reference's per-event update of count_downchannels (countlink.cl:
@@ -437,216 +456,212 @@ __device__ __forceinline__ bool count_event(const slm_params& p, uint32_t e, uin
     return true;
 }
 
-// One thread replays the walks head by head (the pinned sequential order).
-// A repeat record is replayed event by event for its first lap; after a lap
-// every pattern pixel holds a count this walk wrote at most one lap ago,
-// below the running counter, so no later event can stop the walk.  The laps
-// in between only rewrite the same links, flags and growing counts, so they
-// are skipped and the final lap is replayed with its own counter values.
-__global__ void k_count_replay(const slm_params p, uint32_t n, const float2* __restrict__ seeds,
-                               const u64* __restrict__ offsets, const uint32_t* __restrict__ events,
-                               const uint32_t* __restrict__ tail_idx, uint32_t* mapping,
-                               uint32_t* count, uint32_t* link) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    uint32_t last8[CNT_PMAX];
-    for (uint32_t g = 0; g < n; ++g) {
-        const uint32_t head = pixel_of(seed_vec(seeds, g), p);
-        uint32_t counter = 1, prev = head, last = tail_idx[g];
-        uint32_t nd = 0;  // decoded events (for the pattern ring)
-        count[head] = counter++;
-        bool stopped = false;
-        const u64 k_end = offsets[g + 1];
-        for (u64 k = offsets[g]; k < k_end && !stopped; ++k) {
-            const uint32_t wd = events[k];
-            // one thread walks the events: bring the pixels of the event
-            // CNT_PREFETCH ahead into L2 so their loads do not wait on DRAM
-            if (k + CNT_PREFETCH < k_end) {
-                const uint32_t ahead = events[k + CNT_PREFETCH];
-                if (ahead < p.nxy_padded) {  // a pixel, or a count word that is still in the grid
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(count + ahead));
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(mapping + ahead));
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(link + ahead));
-                }
-            }
-            if ((wd & CNT_REPEAT) == 0u) {
-                if (!count_event(p, wd, counter, prev, mapping, count, link)) { last = wd; stopped = true; break; }
-                last8[nd % CNT_PMAX] = wd;
-                nd++;
-                continue;
-            }
-            uint32_t pat_ring[CNT_PMAX];
-            const uint32_t* pat;
-            uint32_t P, reps;
-            if ((wd & CNT_KIND) == CNT_PERIOD) {
-                P = wd & ~CNT_KIND;
-                pat = events + k + 1;
-                k += P;
-                reps = events[++k];
-            } else {
-                P = wd & ~CNT_REPEAT;
-                reps = events[++k];
-                for (uint32_t t = 0; t < P; ++t) pat_ring[t] = last8[(nd - P + t) % CNT_PMAX];
-                pat = pat_ring;
-            }
-            const uint32_t lap = reps < P ? reps : P;
-            for (uint32_t t = 0; t < lap; ++t) {
-                const uint32_t e = pat[t];
-                if (!count_event(p, e, counter, prev, mapping, count, link)) { last = e; stopped = true; break; }
-                last8[nd % CNT_PMAX] = e;
-                nd++;
-            }
-            if (stopped) break;
-            const uint32_t r = reps - lap;  // events after the first lap, from pattern position 0
-            if (r > 0) {
-                // skip to the final lap (events start..r-1) and replay it in order:
-                // every pattern pixel's last link and count assignments fall in
-                // it; flags were set by the first lap
-                const uint32_t c0 = counter;
-                const uint32_t start = r > P ? r - P : 0u;
-                prev = pat[(start + P - 1) % P];
-                for (uint32_t i = start; i < r; ++i) {
-                    const uint32_t e = pat[i % P];
-                    link[prev] = e;
-                    count[e] = c0 + 1 + i;
-                    prev = e;
-                    last8[nd % CNT_PMAX] = e;
-                    nd++;
-                }
-                counter = c0 + r;
-            }
-        }
-        link[prev] = last;
-    }
+// A load whose value nobody waits for: brings *p's line into the L1 cache.
+__device__ __forceinline__ void touch(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
 }
 
-
-// The same replay with one warp: runs of plain events (up to 32) are
-// decided together.  Event i of a run takes counter c + i + 1; the count it
-// compares with is the one an earlier event of the run wrote to the same
-// pixel (c + j + 1, always lower) or else the count loaded before the run,
-// so the first stopping event is a ballot.  Flags (an idempotent update),
-// links (the last writer per pixel wins: the highest lane of a match group
-// writes) and counts are then written in parallel, in the order the single
-// thread would leave them.  Repeat records are replayed by lane 0 as above.
-// __syncwarp orders each run's writes before the next run's loads.
+// One warp replays the walks head by head (the pinned sequential order).
+//
+// Up to 32 events are decided together.  Event i of a run takes counter
+// c + i + 1; the count it compares with is the one an earlier event of the run
+// wrote to the same pixel (c + j + 1, always lower) or else the count loaded
+// before the run, so the first stopping event is a ballot.  Flags (an idempotent
+// update), links (the last writer per pixel wins: the highest lane of a match
+// group writes) and counts are then written in parallel, in the order a single
+// thread would leave them.  __syncwarp orders each run's writes before the next
+// run's loads.
+//
+// A repeat record's first lap joins the run of plain events before it.  After a
+// lap every pattern pixel holds a count this walk wrote at most one lap ago,
+// below the running counter, so no later event can stop the walk: the laps in
+// between only rewrite the same links, flags and growing counts, so they are
+// skipped and the final lap is written with its own counter values.
+//
+// The launch is one serial chain, bound by the latency of each run.  So the
+// heads' words are loaded 32 heads at a time, and the next head's first events, and
+// the lines of the pixels they name, while a head is replayed.  640 heads of 1024^2
+// incised relief, 6354 plain events and 1054 records (1054 runs, the laps by lane
+// 0 before): 2.07 ms, now 1.28, 286 instructions a run of which each waits for the
+// one before; matches for each of the writes' orders, and a dummy value a lane in
+// them, took another 0.3 ms.
 __global__ void __launch_bounds__(32) k_count_replay_warp(const slm_params p, uint32_t n,
                                                           const float2* __restrict__ seeds,
-                                                          const u64* __restrict__ offsets,
+                                                          const u64* __restrict__ n_events,
+                                                          const u64* __restrict__ offsets, uint32_t slot,
                                                           const uint32_t* __restrict__ events,
                                                           const uint32_t* __restrict__ tail_idx, uint32_t* mapping,
                                                           uint32_t* count, uint32_t* link) {
-    if (blockIdx.x != 0) return;
     const unsigned FULL = 0xffffffffu;
-    const unsigned lane = threadIdx.x;
-    const uint32_t dummy = 0xFFFFFFE0u + lane;  // matches no pixel (nxy_padded < 2^32 - 32)
+    const unsigned lane = threadIdx.x, below = (1u << lane) - 1u;
+    // matches no pixel (nxy_padded < 2^32 - 32); one value for all lanes: a match
+    // takes a round a value
+    const uint32_t dummy = 0xFFFFFFE0u;
+    const auto first_lanes = [](uint32_t k) { return k < 32u ? (1u << k) - 1u : 0xffffffffu; };
+    // lane is the highest of `group`
+    const auto last_of = [&](unsigned group) { return (uint32_t)(31 - __clz(group)) == lane; };
     __shared__ uint32_t ring[CNT_PMAX];
-    for (uint32_t g = 0; g < n; ++g) {
-        const uint32_t head = pixel_of(seed_vec(seeds, g), p);
-        uint32_t counter = 1, prev = head, last = tail_idx[g], nd = 0;
-        if (lane == 0) count[head] = counter;
-        counter++;
-        bool stopped = false;
-        u64 k = offsets[g];
-        const u64 k_end = offsets[g + 1];
-        __syncwarp();
-        while (k < k_end && !stopped) {
-            const uint32_t wd0 = events[k];
-            if (wd0 & CNT_REPEAT) {
-                // a repeat record, by lane 0 as the single-thread replay does
-                if (lane == 0) {
-                    uint32_t pat_ring[CNT_PMAX];
-                    const uint32_t* pat;
-                    uint32_t P, reps;
-                    if ((wd0 & CNT_KIND) == CNT_PERIOD) {
-                        P = wd0 & ~CNT_KIND;
-                        pat = events + k + 1;
-                        k += P;
-                        reps = events[++k];
+    for (uint32_t g0 = 0; g0 < n; g0 += 32u) {
+        // lane i: head g0 + i
+        const uint32_t heads = min(32u, n - g0);
+        u64 begin = 0, end = 0;
+        uint32_t head_pixel = 0, tail = 0;
+        if (lane < heads) {
+            const uint32_t g = g0 + lane;
+            begin = slot ? (u64)g * slot : offsets[g];
+            end = slot ? begin + n_events[g] : offsets[g + 1];
+            head_pixel = pixel_of(seed_vec(seeds, g), p);
+            tail = tail_idx[g];
+        }
+        uint32_t ahead = 0;  // the next head's first words
+        {
+            const u64 k = __shfl_sync(FULL, begin, 0) + lane;
+            if (k < __shfl_sync(FULL, end, 0)) ahead = events[k];
+        }
+        for (uint32_t hd = 0; hd < heads; ++hd) {
+            u64 k = __shfl_sync(FULL, begin, hd);
+            const u64 k_end = __shfl_sync(FULL, end, hd);
+            const uint32_t head = __shfl_sync(FULL, head_pixel, hd);
+            uint32_t counter = 1, prev = head, last = __shfl_sync(FULL, tail, hd), nd = 0;
+            uint32_t w = ahead;
+            if (hd + 1u < heads) {
+                const u64 kn = __shfl_sync(FULL, begin, hd + 1u) + lane;
+                const u64 kn_end = __shfl_sync(FULL, end, hd + 1u);
+                ahead = kn < kn_end ? events[kn] : CNT_REPEAT;
+                if (kn + 32u < kn_end) touch(events + kn + 32u);
+            }
+            if (lane == 0) count[head] = counter;
+            counter++;
+            bool stopped = false, first = true;
+            __syncwarp();
+            while (k < k_end && !stopped) {
+                const bool have = k + lane < k_end;
+                if (!first) w = have ? events[k + lane] : 0u;
+                const unsigned pm = __ballot_sync(FULL, have && (w & CNT_REPEAT) == 0u);
+                const uint32_t m = (~pm == 0u) ? 32u : (uint32_t)(__ffs(~pm) - 1);
+                // the record behind the m plain events, if all of it is here
+                uint32_t P = 0, reps = 0, lap = 0, size = 0;
+                bool period = false;
+                if (m < 32u && k + m < k_end) {
+                    const uint32_t wd = __shfl_sync(FULL, w, m);
+                    period = (wd & CNT_KIND) == CNT_PERIOD;
+                    P = wd & ~(period ? CNT_KIND : CNT_REPEAT);
+                    size = period ? (P < 32u ? P + 2u : 33u) : 2u;
+                    if (m + size <= 32u && m + P <= 32u) {
+                        reps = __shfl_sync(FULL, w, m + size - 1u);
+                        lap = min(reps, P);
+                    } else if (m == 0u) {
+                        // a long pattern: by lane 0, event by event
+                        if (lane == 0) {
+                            const uint32_t* pat = events + k + 1;
+                            reps = events[k + 1 + P];
+                            lap = min(reps, P);
+                            for (uint32_t t = 0; t < lap && !stopped; ++t) {
+                                const uint32_t e = pat[t];
+                                if (!count_event(p, e, counter, prev, mapping, count, link)) {
+                                    last = e;
+                                    stopped = true;
+                                }
+                            }
+                            const uint32_t r = reps - lap, start = r > P ? r - P : 0u;
+                            if (!stopped && r > 0u) {
+                                prev = pat[(start + P - 1u) % P];
+                                for (uint32_t i = start; i < r; ++i) {
+                                    const uint32_t e = pat[i % P];
+                                    link[prev] = e;
+                                    count[e] = counter + 1u + i;
+                                    prev = e;
+                                }
+                                counter += r;
+                            }
+                        }
+                        counter = __shfl_sync(FULL, counter, 0);
+                        prev = __shfl_sync(FULL, prev, 0);
+                        last = __shfl_sync(FULL, last, 0);
+                        stopped = __shfl_sync(FULL, stopped ? 1 : 0, 0) != 0;
+                        k += (u64)P + 2u;  // nothing follows a period record
+                        first = false;
+                        __syncwarp();
+                        continue;
                     } else {
-                        P = wd0 & ~CNT_REPEAT;
-                        reps = events[++k];
-                        for (uint32_t t = 0; t < P; ++t) pat_ring[t] = ring[(nd - P + t) % CNT_PMAX];
-                        pat = pat_ring;
-                    }
-                    ++k;
-                    const uint32_t lap = reps < P ? reps : P;
-                    for (uint32_t t = 0; t < lap; ++t) {
-                        const uint32_t e = pat[t];
-                        if (!count_event(p, e, counter, prev, mapping, count, link)) {
-                            last = e;
-                            stopped = true;
-                            break;
-                        }
-                        ring[nd % CNT_PMAX] = e;
-                        nd++;
-                    }
-                    const uint32_t r = reps - lap;
-                    if (!stopped && r > 0) {
-                        const uint32_t c0 = counter;
-                        const uint32_t start = r > P ? r - P : 0u;
-                        prev = pat[(start + P - 1) % P];
-                        for (uint32_t i = start; i < r; ++i) {
-                            const uint32_t e = pat[i % P];
-                            link[prev] = e;
-                            count[e] = c0 + 1 + i;
-                            prev = e;
-                            ring[nd % CNT_PMAX] = e;
-                            nd++;
-                        }
-                        counter = c0 + r;
+                        size = 0u;  // in the next run
                     }
                 }
-                counter = __shfl_sync(FULL, counter, 0);
-                prev = __shfl_sync(FULL, prev, 0);
-                last = __shfl_sync(FULL, last, 0);
-                nd = __shfl_sync(FULL, nd, 0);
-                k = __shfl_sync(FULL, k, 0);
-                stopped = __shfl_sync(FULL, stopped ? 1 : 0, 0) != 0;
+                const uint32_t total = m + lap;
+                uint32_t e = w;
+                if (lap) {
+                    const uint32_t t = lane - m;  // the event of the lap
+                    const int from = period ? (int)(m + 1u + t) : (int)(m + t) - (int)P;
+                    const uint32_t there = __shfl_sync(FULL, w, from & 31);
+                    if (lane >= m) e = from >= 0 ? there : ring[(nd + (uint32_t)from) % CNT_PMAX];
+                }
+                const bool in = lane < total;
+                if (!in) e = dummy;
+                const uint32_t c_loaded = in ? count[e] : 0u;
+                const uint32_t flags = in ? mapping[e] : 0u;
+                const unsigned same = __match_any_sync(FULL, e), earlier = same & below;
+                const uint32_t mine = counter + lane + 1u;
+                const uint32_t seen = earlier ? counter + (uint32_t)(31 - __clz(earlier)) + 1u : c_loaded;
+                const unsigned stops = __ballot_sync(FULL, in && mine < seen);
+                const uint32_t n_pass = stops ? (uint32_t)(__ffs(stops) - 1) : total;  // counts, prev, ring
+                const uint32_t n_proc = stops ? n_pass + 1u : total;                   // flags and links
+                uint32_t prev_i = __shfl_up_sync(FULL, e, 1);
+                if (lane == 0) prev_i = prev;
+                if (lane < n_proc) mapping[e] = (flags & ~p.is_channelhead) | p.is_thinchannel;
+                // the lanes that come from the same pixel: one up from those of
+                // that pixel (and lane 0, from the run before)
+                const unsigned from_prev = __ballot_sync(FULL, e == prev) << 1 | 1u;
+                unsigned siblings = __shfl_up_sync(FULL, same, 1) << 1;
+                if (lane == 0) siblings = from_prev;
+                if (lane < n_proc && last_of(siblings & first_lanes(n_proc))) link[prev_i] = e;
+                if (lane < n_pass && last_of(same & first_lanes(n_pass))) count[e] = mine;
+                __syncwarp();  // the ring has been read
+                if (lane < n_pass && lane + CNT_PMAX >= n_pass) ring[(nd + lane) % CNT_PMAX] = e;
+                if (n_pass > 0u) prev = __shfl_sync(FULL, e, n_pass - 1u);
+                nd += n_pass;
+                counter += n_pass;
+                if (stops) {
+                    last = __shfl_sync(FULL, e, n_pass);
+                    stopped = true;
+                } else if (reps > lap) {
+                    // events start .. r-1 of the laps that follow the first one, by
+                    // lanes 0 .. cnt-1: lane j has pattern position q, and a set of
+                    // positions is turned by `turn` to be one of those lanes
+                    const uint32_t r = reps - lap, start = r > P ? r - P : 0u, cnt = r - start;
+                    const uint32_t turn = start % P;
+                    uint32_t q = turn + lane;
+                    if (q >= P) q -= P;
+                    const bool writes = lane < cnt;
+                    const uint32_t at = writes ? m + q : 0u, from = writes ? m + (q == 0u ? P - 1u : q - 1u) : 0u;
+                    const uint32_t ej = __shfl_sync(FULL, e, at), pj = __shfl_sync(FULL, e, from);
+                    const auto turned = [&](unsigned lanes, uint32_t by) {
+                        const unsigned set = (lanes >> m) & first_lanes(P);
+                        return (set >> by | set << (P - by)) & first_lanes(cnt);
+                    };
+                    const unsigned of_e = turned(__shfl_sync(FULL, same, at), turn);
+                    const unsigned of_p = turned(__shfl_sync(FULL, same, from), turn == 0u ? P - 1u : turn - 1u);
+                    __syncwarp();
+                    if (writes && last_of(of_p)) link[pj] = ej;
+                    if (writes && last_of(of_e)) count[ej] = counter + 1u + start + lane;
+                    if (writes && lane + CNT_PMAX >= cnt) ring[(nd + lane) % CNT_PMAX] = ej;
+                    prev = __shfl_sync(FULL, ej, cnt - 1u);
+                    nd += cnt;
+                    counter += r;
+                }
+                k += m + size;
+                first = false;
                 __syncwarp();
-                continue;
             }
-            // a run of plain events: the prefix of events[k ..] up to a record
-            uint32_t e = dummy;
-            bool plain = false;
-            if (k + lane < k_end) {
-                const uint32_t w = events[k + lane];
-                plain = (w & CNT_REPEAT) == 0u;
-                if (plain) e = w;
-            }
-            const unsigned pm = __ballot_sync(FULL, plain);
-            const uint32_t m = (~pm == 0u) ? 32u : (uint32_t)(__ffs(~pm) - 1);
-            const bool in = lane < m;
-            if (!in) e = dummy;
-            const uint32_t c_loaded = in ? count[e] : 0u;
-            const unsigned same = __match_any_sync(FULL, e);
-            const unsigned earlier = same & ((1u << lane) - 1u);
-            const uint32_t mine = counter + lane + 1u;
-            const uint32_t seen = earlier ? counter + (uint32_t)(31 - __clz(earlier)) + 1u : c_loaded;
-            const unsigned stops = __ballot_sync(FULL, in && mine < seen);
-            const uint32_t s_at = stops ? (uint32_t)(__ffs(stops) - 1) : m;
-            const uint32_t n_proc = stops ? s_at + 1u : m;  // flags and links
-            const uint32_t n_pass = s_at;                   // counts, prev, ring
-            uint32_t prev_i = __shfl_up_sync(FULL, e, 1);
-            if (lane == 0) prev_i = prev;
-            if (lane < n_proc) mapping[e] = (mapping[e] & ~p.is_channelhead) | p.is_thinchannel;
-            const unsigned lm = __match_any_sync(FULL, lane < n_proc ? prev_i : dummy);
-            if (lane < n_proc && (uint32_t)(31 - __clz(lm)) == lane) link[prev_i] = e;
-            const unsigned cm = __match_any_sync(FULL, lane < n_pass ? e : dummy);
-            if (lane < n_pass && (uint32_t)(31 - __clz(cm)) == lane) count[e] = mine;
-            if (lane < n_pass && lane + CNT_PMAX >= n_pass) ring[(nd + lane) % CNT_PMAX] = e;
-            const uint32_t e_last_pass = __shfl_sync(FULL, e, n_pass > 0 ? n_pass - 1 : 0);
-            if (n_pass > 0) prev = e_last_pass;
-            nd += n_pass;
-            counter += n_pass;
-            if (stops) {
-                last = __shfl_sync(FULL, e, s_at);
-                stopped = true;
-            }
-            k += n_proc;
+            if (lane == 0) link[prev] = last;
             __syncwarp();
+            // the next head's pixels: after this head's last stores, so that its
+            // lines are not fetched before they are written
+            if ((ahead & CNT_REPEAT) == 0u && ahead < p.nxy_padded) {
+                touch(count + ahead);
+                touch(mapping + ahead);
+            }
         }
-        if (lane == 0) link[prev] = last;
-        __syncwarp();
     }
 }
 
@@ -751,15 +766,14 @@ k_walks(const __grid_constant__ slm_params p, const __grid_constant__ WalkGrid w
     }
 }
 
-// Items of a warp: an even share of the warps that the SMs hold (28 each), up
+// Items of a warp: an even share (walk_share) of the warps that the SMs hold, up
 // to 256: few walks are spread a few to a warp, whose steps take turns with its
 // lanes' different branches, and many refill their lanes.  Blocks of 64 threads,
 // so that one wave of them fills the SMs (with 256 a quarter of the flank walks'
 // blocks waited for a second: 4.08, now 2.65 ms for 1024^2 incised relief).
 template <class W>
 static void launch_walks(const slm_params& p, const W& w, uint32_t n, cudaStream_t s) {
-    const uint32_t wanted = (uint32_t)num_sms() * 28u;
-    const uint32_t per_warp = std::min(256u, (n + wanted - 1) / wanted);
+    const uint32_t per_warp = std::min(256u, walk_share(n));
     const uint32_t warps = (n + per_warp - 1) / per_warp;
     k_walks<W><<<(warps + 1) / 2, 64, 0, s>>>(p, make_walk_grid(p), w, n, per_warp);
 }
@@ -2070,14 +2084,25 @@ int slm_count_downchannels(const slm_params* p, uint32_t n, const float* seed_po
     u64* n_events = reinterpret_cast<u64*>(workspace);
     u64* offsets = n_events + n;
     uint32_t* tails = reinterpret_cast<uint32_t*>(offsets + n + 1);
-    uint32_t* events = tails + n;
-    k_count_paths<<<blocks_for(n, 128), 128, 0, SS>>>(*p, make_walk_grid(*p), n, F2(seed_point), mask, F2(uv), n_events,
-                                                     nullptr, nullptr, nullptr);
+    uint32_t* too_long = tails + n;
+    uint32_t* events = too_long + 1;
+    SLM_REQUIRE(p->nxy_padded < 0xFFFFFFE0u, "grid too large for the count replay");
+    // The paths into equal shares of the workspace; if one does not fit, walked
+    // again into contiguous ranges.
+    const u64 room = (workspace_bytes - slm_count_downchannels_workspace(n, 0)) / sizeof(uint32_t);
+    uint32_t slot = (uint32_t)std::max<u64>(1u, std::min<u64>(room / n, 0x7fffffffu));
+    const uint32_t per_warp = std::min(32u, walk_share(n)), warps = (n + per_warp - 1) / per_warp;
+    SLM_CUDA(cudaMemsetAsync(too_long, 0, sizeof(uint32_t), SS));
+    k_count_paths<<<(warps + 1) / 2, 64, 0, SS>>>(*p, make_walk_grid(*p), n, per_warp, F2(seed_point), mask, F2(uv),
+                                                 n_events, nullptr, slot, room < n ? nullptr : events, tails,
+                                                 too_long);
     SLM_LAUNCHED("k_count_paths");
     k_exclusive_scan<<<1, 1024, 0, SS>>>(n_events, n, offsets);
     SLM_LAUNCHED("k_exclusive_scan");
     u64 total = 0;
+    uint32_t walk_again = 0;
     SLM_CUDA(cudaMemcpyAsync(&total, offsets + n, sizeof(u64), cudaMemcpyDeviceToHost, SS));
+    SLM_CUDA(cudaMemcpyAsync(&walk_again, too_long, sizeof(uint32_t), cudaMemcpyDeviceToHost, SS));
     SLM_CUDA(cudaStreamSynchronize(SS));
     const size_t need = slm_count_downchannels_workspace(n, total);
     if (required_bytes) *required_bytes = need;
@@ -2086,11 +2111,14 @@ int slm_count_downchannels(const slm_params* p, uint32_t n, const float* seed_po
                   (unsigned long long)total);
         return SLM_ERR_CAPACITY;
     }
-    k_count_paths<<<blocks_for(n, 128), 128, 0, SS>>>(*p, make_walk_grid(*p), n, F2(seed_point), mask, F2(uv), nullptr,
-                                                     offsets, events, tails);
-    SLM_LAUNCHED("k_count_paths");
-    SLM_REQUIRE(p->nxy_padded < 0xFFFFFFE0u, "grid too large for the count replay");
-    k_count_replay_warp<<<1, 32, 0, SS>>>(*p, n, F2(seed_point), offsets, events, tails, mapping, count, link);
+    if (walk_again || room < n) {
+        slot = 0;
+        k_count_paths<<<(warps + 1) / 2, 64, 0, SS>>>(*p, make_walk_grid(*p), n, per_warp, F2(seed_point), mask,
+                                                     F2(uv), n_events, offsets, 0u, events, tails, too_long);
+        SLM_LAUNCHED("k_count_paths");
+    }
+    k_count_replay_warp<<<1, 32, 0, SS>>>(*p, n, F2(seed_point), n_events, offsets, slot, events, tails, mapping,
+                                         count, link);
     SLM_LAUNCHED("k_count_replay_warp");
     return SLM_OK;
 }

@@ -38,7 +38,8 @@ SPECS = {
 FLANK_PATH_BUDGET = None
 FLANK_PATH_MAX = 96 << 30
 _MIN_WS = {
-    "count_downchannels": lambda L, p, n: L.slm_count_downchannels_workspace(n, 0),
+    # 128 words a head, so that most heads' paths are walked once
+    "count_downchannels": lambda L, p, n: L.slm_count_downchannels_workspace(n, 128 * int(n)),
     "flag_downchannels": lambda L, p, n: L.slm_flag_downchannels_workspace(n, p.nxy_padded),
     "fix_right_flanks": lambda L, p, n: L.slm_fix_flanks_workspace(n, p.nxy_padded, 0),
     "fix_left_flanks": lambda L, p, n: L.slm_fix_flanks_workspace(n, p.nxy_padded, 0),

@@ -399,3 +399,36 @@ def test_mapping_walks_one_to_a_warp_and_refilled(kw):
     run = DeviceVsOracle()
     assert M.map_channels_segments(None, info, data, runner=run)
     assert run.mismatches == [], run.mismatches
+
+
+@pytest.mark.parametrize("radius", [0.6, 2.0, 3.2, 4.0, 7.0])
+def test_count_downchannels_on_limit_cycles(radius):
+    """Heads around a vortex whose flow closes on a circle: period records of
+    a few events and of more than a warp holds, joined by walks that stop at
+    a longer one's counts."""
+    _, info, data = pipeline_case(nx=60, ny=50, seed=8)
+    x, y = np.meshgrid(np.arange(data.mask_array.shape[0]) - 31.3, np.arange(data.mask_array.shape[1]) - 26.1,
+                       indexing="ij")
+    r = np.hypot(x, y)
+    pull = np.clip(radius - r, -1.0, 1.0)
+    uv = np.stack((-y + pull * x, x + pull * y), axis=-1) / np.maximum(r, 1e-3)[..., None]
+    data.uv_array = np.ascontiguousarray(uv / np.linalg.norm(uv, axis=-1, keepdims=True).clip(1e-6), dtype=np.float32)
+    data.count_array = np.zeros(data.mask_array.shape, np.uint32)
+    data.link_array = np.zeros(data.mask_array.shape, np.uint32)
+    heads = np.argwhere(~data.mask_array & (r < 20))[::7]
+    data.mapping_array[heads[:, 0], heads[:, 1]] |= info.is_channelhead | info.is_channel
+    run = DeviceVsOracle()
+    assert M.count_downchannels(None, info, data, runner=run)
+    assert run.mismatches == [], run.mismatches
+
+
+def test_count_downchannels_paths_walked_again(monkeypatch):
+    """With the least workspace, then with exactly the events' total (uneven
+    paths, so they do not fit equal shares), counts and links are the oracle's."""
+    from slm_b200 import map_kernels
+    monkeypatch.setitem(map_kernels._MIN_WS, "count_downchannels",
+                        lambda L, p, n: L.slm_count_downchannels_workspace(n, 0))
+    info, data = incised_pipeline_case(seed=6)
+    run = DeviceVsOracle()
+    assert M.map_channels_segments(None, info, data, runner=run)
+    assert run.mismatches == [], run.mismatches
