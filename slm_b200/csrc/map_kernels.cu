@@ -264,12 +264,6 @@ __global__ void __launch_bounds__(1024) k_prune_channel_heads(const slm_params p
     }
 }
 
-// n items spread over the warps that the SMs hold of the walk kernels (28 each)
-static uint32_t walk_share(uint32_t n) {
-    const uint32_t warps = (uint32_t)num_sms() * 28u;
-    return n / warps + (n % warps ? 1u : 0u);
-}
-
 // ------------------------------------------------------------------ count / flag
 // Phase A of count_downchannels: the pixels each head's walk enters, in order,
 // up to the walk's state-independent end; with events == nullptr only counts.
@@ -773,7 +767,7 @@ k_walks(const __grid_constant__ slm_params p, const __grid_constant__ WalkGrid w
 // blocks waited for a second: 4.08, now 2.65 ms for 1024^2 incised relief).
 template <class W>
 static void launch_walks(const slm_params& p, const W& w, uint32_t n, cudaStream_t s) {
-    const uint32_t per_warp = std::min(256u, walk_share(n));
+    const uint32_t per_warp = walk_share(n, 256u);
     const uint32_t warps = (n + per_warp - 1) / per_warp;
     k_walks<W><<<(warps + 1) / 2, 64, 0, s>>>(p, make_walk_grid(p), w, n, per_warp);
 }
@@ -2091,7 +2085,7 @@ int slm_count_downchannels(const slm_params* p, uint32_t n, const float* seed_po
     // again into contiguous ranges.
     const u64 room = (workspace_bytes - slm_count_downchannels_workspace(n, 0)) / sizeof(uint32_t);
     uint32_t slot = (uint32_t)std::max<u64>(1u, std::min<u64>(room / n, 0x7fffffffu));
-    const uint32_t per_warp = std::min(32u, walk_share(n)), warps = (n + per_warp - 1) / per_warp;
+    const uint32_t per_warp = walk_share(n), warps = (n + per_warp - 1) / per_warp;
     SLM_CUDA(cudaMemsetAsync(too_long, 0, sizeof(uint32_t), SS));
     k_count_paths<<<(warps + 1) / 2, 64, 0, SS>>>(*p, make_walk_grid(*p), n, per_warp, F2(seed_point), mask, F2(uv),
                                                  n_events, nullptr, slot, room < n ? nullptr : events, tails,

@@ -39,6 +39,7 @@
 // or the draws' reduction) measured 2 to 5 % slower, fewer or more resident
 // warps (24, 36, 38, 40 against 32 per SM) 0 to 4 % slower.
 #pragma once
+#include "capi_util.cuh"
 #include "trace_common.cuh"
 #include "unit_math.cuh"
 
@@ -411,6 +412,16 @@ static inline WalkGrid make_walk_grid(const slm_params& p) {
     w.fast = fast_params(p) &&
              fast_grid(p.nx_padded, p.ny_padded, 0u, p.combo_factor, p.dt_max, p.trajectory_resolution);
     return w;
+}
+
+// Walks of a warp when n are spread evenly over the warps that the SMs hold of
+// the walk kernels (28 each), `most` at most.  A launch of few walks takes as
+// long as the longest of them, and a warp's steps take turns with its lanes'
+// different branches.
+static inline uint32_t walk_share(uint32_t n, uint32_t most = 32u) {
+    const uint32_t warps = (uint32_t)num_sms() * 28u;
+    const uint32_t share = n / warps + (n % warps ? 1u : 0u);
+    return share < most ? share : most;
 }
 
 template <int ORDER>

@@ -334,3 +334,16 @@ def test_fields_refill_takes_every_trajectory_once(block, size, max_length, chun
         got.append([t.cpu().numpy() for t in (slc, slt, steps, work[1:3])])
     for plain, persistent in zip(*got):
         assert np.array_equal(plain, persistent)
+
+
+@pytest.mark.parametrize("n", [1, 33, 4145, 9001])
+def test_trajectories_however_they_share_warps(n):
+    """Recorded trajectories with one, some and a ragged number of lanes of a
+    warp in use (the share follows their number) are the oracle's."""
+    c = Case(nx=110, ny=90, seed=23, step=0.5, max_length=8.0, n_traj_seeds=n)
+    prm = c.params("INTEGRATE_TRAJECTORY", np.float32(1.0))
+    ot, on, ol, _ = O.integrate_trajectory(prm, n, c.seeds, c.mask, c.uv, n_threads=4)
+    t, nn, ll = _gpu_traj(c, prm, n)
+    assert np.array_equal(on, nn) and np.array_equal(ol.view(np.uint32), ll.view(np.uint32))
+    for k in range(n):
+        assert np.array_equal(ot[k, :on[k]], t[k, :nn[k]]), k
