@@ -1570,7 +1570,7 @@ k_flank_settle(const __grid_constant__ slm_params p, uint32_t g0, uint32_t n, ui
     BackLane b;
     bool back = false;
     w.alive = false;
-    bool drained = false;
+    bool drained = false, stalled = false;
     for (uint32_t pass = 0;; ++pass) {
         // a lane that gave up stops every warp (the caller falls back)
         if ((pass & 255u) == 0u) {
@@ -1580,7 +1580,13 @@ k_flank_settle(const __grid_constant__ slm_params p, uint32_t g0, uint32_t n, ui
         }
         if (!drained) {
             const unsigned idle = __ballot_sync(FULL, !w.alive);
-            if (idle) {
+            // an item costs the warp a queue atomic and three dependent loads, so
+            // lanes are filled eight at a time, or when the warp only waited (no
+            // lane waits for an item not yet taken: they are taken ascending).
+            // Right flanks of 1024^2 incised relief: 1.82 ms one at a time, 1.72;
+            // 4 and 14 at a time 1.78 and 1.75; fewer or, with spills, more
+            // resident warps than 40 an SM are slower (24: 2.2, 48: 1.9)
+            if (__popc(idle) >= 8 || (stalled && idle)) {
                 const int leader = __ffs(idle) - 1;
                 uint32_t head = 0;
                 if ((int)lane == leader) head = atomicAdd(queue_head, (uint32_t)__popc(idle));
@@ -1664,7 +1670,8 @@ k_flank_settle(const __grid_constant__ slm_params p, uint32_t g0, uint32_t n, ui
         }
         // a warp whose every lane only waited backs off, leaving the issue
         // slots to warps that scan
-        if (__all_sync(FULL, idle_pass)) __nanosleep(64);
+        stalled = __all_sync(FULL, idle_pass);
+        if (stalled) __nanosleep(64);
     }
 }
 
