@@ -393,3 +393,20 @@ def test_bias_grad_column_sums(rows, cols):
     want = dz.double().sum(0) + 0.5
     bound = (rows / 256 + 301) * 2.0 ** -24 * (dz.double().abs().sum(0) + 0.5)
     assert torch.all((db.double() - want).abs() <= bound)
+
+
+@pytest.mark.parametrize("block,nx,ny,n", [(64, 130, 67, 130 * 67), (64, 64, 64, 4096), (64, 64, 64, 4097), (16, 33, 50, 1650),
+                                           (24, 50, 49, 2400), (8, 40, 40, 1600), (72, 100, 90, 5000), (64, 64, 64, 1)])
+def test_spatial_order_parts_of_blocks(block, nx, ny, n):
+    """Inside blocks of 16 to 64 pixels with at most 4096 seeds the order goes
+    by 8 x 8 pixel parts; it is a permutation by blocks everywhere."""
+    rng = np.random.default_rng(12)
+    seeds = np.stack([rng.integers(0, nx, n), rng.integers(0, ny, n)], 1).astype(np.float32)
+    order = S.spatial_order(torch.from_numpy(seeds).to(DEV), n, nx, ny, block=block).cpu().numpy().astype(np.int64)
+    assert np.array_equal(np.sort(order), np.arange(n))
+    x, y = seeds[order].astype(np.int64).T
+    key = x // block * -(-ny // block) + y // block
+    assert np.all(np.diff(key) >= 0)
+    if 8 < block <= 64:
+        held = np.bincount(key)[key] <= 4096
+        assert np.all(np.diff((key * 64 + x % block // 8 * 8 + y % block // 8)[held]) >= 0)
