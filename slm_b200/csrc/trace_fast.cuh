@@ -31,7 +31,7 @@
 // issue slots of the bilinear sums and the step's products.
 //
 // Measured (B200, both directions of 1024^2 incised relief, 2x2 seeds, RK4):
-// 815 -> 428 thread instructions per step; 4096^2 fan terrain, 1.64e10 RK4
+// 815 -> 414 thread instructions per step; 4096^2 fan terrain, 1.64e10 RK4
 // steps: 505 -> 274 ms; 256^2 hills, RK2: 11.9 -> 6.2 ms.  What is left is
 // bound by the float units (80 % of the issue slots' worth of work: packed
 // operations take two cycles, the generator's wide products four), so
