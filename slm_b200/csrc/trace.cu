@@ -212,7 +212,9 @@ __device__ __forceinline__ void field_step(FieldLane& s, const uint8_t* __restri
         s.a = st.next;
         s.t = st.t;
         dl = quantised_length(__fmaf_rn(st.d2.y, st.d2.y, st.d2.x * st.d2.x));
-        idx = st.off >> 3;
+        // a batch's tiles may lie beyond the byte offsets' range (their steps are
+        // then step_exact's); a single grid that is traced fast does not
+        idx = GATED ? st.idx : st.off >> 3;
         s.alive = load_if(on, mask + idx) == 0u;
     } else {
         const Step st = rk_step<ORDER, true>(s.a, s.dt, s.rng, uv + G.base, p, G.g);

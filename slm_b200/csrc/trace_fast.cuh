@@ -289,7 +289,8 @@ __device__ __forceinline__ float quant_fast(float v, const FastConst& k) {
 struct FastStep {
     Vec2 d1, d2, next, u1;
     F2 t;          // 2^23 + pixel of next
-    uint32_t off;  // byte offset of that pixel's vector
+    uint32_t off;  // byte offset of that pixel's vector; on a grid that fast_grid admits
+    uint32_t idx;  // the pixel, on any grid (a byte offset wraps from pixel 2^29 on)
     uint32_t rng;
 };
 
@@ -300,7 +301,7 @@ __device__ __noinline__ FastStep step_exact(Vec2 a, float dt, uint32_t rng, floa
     const Geo g{nxp, nyp, cf, 0.0f, 0.0f, 0.0f};  // the step itself reads neither DT_MAX nor GRID_SCALE
     const Step st = rk_step<ORDER, JITTER>(a, dt, rng, uv + base, p, g);
     return FastStep{st.d1, st.d2, st.next, st.u1, pixel_magic_clamped(st.next, p.pad_width_pp5, nxp, nyp),
-                    8u * (base + st.idx), rng};
+                    8u * (base + st.idx), base + st.idx, rng};
 }
 
 // One RK step from a0 (pixel t0 - 2^23, at byte offset off0 of the array uv)
@@ -322,6 +323,7 @@ __device__ __forceinline__ bool step_fast(Vec2 a0, F2 t0, uint32_t off0, float d
         o.next = a0;
         o.t = t0;
         o.off = off0;
+        o.idx = off0 >> 3;
         o.rng = rng;
         return false;
     }
@@ -362,6 +364,7 @@ __device__ __forceinline__ bool step_fast(Vec2 a0, F2 t0, uint32_t off0, float d
     const F2 next = add2(a, pack2(o.d2.x, o.d2.y));
     o.t = add2_rz(add2(next, as_f2(k.pp5)), as_f2(k.magic));
     o.off = offset_from_magic(o.t, f);
+    o.idx = o.off >> 3;
     o.rng = rng;
     unpack2(next, o.next.x, o.next.y);
     unpack2(k1, o.u1.x, o.u1.y);
@@ -434,7 +437,7 @@ __device__ __forceinline__ Step plain_step(Vec2 a, float dt, const float2* __res
         ok = step_fast<ORDER, false, false>(a, t, offset_from_magic(t, w.f), dt, p.combo_factor, 0u, uv, w.f, w.k, st);
     }
     if (!ok) st = step_exact<ORDER, false>(a, dt, 0u, p.combo_factor, uv, 0u, p, p.nx_padded, p.ny_padded);
-    return Step{st.d1, st.d2, st.u1, st.next, st.off >> 3};
+    return Step{st.d1, st.d2, st.u1, st.next, st.idx};
 }
 
 // |d| of a quantised step

@@ -104,3 +104,40 @@ def test_autotune_picks_and_caches(tmp_path):
     b.trace(L)
     torch.cuda.synchronize()
     assert torch.equal(b.acc, ref)
+
+
+def test_tiles_beyond_pixel_2_to_the_29():
+    """Tiles that straddle, follow and precede pixel 2^29 of a batch (where the
+    byte offset of a pixel's vector no longer fits 32 bits): each tile's sums
+    are the oracle's, and no other pixel is written."""
+    tiles = [batch.make_tile(synth.tile_dtm(nx, ny, 90 + i), density=2, step=0.5, max_steps=60)
+             for i, (nx, ny) in enumerate([(30, 25), (40, 33), (21, 44)])]
+    b = batch.TileBatch(tiles, DEV, 2)
+    n_px = (1 << 29) + 64 + 4096
+    at = [100, (1 << 29) - 900, (1 << 29) + 64 + 1000]
+    uv = torch.zeros((n_px, 2), dtype=torch.float32, device=DEV)
+    mask = torch.zeros(n_px, dtype=torch.uint8, device=DEV)
+    sizes = [int(t.mask.size) for t in tiles]
+    assert at[1] + sizes[1] > 1 << 29 and at[2] + sizes[2] <= n_px and at[1] + sizes[1] <= at[2]
+    for d in range(2):
+        table = b.tables[d].cpu().numpy().copy()
+        entries = (batch.SlmTile * len(tiles)).from_buffer(table)
+        for k, o in enumerate(at):
+            entries[k].grid_offset = o
+        b.tables[d] = torch.from_numpy(table).to(DEV)
+    for t, o, n in zip(tiles, at, sizes):
+        uv[o:o + n] = torch.from_numpy(t.uv.reshape(-1, 2)).to(DEV)
+        mask[o:o + n] = torch.from_numpy(t.mask.reshape(-1).view(np.uint8)).to(DEV)
+    b.uv, b.mask = uv, mask
+    for integrator, d, sign in ((2, 0, 1.0), (4, 1, -1.0)):
+        b.integrator = integrator
+        acc = torch.zeros((2, n_px), dtype=torch.int64, device=DEV)
+        b.acc = {(d, 0): acc[0].view(torch.uint64), (d, 1): acc[1].view(torch.uint64)}
+        b.trace_direction(d)
+        torch.cuda.synchronize()
+        want = [_oracle(t, sign, integrator) for t in tiles]
+        for (slc, slt, _), o, n in zip(want, at, sizes):
+            assert np.array_equal(acc[0, o:o + n].cpu().numpy().view(np.uint64), slc)
+            assert np.array_equal(acc[1, o:o + n].cpu().numpy().view(np.uint64), slt)
+        assert int(acc[0].sum()) == sum(int(w[0].sum()) for w in want)
+        assert int(acc[1].sum()) == sum(int(w[1].sum()) for w in want)

@@ -432,3 +432,76 @@ def test_count_downchannels_paths_walked_again(monkeypatch):
     run = DeviceVsOracle()
     assert M.map_channels_segments(None, info, data, runner=run)
     assert run.mismatches == [], run.mismatches
+
+
+def test_walks_beyond_pixel_2_to_the_29():
+    """Recorded trajectories and labelled hillslope walks around pixel 2^29 of a
+    grid (where the byte offset of a pixel's vector no longer fits 32 bits).
+    The flow is a patch at the low columns of the last rows, so the oracle's
+    grid holds only those columns: coordinates, and so every step, are the
+    same."""
+    import ctypes
+
+    import torch
+
+    from cases import Case
+    from slm_b200 import kernels, map_kernels
+    cols, nyp, nxp = 40, 22400, 24000
+    first = nxp - 100  # the patch's first row; pixel 2^29 is in row 23967
+    assert first * nyp < 1 << 29 < nxp * nyp and (1 << 29) // nyp < nxp - 20
+    c = Case(nx=96, ny=cols - 4, seed=12, step=0.5, max_length=60.0)
+    c.info.set_xy(nxp - 4, cols - 4, 2)
+    uv = np.zeros((nxp, cols, 2), np.float32)
+    uv[first:] = c.uv
+    mask = np.ones((nxp, cols), bool)
+    mask[first:] = c.mask
+    rng = np.random.default_rng(5)
+    seeds = np.ascontiguousarray(c.seeds[rng.choice(c.seeds.shape[0], 300, replace=False)])
+    seeds[:, 0] += first
+    c.info.n_seed_points = np.uint32(seeds.shape[0])
+    n = seeds.shape[0]
+
+    def wide(prm):
+        big = type(prm).from_buffer_copy(prm)
+        big.ny_padded, big.nxy_padded = nyp, nxp * nyp
+        return big
+
+    uv_d = torch.zeros((nxp, nyp, 2), dtype=torch.float32, device="cuda")
+    uv_d[first:, :cols] = torch.from_numpy(uv[first:]).cuda()
+    mask_d = torch.zeros((nxp, nyp), dtype=torch.uint8, device="cuda")  # nothing but the patch's own mask stops a walk
+    mask_d[first:, :cols] = torch.from_numpy(mask[first:].view(np.uint8)).cuda()
+    seeds_d = torch.from_numpy(seeds).cuda()
+    for integrator in (2, 4):
+        prm = c.params("INTEGRATE_TRAJECTORY", np.float32(1.0))
+        ot, on, ol, _ = O.integrate_trajectory(prm, n, seeds, mask, uv, integrator=integrator)
+        traj = torch.zeros(n * prm.max_n_steps * 2, dtype=torch.int8, device="cuda")
+        nsteps = torch.zeros(n, dtype=torch.uint16, device="cuda")
+        length = torch.zeros(n, dtype=torch.float32, device="cuda")
+        kernels.integrate_trajectory(wide(prm), n, seeds_d, mask_d, uv_d, traj, nsteps, length, integrator)
+        t, nn = traj.cpu().numpy().reshape(n, -1, 2), nsteps.cpu().numpy()
+        assert np.array_equal(on, nn)
+        assert np.array_equal(ol.view(np.uint32), length.cpu().numpy().view(np.uint32))
+        for k in range(n):
+            assert np.array_equal(ot[k, :on[k]], t[k, :nn[k]]), k
+
+    prm = M.kernel_params(c.info, "SEGMENT_HILLSLOPES")
+    mapping = np.zeros((nxp, cols), np.uint32)
+    thin = ~mask & (rng.random(mask.shape) < 0.08)
+    mapping[thin] = c.info.is_thinchannel
+    label = np.zeros((nxp, cols), np.uint32)
+    label[thin] = rng.integers(1, 1 << 20, int(thin.sum()))
+    mapping_d = torch.zeros((nxp, nyp), dtype=torch.int32, device="cuda")
+    mapping_d[first:, :cols] = torch.from_numpy(mapping[first:].view(np.int32)).cuda()
+    label_d = torch.zeros((nxp, nyp), dtype=torch.int32, device="cuda")
+    label_d[first:, :cols] = torch.from_numpy(label[first:].view(np.int32)).cuda()
+    none = np.zeros(1, np.uint32)
+    oracle_runner("segment_hillslopes", prm, seeds, [mask, uv, mapping, none, none, label])
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    map_kernels.run_device("segment_hillslopes", wide(prm), seeds_d, n,
+                           [mask_d, uv_d, mapping_d.view(torch.uint32), None, None, label_d.view(torch.uint32)],
+                           stream=st)
+    got = label_d[first:, :cols].cpu().numpy().view(np.uint32)
+    assert int((got != 0).sum()) > int(thin.sum())
+    assert np.array_equal(got, label[first:])
+    label_d[first:, :cols] = 0
+    assert not bool(label_d.any())
