@@ -108,7 +108,7 @@ struct FieldStart {
 // jittertrajectory.cl:56-62), on the grid of geometry g and first pixel
 // `base`; false if it lies on a masked pixel (a trajectory without visits or
 // steps).
-template <bool FAST>
+template <int FORM>
 __device__ __forceinline__ bool start_at(FieldStart& st, float2 c, uint32_t rng_idx, uint32_t sub,
                                          const uint8_t* __restrict__ mask, const slm_params& p, const Geo& g,
                                          uint32_t base) {
@@ -119,13 +119,13 @@ __device__ __forceinline__ bool start_at(FieldStart& st, float2 c, uint32_t rng_
     st.rng = seed_rng(rng_idx);
     // the fast draws form (state + 1) * A without wrapping the sum: the state
     // whose successor wraps to 0 has the same successor as the modulus - 1
-    if (FAST && st.rng == 0xffffffffu) st.rng = LEHMER_M - 1u;
+    if (FORM && st.rng == 0xffffffffu) st.rng = LEHMER_M - 1u;
     st.idx = base + pixel_of(st.a, p, g);
     return __ldg(mask + st.idx) == 0;
 }
 
 // Put the lane on the trajectory `st` of the grid G: its first visit.
-template <bool FAST>
+template <int FORM>
 __device__ __forceinline__ void field_begin(FieldLane& s, const FieldStart& st, const slm_params& p,
                                             const FieldGrid& G, Acc& acc, u64* __restrict__ slc,
                                             u64* __restrict__ slt) {
@@ -135,7 +135,7 @@ __device__ __forceinline__ void field_begin(FieldLane& s, const FieldStart& st, 
     s.dt = G.g.dt_max;
     s.n = 0;
     s.item = st.item;
-    if (FAST) {
+    if (FORM) {
         s.t = pixel_magic_clamped(s.a, p.pad_width_pp5, G.g.nxp, G.g.nyp);
         s.off = 8u * st.idx;
     }
@@ -161,7 +161,7 @@ __device__ __forceinline__ void split_item(u64 item, uint32_t dd, uint32_t& pos,
 // `order` (optional) maps queue positions to seed indices, so trajectories can
 // be traced in any order; the RNG stream still follows the seed index, so no
 // trajectory changes.
-template <bool FAST>
+template <int FORM>
 __device__ __forceinline__ bool start_of(FieldStart& st, u64 item, uint32_t seed_begin,
                                          const float2* __restrict__ seeds, const uint32_t* __restrict__ order,
                                          const uint8_t* __restrict__ mask, const slm_params& p, const Geo& g) {
@@ -170,19 +170,19 @@ __device__ __forceinline__ bool start_of(FieldStart& st, u64 item, uint32_t seed
     split_item(item, d * d, pos, sub);
     const uint32_t seed_idx = order ? __ldg(order + seed_begin + pos) : seed_begin + pos;
     st.item = (uint32_t)item;
-    return start_at<FAST>(st, __ldg(seeds + seed_idx), seed_idx, sub, mask, p, g, 0u);
+    return start_at<FORM>(st, __ldg(seeds + seed_idx), seed_idx, sub, mask, p, g, 0u);
 }
 
 // One pass of the while loop of jittered_trajectory with
 // runge_kutta_step_write_sl_data (rungekutta.cl:163-186).  The Euler branch
-// of that loop is unreachable (get_array_idx clamps into the grid).  FAST:
-// the launch meets fast_params, and the grid fast_grid (GATED: or it has no
-// interior, so that every step is rk_step's).
+// of that loop is unreachable (get_array_idx clamps into the grid).  FORM, but
+// for STEP_GENERAL: the launch meets fast_params, and the grid fast_grid
+// (GATED: or it has no interior, so that every step is rk_step's).
 //
 // All lanes of a warp run it together (WARP): those without a live trajectory
 // compute along on whatever point they have, reading within the grid, and
 // leave no visit and no count.
-template <int ORDER, bool FAST, bool GATED, bool WARP>
+template <int ORDER, int FORM, bool GATED, bool WARP>
 __device__ __forceinline__ void field_step(FieldLane& s, const uint8_t* __restrict__ mask,
                                            const float2* __restrict__ uv, const slm_params& p,
                                            const FastConst& k, const FieldGrid& G, Acc& acc,
@@ -190,9 +190,9 @@ __device__ __forceinline__ void field_step(FieldLane& s, const uint8_t* __restri
     float dl, dt;
     uint32_t idx;
     const bool on = !WARP || s.alive;
-    if (FAST) {
+    if (FORM) {
         FastStep st;
-        const bool ok = step_fast<ORDER, true, GATED>(s.a, s.t, s.off, s.dt, G.g.cf, s.rng, uv, G.f, k, st);
+        const bool ok = step_fast<ORDER, FORM, GATED>(s.a, s.t, s.off, s.dt, G.g.cf, s.rng, uv, G.f, k, st);
         float ex = st.d2.x - st.d1.x, ey = st.d2.y - st.d1.y;
         dt = G.g.dt_max;
         // rare: a guard failed, or the next dt is not DT_MAX by the cheap test
@@ -267,7 +267,7 @@ __device__ __forceinline__ void count_trajectory(LaneCount& c, FieldLane& s) {
     s.n = 0;
 }
 
-template <int ORDER, bool RECORD, bool FAST>
+template <int ORDER, bool RECORD, int FORM>
 __global__ void __launch_bounds__(256, FIELD_BLOCKS)
 k_fields_plain(const __grid_constant__ slm_params p, const __grid_constant__ FastGeo f,
                const __grid_constant__ FastConst k, const float2* __restrict__ seeds, uint32_t seed_begin,
@@ -284,11 +284,11 @@ k_fields_plain(const __grid_constant__ slm_params p, const __grid_constant__ Fas
         s.alive = false;
         s.n = 0;
         s.item = (uint32_t)item;
-        if (start_of<FAST>(st, item, seed_begin, seeds, order, mask, p, G.g))
-            field_begin<FAST>(s, st, p, G, acc, slc, slt);
+        if (start_of<FORM>(st, item, seed_begin, seeds, order, mask, p, G.g))
+            field_begin<FORM>(s, st, p, G, acc, slc, slt);
         c.ntraj = 1;
         while (s.alive) {
-            field_step<ORDER, FAST, false, false>(s, mask, uv, p, k, G, acc, slc, slt);
+            field_step<ORDER, FORM, false, false>(s, mask, uv, p, k, G, acc, slc, slt);
         }
         record_end<RECORD>(s, item_steps);
         count_trajectory(c, s);
@@ -320,7 +320,7 @@ k_fields_plain(const __grid_constant__ slm_params p, const __grid_constant__ Fas
 // 4096^2 fan terrain, RK4 (122 steps a trajectory): 289 -> 274 ms; odd incised
 // relief, RK4 (92): 43.7 -> 41.3 ms; 256^2 hills, RK2 (880): 6.5 -> 6.2 ms; 24
 // tiles, RK2 (740): 104 -> 94.5 ms (make_fast_geo's wider interior included).
-template <int ORDER, bool RECORD, bool FAST, bool GATED, class Prepare, class Place>
+template <int ORDER, bool RECORD, int FORM, bool GATED, class Prepare, class Place>
 __device__ __forceinline__ void field_loop(FieldLane& s, LaneCount& c, Acc& acc, FieldGrid& G, u64 n_items,
                                            uint32_t refill_min, const slm_params& p, const FastConst& k,
                                            const uint8_t* __restrict__ mask, const float2* __restrict__ uv,
@@ -362,7 +362,7 @@ __device__ __forceinline__ void field_loop(FieldLane& s, LaneCount& c, Acc& acc,
                 const FieldStart st = stash[held - 1u - rank];
                 place(st);
                 count_trajectory(c, s);
-                field_begin<FAST>(s, st, p, G, acc, slc, slt);
+                field_begin<FORM>(s, st, p, G, acc, slc, slt);
                 if (RECORD && !s.alive) record_end<RECORD>(s, item_steps);
             }
             __syncwarp();  // the stash is read before it is written again
@@ -373,12 +373,12 @@ __device__ __forceinline__ void field_loop(FieldLane& s, LaneCount& c, Acc& acc,
         if (live == 0u) break;
         const int keep = held == 0u && drained ? 0 : 32 - (int)refill_min;
         do {
-            if (FAST) {
+            if (FORM) {
                 const bool on = s.alive;
-                field_step<ORDER, FAST, GATED, true>(s, mask, uv, p, k, G, acc, slc, slt);
+                field_step<ORDER, FORM, GATED, true>(s, mask, uv, p, k, G, acc, slc, slt);
                 if (RECORD && on && !s.alive) record_end<RECORD>(s, item_steps);
             } else if (s.alive) {
-                field_step<ORDER, FAST, GATED, false>(s, mask, uv, p, k, G, acc, slc, slt);
+                field_step<ORDER, FORM, GATED, false>(s, mask, uv, p, k, G, acc, slc, slt);
                 if (RECORD && !s.alive) record_end<RECORD>(s, item_steps);
             }
             live = __ballot_sync(FULL, s.alive);
@@ -393,7 +393,7 @@ __device__ __forceinline__ void field_end(FieldLane& s, LaneCount& c, Acc& acc, 
     warp_add_counters(c.steps, c.ntraj, work);
 }
 
-template <int ORDER, bool RECORD, bool FAST>
+template <int ORDER, bool RECORD, int FORM>
 __global__ void __launch_bounds__(256, FIELD_BLOCKS)
 k_fields_persistent(const __grid_constant__ slm_params p, const __grid_constant__ FastGeo f,
                     const __grid_constant__ FastConst k, const float2* __restrict__ seeds, uint32_t seed_begin,
@@ -405,9 +405,9 @@ k_fields_persistent(const __grid_constant__ slm_params p, const __grid_constant_
     FieldLane s{};
     Acc acc{0u, 0u, 0ull};
     LaneCount c{0ull, 0ull};
-    field_loop<ORDER, RECORD, FAST, false>(
+    field_loop<ORDER, RECORD, FORM, false>(
         s, c, acc, G, n_items, refill_min, p, k, mask, uv, slc, slt, work, item_steps,
-        [&](u64 item, FieldStart& st) { return start_of<FAST>(st, item, seed_begin, seeds, order, mask, p, G.g); },
+        [&](u64 item, FieldStart& st) { return start_of<FORM>(st, item, seed_begin, seeds, order, mask, p, G.g); },
         [](const FieldStart&) {});
     field_end(s, c, acc, slc, slt, work);
 }
@@ -420,7 +420,7 @@ k_fields_persistent(const __grid_constant__ slm_params p, const __grid_constant_
 // direction value of the step) and its accumulator offset (0, or up_stride
 // for the upstream slc/slt); every trajectory is the single-direction
 // kernels'.
-template <int ORDER, bool FAST>
+template <int ORDER, int FORM>
 __global__ void __launch_bounds__(256, FIELD_BLOCKS)
 k_fields_pair(const __grid_constant__ slm_params p, const __grid_constant__ FastGeo f,
               const __grid_constant__ FastConst k, float cf_up, const float2* __restrict__ seeds,
@@ -434,12 +434,12 @@ k_fields_pair(const __grid_constant__ slm_params p, const __grid_constant__ Fast
     Acc acc{0u, 0u, 0ull};
     LaneCount c{0ull, 0ull};
     u64 steps_up = 0;
-    field_loop<ORDER, false, FAST, false>(
+    field_loop<ORDER, false, FORM, false>(
         s, c, acc, G, 2 * n_items, refill_min, p, k, mask, uv, slc, slt, work, nullptr,
         [&](u64 item, FieldStart& st) {
             const bool up = item >= n_items;
             st.tag = up;
-            return start_of<FAST>(st, up ? item - n_items : item, seed_begin, seeds, up ? order_up : order, mask, p,
+            return start_of<FORM>(st, up ? item - n_items : item, seed_begin, seeds, up ? order_up : order, mask, p,
                                   G.g);
         },
         [&](const FieldStart& st) {
@@ -475,7 +475,7 @@ __device__ __forceinline__ uint32_t find_tile(const slm_tile* __restrict__ tiles
 // trajectory is computed exactly as a single-grid launch on its tile computes
 // it (RNG stream of the tile-local seed index).  work[3] receives 1 if a seed
 // falls outside its tile's range (an inconsistent table).
-template <int ORDER, bool RECORD, bool FAST>
+template <int ORDER, bool RECORD, int FORM>
 __global__ void __launch_bounds__(256, FIELD_BLOCKS)
 k_fields_batched(const __grid_constant__ slm_params p, const __grid_constant__ FastConst k, const slm_tile* __restrict__ tiles, uint32_t n_tiles,
                  const float2* __restrict__ seeds, u64 n_items, const uint8_t* __restrict__ mask,
@@ -491,7 +491,7 @@ k_fields_batched(const __grid_constant__ slm_params p, const __grid_constant__ F
         return make_geo(__ldg(&T.nx_padded), __ldg(&T.ny_padded), __ldg(&T.combo_factor), __ldg(&T.dt_max),
                         __ldg(&T.grid_scale));
     };
-    field_loop<ORDER, RECORD, FAST, true>(
+    field_loop<ORDER, RECORD, FORM, true>(
         s, c, acc, G, n_items, refill_min, p, k, mask, uv, slc, slt, work, item_steps,
         [&](u64 item, FieldStart& st) {
             uint32_t pos, sub;
@@ -505,14 +505,14 @@ k_fields_batched(const __grid_constant__ slm_params p, const __grid_constant__ F
                 atomicOr(reinterpret_cast<unsigned long long*>(work + 3), 1ull);
                 return false;
             }
-            return start_at<FAST>(st, __ldg(seeds + seed), local, sub, mask, p, tile_geo(T),
+            return start_at<FORM>(st, __ldg(seeds + seed), local, sub, mask, p, tile_geo(T),
                                   (uint32_t)__ldg(&T.grid_offset));
         },
         [&](const FieldStart& st) {
             const slm_tile& T = tiles[st.tag];
             G.g = tile_geo(T);
             G.base = (uint32_t)__ldg(&T.grid_offset);
-            if (FAST) {
+            if (FORM) {
                 G.f = make_fast_geo(G.g.nxp, G.g.nyp, G.g.gs, G.g.dt_max, p.adjusted_max_error, G.base);
                 // a tile the fast step cannot take has no interior pixel
                 if (!fast_grid(G.g.nxp, G.g.nyp, G.base, G.g.cf, G.g.dt_max, p.trajectory_resolution))
@@ -662,10 +662,12 @@ __global__ void k_fields_finish(const u64* __restrict__ acc, uint32_t nxy, uint3
 
 using namespace slm;
 
-// The launch's steps can be evaluated by step_fast (else rk_step, the general form).
-static bool fast_steps(const slm_params& p) {
-    return fast_params(p) &&
-           fast_grid(p.nx_padded, p.ny_padded, 0u, p.combo_factor, p.dt_max, p.trajectory_resolution);
+// The form of a single-grid launch's steps: STEP_GENERAL where the grid is not
+// one for step_fast.
+static StepForm form_of(const slm_params& p) {
+    return fast_grid(p.nx_padded, p.ny_padded, 0u, p.combo_factor, p.dt_max, p.trajectory_resolution)
+               ? jittered_form(p)
+               : STEP_GENERAL;
 }
 
 static FastGeo fast_geo_of(const slm_params& p) {
@@ -702,22 +704,22 @@ static uint32_t refill_min(const slm_launch& L) {
     return L.chunk <= 1 ? 1u : (L.chunk >= 32 ? 32u : (uint32_t)L.chunk);
 }
 
-template <int ORDER, bool RECORD, bool FAST>
+template <int ORDER, bool RECORD, int FORM>
 static int launch_fields(const slm_params* p, const slm_launch& L, int block, const float2* sp,
                          uint32_t begin, u64 n_items, const uint8_t* mask, const float2* u2, u64* slc,
                          u64* slt, u64* work, const uint32_t* order, uint16_t* rec, cudaStream_t s) {
     if (L.schedule == SLM_SCHED_PLAIN) {
         const u64 grid = (n_items + block - 1) / block;
         SLM_REQUIRE(grid < (1ull << 31), "too many trajectories for one launch");
-        k_fields_plain<ORDER, RECORD, FAST><<<(unsigned)grid, block, 0, s>>>(*p, fast_geo_of(*p), make_fast_const(*p), sp, begin, n_items, mask, u2,
+        k_fields_plain<ORDER, RECORD, FORM><<<(unsigned)grid, block, 0, s>>>(*p, fast_geo_of(*p), make_fast_const(*p), sp, begin, n_items, mask, u2,
                                                                             slc, slt, work, order, rec);
         SLM_LAUNCHED("k_fields_plain");
     } else if (L.schedule == SLM_SCHED_PERSISTENT) {
         int per_sm = 0;
-        const int rc = blocks_per_sm(L, (const void*)k_fields_persistent<ORDER, RECORD, FAST>, block, &per_sm);
+        const int rc = blocks_per_sm(L, (const void*)k_fields_persistent<ORDER, RECORD, FORM>, block, &per_sm);
         if (rc) return rc;
         const unsigned grid = (unsigned)(num_sms() * per_sm);
-        k_fields_persistent<ORDER, RECORD, FAST><<<grid, block, 0, s>>>(*p, fast_geo_of(*p), make_fast_const(*p), sp, begin, n_items, mask, u2, slc, slt,
+        k_fields_persistent<ORDER, RECORD, FORM><<<grid, block, 0, s>>>(*p, fast_geo_of(*p), make_fast_const(*p), sp, begin, n_items, mask, u2, slc, slt,
                                                                         work, order, rec, refill_min(L));
         SLM_LAUNCHED("k_fields_persistent");
     } else {
@@ -727,27 +729,31 @@ static int launch_fields(const slm_params* p, const slm_launch& L, int block, co
     return SLM_OK;
 }
 
-template <int ORDER, bool RECORD, bool FAST>
+template <int ORDER, bool RECORD, int FORM>
 static int launch_batched(const slm_params* p, const slm_launch& L, int block, const slm_tile* tiles,
                           uint32_t n_tiles, const float2* sp, u64 n_items, const uint8_t* mask,
                           const float2* u2, u64* slc, u64* slt, u64* work, const uint32_t* order,
                           uint16_t* rec, cudaStream_t s) {
     int per_sm = 0;
-    const int rc = blocks_per_sm(L, (const void*)k_fields_batched<ORDER, RECORD, FAST>, block, &per_sm);
+    const int rc = blocks_per_sm(L, (const void*)k_fields_batched<ORDER, RECORD, FORM>, block, &per_sm);
     if (rc) return rc;
     const unsigned grid = (unsigned)(num_sms() * per_sm);
-    k_fields_batched<ORDER, RECORD, FAST><<<grid, block, 0, s>>>(*p, make_fast_const(*p), tiles, n_tiles, sp, n_items, mask, u2, slc, slt,
+    k_fields_batched<ORDER, RECORD, FORM><<<grid, block, 0, s>>>(*p, make_fast_const(*p), tiles, n_tiles, sp, n_items, mask, u2, slc, slt,
                                                                 work, order, rec, refill_min(L));
     SLM_LAUNCHED("k_fields_batched");
     return SLM_OK;
 }
 
-// f<ORDER, RECORD, FAST>(...) for run-time values of the three
-#define SLM_FIELDS_DISPATCH(f, rk4, record, fast, ...)                                             \
-    ((rk4) ? ((record) ? ((fast) ? f<4, true, true>(__VA_ARGS__) : f<4, true, false>(__VA_ARGS__))    \
-                       : ((fast) ? f<4, false, true>(__VA_ARGS__) : f<4, false, false>(__VA_ARGS__))) \
-           : ((record) ? ((fast) ? f<2, true, true>(__VA_ARGS__) : f<2, true, false>(__VA_ARGS__))    \
-                       : ((fast) ? f<2, false, true>(__VA_ARGS__) : f<2, false, false>(__VA_ARGS__))))
+// f<ORDER, RECORD, FORM>(...) for run-time values of the three
+#define SLM_FORM_DISPATCH(f, order, record, form, ...)                     \
+    ((form) == STEP_JITTERED ? f<order, record, STEP_JITTERED>(__VA_ARGS__) \
+     : (form) == STEP_FAINT  ? f<order, record, STEP_FAINT>(__VA_ARGS__)    \
+                             : f<order, record, STEP_GENERAL>(__VA_ARGS__))
+#define SLM_FIELDS_DISPATCH(f, rk4, record, form, ...)                          \
+    ((rk4) ? ((record) ? SLM_FORM_DISPATCH(f, 4, true, form, __VA_ARGS__)        \
+                       : SLM_FORM_DISPATCH(f, 4, false, form, __VA_ARGS__))      \
+           : ((record) ? SLM_FORM_DISPATCH(f, 2, true, form, __VA_ARGS__)        \
+                       : SLM_FORM_DISPATCH(f, 2, false, form, __VA_ARGS__)))
 
 extern "C" {
 
@@ -789,7 +795,7 @@ int slm_integrate_fields_scheduled(const slm_params* p, const slm_launch* launch
     const float2* sp = reinterpret_cast<const float2*>(seed_point);
     const float2* u2 = reinterpret_cast<const float2*>(uv);
     u64* w = (u64*)workspace;
-    return SLM_FIELDS_DISPATCH(launch_fields, L.integrator == SLM_RK4, item_steps != nullptr, fast_steps(*p), p, L, block,
+    return SLM_FIELDS_DISPATCH(launch_fields, L.integrator == SLM_RK4, item_steps != nullptr, form_of(*p), p, L, block,
                                sp, begin, n_items, mask, u2, (u64*)slc, (u64*)slt, w, seed_order, item_steps, s);
 }
 
@@ -831,9 +837,11 @@ int slm_integrate_fields_pair(const slm_params* p_down, const slm_params* p_up, 
     const u64 n_items = (u64)(p_down->n_seed_points - begin) * dd;
     const float2* sp = reinterpret_cast<const float2*>(seed_point);
     const float2* u2 = reinterpret_cast<const float2*>(uv);
-    const bool rk4 = L.integrator == SLM_RK4, fast = fast_steps(*p_down);
-    const auto kernel = rk4 ? (fast ? k_fields_pair<4, true> : k_fields_pair<4, false>)
-                            : (fast ? k_fields_pair<2, true> : k_fields_pair<2, false>);
+    const bool rk4 = L.integrator == SLM_RK4;
+    const StepForm form = form_of(*p_down);
+    const auto kernel = form == STEP_JITTERED ? (rk4 ? k_fields_pair<4, STEP_JITTERED> : k_fields_pair<2, STEP_JITTERED>)
+                        : form == STEP_FAINT  ? (rk4 ? k_fields_pair<4, STEP_FAINT> : k_fields_pair<2, STEP_FAINT>)
+                                              : (rk4 ? k_fields_pair<4, STEP_GENERAL> : k_fields_pair<2, STEP_GENERAL>);
     int per_sm = 0;
     rc = blocks_per_sm(L, (const void*)kernel, block, &per_sm);
     if (rc) return rc;
@@ -875,7 +883,7 @@ int slm_integrate_fields_batched(const slm_params* p, const slm_launch* launch, 
     const float2* sp = reinterpret_cast<const float2*>(seed_point);
     const float2* u2 = reinterpret_cast<const float2*>(uv);
     u64* w = (u64*)workspace;
-    return SLM_FIELDS_DISPATCH(launch_batched, L.integrator == SLM_RK4, item_steps != nullptr, fast_params(*p), p, L, block,
+    return SLM_FIELDS_DISPATCH(launch_batched, L.integrator == SLM_RK4, item_steps != nullptr, jittered_form(*p), p, L, block,
                                tiles, n_tiles, sp, n_items, mask, u2, (u64*)slc, (u64*)slt, w, seed_order, item_steps, s);
 }
 

@@ -7,8 +7,9 @@
 // four bilinear samples.  Here a step is evaluated without any of them and
 // with one test at its end: the step's values are those of rk_step bit for
 // bit when every guard below holds, and a lane for which one does not hold
-// (a sample next to the grid's edge, a NaN, an overflow, a component below
-// 2^-30, one generator state in 10^9) evaluates the step again with rk_step.
+// (a sample next to the grid's edge, a NaN, an overflow, a jittered component
+// below 2^-30, one generator state in 10^9) evaluates the step again with
+// rk_step.
 //
 // What makes each shortcut exact:
 //
@@ -90,14 +91,33 @@ __device__ __forceinline__ float min3_nan(float a, float b, float c) {
 
 constexpr float FAST_MAGIC = 8388608.0f;           // 2^23
 constexpr uint32_t FAST_MAGIC_BITS = 0x4B000000u;  // its bit pattern
-constexpr float FAST_S_MIN = 0x1p-60f;             // least square of a component
+constexpr float FAST_S_MIN = 0x1p-60f;             // least square of a vector or a jittered component
+constexpr uint32_t FAST_C_BITS = 0x21800000u;      // 2^-60, the least component that is not zero
+constexpr float FAST_JITTER = 0x1p-8f;             // least magnitude of STEP_JITTERED
 
 constexpr uint32_t LEHMER_M = 0xfffffffbu;
+
+// How a launch forms its steps.  A flow component that is exactly 0 is nothing
+// unusual (planes along an axis, and relief in whole metres or centimetres), so
+// no form may leave such steps to step_exact: a plane along an axis, RK4, then
+// took 401 ms where one oblique to the axes took 134 (rk_step for all: 305).
+//
+//   STEP_JITTERED  the components after the jitter are tested: at least 2^-30
+//                  each.  That covers the flow's own: where one is too small
+//                  for an exact quotient (below 2^-103, or its quotient not
+//                  normal), its unit component is below 2^-72, and the
+//                  jittered one, at least 2^-30, is the jitter alone.
+//   STEP_FAINT     a jitter below 2^-8, or none, may leave a component at 0 or
+//                  next to it: components before and after it are tested to be
+//                  0 or at least 2^-60, which takes one instruction and a half
+//                  a stage more (1 % of the time of a launch).
+//   STEP_PLAIN     no jitter and no second normalisation; tested as STEP_FAINT.
+enum StepForm : int { STEP_GENERAL = 0, STEP_JITTERED = 1, STEP_FAINT = 2, STEP_PLAIN = 3 };
 
 // u / |u| as rk_step forms it: |u| = sqrt(x*x + y*y), both components divided
 // by it.  Exact, but for the sign of a zero component (which no later value
 // depends on), when s = x*x + y*y >= 2^-60 is finite and each component is
-// zero or at least 2^-103: the residuals are then exact.
+// zero or at least 2^-60: the residuals are then exact and the quotients normal.
 __device__ __forceinline__ F2 unit_fast(F2 u, float& xx, float& yy, float& s) {
     unpack2(mul2(u, u), xx, yy);
     s = __fadd_rn(xx, yy);
@@ -206,6 +226,11 @@ __host__ __device__ __forceinline__ bool fast_params(const slm_params& p) {
            p.adjusted_max_error >= 0.0f && p.pad_width < (1u << 20);
 }
 
+// The form of a jittered launch whose grids fast_grid admits.
+static inline StepForm jittered_form(const slm_params& p) {
+    return !fast_params(p) ? STEP_GENERAL : fabsf(p.jitter_magnitude) >= FAST_JITTER ? STEP_JITTERED : STEP_FAINT;
+}
+
 // 2^23 + clamped pixel index of a position, per axis (get_array_idx); the
 // clamp written so that NaN gives pixel 0, as axis_index
 __device__ __forceinline__ F2 pixel_magic_clamped(Vec2 a, float pp5, uint32_t nxp, uint32_t nyp) {
@@ -248,28 +273,42 @@ __device__ __forceinline__ uint32_t lehmer_fast(uint32_t s) {
     return y < lo ? y + 5u : y;
 }
 
-// Guards gathered over one step: the least square of a sampled component or
-// sum of squares of a jittered vector (NaN if one is), the largest state.
+// Guards gathered over one step: the least sum of squares of a flow vector or
+// square of a jittered component (NaN if one is), the least pattern of a
+// component less 1 (a zero's wraps to the largest), the largest state.
 struct FastGuard {
     float smallest;
+    uint32_t component;
     uint32_t state;
 };
 
-// The unit flow vector at a stage's point, jittered.
-template <bool JITTER>
-__device__ __forceinline__ F2 stage_fast(F2 a, F2 floor2, uint32_t off, uint32_t& rng, FastGuard& gd, float& sj,
+__device__ __forceinline__ void guard_components(FastGuard& gd, F2 v) {
+    float x, y;
+    unpack2(v, x, y);
+    gd.component = __viaddmin_u32(__float_as_uint(fminf(fabsf(x), fabsf(y))), 0xffffffffu, gd.component);
+}
+
+// The unit flow vector at a stage's point, jittered; s: the flow's sum of squares.
+template <int FORM>
+__device__ __forceinline__ F2 stage_fast(F2 a, F2 floor2, uint32_t off, uint32_t& rng, FastGuard& gd, float& s,
                                          const float2* __restrict__ uv, const FastGeo& f, const FastConst& k) {
-    float xx, yy;
-    F2 u = unit_fast(taps_fast(a, floor2, off, uv, f, k), xx, yy, sj);
-    gd.smallest = min3_nan(gd.smallest, xx, yy);
-    if (JITTER) {
+    float xx, yy, sj;
+    const F2 flow = taps_fast(a, floor2, off, uv, f, k);
+    F2 u = unit_fast(flow, xx, yy, s);
+    if (FORM != STEP_JITTERED) guard_components(gd, flow);
+    if (FORM == STEP_PLAIN) return u;
+    if (FORM == STEP_JITTERED || k.mag.x != 0.0f) {
         const uint32_t r0 = lehmer_fast(rng), r1 = lehmer_fast(r0);
         rng = r1;
         gd.state = max(gd.state, max(r0, r1));
         // r * 2^-32 - 1/2 in one rounding (the product is exact)
         const F2 r = fma2(pack2(__uint2float_rn(r0), __uint2float_rn(r1)), as_f2(k.draw), as_f2(k.draw0));
-        u = unit_fast(add2_product(mul2(r, as_f2(k.mag)), u, k), xx, yy, sj);
+        u = add2_product(mul2(r, as_f2(k.mag)), u, k);
     }
+    if (FORM == STEP_FAINT) guard_components(gd, u);
+    u = unit_fast(u, xx, yy, sj);
+    if (FORM == STEP_JITTERED) gd.smallest = min3_nan(gd.smallest, xx, yy);
+    else gd.smallest = min3_nan(gd.smallest, sj, sj);
     return u;
 }
 
@@ -308,7 +347,7 @@ __device__ __noinline__ FastStep step_exact(Vec2 a, float dt, uint32_t rng, floa
 // with time step dt; true if every guard held and the values are rk_step's.
 // GATED: a lane outside the interior reads nothing (its grid may have none) and
 // stays where it is; else it reads its clamped pixel's taps.
-template <int ORDER, bool JITTER, bool GATED>
+template <int ORDER, int FORM, bool GATED>
 __device__ __forceinline__ bool step_fast(Vec2 a0, F2 t0, uint32_t off0, float dt, float cf, uint32_t rng,
                                           const float2* __restrict__ uv, const FastGeo& f, const FastConst& k,
                                           FastStep& o) {
@@ -328,9 +367,9 @@ __device__ __forceinline__ bool step_fast(Vec2 a0, F2 t0, uint32_t off0, float d
         return false;
     }
     uint32_t off = min(off0, f.off_last);
-    FastGuard gd{FAST_S_MIN, 0u};
-    float s1, s2, s3, s4;  // sums of squares of the stages' last vectors
-    const F2 k1 = stage_fast<JITTER>(a, fl, off, rng, gd, s1, uv, f, k);
+    FastGuard gd{FAST_S_MIN, 0xffffffffu, 0u};
+    float s1, s2, s3, s4;  // sums of squares of the stages' flow vectors
+    const F2 k1 = stage_fast<FORM>(a, fl, off, rng, gd, s1, uv, f, k);
     const F2 h1 = mul2(mul2(k1, cf2), dt2);
     float hx, hy, sx, sy;
     unpack2(h1, hx, hy);
@@ -340,20 +379,20 @@ __device__ __forceinline__ bool step_fast(Vec2 a0, F2 t0, uint32_t off0, float d
         const F2 d1 = pack2(o.d1.x, o.d1.y);
         const F2 b = add2(a, d1);
         locate_fast(b, f, k, fl, off);
-        const F2 k2 = stage_fast<JITTER>(b, fl, off, rng, gd, s2, uv, f, k);
+        const F2 k2 = stage_fast<FORM>(b, fl, off, rng, gd, s2, uv, f, k);
         gd.smallest = min3_nan(gd.smallest, s1, s2);
         unpack2(mul2(as_f2(k.half), add2_product(mul2(mul2(k2, cf2), dt2), d1, k)), sx, sy);
     } else {
         const F2 b = fma2(as_f2(k.half), h1, a);
         locate_fast(b, f, k, fl, off);
-        const F2 h2 = mul2(mul2(stage_fast<JITTER>(b, fl, off, rng, gd, s2, uv, f, k), cf2), dt2);
+        const F2 h2 = mul2(mul2(stage_fast<FORM>(b, fl, off, rng, gd, s2, uv, f, k), cf2), dt2);
         gd.smallest = min3_nan(gd.smallest, s1, s2);
         const F2 c = fma2(as_f2(k.half), h2, a);
         locate_fast(c, f, k, fl, off);
-        const F2 h3 = mul2(mul2(stage_fast<JITTER>(c, fl, off, rng, gd, s3, uv, f, k), cf2), dt2);
+        const F2 h3 = mul2(mul2(stage_fast<FORM>(c, fl, off, rng, gd, s3, uv, f, k), cf2), dt2);
         const F2 d = add2_product(h3, a, k);
         locate_fast(d, f, k, fl, off);
-        const F2 h4 = mul2(mul2(stage_fast<JITTER>(d, fl, off, rng, gd, s4, uv, f, k), cf2), dt2);
+        const F2 h4 = mul2(mul2(stage_fast<FORM>(d, fl, off, rng, gd, s4, uv, f, k), cf2), dt2);
         gd.smallest = min3_nan(gd.smallest, s3, s4);
         const F2 w = add2_product(h4, fma2(as_f2(k.two), h3, fma2(as_f2(k.two), h2, h1)), k);
         // div6 without its range test: below 2^-120 both quantise to 0
@@ -369,7 +408,8 @@ __device__ __forceinline__ bool step_fast(Vec2 a0, F2 t0, uint32_t off0, float d
     unpack2(next, o.next.x, o.next.y);
     unpack2(k1, o.u1.x, o.u1.y);
     bool ok = (gd.smallest >= FAST_S_MIN) & inside;
-    if (JITTER) ok = ok & (gd.state < LEHMER_M);
+    if (FORM != STEP_JITTERED) ok = ok & (gd.component >= FAST_C_BITS - 1u);
+    if (FORM != STEP_PLAIN) ok = ok & (gd.state < LEHMER_M);
     else ok = ok & (fabsf(sx) < 1.0f) & (fabsf(sy) < 1.0f);  // an infinite sum of squares gives NaN here
     return ok;
 }
@@ -434,7 +474,7 @@ __device__ __forceinline__ Step plain_step(Vec2 a, float dt, const float2* __res
     bool ok = false;
     if (w.fast) {
         const F2 t = pixel_magic_clamped(a, p.pad_width_pp5, p.nx_padded, p.ny_padded);
-        ok = step_fast<ORDER, false, false>(a, t, offset_from_magic(t, w.f), dt, p.combo_factor, 0u, uv, w.f, w.k, st);
+        ok = step_fast<ORDER, STEP_PLAIN, false>(a, t, offset_from_magic(t, w.f), dt, p.combo_factor, 0u, uv, w.f, w.k, st);
     }
     if (!ok) st = step_exact<ORDER, false>(a, dt, 0u, p.combo_factor, uv, 0u, p, p.nx_padded, p.ny_padded);
     return Step{st.d1, st.d2, st.u1, st.next, st.idx};
