@@ -48,6 +48,15 @@ DENSE_SEEDS = 16384
 DENSE_PIXELS_PER_SEED = 6
 
 
+def grid_form(n, nxp, nyp):
+    """Whether predictions of n seeds are formed once per pixel: enough seeds,
+    and a grid within slm_cnn_infer_grid's limits (a side below 2^24 pixels,
+    fewer than 2^32 in all); slm_cnn_infer takes any other."""
+    pixels = nxp * nyp
+    return (nxp < 1 << 24 and nyp < 1 << 24 and pixels < 1 << 32
+            and n >= DENSE_SEEDS and n * DENSE_PIXELS_PER_SEED >= pixels)
+
+
 def _stream(stream=None):
     s = stream if stream is not None else torch.cuda.current_stream()
     return ctypes.c_void_p(s.cuda_stream)
@@ -242,7 +251,7 @@ class LengthModel:
             out = torch.empty((n, 2), dtype=torch.float32, device=self.device)
         args = (ptr(uv), int(nxp), int(nyp), int(pad), ptr(seeds), ptr(visit), int(n),
                 ptr(W["w1"]), ptr(W["b1"]), ptr(W["w2"]), ptr(W["b2"]), ptr(W["w3"]), ptr(W["b3"]), ptr(out))
-        if n >= DENSE_SEEDS and n * DENSE_PIXELS_PER_SEED >= int(nxp) * int(nyp):
+        if grid_form(int(n), int(nxp), int(nyp)):
             need = int(self.L.slm_cnn_infer_grid_workspace(int(nxp), int(nyp)))
             ws = torch.empty(need, dtype=torch.uint8, device=self.device)
             if stream is not None:

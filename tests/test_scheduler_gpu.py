@@ -410,3 +410,24 @@ def test_spatial_order_parts_of_blocks(block, nx, ny, n):
     if 8 < block <= 64:
         held = np.bincount(key)[key] <= 4096
         assert np.all(np.diff((key * 64 + x % block // 8 * 8 + y % block // 8)[held]) >= 0)
+
+
+def test_predict_on_a_grid_too_long_for_the_grid_form():
+    """A side of 2^24 pixels is beyond the grid form's limits: however many seeds
+    ask, predict gives what the per-seed kernel gives."""
+    import ctypes
+
+    from slm_b200 import _lib
+    nxp, n = 1 << 24, 3 << 20
+    g = torch.Generator(device=DEV).manual_seed(8)
+    uv = torch.randn((nxp, 1, 2), generator=g, device=DEV)
+    seeds = torch.zeros((n, 2), device=DEV)
+    seeds[:, 0] = torch.randint(0, nxp, (n,), generator=g, device=DEV)
+    m = S.LengthModel(DEV, _weights(4))
+    got = m.predict(uv, nxp, 1, 0, seeds, n)
+    ref = torch.full((n, 2), float("nan"), device=DEV)
+    P, W = _lib.ptr, m.W
+    _lib.check(m.L.slm_cnn_infer(P(uv), nxp, 1, 0, P(seeds), None, n, P(W["w1"]), P(W["b1"]), P(W["w2"]), P(W["b2"]),
+                                 P(W["w3"]), P(W["b3"]), P(ref),
+                                 ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    assert torch.equal(got, ref)
