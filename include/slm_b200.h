@@ -523,8 +523,9 @@ int slm_cnn_infer(const float* uv, uint32_t nx_padded, uint32_t ny_padded, uint3
  * slm_cnn_infer_grid_workspace bytes; a seed's patch depends only on its
  * pixel) and then picked for the seeds; seeds whose pixel is off the grid go
  * through slm_cnn_infer's kernel.  Equal to slm_cnn_infer but for the order
- * of the last layer's fp32 sums.  Cheaper from about one seed in eight
- * pixels on.  Each side below 2^24 pixels, fewer than 2^32 in all. */
+ * of the last layer's fp32 sums.  Cheaper from about one seed in sixteen
+ * pixels on (one in ten on grids of 512 x 512, one in two on 128 x 128).  Each
+ * side below 2^24 pixels, fewer than 2^32 in all. */
 size_t slm_cnn_infer_grid_workspace(uint32_t nx_padded, uint32_t ny_padded);
 int slm_cnn_infer_grid(const float* uv, uint32_t nx_padded, uint32_t ny_padded, uint32_t pad,
                        const float* seed_point, const uint32_t* index, uint32_t n,

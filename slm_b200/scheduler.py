@@ -40,12 +40,15 @@ SHAPES = (("w1", (32, 32)), ("b1", (32,)), ("w2", (128, 64)), ("b2", (64,)),
 N_PARAMS = sum(int(np.prod(s)) for _, s in SHAPES)
 N_BINS = 1024
 # Predictions of n seeds are formed once per pixel (slm_cnn_infer_grid) from
-# DENSE_SEEDS seeds on, when the grid has at most DENSE_PIXELS_PER_SEED pixels
-# for each: a B200 takes 0.29 ms for the 3.1 M pixels of a 1500 x 2048 grid
-# however many seeds ask, the per-seed kernel 1.1 ns a seed and 0.04 ms at least
-# (3.49 ms for every pixel, 0.54 ms for one in 8, 0.31 ms for one in 16).
-DENSE_SEEDS = 16384
-DENSE_PIXELS_PER_SEED = 6
+# DENSE_SEEDS seeds and one in DENSE_PIXELS_PER_SEED pixels on.  On a B200 that
+# form takes 0.08 ns a pixel and 0.04 ms, however many seeds ask; the per-seed
+# kernel 1.1 to 1.3 ns a seed and 0.04 ms at least.  Measured, one in so many
+# pixels (grid / per seed, ms): 3000 x 4096 16: 0.97 / 1.02, 20: 0.97 / 0.83;
+# 1500 x 2048 16: 0.28 / 0.31, 20: 0.28 / 0.26; 512 x 512 10: 0.069 / 0.070,
+# 12: 0.069 / 0.068; 300 x 400 6: 0.060 / 0.069, 8: 0.060 / 0.056; 128 x 128 1:
+# 0.048 / 0.055, 2: 0.047 / 0.042.
+DENSE_SEEDS = 8192
+DENSE_PIXELS_PER_SEED = 16
 
 
 def grid_form(n, nxp, nyp):
@@ -54,7 +57,7 @@ def grid_form(n, nxp, nyp):
     fewer than 2^32 in all); slm_cnn_infer takes any other."""
     pixels = nxp * nyp
     return (nxp < 1 << 24 and nyp < 1 << 24 and pixels < 1 << 32
-            and n >= DENSE_SEEDS and n * DENSE_PIXELS_PER_SEED >= pixels)
+            and n >= DENSE_SEEDS + pixels // DENSE_PIXELS_PER_SEED)
 
 
 def _stream(stream=None):

@@ -431,3 +431,11 @@ def test_predict_on_a_grid_too_long_for_the_grid_form():
                                  P(W["w3"]), P(W["b3"]), P(ref),
                                  ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
     assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("n,nxp,nyp,want", [
+    (8192, 1, 1, True), (8191, 1, 1, False), (8192 + 65536, 1024, 1024, True), (8191 + 65536, 1024, 1024, False),
+    (1 << 28, (1 << 24) - 1, 100, True), (1 << 28, 1 << 24, 100, False), (1 << 28, 100, 1 << 24, False),
+    (1 << 31, 1 << 16, 1 << 16, False), (1 << 31, 1 << 16, (1 << 16) - 1, True)])
+def test_rule_of_the_grid_form(n, nxp, nyp, want):
+    assert S.grid_form(n, nxp, nyp) is want
