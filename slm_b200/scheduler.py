@@ -254,9 +254,14 @@ class LengthModel:
             out = torch.empty((n, 2), dtype=torch.float32, device=self.device)
         args = (ptr(uv), int(nxp), int(nyp), int(pad), ptr(seeds), ptr(visit), int(n),
                 ptr(W["w1"]), ptr(W["b1"]), ptr(W["w2"]), ptr(W["b2"]), ptr(W["w3"]), ptr(W["b3"]), ptr(out))
+        ws = None
         if grid_form(int(n), int(nxp), int(nyp)):
             need = int(self.L.slm_cnn_infer_grid_workspace(int(nxp), int(nyp)))
-            ws = torch.empty(need, dtype=torch.uint8, device=self.device)
+            try:
+                ws = torch.empty(need, dtype=torch.uint8, device=self.device)
+            except torch.cuda.OutOfMemoryError:
+                pass  # 8 bytes a pixel; the per-seed kernel needs none
+        if ws is not None:
             if stream is not None:
                 ws.record_stream(stream)
             check(self.L.slm_cnn_infer_grid(*args, ptr(ws), need, _stream(stream)))

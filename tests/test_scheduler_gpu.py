@@ -439,3 +439,30 @@ def test_predict_on_a_grid_too_long_for_the_grid_form():
     (1 << 31, 1 << 16, 1 << 16, False), (1 << 31, 1 << 16, (1 << 16) - 1, True)])
 def test_rule_of_the_grid_form(n, nxp, nyp, want):
     assert S.grid_form(n, nxp, nyp) is want
+
+
+def test_predict_without_memory_for_the_grid_form(monkeypatch):
+    """Where the grid form's workspace cannot be had, predict takes the per-seed
+    kernel, which needs none."""
+    nxp, nyp = 150, 130
+    n = nxp * nyp
+    g = torch.Generator(device=DEV).manual_seed(9)
+    uv = torch.randn((nxp, nyp, 2), generator=g, device=DEV)
+    p = torch.arange(n, device=DEV)
+    seeds = torch.stack((p // nyp, p % nyp), 1).to(torch.float32).contiguous()
+    m = S.LengthModel(DEV, _weights(4))
+    assert n >= 8192 + n // 16
+    want = m.predict(uv, nxp, nyp, 0, seeds, n)
+    need, empty = int(m.L.slm_cnn_infer_grid_workspace(nxp, nyp)), torch.empty
+    refused = []
+
+    def short_of_memory(*args, **kw):
+        if args and args[0] == need:
+            refused.append(need)
+            raise torch.cuda.OutOfMemoryError("out of memory")
+        return empty(*args, **kw)
+
+    monkeypatch.setattr(torch, "empty", short_of_memory)
+    got = m.predict(uv, nxp, nyp, 0, seeds, n)
+    assert refused
+    assert torch.allclose(got, want, rtol=1e-4, atol=1e-4)
