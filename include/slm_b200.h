@@ -522,8 +522,7 @@ int slm_cnn_infer(const float* uv, uint32_t nx_padded, uint32_t ny_padded, uint3
  * the padded grid into workspace (device, 8-byte aligned,
  * slm_cnn_infer_grid_workspace bytes; a seed's patch depends only on its
  * pixel) and then picked for the seeds; seeds whose pixel is off the grid go
- * through slm_cnn_infer's kernel.  Equal to slm_cnn_infer but for the order
- * of the last layer's fp32 sums.  Cheaper from about one seed in sixteen
+ * through slm_cnn_infer's kernel.  Bit for bit slm_cnn_infer's.  Cheaper from about one seed in sixteen
  * pixels on (one in ten on grids of 512 x 512, one in two on 128 x 128).  Each
  * side below 2^24 pixels, fewer than 2^32 in all. */
 size_t slm_cnn_infer_grid_workspace(uint32_t nx_padded, uint32_t ny_padded);

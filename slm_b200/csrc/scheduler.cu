@@ -301,8 +301,10 @@ k_cnn_infer(const float2* __restrict__ uv, uint32_t nxp, uint32_t nyp, uint32_t 
             }
             __syncwarp();
         }
-        // dense: M = 16 seeds, K = 256, N = 8 (2 used)
-        float c3[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        // dense: M = 16 seeds, K = 256, N = 8 (2 used); the four positions' 64
+        // products are summed apart and then added, as k_cnn_grid has them, so
+        // a seed's prediction does not depend on which of the two forms it
+        float c3[4][4] = {};
 #pragma unroll
         for (int ks = 0; ks < 16; ++ks) {
             uint32_t a[4];
@@ -310,22 +312,25 @@ k_cnn_infer(const float2* __restrict__ uv, uint32_t nxp, uint32_t nyp, uint32_t 
             a[1] = S.x3[warp][gid + 8][ks * 8 + tig];
             a[2] = S.x3[warp][gid][ks * 8 + tig + 4];
             a[3] = S.x3[warp][gid + 8][ks * 8 + tig + 4];
-            mma_bf16(c3, a, S.w3[gid][ks * 8 + tig], S.w3[gid][ks * 8 + tig + 4]);
+            mma_bf16(c3[ks >> 2], a, S.w3[gid][ks * 8 + tig], S.w3[gid][ks * 8 + tig + 4]);
         }
+        float y[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) y[r] = (((c3[0][r] + c3[1][r]) + c3[2][r]) + c3[3][r]) + S.b3[r & 1];
         if (tig == 0) {
             const uint32_t s0 = grp * 16 + gid, s1 = s0 + 8;
             if (s0 < n) {
                 const size_t o = index ? __ldg(index + s0) : s0;
                 if (!outside || off_grid(seeds[o], nxp, nyp, pad)) {
-                    out[2 * o] = c3[0] + S.b3[0];
-                    out[2 * o + 1] = c3[1] + S.b3[1];
+                    out[2 * o] = y[0];
+                    out[2 * o + 1] = y[1];
                 }
             }
             if (s1 < n) {
                 const size_t o = index ? __ldg(index + s1) : s1;
                 if (!outside || off_grid(seeds[o], nxp, nyp, pad)) {
-                    out[2 * o] = c3[2] + S.b3[0];
-                    out[2 * o + 1] = c3[3] + S.b3[1];
+                    out[2 * o] = y[2];
+                    out[2 * o + 1] = y[3];
                 }
             }
         }
@@ -344,8 +349,8 @@ k_cnn_infer(const float2* __restrict__ uv, uint32_t nxp, uint32_t nyp, uint32_t 
 //   out(P) = b3 + sum over u of W3_u A2(P - 8 + 8(ui, uj))
 //
 // 9.8 k products per pixel against 50 k per seed, and no patch gathers (2 KB
-// per seed).  The products, their order and the roundings are k_cnn_infer's up
-// to the dense layer, whose four positions are summed apart and then added.
+// per seed).  The products, their order and the roundings are k_cnn_infer's,
+// whose dense layer sums the four positions apart as well: same bits.
 //
 // A block walks down a strip of GRID_OUT columns, GRID_ROWS rows at a time.
 // A1 and the dense layer's partial sums D stay in rings of rows in shared

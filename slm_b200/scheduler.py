@@ -248,7 +248,8 @@ class LengthModel:
     def predict(self, uv, nxp, nyp, pad, seeds, n, out=None, visit=None, stream=None):
         """Fused tensor-core inference: predictions [n][2] (down, up).
         ``visit`` (uint32 [n], optional): the order the seeds are processed
-        in, e.g. ``spatial_order(...)``, for cache locality of the patches."""
+        in, e.g. ``spatial_order(...)``, for cache locality of the patches.
+        A seed's prediction is the same bits however many are asked for."""
         W = self.W
         if out is None:
             out = torch.empty((n, 2), dtype=torch.float32, device=self.device)

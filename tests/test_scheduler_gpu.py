@@ -466,3 +466,19 @@ def test_predict_without_memory_for_the_grid_form(monkeypatch):
     got = m.predict(uv, nxp, nyp, 0, seeds, n)
     assert refused
     assert torch.allclose(got, want, rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.parametrize("nxp,nyp,pad", [(130, 131, 2), (97, 203, 0)])
+def test_predictions_do_not_depend_on_how_many_are_asked_for(nxp, nyp, pad):
+    """The whole grid (formed once per pixel) and a few of its seeds (formed per
+    seed) give the same bits."""
+    n = nxp * nyp
+    g = torch.Generator(device=DEV).manual_seed(n)
+    uv = torch.randn((nxp, nyp, 2), generator=g, device=DEV)
+    p = torch.randperm(n, generator=g, device=DEV)
+    seeds = (torch.stack((p // nyp, p % nyp), 1) - pad).to(torch.float32).contiguous()
+    m = S.LengthModel(DEV, _weights(6))
+    few = seeds[:1237].contiguous()
+    assert n >= 16384  # the grid form is taken
+    whole = m.predict(uv, nxp, nyp, pad, seeds, n)
+    assert torch.equal(m.predict(uv, nxp, nyp, pad, few, 1237), whole[:1237])
