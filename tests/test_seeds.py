@@ -117,3 +117,42 @@ def test_reservation_rounds_equal_sequential_swaps(n, seed):
             perm[i], perm[j] = perm[j], perm[i]
         assert np.array_equal(got, rows[perm])
     assert rounds <= max(4, 8 * int(np.log2(max(n, 2))))
+
+
+def _rows_by_links(js):
+    """The device list's permutation restated: with next(r) the least i > r with
+    js[i] = js[r] and first(p) the least i > p with js[i] = p, row r ends with
+    the initial row js[r] if there is no next(r), else with next(r) followed
+    through first() to its end."""
+    n = js.shape[0]
+    chain, first = {}, np.full(n, n, np.int64)
+    for i in range(1, n):  # (the chains' order does not matter)
+        chain.setdefault(int(js[i]), []).append(i)
+        if js[i] != i:
+            first[js[i]] = min(first[js[i]], i)
+    out = np.empty(n, np.int64)
+    for r in range(n):
+        j = int(js[r]) if r else 0
+        later = [i for i in chain.get(j, ()) if i > r]
+        q, i = j, min(later) if later else n
+        while i < n:
+            q, i = i, int(first[i])
+        out[r] = q
+    return out
+
+
+@pytest.mark.parametrize("kind", ["drawn", "own row", "first row", "row before", "few targets"])
+@pytest.mark.parametrize("n", [1, 2, 3, 17, 1000, 20_000])
+def test_rows_by_links_equal_sequential_swaps(n, kind):
+    """Row by row, the links give the sequential shuffle's rows for any partners
+    j(i) in [0, i]: drawn ones, and ones that share targets as much as can be."""
+    if n > 1000 and kind in ("first row", "few targets"):
+        n = 2000  # (chains of n links: quadratic)
+    i = np.arange(n, dtype=np.int64)
+    rng = np.random.default_rng(n)
+    js = {"drawn": np.floor(rng.random(n) * (i + 1)).astype(np.int64), "own row": i.copy(), "first row": 0 * i,
+          "row before": np.maximum(i - 1, 0), "few targets": np.minimum(i, rng.integers(0, 3, n))}[kind]
+    perm = np.arange(n)
+    for k in range(n - 1, 0, -1):
+        perm[k], perm[js[k]] = perm[js[k]], perm[k]
+    assert np.array_equal(_rows_by_links(js), perm)
