@@ -221,6 +221,13 @@ int slm_selftest_div6(uint64_t* counts, void* stream);
  * bit pattern + 1 (0: none).  Asynchronous. */
 int slm_selftest_unit(uint64_t* counts, void* stream);
 
+/* slm_selftest_packed -- no counterpart in the reference: checks on the device
+ * that the fast step's packed product and sum round twice, as the scalar
+ * operations do, over 2^24 pairs of triples.  counts: DEVICE [2] uint64: pairs
+ * that differ, and pairs whose fused result would (so that the inputs can tell
+ * the two).  Asynchronous. */
+int slm_selftest_packed(uint64_t* counts, void* stream);
+
 /* slm_selftest_cvt_i8 -- no counterpart in the reference: checks on the
  * device, over all 2^32 float bit patterns, that the tracer's float -> char
  * conversion (one range test around the device's saturating conversion)

@@ -1059,6 +1059,42 @@ __global__ void k_selftest_unit(u64* counts) {
     }
 }
 
+// a float in [1/2, 8) of either sign from a hash of x
+__device__ __forceinline__ float hashed_float(uint32_t x) {
+    x = (x ^ (x >> 16)) * 0x7feb352du;
+    x = (x ^ (x >> 15)) * 0x846ca68bu;
+    x ^= x >> 16;
+    return __uint_as_float((x & 0x807fffffu) | (((x >> 23 & 3u) + 126u) << 23));
+}
+
+// counts[0] += pairs of a * b + c for which the packed product and sum are not
+// the scalar ones, counts[1] += pairs for which a fused operation is not
+__global__ void k_selftest_packed(const __grid_constant__ FastConst k, u64* counts) {
+    const uint32_t i = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
+    const float a = hashed_float(i), b = hashed_float(i + 1u), c = hashed_float(i + 2u), d = hashed_float(i + 3u);
+    const float x = __fadd_rn(__fmul_rn(a, b), c), y = __fadd_rn(__fmul_rn(d, b), a);
+    float px, py;
+    unpack2(add2_product(mul2(pack2(a, d), pack2(b, b)), pack2(c, a), k), px, py);
+    const unsigned bad = __ballot_sync(0xffffffffu, px != x || py != y);
+    const unsigned fused = __ballot_sync(0xffffffffu, __fmaf_rn(a, b, c) != x || __fmaf_rn(d, b, a) != y);
+    if ((threadIdx.x & 31u) == 0u) {
+        if (bad) atomicAdd(counts, (u64)__popc(bad));
+        if (fused) atomicAdd(counts + 1, (u64)__popc(fused));
+    }
+}
+
+extern "C" int slm_selftest_packed(uint64_t* counts, void* stream) {
+    clear_error();
+    SLM_REQUIRE(counts && aligned(counts, 8), "counts must be two 8-byte aligned device words");
+    cudaStream_t s = (cudaStream_t)stream;
+    SLM_CUDA(cudaMemsetAsync(counts, 0, 2 * sizeof(uint64_t), s));
+    slm_params p{};
+    p.trajectory_resolution = 128;
+    k_selftest_packed<<<1u << 16, 256, 0, s>>>(make_fast_const(p), (u64*)counts);
+    SLM_LAUNCHED("k_selftest_packed");
+    return SLM_OK;
+}
+
 extern "C" int slm_selftest_unit(uint64_t* counts, void* stream) {
     clear_error();
     SLM_REQUIRE(counts && aligned(counts, 8), "counts must be two 8-byte aligned device words");

@@ -1,10 +1,9 @@
 // trace_fast.cuh -- the RK step of trace_common.cuh as straight-line code.
 //
 // The tracers are bound by instruction issue, not by memory: the plain form
-// of a jittered RK4 step (rk_step) is 815 thread instructions, most of them
-// the 17 IEEE divisions and 10 square roots, each with a range check, a branch
-// around its slow path and a convergence barrier, and the index clamps of the
-// four bilinear samples.  Here a step is evaluated without any of them and
+// of a jittered RK4 step (rk_step), with its 17 IEEE divisions, 10 square roots
+// and the index clamps of the four bilinear samples, executes 815 thread
+// instructions (ncu).  Here a step is evaluated without any of them and
 // with one test at its end: the step's values are those of rk_step bit for
 // bit when every guard below holds, and a lane for which one does not hold
 // (a sample next to the grid's edge, a NaN, an overflow, a jittered component
@@ -199,10 +198,10 @@ static inline FastConst make_fast_const(const slm_params& p) {
 
 __device__ __forceinline__ F2 as_f2(const float2& v) { return pack2(v.x, v.y); }
 
-// a + m where m is a product of its own rounding: the assembler joins a packed
-// product and the packed sum that follows into one fused operation whatever
-// its contraction flag says, so the sum is written as m * 1 + a with a 1 it
-// cannot see (exact, and one instruction as well).
+// a + m where m is a product of its own rounding.  With add2(mul2(..), a) here
+// (contraction is switched off) 8.6 M of the 16.8 M pairs of slm_selftest_packed
+// come out as a fused operation's, and the oracle's sums are missed; as m * 1 + a
+// with a 1 that is a kernel argument every pair is rounded twice.
 __device__ __forceinline__ F2 add2_product(F2 m, F2 a, const FastConst& k) { return fma2(m, as_f2(k.one), a); }
 
 // Whether a grid's steps can be evaluated by step_fast: quantised steps below

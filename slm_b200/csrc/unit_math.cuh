@@ -1,6 +1,6 @@
 // unit_math.cuh -- correctly rounded square roots, reciprocals and quotients of
-// vector lengths from one reciprocal square root estimate, without the range
-// checks and slow-path branches of the IEEE operations.
+// vector lengths from one reciprocal square root estimate, without a test or a
+// branch (the callers' guards keep the operands in range).
 //
 // The method is P. Markstein's ("Computation of elementary functions on the
 // IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990): an estimate

@@ -430,3 +430,15 @@ def test_flow_along_an_axis_costs_no_more_a_step(jitter, integrator):
             ms = _ms(lambda: kernels.integrate_fields(prm, seeds, mask, uv, slc, slt, work, integrator=integrator))
             per_step.append(ms / int(work[1].item()))
     assert max(per_step[:2]) < 1.6 * per_step[2], per_step
+
+
+def test_packed_product_and_sum_round_twice():
+    import ctypes
+
+    from slm_b200 import _lib
+    counts = torch.zeros(2, dtype=torch.uint64, device=DEV)
+    _lib.check(_lib.load().slm_selftest_packed(_lib.ptr(counts),
+                                               ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    bad, fused = (int(v) for v in counts.view(torch.int64).cpu().tolist())
+    assert bad == 0 and fused > 1 << 20
