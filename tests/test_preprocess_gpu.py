@@ -205,3 +205,37 @@ def test_preprocess_without_the_optional_outputs():
                                           ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
     torch.cuda.synchronize()
     assert torch.equal(uv, full.uv_array)
+
+
+@pytest.mark.parametrize("pad,normalize", [(2, True), (0, False)])
+def test_preprocess_of_level_ground(pad, normalize):
+    """Level everywhere, level on one side, and steps of whole metres."""
+    rolling = _roi(90, 75, 34)
+    for roi in (np.full((60, 70), 5.0, np.float32), np.where(np.arange(75) < 30, rolling, np.float32(90.0)),
+                np.round(rolling), np.round(rolling).astype(np.float64)):
+        o = D.conditioned_uv(roi, 2.0, pad, do_normalize_speed=normalize)
+        r = _gpu(roi, 2.0, pad, normalize)
+        for k in EXACT:
+            assert _same(getattr(r, k), o[k]), k
+        _slope_close(r.slope_array, o["slope_array"])
+
+
+def test_preprocess_of_level_ground_costs_no_more():
+    """A pixel without gradient does not go through the double path: level ground
+    takes what relief takes (measured 0.9; 1.4 with the double path)."""
+    import torch
+    rolling = torch.from_numpy(_roi(1500, 1400, 35, noise=0.05)).cuda()
+
+    def ms(roi):
+        times = []
+        for _ in range(12):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            for _ in range(8):
+                _gpu(roi, 1.0, 2, download=False)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return sorted(times[2:])[5]
+
+    assert ms(torch.full_like(rolling, 3.0)) < 1.25 * ms(rolling)
