@@ -283,13 +283,18 @@ int slm_histogram_univariate(const slm_params* p, const float* sl, uint32_t n_da
     if (rc) return rc;
     if (n_data == 0) return SLM_OK;
     SLM_REQUIRE(sl && hist, "NULL buffer");
-    // Counted in shared memory where the bins fit and a block's values are at
-    // least four a bin (below that, adding the bins up costs more than the
-    // atomics it saves); as many blocks as that leaves, two an SM at most.
-    const uint32_t by_values = n_data / std::max(4u * p->n_hist_bins, 4096u);
+    // Counting in memory takes n / bins (the queue of atomics at a popular bin),
+    // counting in shared memory a block's values, four a bin, and its bins at the
+    // end: bins.  The lines cross at n ~ bins^2 / 180, and not below 16384 values,
+    // where both are a few us.  Measured, us (memory / shared): 64 bins, 9000
+    // values 2.9 / 3.7, 20000 5.1 / 3.9; 2048 bins, 40000 5.3 / 6.1, 60000 7.9 /
+    // 5.6; 4096 bins, 100000 7.7 / 8.7, 200000 14.5 / 8.6; 8192 bins, 200000 7.9 /
+    // 15.5, 400000 15.6 / 15.5; 12288 bins, 60000 2.8 / 25.7, 1 M 27.2 / 22.0.
+    // As many blocks as four values a bin leave, two an SM at most.
+    const uint64_t bins = p->n_hist_bins;
     const uint32_t wide = (uint32_t)num_sms() * 2u;
-    if (by_values >= 1 && p->n_hist_bins <= 12288u) {
-        const unsigned grid = std::min(by_values, wide);
+    if (bins <= 12288u && n_data >= 16384u + bins * bins / 180u) {
+        const unsigned grid = std::min(n_data / std::max(4u * p->n_hist_bins, 4096u), wide);
         k_histogram_univariate<true><<<grid, HIST_BLOCK, p->n_hist_bins * sizeof(uint32_t), (cudaStream_t)stream>>>(
             *p, sl, n_data, hist);
     } else {
