@@ -298,7 +298,7 @@ int slm_histogram_univariate(const slm_params* p, const float* sl, uint32_t n_da
         k_histogram_univariate<true><<<grid, HIST_BLOCK, p->n_hist_bins * sizeof(uint32_t), (cudaStream_t)stream>>>(
             *p, sl, n_data, hist);
     } else {
-        const unsigned grid = std::min((n_data + HIST_BLOCK - 1) / HIST_BLOCK, wide * 8u);
+        const unsigned grid = std::min((n_data - 1u) / HIST_BLOCK + 1u, wide * 8u);
         k_histogram_univariate<false><<<grid, HIST_BLOCK, 0, (cudaStream_t)stream>>>(*p, sl, n_data, hist);
     }
     SLM_LAUNCHED("k_histogram_univariate");

@@ -196,3 +196,21 @@ def test_univariate_histogram_of_few_values_in_many_bins():
         return sorted(times)[4]
 
     assert us(12288) < 3.0 * us(16384)
+
+
+def test_univariate_histogram_of_as_many_values_as_a_count_holds():
+    """2^32 - 400 values: a chunk sixteen times over, but for its last 400."""
+    nb, chunk, cut = 16384, 1 << 28, 400
+    d, _ = univariate("gaussian", n_hist_bins=nb, n_pdf_points=64, n=20000, bandwidth=6.0)
+    prm = kde.kde_params(d, "pdf_univariate")
+    lo, span = float(d.logx_min), float(d.logx_range)
+    data = torch.empty(16 * chunk, dtype=torch.float32, device="cuda")
+    data[:chunk].uniform_(lo, lo + span, generator=torch.Generator(device="cuda").manual_seed(3))
+    for k in range(1, 16):
+        data[k * chunk:(k + 1) * chunk] = data[:chunk]
+    hist = [torch.zeros(nb, dtype=torch.uint32, device="cuda") for _ in range(3)]
+    for h, part in zip(hist, (data[:chunk], data[chunk - cut:chunk], data[:16 * chunk - cut])):
+        kernels.histogram_univariate(prm, part, h)
+    one, last, whole = (h.cpu().numpy().astype(np.int64) for h in hist)
+    assert one.sum() == chunk and last.sum() == cut
+    assert np.array_equal(whole, 16 * one - last)
