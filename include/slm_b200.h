@@ -549,7 +549,7 @@ int slm_order_by_prediction(const float* pred, uint32_t stride, uint32_t col, ui
  * same time share uv / mask / slc / slt cache lines.  With pred (NULL: none),
  * the seeds whose pred[i*stride+col] >= threshold come first, each class in
  * spatial order.  Blocks of 9 to 64 pixels a side that hold at most 4096 seeds
- * go by 8 x 8 pixel parts inside.  bins: scratch of slm_order_spatial_bins(...) uint32. */
+ * go by 8 x 8 pixel parts inside (from one seed in 256 pixels on).  bins: scratch of slm_order_spatial_bins(...) uint32. */
 uint32_t slm_order_spatial_bins(uint32_t nx, uint32_t ny, uint32_t block_px, int with_prediction);
 int slm_order_spatial(const float* seed_point, uint32_t n, uint32_t nx, uint32_t ny,
                       uint32_t block_px, const float* pred, uint32_t stride, uint32_t col,

@@ -679,7 +679,13 @@ __global__ void k_key_scatter(K key, uint32_t n, uint32_t nb, uint32_t* __restri
 // to 3 %.  16 pixel parts gain two thirds of that, 4 pixel parts the same; the
 // parts as bins of the counting sort itself leave its shared counts (3.1e6 seeds:
 // 49, here 37 us more).
-constexpr uint32_t PART_PX = 8, PART_MAX_BLOCK = 64;
+//
+// Seeds sparser than one in PART_SPARSE pixels share no lines whatever their
+// order.  4096^2 fan, RK4, order and trace in ms without / with parts: one seed
+// in 64 pixels 0.027 + 8.84 / 0.044 + 8.00, in 256 0.018 + 4.70 / 0.035 + 4.65,
+// in 1024 0.016 + 4.15 / 0.032 + 4.13; incised relief, RK2: in 64 0.015 + 3.76 /
+// 0.020 + 3.64, in 256 0.013 + 3.52 / 0.019 + 3.56.
+constexpr uint32_t PART_PX = 8, PART_MAX_BLOCK = 64, PART_SPARSE = 256;
 constexpr uint32_t PART_PER = 16, PART_SEEDS = 256 * PART_PER;  // seeds a block of threads holds
 __global__ void __launch_bounds__(256) k_part_order(SpatialKey key, const uint32_t* __restrict__ ends,
                                                     uint32_t* __restrict__ order) {
@@ -912,6 +918,7 @@ int slm_order_spatial(const float* seed_point, uint32_t n, uint32_t nx, uint32_t
                    stride, col, threshold};
     const int rc = counting_order(key, n, nb, bins, order, (cudaStream_t)stream);
     if (rc || block_px <= PART_PX || block_px > PART_MAX_BLOCK || nb > 0x7fffffffu) return rc;
+    if ((uint64_t)n * PART_SPARSE < (uint64_t)nx * ny) return rc;
     k_part_order<<<nb, 256, 0, (cudaStream_t)stream>>>(key, bins, order);  // (the scatter left the bins' ends)
     SLM_LAUNCHED("k_part_order");
     return SLM_OK;

@@ -290,7 +290,8 @@ def spatial_order(seeds, n, nx, ny, block=SPATIAL_BLOCK, pred=None, col=0, thres
                   bins=None, stream=None):
     """Seed order by ``block`` x ``block`` pixel block of the nx x ny grid
     (uint32 [n]); with ``pred`` [n][2], seeds predicted >= ``threshold`` first.
-    Blocks of up to 64 pixels go by 8 x 8 pixel parts inside.
+    Blocks of up to 64 pixels go by 8 x 8 pixel parts inside, where at least
+    one pixel in 256 has a seed.
 
     Trajectories traced together then share cache lines of uv / mask /
     slc / slt: on grids larger than L2 this is what keeps the tracer
