@@ -120,7 +120,7 @@ k_bias_grad(const float* __restrict__ dz, size_t rows, int cols, uint32_t width,
             const float* p = cluster.map_shared_rank(&part[0][0], b);
             for (uint32_t w = 0; w < BIAS_THREADS / 32; ++w) t += p[w * 32 + lane];
         }
-        db[c] += t;
+        atomicAdd(db + c, t);  // (gradients of several streams may add into one db)
     }
     cluster.sync();  // the other blocks' shared memory stays until it is read
 }

@@ -510,3 +510,21 @@ def test_spatial_order_of_sparse_seeds_is_one_sort():
         return sorted(times)[4]
 
     assert ms(64) < 1.6 * ms(72)
+
+
+def test_bias_grads_of_two_streams_add_into_one():
+    """Launches that overlap on the device add into the same sums, as whole
+    numbers that fp32 holds: none is lost."""
+    import ctypes
+
+    from slm_b200 import _lib
+    rows, cols, times = 1024, 32, 300
+    dz = torch.ones((rows, cols), device=DEV)
+    db = torch.zeros(cols, device=DEV)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    for _ in range(times):
+        for s in streams:
+            _lib.check(_lib.load().slm_bias_grad(_lib.ptr(dz), rows, cols, _lib.ptr(db), ctypes.c_void_p(s.cuda_stream)))
+    torch.cuda.synchronize()
+    assert torch.all(db == 2.0 * times * rows)
