@@ -81,48 +81,53 @@ __global__ void k_relu_backward(const float* __restrict__ da, const float* __res
     if (i < n) dz[i] = z[i] > 0.0f ? da[i] : 0.0f;
 }
 
-// Column sums of dZ [rows][cols] added into db[cols].  A cluster of BIAS_CTAS
-// blocks takes 32 columns (one a lane, so rows are read whole; with fewer
-// columns a warp reads 32 / width rows at once), each warp every
-// (BIAS_CTAS * 32)th of the rows; the warps' sums are added in order by the
-// first block, which reads the others' shared memory, so the result does not
-// depend on the order they run in.  65536 x 32: 57 us with a block a column,
-// 22 us now (B200), what the eight SMs read from L2.
+// Column sums of dZ [rows][cols] added into db[cols].  A block, or a cluster of
+// CTAS of them, takes `width` columns, one a lane, so a warp reads 32 / width rows
+// at once, each warp every (CTAS * 32)th of such groups of rows; the warps' sums
+// are added in order by the first block, which reads the others' shared memory,
+// so the result does not depend on the order they run in.
 constexpr uint32_t BIAS_CTAS = 8, BIAS_THREADS = 1024;
 
-__global__ void __cluster_dims__(BIAS_CTAS, 1, 1) __launch_bounds__(BIAS_THREADS)
+template <uint32_t CTAS>
+__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(BIAS_THREADS)
 k_bias_grad(const float* __restrict__ dz, size_t rows, int cols, uint32_t width, float* __restrict__ db) {
     __shared__ float part[BIAS_THREADS / 32][32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t rank = blockIdx.x % BIAS_CTAS;
-    const int c = (int)((blockIdx.x / BIAS_CTAS) * 32u + lane % width);
+    const uint32_t rank = blockIdx.x % CTAS;
+    const int c = (int)((blockIdx.x / CTAS) * width + lane % width);
     const uint32_t per_warp = 32u / width;  // rows a warp reads at once
-    const size_t step = (size_t)BIAS_CTAS * (BIAS_THREADS / 32) * per_warp;
+    const size_t step = (size_t)CTAS * (BIAS_THREADS / 32) * per_warp;
     float s = 0.0f;
     if (c < cols) {
         size_t r = ((size_t)rank * (BIAS_THREADS / 32) + warp) * per_warp + lane / width;
-        for (; r + 15 * step < rows; r += 16 * step) {  // sixteen loads in flight
-            float v[16];
+        float v[16];  // sixteen loads in flight
+        for (; r + 15 * step < rows; r += 16 * step) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] = __ldg(dz + (r + j * step) * cols + c);
 #pragma unroll
             for (int j = 0; j < 16; ++j) s += v[j];
         }
-        for (; r < rows; r += step) s += __ldg(dz + r * cols + c);
+        if (r < rows) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = r + j * step < rows ? __ldg(dz + (r + j * step) * cols + c) : 0.0f;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) s += v[j];
+        }
     }
     for (uint32_t o = width; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     part[warp][lane] = s;
     cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
-    cluster.sync();
+    if (CTAS > 1) cluster.sync();
+    else __syncthreads();
     if (rank == 0 && warp == 0 && lane < width && c < cols) {
         float t = 0.0f;
-        for (uint32_t b = 0; b < BIAS_CTAS; ++b) {
-            const float* p = cluster.map_shared_rank(&part[0][0], b);
+        for (uint32_t b = 0; b < CTAS; ++b) {
+            const float* p = CTAS > 1 ? cluster.map_shared_rank(&part[0][0], b) : &part[0][0];
             for (uint32_t w = 0; w < BIAS_THREADS / 32; ++w) t += p[w * 32 + lane];
         }
         atomicAdd(db + c, t);  // (gradients of several streams may add into one db)
     }
-    cluster.sync();  // the other blocks' shared memory stays until it is read
+    if (CTAS > 1) cluster.sync();  // the other blocks' shared memory stays until it is read
 }
 
 // dY = 2 W (Y - T) inv_n, loss += sum W (Y - T)^2 inv_n (W = 1 without weights)
@@ -785,10 +790,24 @@ int slm_relu_backward(const float* da, const float* z, uint64_t n, float* dz, vo
 int slm_bias_grad(const float* dz, uint64_t rows, int cols, float* db, void* stream) {
     clear_error();
     SLM_REQUIRE(cols > 0, "cols must be > 0");
+    cudaStream_t s = (cudaStream_t)stream;
     uint32_t width = 1;  // lanes side by side on a row
     while (width < 32u && width < (uint32_t)cols) width <<= 1;
-    const unsigned groups = (unsigned)((cols + 31) / 32);
-    k_bias_grad<<<groups * BIAS_CTAS, BIAS_THREADS, 0, (cudaStream_t)stream>>>(dz, rows, cols, width, db);
+    // One block a group of columns while a lane has at most 64 rows with groups
+    // of 8 columns (a memory sector); the widest groups that leave a lane 16.
+    // Above that a cluster of blocks.  Measured, us (a block of 256 threads a column /
+    // a cluster for all sizes / this): 100 x 32 1.6 / 4.8 / 2.6; 1000 x 64 2.6 / 5.5 /
+    // 3.0; 100 x 4096 5.4 / 20.3 / 3.2; 4096 x 64 5.4 / 6.1 / 4.5; 4096 x 2 4.3 / 4.9 /
+    // 3.0; 8192 x 32 8.7 / 7.2 / 7.2; 65536 x 32 56.6 / 21.8 / 21.7.
+    const auto lane_rows = [&](uint32_t w) { return rows / ((BIAS_THREADS / 32u) * (32u / w)); };
+    const uint32_t least = width < 8u ? width : 8u;
+    if (lane_rows(least) < 64u) {
+        while (width > least && lane_rows(width) >= 16u) width >>= 1;
+        k_bias_grad<1><<<((uint32_t)cols + width - 1u) / width, BIAS_THREADS, 0, s>>>(dz, rows, cols, width, db);
+    } else {
+        const uint32_t groups = ((uint32_t)cols + width - 1u) / width;
+        k_bias_grad<BIAS_CTAS><<<groups * BIAS_CTAS, BIAS_THREADS, 0, s>>>(dz, rows, cols, width, db);
+    }
     SLM_LAUNCHED("k_bias_grad");
     return SLM_OK;
 }

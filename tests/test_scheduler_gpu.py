@@ -528,3 +528,54 @@ def test_bias_grads_of_two_streams_add_into_one():
             _lib.check(_lib.load().slm_bias_grad(_lib.ptr(dz), rows, cols, _lib.ptr(db), ctypes.c_void_p(s.cuda_stream)))
     torch.cuda.synchronize()
     assert torch.all(db == 2.0 * times * rows)
+
+
+@pytest.mark.parametrize("rows,cols", [(511, 40), (512, 40), (1023, 9), (2048, 32), (8191, 33), (8192, 33), (16383, 3),
+                                       (16384, 4), (65535, 1), (65536, 1), (100, 4096)])
+def test_bias_grad_by_a_block_and_by_a_cluster(rows, cols):
+    """Sizes on either side of the rules for the group's width and the cluster;
+    the bound of test_bias_grad_column_sums."""
+    import ctypes
+
+    from slm_b200 import _lib
+    g = torch.Generator().manual_seed(rows * 5 + cols)
+    dz = (torch.rand((rows, cols), generator=g) * 2 - 1).to(DEV)
+    db = torch.full((cols,), 0.5, device=DEV)
+    _lib.check(_lib.load().slm_bias_grad(_lib.ptr(dz), rows, cols, _lib.ptr(db),
+                                         ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    want = dz.double().sum(0) + 0.5
+    bound = (rows / 256 + 301) * 2.0 ** -24 * (dz.double().abs().sum(0) + 0.5)
+    assert torch.all((db.double() - want).abs() <= bound)
+
+
+def test_bias_grad_of_few_rows_costs_no_cluster():
+    """Four times the columns of a short array take about as long (3.4 times with
+    clusters of 1024-thread blocks, more of them than the SMs hold)."""
+    import ctypes
+
+    from slm_b200 import _lib
+    L = _lib.load()
+
+    def ms(cols):
+        dz, db = torch.ones((100, cols), device=DEV), torch.zeros(cols, device=DEV)
+
+        def call():
+            _lib.check(L.slm_bias_grad(_lib.ptr(dz), 100, cols, _lib.ptr(db),
+                                       ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        call()
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            for _ in range(20):
+                call()
+        times = []
+        for _ in range(9):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            g.replay()
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return sorted(times)[4]
+
+    assert ms(4096) < 2.0 * ms(1000)
