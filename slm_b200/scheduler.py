@@ -46,8 +46,9 @@ N_BINS = 1024
 # pixels (grid / per seed, ms): 3000 x 4096 16: 0.97 / 1.02, 20: 0.97 / 0.83;
 # 1500 x 2048 16: 0.28 / 0.31, 20: 0.28 / 0.26; 512 x 512 10: 0.069 / 0.070,
 # 12: 0.069 / 0.068; 300 x 400 6: 0.060 / 0.069, 8: 0.060 / 0.056; 128 x 128 1:
-# 0.048 / 0.055, 2: 0.047 / 0.042.
-DENSE_SEEDS = 8192
+# 0.048 / 0.055, 2: 0.047 / 0.042.  The per-seed kernel takes 9472 seeds at once
+# (64 an SM): up to there the grid form, at best as fast, is not taken.
+DENSE_SEEDS = 9216
 DENSE_PIXELS_PER_SEED = 16
 
 

@@ -434,7 +434,7 @@ def test_predict_on_a_grid_too_long_for_the_grid_form():
 
 
 @pytest.mark.parametrize("n,nxp,nyp,want", [
-    (8192, 1, 1, True), (8191, 1, 1, False), (8192 + 65536, 1024, 1024, True), (8191 + 65536, 1024, 1024, False),
+    (9216, 1, 1, True), (9215, 1, 1, False), (9216 + 65536, 1024, 1024, True), (9215 + 65536, 1024, 1024, False),
     (1 << 28, (1 << 24) - 1, 100, True), (1 << 28, 1 << 24, 100, False), (1 << 28, 100, 1 << 24, False),
     (1 << 31, 1 << 16, 1 << 16, False), (1 << 31, 1 << 16, (1 << 16) - 1, True)])
 def test_rule_of_the_grid_form(n, nxp, nyp, want):
@@ -451,7 +451,7 @@ def test_predict_without_memory_for_the_grid_form(monkeypatch):
     p = torch.arange(n, device=DEV)
     seeds = torch.stack((p // nyp, p % nyp), 1).to(torch.float32).contiguous()
     m = S.LengthModel(DEV, _weights(4))
-    assert n >= 8192 + n // 16
+    assert n >= 9216 + n // 16
     want = m.predict(uv, nxp, nyp, 0, seeds, n)
     need, empty = int(m.L.slm_cnn_infer_grid_workspace(nxp, nyp)), torch.empty
     refused = []
