@@ -205,15 +205,17 @@ k_preprocess(const T* __restrict__ roi, int nx, int ny, int rows, float pixel_si
         gv = quotient_from(gy, pixel_size, pixel_rcp);
         Vel w{-gu, -gv, 1.0f};
         const bool whole = (gu != 0.0f || gx == 0.0f) && (gv != 0.0f || gy == 0.0f);
-        // no gradient at all: w is what the definition gives (speed_of).  Level
-        // ground is common, in rounded heights above all: with its double path
-        // 2000 x 2001 level pixels took 219 us, where relief takes 144; they take 128 now
-        const bool level = whole && gu == 0.0f && gv == 0.0f;
-        if (!(whole && unit_of_fast(w.u, w.v, w.raw)) && !level) {
-            gu = __fdiv_rn(gx, pixel_size);
-            gv = __fdiv_rn(gy, pixel_size);
-            const float3 e = unit_of_exact(-gu, -gv);
-            w = Vel{e.x, e.y, e.z};
+        if (!whole || !unit_of_fast(w.u, w.v, w.raw)) {
+            // No gradient at all: w is what the definition gives (speed_of).
+            // Level ground is common, in rounded heights above all: with its
+            // double path 2000 x 2001 level pixels took 219 us, where relief
+            // takes 144; they take 128 now.
+            if (!whole || gu != 0.0f || gv != 0.0f) {
+                gu = __fdiv_rn(gx, pixel_size);
+                gv = __fdiv_rn(gy, pixel_size);
+                const float3 e = unit_of_exact(-gu, -gv);
+                w = Vel{e.x, e.y, e.z};
+            }
         }
         return w;
     };
