@@ -16,7 +16,7 @@
 // reads the accumulators with tcgen05.ld: warp w owns tensor-memory lanes
 // (= rows) 32w..32w+31.
 //
-// The products are small (10 GFLOP a training step); what a launch takes is the
+// The products are small (1.2 GFLOP a training step of 4096 samples); what a launch takes is the
 // conversion.  A thread therefore converts eight k of one row at a time: one
 // 16-byte shared store (a row of a core matrix, so a warp's 32 rows are free
 // of bank conflicts) and eight loads in flight, two 16-byte ones where K runs

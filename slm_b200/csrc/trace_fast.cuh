@@ -30,9 +30,9 @@
 // (each half rounded as the scalar instruction rounds it), which halve the
 // issue slots of the bilinear sums and the step's products.
 //
-// Measured (B200, both directions of 1024^2 incised relief, 2x2 seeds, RK4):
-// 815 -> 414 thread instructions per step; 4096^2 fan terrain, 1.64e10 RK4
-// steps: 505 -> 274 ms; 256^2 hills, RK2: 11.9 -> 6.2 ms.  What is left is
+// Measured (B200, both directions, RK4): 815 -> 414 thread instructions per step
+// on 4096^2 fan terrain with one trajectory a seed (421 on 1024^2 incised relief,
+// 2x2); 2x2, 1.64e10 steps: 505 -> 274 ms; 256^2 hills, RK2: 11.9 -> 6.2 ms.  What is left is
 // bound by the float units (80 % of the issue slots' worth of work: packed
 // operations take two cycles, the generator's wide products four), so
 // variants that trade slots for float work (wide products for the addresses
